@@ -21,12 +21,16 @@
 #include <vector>
 
 #include "gb_ntt.cuh"
+#include "gb_fr_shoup.cuh"
 
 namespace gb {
 
 static constexpr int kPassBits = 10;
 
-// CTAs per SM the staged passes are compiled for (their register budget)
+// CTAs per SM the staged passes are compiled for (their register budget).  A
+// pass is bound by the multiply-add pipe, and two CTAs leave it waiting for
+// loads and barriers more often than three: 16 transforms of 2^20 take
+// 2.49 ms with 2 (no register spilled) and 2.34 ms with 3 (24 words spilled).
 #ifndef GB_NTT_MIN_BLOCKS
 #define GB_NTT_MIN_BLOCKS 3
 #endif
@@ -41,6 +45,20 @@ fr_t host_fr_from_u64(uint64_t v)
 }
 
 fr_t host_fr_inverse(const fr_t &a) { return a.inverse(); }
+
+// 2^-k: k halvings mod r of one, a small part of a Fermat inversion's time
+// (the whole of a resident 2^12 inverse transform took 40 us on the host side
+// with the latter)
+static fr_t host_fr_pow2_inverse(uint32_t k)
+{
+    fr_t a = fr_t::one();
+    const fr_t m = fr_t::modulus();
+    while (k--) {
+        if (a.v[0] & 1u) mp_add<8>(a.v, a.v, m.v);  // below 2r, which fits
+        for (int i = 0; i < 8; i++) a.v[i] = (a.v[i] >> 1) | (i < 7 ? a.v[i + 1] << 31 : 0u);
+    }
+    return a;
+}
 
 fr_t host_omega(uint32_t log_n, bool inverse)
 {
@@ -183,6 +201,18 @@ __global__ void ntt_dif_pass_reg_kernel(fr_t *data, uint32_t log_n, int s_hi, in
 // butterflies whose local index is t' mod 2^p:
 //     w^(((t' << s_lo) + lo) << (log_n - 1 - s_lo - p))
 // (entry 0 is unused).  A pass with s_lo = 0 has the single chunk lo = 0.
+// Every twiddle is kept plain and with its quotient floor(w 2^256 / r) for
+// the prepared product (gb_fr_shoup.cuh), so a chunk is four runs of 2^(g-1)
+// entries: plain then quotient of the entries below 2^(g-1), then plain and
+// quotient of those from 2^(g-1) on, which the pass's first stage alone
+// reads.  The data exchanged between groups is written over that second half
+// once the first group is done, so a CTA needs 64 bytes of shared memory an
+// element and three CTAs fit an SM.
+//
+// The first group's values come straight from global memory into registers
+// and the last group's go straight back, one 32-byte access an element; in
+// between the values cross the block through shared memory, or only a warp
+// where a group's warp holds whole runs of 2^(5 + EL) elements.
 //
 // Shared memory is addressed in 16-byte chunks.  Element t of a sub-block
 // occupies chunks 2t and 2t+1 of its 128-byte row r = t/4, permuted inside
@@ -217,13 +247,18 @@ __device__ __forceinline__ void ntt_st(uint4 *s, uint32_t t, uint32_t x, const f
 }
 
 // Butterfly arithmetic of the staged passes.  The values between stages and
-// passes are kept in [0, 2r) (Harvey's lazy butterflies): a product x * w
-// with x < 2r and a twiddle w < r is below 2r without the Montgomery
-// product's final subtraction, and sums and differences are reduced mod 2r;
-// the last pass reduces its outputs to [0, r).  Measured on GB300 this makes
-// the transform 7% faster than reducing every result; GB_NTT_EAGER selects
-// the fully reduced form.
-#if !defined(GB_NTT_EAGER)
+// passes are kept in [0, 2r) (Harvey's lazy butterflies): the prepared product
+// of x < 2r by a twiddle is below 2r, and sums and differences are reduced
+// mod 2r; the last pass reduces its outputs to [0, r).
+//
+// A pass is bound by the multiply-add pipe, where a 32 x 32 -> 64 product
+// takes 4 cycles a warp and a 32-bit one 2.  A Montgomery product needs 120
+// of the former and about 140 carry additions; the prepared product
+// (gb_fr_shoup.cuh) 79 and 21 of the latter and 50 additions, for a second
+// 32-byte word per twiddle.  Measured alone on all SMs, 65.8 -> 96.8 G
+// products/s; 16 transforms of 2^20, 3.53 -> 2.34 ms with the register paths
+// of ntt_tw_piece (2.37 ms of 3.15 came from those), 8 coset extensions
+// 2^18 -> 2^20 1.80 -> 1.08 ms.
 __device__ __forceinline__ fr_t bfly_add(const fr_t &a, const fr_t &b)
 {
     fr_t r;
@@ -259,40 +294,40 @@ __device__ __forceinline__ fr_t bfly_add(const fr_t &a, const fr_t &b)
 
 __device__ __forceinline__ fr_t bfly_sub(const fr_t &a, const fr_t &b)
 {
+    // the addition of 2r is predicated on the borrow: no selects
     fr_t r;
-    uint32_t d[8], t[8], br;
-    asm("sub.cc.u32 %0, %9, %17;\n\t"
-        "subc.cc.u32 %1, %10, %18;\n\t"
-        "subc.cc.u32 %2, %11, %19;\n\t"
-        "subc.cc.u32 %3, %12, %20;\n\t"
-        "subc.cc.u32 %4, %13, %21;\n\t"
-        "subc.cc.u32 %5, %14, %22;\n\t"
-        "subc.cc.u32 %6, %15, %23;\n\t"
-        "subc.cc.u32 %7, %16, %24;\n\t"
-        "subc.u32 %8, 0, 0;"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(br)
+    asm("{\n\t.reg .pred p;\n\t.reg .u32 br;\n\t"
+        "sub.cc.u32 %0, %8, %16;\n\t"
+        "subc.cc.u32 %1, %9, %17;\n\t"
+        "subc.cc.u32 %2, %10, %18;\n\t"
+        "subc.cc.u32 %3, %11, %19;\n\t"
+        "subc.cc.u32 %4, %12, %20;\n\t"
+        "subc.cc.u32 %5, %13, %21;\n\t"
+        "subc.cc.u32 %6, %14, %22;\n\t"
+        "subc.cc.u32 %7, %15, %23;\n\t"
+        "subc.u32 br, 0, 0;\n\t"
+        "setp.ne.u32 p, br, 0;\n\t"
+        "@p add.cc.u32 %0, %0, 0x00000002;\n\t"
+        "@p addc.cc.u32 %1, %1, 0xfffffffe;\n\t"
+        "@p addc.cc.u32 %2, %2, 0xfffcb7fd;\n\t"
+        "@p addc.cc.u32 %3, %3, 0xa77b4805;\n\t"
+        "@p addc.cc.u32 %4, %4, 0x1343b00a;\n\t"
+        "@p addc.cc.u32 %5, %5, 0x6673b010;\n\t"
+        "@p addc.cc.u32 %6, %6, 0x533afa90;\n\t"
+        "@p addc.u32 %7, %7, 0xe7db4ea6;\n\t}"
+        : "=&r"(r.v[0]), "=&r"(r.v[1]), "=&r"(r.v[2]), "=&r"(r.v[3]), "=&r"(r.v[4]), "=&r"(r.v[5]), "=&r"(r.v[6]),
+          "=&r"(r.v[7])
         : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
           "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
-    asm("add.cc.u32 %0, %8, 0x00000002;\n\t"
-        "addc.cc.u32 %1, %9, 0xfffffffe;\n\t"
-        "addc.cc.u32 %2, %10, 0xfffcb7fd;\n\t"
-        "addc.cc.u32 %3, %11, 0xa77b4805;\n\t"
-        "addc.cc.u32 %4, %12, 0x1343b00a;\n\t"
-        "addc.cc.u32 %5, %13, 0x6673b010;\n\t"
-        "addc.cc.u32 %6, %14, 0x533afa90;\n\t"
-        "addc.u32 %7, %15, 0xe7db4ea6;"
-        : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
-        : "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]), "r"(d[4]), "r"(d[5]), "r"(d[6]), "r"(d[7]));
-#pragma unroll
-    for (int i = 0; i < 8; i++) r.v[i] = br ? t[i] : d[i];
     return r;
 }
 
-__device__ __forceinline__ fr_t bfly_mul(const fr_t &x, const fr_t &w)
+// x * w for a twiddle w prepared with v = floor(w 2^256 / r)
+__device__ __forceinline__ fr_t bfly_mul(const fr_t &x, const fr_t &w, const fr_t &v)
 {
     fr_t r;
 #if defined(__CUDA_ARCH__)
-    mont_mul_device<FrCfg, false>(r.v, x.v, w.v);
+    fr_mul_prepared(r.v, x.v, w.v, v.v);
 #endif
     return r;
 }
@@ -303,12 +338,6 @@ __device__ __forceinline__ fr_t bfly_out(fr_t v)
     fr_t::reduce_once(v.v, 0);
     return v;
 }
-#else
-__device__ __forceinline__ fr_t bfly_add(const fr_t &a, const fr_t &b) { return a + b; }
-__device__ __forceinline__ fr_t bfly_sub(const fr_t &a, const fr_t &b) { return a - b; }
-__device__ __forceinline__ fr_t bfly_mul(const fr_t &x, const fr_t &w) { return x * w; }
-__device__ __forceinline__ fr_t bfly_out(fr_t v) { return v; }
-#endif
 
 // chunk(t, h, x) = lin(t) ^ h ^ x, with lin linear over GF(2) in the bits
 // of t: addresses of elements whose indices differ in known bits are found
@@ -342,47 +371,50 @@ __device__ __forceinline__ void ntt_st_c(uint4 *s, uint32_t c, const fr_t &v)
 // images of single bits.  The butterflies of one stage that share a twiddle
 // (same local index mod 2^p) read it once.
 template <int EL, int R>
-__device__ __forceinline__ void ntt_tw_group(uint4 *sd, const uint4 *stw, uint32_t u, int B, uint32_t twist,
-                                             bool lo_zero)
+__device__ __forceinline__ uint32_t ntt_tl0(uint32_t u, int B)
+{
+    const uint32_t rest0 = u << (EL - R);
+    return (rest0 & ((1u << B) - 1)) | ((rest0 >> B) << (B + R));
+}
+
+// local index of element k, less tl[0]'s bits
+template <int EL, int R>
+__device__ __forceinline__ uint32_t ntt_tk(int k, int B)
+{
+    return ((uint32_t)k >> R) | (((uint32_t)k & ((1u << R) - 1)) << B);
+}
+
+// the group's R stages on the thread's values; `st` is the sub-block's
+// twiddle chunk (see the table's layout above), g its number of stages
+template <int EL, int R>
+__device__ __forceinline__ void ntt_tw_stages(fr_t *x, const uint4 *st, uint32_t u, int B, int g, bool lo_zero)
 {
     constexpr int E = 1 << EL;
-    const uint32_t rest0 = u << (EL - R);
-    const uint32_t tl0 = (rest0 & ((1u << B) - 1)) | ((rest0 >> B) << (B + R));
-    const uint32_t base = ntt_lin(tl0) ^ twist;
+    const uint32_t tl0 = ntt_tl0<EL, R>(u, B);
+    const uint32_t sub = 1u << g;
     uint32_t img_b[R];  // lin(1 << (B + j))
 #pragma unroll
     for (int j = 0; j < R; j++) img_b[j] = ntt_lin(1u << (B + j));
-    // lin of the bits k >> R (below B): constants
-    auto img_lo = [](uint32_t v) { return ntt_lin(v); };
-    uint32_t off[E];
-    fr_t x[E];
 #pragma unroll
-    for (int k = 0; k < E; k++) {
-        uint32_t o = img_lo((uint32_t)k >> R);
-#pragma unroll
-        for (int j = 0; j < R; j++)
-            if ((k >> j) & 1) o ^= img_b[j];
-        off[k] = o;
-        x[k] = ntt_ld_c(sd, base ^ o);
-    }
-#pragma unroll
-    for (int st = 0; st < R; st++) {
-        const int p = B + R - 1 - st;  // local bit of this stage
-        const int lh = R - 1 - st, hk = 1 << lh;
+    for (int s = 0; s < R; s++) {
+        const int p = B + R - 1 - s;  // local bit of this stage
+        const int lh = R - 1 - s, hk = 1 << lh;
+        const uint4 *stw = st + (s == 0 && p == g - 1 ? sub : 0), *stv = stw + sub;
         // twiddle entry of key (kl, kr): m = 2^p ^ (tl0 mod 2^p) ^ kr ^ (kl << B)
         const uint32_t tp0 = tl0 & ((1u << p) - 1);
         const uint32_t tbase = ntt_lin((1u << p) ^ tp0);
-        fr_t w[E / 2];
+        fr_t w[E / 2], v[E / 2];
         bool one[E / 2];
 #pragma unroll
         for (int key = 0; key < (hk << (EL - R)); key++) {
             const uint32_t kl = (uint32_t)key & (hk - 1), kr = (uint32_t)key >> lh;
-            uint32_t o = img_lo(kr);
+            uint32_t o = ntt_lin(kr);
 #pragma unroll
             for (int j = 0; j < lh; j++)
                 if ((kl >> j) & 1) o ^= img_b[j];
             one[key] = lo_zero && (tp0 | kr | kl) == 0;
             w[key] = ntt_ld_c(stw, tbase ^ o);
+            v[key] = ntt_ld_c(stv, tbase ^ o);
         }
 #pragma unroll
         for (int k = 0; k < E; k++) {
@@ -392,13 +424,30 @@ __device__ __forceinline__ void ntt_tw_group(uint4 *sd, const uint4 *stw, uint32
                 const fr_t a = x[k], c = x[k1];
                 x[k] = bfly_add(a, c);
                 fr_t diff = bfly_sub(a, c);
-                if (!one[key]) diff = bfly_mul(diff, w[key]);
+                if (!one[key]) diff = bfly_mul(diff, w[key], v[key]);
                 x[k1] = diff;
             }
         }
     }
+}
+
+// the thread's values of a group to or from the sub-block's data area
+template <int EL, int R, bool STORE>
+__device__ __forceinline__ void ntt_tw_exchange(fr_t *x, uint4 *sd, uint32_t u, int B, uint32_t twist)
+{
+    const uint32_t base = ntt_lin(ntt_tl0<EL, R>(u, B)) ^ twist;
+    uint32_t img_b[R];
 #pragma unroll
-    for (int k = 0; k < E; k++) ntt_st_c(sd, base ^ off[k], x[k]);
+    for (int j = 0; j < R; j++) img_b[j] = ntt_lin(1u << (B + j));
+#pragma unroll
+    for (int k = 0; k < 1 << EL; k++) {
+        uint32_t o = ntt_lin((uint32_t)k >> R);
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if ((k >> j) & 1) o ^= img_b[j];
+        if (STORE) ntt_st_c(sd, base ^ o, x[k]);
+        else x[k] = ntt_ld_c(sd, base ^ o);
+    }
 }
 
 // Spin limits of the twiddle copy's waits.  The first wait gives up after
@@ -441,7 +490,44 @@ struct ntt_factors {
     int on;
     const fr_t *pw_lo = nullptr, *pw_hi = nullptr;
     uint32_t lo_bits = 0;
+    fr_t w[3] = {}, v[3] = {};  // on == 1: f plain, and its quotients floor(w 2^256 / r)
 };
+
+// r = a * b mod 2^256
+GB_HD void mul_low256(uint32_t *r, const uint32_t *a, const uint32_t *b)
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) r[i] = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        uint64_t c = 0;
+#pragma unroll
+        for (int j = 0; i + j < 8; j++) {
+            c += (uint64_t)a[i] * b[j] + r[i + j];
+            r[i + j] = (uint32_t)c;
+            c >>= 32;
+        }
+    }
+}
+
+// The plain form w of a Montgomery-form constant and floor(w 2^256 / r).  The
+// Montgomery form is w 2^256 mod r, so the quotient is (w 2^256 - Montgomery
+// form) / r, an exact division: mod 2^256 it is the Montgomery form times
+// -1/r.
+GB_HD void prepare_constant(const fr_t &mont, fr_t &w, fr_t &v)
+{
+    const uint32_t neg_inv[8] = {0xffffffffu, 0xfffffffeu, 0xfffe5bfdu, 0x53ba5bffu,
+                                 0x0004ec06u, 0x181b2c17u, 0xd7bf2839u, 0x3d443ab0u};  // -1/r mod 2^256
+    w = mont.from_mont();
+    mul_low256(v.v, mont.v, neg_inv);
+}
+
+static ntt_factors period3_factors(const fr_t &f0, const fr_t &f1, const fr_t &f2)
+{
+    ntt_factors fac{{f0, f1, f2}, 1};
+    for (int k = 0; k < 3; k++) prepare_constant(fac.f[k], fac.w[k], fac.v[k]);
+    return fac;
+}
 
 __device__ __forceinline__ fr_t ntt_factor(const ntt_factors &fac, size_t i)
 {
@@ -456,6 +542,48 @@ __device__ __forceinline__ fr_t ntt_factor(const ntt_factors &fac, size_t i)
         for (int w = 0; w < 8; w++) f.v[w] = c == 0 ? fac.f[0].v[w] : c == 1 ? fac.f[1].v[w] : fac.f[2].v[w];
     }
     return f;
+}
+
+// x (below 2r) times position i's factor, below 2r; i < 2^32
+__device__ __forceinline__ fr_t ntt_scaled(const fr_t &x, const ntt_factors &fac, size_t i)
+{
+    if (fac.on == 2) return x * ntt_factor(fac, i);
+    const uint32_t c = (uint32_t)i % 3u;
+    fr_t w, v;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        w.v[k] = c == 0 ? fac.w[0].v[k] : c == 1 ? fac.w[1].v[k] : fac.w[2].v[k];
+        v.v[k] = c == 0 ? fac.v[0].v[k] : c == 1 ? fac.v[1].v[k] : fac.v[2].v[k];
+    }
+    return bfly_mul(x, w, v);
+}
+
+// one 32-byte access (a whole sector); L2 reads past L1, for values that
+// other CTAs of the same launch wrote
+template <bool L2>
+__device__ __forceinline__ fr_t ntt_ldg(const fr_t *p)
+{
+    fr_t r;
+    if (L2)
+        asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
+                       "=r"(r.v[6]), "=r"(r.v[7])
+                     : "l"(p)
+                     : "memory");
+    else
+        asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
+                       "=r"(r.v[6]), "=r"(r.v[7])
+                     : "l"(p)
+                     : "memory");
+    return r;
+}
+
+__device__ __forceinline__ void ntt_stg(fr_t *p, const fr_t &r)
+{
+    asm volatile("st.global.v8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"r"(r.v[0]), "r"(r.v[1]), "r"(r.v[2]),
+                 "r"(r.v[3]), "r"(r.v[4]), "r"(r.v[5]), "r"(r.v[6]), "r"(r.v[7]), "l"(p)
+                 : "memory");
 }
 
 // The input of a fused first pass: `count` polynomials of in_len values
@@ -498,80 +626,72 @@ __device__ __forceinline__ bool ntt_tw_piece(const fr_t *src, fr_t *dst, uint32_
                                              size_t cta, uint4 *smem, uint32_t mbar, uint32_t parity, int &copy_ok,
                                              uint32_t *status, unsigned spins, const ntt_input &in = ntt_input{})
 {
+    constexpr int E = 1 << EL;
     const int s_lo = s_hi - g + 1;
-    const uint32_t sub = 1u << g, Q = 1u << q, nd = Q << g;
+    const uint32_t sub = 1u << g, nd = sub << q;
     const size_t n = (size_t)1 << log_n;
     const uint32_t tw_entries = s_lo > 0 ? nd : sub;
-    uint4 *sd = smem;
-    uint4 *stw = smem + 2 * (size_t)nd;
     const int nb_log = (int)log_n - g;                 // log2 sub-blocks per transform
     const size_t total = count << nb_log;              // sub-blocks in the batch
-    const bool q_fast = !LAST || nb_log >= q;          // LAST: Q adjacent columns of one transform
 
     size_t poly = 0, b0 = 0;
     const fr_t *twsrc = twt;
     if (s_lo > 0) {
         poly = cta % count;
         b0 = (size_t)(cta / count) << q;
-        twsrc = twt + ((b0 & (((size_t)1 << s_lo) - 1)) << g);
+        twsrc = twt + ((b0 & (((size_t)1 << s_lo) - 1)) << (g + 1));
     } else {
         b0 = cta << q;
     }
 
     if (threadIdx.x == 0) {
-        // the previous piece's generic reads of the twiddle buffer are done
+        // the previous piece's generic accesses of the buffer are done
         // (barrier); order them before the async-proxy write
         if (QUEUE) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const uint32_t bytes = tw_entries * (uint32_t)sizeof(fr_t);
+        const uint32_t bytes = 2 * tw_entries * (uint32_t)sizeof(fr_t);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
         asm volatile(
             "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                (uint32_t)__cvta_generic_to_shared(stw)),
+                (uint32_t)__cvta_generic_to_shared(smem)),
             "l"(twsrc), "r"(bytes), "r"(mbar)
             : "memory");
     }
 
-    // gather the sub-blocks into shared memory
-    for (uint32_t idx = threadIdx.x; idx < nd; idx += blockDim.x) {
-        uint32_t qq, t;
-        size_t addr;
-        bool valid = true;
-        if (s_lo > 0) {
-            qq = idx & (Q - 1);
-            t = idx >> q;
-            const size_t b = b0 + qq;
-            addr = poly * n + ((b >> s_lo) << (s_hi + 1)) + (b & (((size_t)1 << s_lo) - 1)) + ((size_t)t << s_lo);
-        } else {
-            qq = idx >> g;
-            t = idx & (sub - 1);
-            const size_t F = b0 + qq;
-            valid = F < total;
-            if (LAST) {
-                const size_t col = F & (((size_t)1 << nb_log) - 1);
-                addr = ((F >> nb_log) << log_n) + ((size_t)brev_bits((uint32_t)col, nb_log) << g) + t;
-            } else {
-                addr = (F << g) + t;
-            }
-        }
-        fr_t v = fr_t::zero();
+    const uint32_t per_sub = sub >> EL;  // threads per sub-block; nd >> EL threads take part
+    const bool part = !QUEUE || threadIdx.x < (nd >> EL);
+    const uint32_t qq = part ? threadIdx.x / per_sub : 0, u = threadIdx.x % per_sub;
+    const size_t F = b0 + qq;
+    const bool valid = part && (s_lo > 0 || F < total);
+    const size_t col = F & (((size_t)1 << nb_log) - 1);
+    // address of the sub-block's element t: in0 + (t << s_lo) (s_lo = 0 when
+    // the sub-block is contiguous)
+    size_t in0;
+    if (s_lo > 0)
+        in0 = poly * n + ((F >> s_lo) << (s_hi + 1)) + (F & (((size_t)1 << s_lo) - 1));
+    else if (LAST)
+        in0 = ((F >> nb_log) << log_n) + ((size_t)brev_bits((uint32_t)col, nb_log) << g);
+    else
+        in0 = F << g;
+
+    // the first group's values: the remainder of g by EL, at the top bits
+    const int r1 = g % EL ? g % EL : EL, B1 = g - r1;
+    fr_t x[E];
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        x[k] = fr_t::zero();
+        if (!valid) continue;
+        const uint32_t t = (u << (EL - r1)) | ((uint32_t)k >> r1) | (((uint32_t)k & ((1u << r1) - 1)) << B1);
+        const size_t addr = in0 + ((size_t)t << s_lo);
         if (LOADF) {
             // first pass: s_hi = log_n - 1, so the position is addr - poly * n
             const size_t i = addr - poly * n;
             if (i < in.in_len) {
-                v = in.src[poly * in.in_len + i];
-                if (in.fac.on) v = v * ntt_factor(in.fac, i);
+                x[k] = ntt_ldg<false>(in.src + poly * in.in_len + i);
+                if (in.fac.on) x[k] = ntt_scaled(x[k], in.fac, i);
             }
-        } else if (valid) {
-            if (QUEUE) {
-                const uint4 *p = reinterpret_cast<const uint4 *>(src + addr);
-                const uint4 lo = __ldcg(p), hi = __ldcg(p + 1);
-                v.v[0] = lo.x, v.v[1] = lo.y, v.v[2] = lo.z, v.v[3] = lo.w;
-                v.v[4] = hi.x, v.v[5] = hi.y, v.v[6] = hi.z, v.v[7] = hi.w;
-            } else {
-                v = src[addr];
-            }
+        } else {
+            x[k] = ntt_ldg<QUEUE>(src + addr);
         }
-        ntt_st(sd + 2 * (size_t)qq * sub, t, ntt_twist(qq & 7u), v);
     }
     if (threadIdx.x == 0) {
         bool ok = mbar_wait(mbar, parity, spins);
@@ -584,71 +704,50 @@ __device__ __forceinline__ bool ntt_tw_piece(const fr_t *src, fr_t *dst, uint32_
     __syncthreads();
     if (!copy_ok) return false;
 
-    // radix-2^EL groups; the remainder group first, at the top bits
-    {
-        const uint32_t per_sub = sub >> EL;  // threads per sub-block; nd >> EL threads take part
-        const bool part = !QUEUE || threadIdx.x < (nd >> EL);
-        const uint32_t qq = part ? threadIdx.x / per_sub : 0, ul = threadIdx.x % per_sub;
-        uint4 *sdq = sd + 2 * (size_t)qq * sub;
-        const uint4 *stq = stw + (s_lo > 0 ? 2 * (size_t)qq * sub : 0);
-        const uint32_t twist = ntt_twist(qq & 7u);
-        const bool lo_zero = s_lo == 0 || (((b0 + qq) & (((size_t)1 << s_lo) - 1)) == 0);
-        int top = g;
-        const int rem = g % EL;
-        if (rem) {
-            if (!part) {
-            } else if (EL == 3 && rem == 2) {
-                ntt_tw_group<EL, (EL == 3 ? 2 : 1)>(sdq, stq, ul, g - rem, twist, lo_zero);
-            } else {
-                ntt_tw_group<EL, 1>(sdq, stq, ul, g - rem, twist, lo_zero);
-            }
-            top -= rem;
-            __syncthreads();
+    const uint4 *st = smem + (s_lo > 0 ? 4 * (size_t)qq * sub : 0);
+    uint4 *sd = smem + 2 * (size_t)sub + (s_lo > 0 ? 4 : 2) * (size_t)qq * sub;
+    const uint32_t twist = ntt_twist(qq & 7u);
+    const bool lo_zero = s_lo == 0 || (F & (((size_t)1 << s_lo) - 1)) == 0;
+    if (part) {
+        if (r1 == EL) ntt_tw_stages<EL, EL>(x, st, u, B1, g, lo_zero);
+        else if (EL == 3 && r1 == 2) ntt_tw_stages<EL, (EL == 3 ? 2 : 1)>(x, st, u, B1, g, lo_zero);
+        else ntt_tw_stages<EL, 1>(x, st, u, B1, g, lo_zero);
+    }
+    if (B1 > 0) {
+        __syncthreads();  // the first stage's twiddles are read: the data area lies over them
+        if (part) {
+            if (r1 == EL) ntt_tw_exchange<EL, EL, true>(x, sd, u, B1, twist);
+            else if (EL == 3 && r1 == 2) ntt_tw_exchange<EL, (EL == 3 ? 2 : 1), true>(x, sd, u, B1, twist);
+            else ntt_tw_exchange<EL, 1, true>(x, sd, u, B1, twist);
         }
-        while (top > 0) {
-            if (part) ntt_tw_group<EL, EL>(sdq, stq, ul, top - EL, twist, lo_zero);
-            top -= EL;
-            __syncthreads();
+        for (int B = B1 - EL;; B -= EL) {
+            // with the previous group at or below bit 5 a warp holds the same
+            // 2^(5 + EL) elements before and after the exchange
+            if (B + (B == B1 - EL ? r1 : EL) <= 5 && (B != B1 - EL || r1 == EL)) __syncwarp();
+            else __syncthreads();
+            if (part) {
+                ntt_tw_exchange<EL, EL, false>(x, sd, u, B, twist);
+                ntt_tw_stages<EL, EL>(x, st, u, B, g, lo_zero);
+            }
+            if (B == 0) break;
+            if (part) ntt_tw_exchange<EL, EL, true>(x, sd, u, B, twist);
         }
     }
 
-    // write back
-    for (uint32_t idx = threadIdx.x; idx < nd; idx += blockDim.x) {
-        uint32_t qq, t;
-        size_t addr;
-        if (s_lo > 0) {
-            qq = idx & (Q - 1);
-            t = idx >> q;
-            const size_t b = b0 + qq;
-            addr = poly * n + ((b >> s_lo) << (s_hi + 1)) + (b & (((size_t)1 << s_lo) - 1)) + ((size_t)t << s_lo);
-        } else if (!LAST) {
-            qq = idx >> g;
-            t = idx & (sub - 1);
-            if (b0 + qq >= total) continue;
-            addr = ((b0 + qq) << g) + t;
-        } else {
-            uint32_t r;  // output row
-            if (q_fast) {
-                qq = idx & (Q - 1);
-                r = idx >> q;
+    // the last group ends at bit 0: element k is local index u * E + k
+    if (valid) {
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const uint32_t t = (u << EL) | (uint32_t)k;
+            if (!LAST) {
+                ntt_stg(dst + in0 + ((size_t)t << s_lo), x[k]);
             } else {
-                qq = idx >> g;
-                r = idx & (sub - 1);
+                const size_t i_nat = ((size_t)brev_bits(t, g) << nb_log) + col;
+                fr_t v = x[k];
+                if (fac.on) v = ntt_scaled(v, fac, i_nat);
+                ntt_stg(dst + ((F >> nb_log) << log_n) + i_nat, bfly_out(v));
             }
-            const size_t F = b0 + qq;
-            if (F >= total) continue;
-            t = brev_bits(r, g);
-            const size_t col = F & (((size_t)1 << nb_log) - 1);
-            const size_t i_nat = ((size_t)r << nb_log) + col;
-            addr = ((F >> nb_log) << log_n) + i_nat;
-            fr_t v = ntt_ld(sd + 2 * (size_t)qq * sub, t, ntt_twist(qq & 7u));
-            // x * f with x < 2r, f < r is fully reduced by the product
-            if (!fac.on) v = bfly_out(v);
-            else v = v * ntt_factor(fac, i_nat);
-            dst[addr] = v;
-            continue;
         }
-        dst[addr] = ntt_ld(sd + 2 * (size_t)qq * sub, t, ntt_twist(qq & 7u));
     }
     return true;
 }
@@ -800,9 +899,16 @@ __global__ void pass_twiddle_kernel(fr_t *out, const fr_t *__restrict__ tw, uint
         const size_t e = ((tp << s_lo) + lo) << (log_n - 1 - s_lo - p);
         v = tw[e];
     }
-    uint4 *o = reinterpret_cast<uint4 *>(out + (lo << g));
-    o[ntt_chunk(m, 0, 0)] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
-    o[ntt_chunk(m, 1, 0)] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
+    fr_t w, quo;
+    prepare_constant(v, w, quo);
+    // runs of sub / 2 entries (sub uint4 each): entries from sub / 2 on lie
+    // one run further than their index, quotients one run behind their plain
+    // value
+    uint4 *o = reinterpret_cast<uint4 *>(out + (lo << (g + 1))) + (m >= sub / 2 ? sub : 0), *oq = o + sub;
+    o[ntt_chunk(m, 0, 0)] = make_uint4(w.v[0], w.v[1], w.v[2], w.v[3]);
+    o[ntt_chunk(m, 1, 0)] = make_uint4(w.v[4], w.v[5], w.v[6], w.v[7]);
+    oq[ntt_chunk(m, 0, 0)] = make_uint4(quo.v[0], quo.v[1], quo.v[2], quo.v[3]);
+    oq[ntt_chunk(m, 1, 0)] = make_uint4(quo.v[4], quo.v[5], quo.v[6], quo.v[7]);
 }
 
 __device__ __forceinline__ size_t bitrev_n(size_t x, uint32_t bits)
@@ -1018,7 +1124,7 @@ const fr_t *pass_twiddles(uint32_t log_n, bool inverse, int s_hi, int g, const f
     const size_t chunks = s_lo > 0 ? (size_t)1 << s_lo : 1;
     const size_t entries = chunks << g;
     fr_t *t = nullptr;
-    GB_CUDA_OK(cudaMalloc(&t, entries * sizeof(fr_t)));
+    GB_CUDA_OK(cudaMalloc(&t, 2 * entries * sizeof(fr_t)));
     pass_twiddle_kernel<<<blocks_for(entries, 256), 256, 0, s>>>(t, tw, log_n, s_lo, g, chunks);
     GB_CHECK_LAUNCH();
     GB_CUDA_OK(cudaStreamSynchronize(s));
@@ -1069,8 +1175,8 @@ static void ntt_staged(fr_t *d, uint32_t log_n, size_t count, bool inverse, cons
         while (q > 0 && ctas_for(q) < 2 * (size_t)sm_count()) q--;
         ctas = ctas_for(q);
         const uint32_t nd = 1u << (g + q);
-        const uint32_t tw_entries = s_lo > 0 ? nd : 1u << g;
-        const size_t smem = ((size_t)nd + tw_entries) * sizeof(fr_t);
+        // the twiddle chunks; a single chunk's data areas go past its first half
+        const size_t smem = (s_lo > 0 ? 2 * (size_t)nd : ((size_t)1 << g) + nd) * sizeof(fr_t);
         const unsigned threads = nd >> el;
         const bool fused = in && i == 0;
         const ntt_input &pin = fused ? *in : no_in;
@@ -1280,7 +1386,7 @@ void ntt_inplace(fr_t *d, uint32_t log_n, size_t count, bool inverse, const fr_t
                  cudaStream_t s)
 {
     ntt_factors fac{{fr_t::one(), fr_t::one(), fr_t::one()}, 0};
-    if (scale) fac = ntt_factors{{*scale, *scale, *scale}, 1};
+    if (scale) fac = period3_factors(*scale, *scale, *scale);
     ntt_apply(d, log_n, count, inverse, fac, status, s);
 }
 
@@ -1394,7 +1500,7 @@ void launch_coeff_to_extended_prepare(fr_t *out, const fr_t *in, const fr_t &fir
 static void ntt_ref(fr_t *d, uint32_t log_n, size_t count, bool inverse, uint32_t *status, cudaStream_t s)
 {
     if (inverse) {
-        fr_t ninv = host_fr_inverse(host_fr_from_u64((uint64_t)1 << log_n));
+        fr_t ninv = host_fr_pow2_inverse(log_n);
         ntt_inplace(d, log_n, count, true, &ninv, status, s);
     } else {
         ntt_inplace(d, log_n, count, false, nullptr, status, s);
@@ -1408,8 +1514,8 @@ static void ntt_ref_zeta(fr_t *d, uint32_t log_n, size_t count, bool inverse, co
                          const fr_t &second, uint32_t *status, cudaStream_t s)
 {
     fr_t sc = scale;
-    if (inverse) sc = sc * host_fr_inverse(host_fr_from_u64((uint64_t)1 << log_n));
-    const ntt_factors fac{{sc, sc * first, sc * second}, 1};
+    if (inverse) sc = sc * host_fr_pow2_inverse(log_n);
+    const ntt_factors fac = period3_factors(sc, sc * first, sc * second);
     ntt_apply(d, log_n, count, inverse, fac, status, s);
 }
 
@@ -1420,7 +1526,7 @@ static void ntt_ref_zeta(fr_t *d, uint32_t log_n, size_t count, bool inverse, co
 static void c2e_zeta(fr_t *out, const fr_t *in, size_t input_len, size_t count, uint32_t ext_log_n,
                      const fr_t &first, const fr_t &second, uint32_t *status, cudaStream_t s)
 {
-    const ntt_factors infac{{fr_t::one(), first, second}, 1};
+    const ntt_factors infac = period3_factors(fr_t::one(), first, second);
     const ntt_factors none{{fr_t::one(), fr_t::one(), fr_t::one()}, 0};
     ntt_padded(out, in, input_len, count, ext_log_n, infac, none, status, s);
 }
@@ -1448,7 +1554,7 @@ static void ntt_coset(fr_t *d, uint32_t log_n, size_t count, bool inverse, const
         c2e_coset(d, d, n, count, log_n, shift, status, s);
         return;
     }
-    const fr_t ninv = host_fr_inverse(host_fr_from_u64((uint64_t)n));
+    const fr_t ninv = host_fr_pow2_inverse(log_n);
     const ntt_factors outfac = power_factors(host_fr_inverse(shift), ninv, n, s);
     ntt_apply(d, log_n, count, true, outfac, status, s);
 }
@@ -1564,13 +1670,13 @@ RustError midnight_sppark_bls12_381_fr_device_coeff_to_extended_batch(void **out
     size_t output_len = (size_t)1 << extended_log_n;
     if (input_len > output_len) return make_error(-1, "input length exceeds extended domain length");
     cudaStream_t s = lane_stream();
+    lane_check();  // of the lane's earlier work: this call's own waits are reported by a later one
     ntt_status st;
     dev_buf<fr_t> din(input_len * count, s);
     h2d(din, inputs, input_len * count * sizeof(fr_t), s);
     fr_device_vec *v = device_vec_new(output_len * count, s);
     try {
         c2e_zeta(v->values, din, input_len, count, extended_log_n, first, second, st.ptr(), s);
-        lane_check();
         device_vec_mark_ready(v, s);
     } catch (...) {
         device_vec_delete(v);
@@ -1597,12 +1703,12 @@ RustError midnight_sppark_bls12_381_fr_device_coeff_to_extended_from_device_batc
     size_t output_len = (size_t)1 << extended_log_n;
     if (input_len > output_len) return make_error(-1, "input length exceeds extended domain length");
     cudaStream_t s = lane_stream();
+    lane_check();  // of the lane's earlier work: this call's own waits are reported by a later one
     device_vec_wait(src, s);
     ntt_status st;
     fr_device_vec *v = device_vec_new(output_len * count, s);
     try {
         c2e_zeta(v->values, src->values, input_len, count, extended_log_n, first, second, st.ptr(), s);
-        lane_check();
         device_vec_mark_ready(v, s);
     } catch (...) {
         device_vec_delete(v);
@@ -1627,10 +1733,10 @@ RustError midnight_sppark_bls12_381_fr_device_vec_ntt_zeta(void *device_vec, uin
     // a single value is returned unscaled, as the reference does (.cu:3296-3298)
     if (log_n == 0) return ok();
     cudaStream_t s = lane_stream();
+    lane_check();  // of the lane's earlier work: this call's own waits are reported by a later one
     device_vec_wait(v, s);
     ntt_status st;
     ntt_ref_zeta(v->values, log_n, 1, inverse, scale, first, second, st.ptr(), s);
-    lane_check();
     device_vec_mark_ready(v, s);
     return ok();
     GB_ENTRY_END
@@ -1650,10 +1756,10 @@ RustError midnight_sppark_bls12_381_fr_device_vec_ntt_zeta_batch(void *device_ve
     if (count > SIZE_MAX / n) return make_error((int)cudaErrorInvalidValue, "resident NTT batch size overflow");
     if (v->len != n * count) return make_error((int)cudaErrorInvalidValue, "resident NTT batch length mismatch");
     cudaStream_t s = lane_stream();
+    lane_check();  // of the lane's earlier work: this call's own waits are reported by a later one
     device_vec_wait(v, s);
     ntt_status st;
     ntt_ref_zeta(v->values, log_n, count, inverse, scale, first, second, st.ptr(), s);
-    lane_check();
     device_vec_mark_ready(v, s);
     return ok();
     GB_ENTRY_END
@@ -1685,6 +1791,7 @@ RustError gb_fr_device_vec_ntt_ragged(void *device_vec, const size_t *offsets, c
             return make_error((int)cudaErrorInvalidValue, "ragged NTT polynomials overlap");
     if (count == 0) return ok();
     cudaStream_t s = lane_stream();
+    lane_check();  // of the lane's earlier work: this call's own waits are reported by a later one
     device_vec_wait(v, s);
     ntt_status st;
     std::vector<size_t> q_off;
@@ -1698,13 +1805,12 @@ RustError gb_fr_device_vec_ntt_ragged(void *device_vec, const size_t *offsets, c
             continue;
         }
         fr_t sc = scale;
-        if (inverse) sc = sc * host_fr_inverse(host_fr_from_u64((uint64_t)1 << log_ns[j]));
+        if (inverse) sc = sc * host_fr_pow2_inverse(log_ns[j]);
         q_off.push_back(offsets[j]);
         q_log.push_back(log_ns[j]);
-        q_fac.push_back(ntt_factors{{sc, sc * first, sc * second}, 1});
+        q_fac.push_back(period3_factors(sc, sc * first, sc * second));
     }
     ntt_ragged(v->values, q_off.data(), q_log.data(), q_fac.data(), q_off.size(), inverse, st.ptr(), s);
-    lane_check();
     device_vec_mark_ready(v, s);
     return ok();
     GB_ENTRY_END
@@ -1724,13 +1830,13 @@ RustError midnight_sppark_bls12_381_fr_device_vec_divide_ntt_zeta(void *device_v
     size_t n = (size_t)1 << log_n;
     if (log_n > 31 || v->len != n) return make_error((int)cudaErrorInvalidValue, "resident NTT length mismatch");
     cudaStream_t s = lane_stream();
+    lane_check();  // of the lane's earlier work: this call's own waits are reported by a later one
     device_vec_wait(v, s);
     ntt_status st;
     dev_buf<fr_t> f(factor_len, s);
     h2d(f, factors, factor_len * sizeof(fr_t), s);
     launch_mul_assign_repeating(v->values, f, factor_len, n, s);
     ntt_ref_zeta(v->values, log_n, 1, true, scale, first, second, st.ptr(), s);
-    lane_check();
     device_vec_mark_ready(v, s);
     return ok();
     GB_ENTRY_END
@@ -1820,12 +1926,12 @@ RustError gb_fr_device_coeff_to_extended_coset_batch(void **out, const void *sou
     const size_t output_len = (size_t)1 << extended_log_n;
     if (input_len > output_len) return make_error(-1, "input length exceeds extended domain length");
     cudaStream_t s = lane_stream();
+    lane_check();  // of the lane's earlier work: this call's own waits are reported by a later one
     device_vec_wait(src, s);
     ntt_status st;
     fr_device_vec *v = device_vec_new(output_len * count, s);
     try {
         c2e_coset(v->values, src->values, input_len, count, extended_log_n, shift, st.ptr(), s);
-        lane_check();
         device_vec_mark_ready(v, s);
     } catch (...) {
         device_vec_delete(v);
@@ -1854,10 +1960,10 @@ RustError gb_fr_device_vec_ntt_coset_batch(void *device_vec, uint32_t log_n, siz
     if (shift.is_zero()) return make_error((int)cudaErrorInvalidValue, "zero coset shift");
     if (log_n == 0) return ok();
     cudaStream_t s = lane_stream();
+    lane_check();  // of the lane's earlier work: this call's own waits are reported by a later one
     device_vec_wait(v, s);
     ntt_status st;
     ntt_coset(v->values, log_n, count, inverse, shift, st.ptr(), s);
-    lane_check();
     device_vec_mark_ready(v, s);
     return ok();
     GB_ENTRY_END
