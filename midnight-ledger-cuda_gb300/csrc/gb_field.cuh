@@ -39,7 +39,7 @@
 #define GB_COLD inline
 #endif
 
-#include "gb_fp_sqr.cuh"
+#include "gb_fp_rows.cuh"
 
 namespace gb {
 
@@ -178,49 +178,8 @@ GB_D void row_mac8(uint32_t *acc, uint32_t x0, uint32_t x1, uint32_t x2, uint32_
 }
 
 // acc += modulus * m, modulus limbs as immediates (no registers held for them)
-#define GB_ROW12_IMM(acc, x0, x1, x2, x3, x4, x5, y)                                                    \
-    asm("mad.lo.cc.u32 %0, %13, %14, %0;\n\t"                                                         \
-        "madc.hi.cc.u32 %1, %13, %14, %1;\n\t"                                                        \
-        "madc.lo.cc.u32 %2, %13, %15, %2;\n\t"                                                        \
-        "madc.hi.cc.u32 %3, %13, %15, %3;\n\t"                                                        \
-        "madc.lo.cc.u32 %4, %13, %16, %4;\n\t"                                                        \
-        "madc.hi.cc.u32 %5, %13, %16, %5;\n\t"                                                        \
-        "madc.lo.cc.u32 %6, %13, %17, %6;\n\t"                                                        \
-        "madc.hi.cc.u32 %7, %13, %17, %7;\n\t"                                                        \
-        "madc.lo.cc.u32 %8, %13, %18, %8;\n\t"                                                        \
-        "madc.hi.cc.u32 %9, %13, %18, %9;\n\t"                                                        \
-        "madc.lo.cc.u32 %10, %13, %19, %10;\n\t"                                                      \
-        "madc.hi.cc.u32 %11, %13, %19, %11;\n\t"                                                      \
-        "addc.u32 %12, %12, 0;"                                                                         \
-        : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]),          \
-          "+r"(acc[6]), "+r"(acc[7]), "+r"(acc[8]), "+r"(acc[9]), "+r"(acc[10]), "+r"(acc[11]),        \
-          "+r"(acc[12])                                                                                 \
-        : "r"(y), "n"(x0), "n"(x1), "n"(x2), "n"(x3), "n"(x4), "n"(x5))
-
-#define GB_ROW8_IMM(acc, x0, x1, x2, x3, y)                                                             \
-    asm("mad.lo.cc.u32 %0, %9, %10, %0;\n\t"                                                          \
-        "madc.hi.cc.u32 %1, %9, %10, %1;\n\t"                                                         \
-        "madc.lo.cc.u32 %2, %9, %11, %2;\n\t"                                                         \
-        "madc.hi.cc.u32 %3, %9, %11, %3;\n\t"                                                         \
-        "madc.lo.cc.u32 %4, %9, %12, %4;\n\t"                                                         \
-        "madc.hi.cc.u32 %5, %9, %12, %5;\n\t"                                                         \
-        "madc.lo.cc.u32 %6, %9, %13, %6;\n\t"                                                         \
-        "madc.hi.cc.u32 %7, %9, %13, %7;\n\t"                                                         \
-        "addc.u32 %8, %8, 0;"                                                                           \
-        : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]),          \
-          "+r"(acc[6]), "+r"(acc[7]), "+r"(acc[8])                                                      \
-        : "r"(y), "n"(x0), "n"(x1), "n"(x2), "n"(x3))
-
 template <class Cfg>
 GB_D void row_mac_mod(uint32_t *acc, int parity, uint32_t m);
-
-template <>
-GB_D void row_mac_mod<FpCfg>(uint32_t *acc, int parity, uint32_t m)
-{
-    typedef FpCfg C;
-    if (parity == 0) GB_ROW12_IMM(acc, C::M0, C::M2, C::M4, C::M6, C::M8, C::M10, m);
-    else GB_ROW12_IMM(acc, C::M1, C::M3, C::M5, C::M7, C::M9, C::M11, m);
-}
 
 template <>
 GB_D void row_mac_mod<FrCfg>(uint32_t *acc, int parity, uint32_t m)
@@ -262,27 +221,6 @@ GB_D void row_mac_mod<FrCfg>(uint32_t *acc, int parity, uint32_t m)
 
 // even[0..N-1] = even[1..N] + odd[0..N-1], even[N] = odd[N] + carry: the
 // division by 2^32 that ends each CIOS step, as one carry chain
-GB_D void fold12(uint32_t *e, const uint32_t *o)
-{
-    asm("add.cc.u32 %0, %1, %13;\n\t"
-        "addc.cc.u32 %1, %2, %14;\n\t"
-        "addc.cc.u32 %2, %3, %15;\n\t"
-        "addc.cc.u32 %3, %4, %16;\n\t"
-        "addc.cc.u32 %4, %5, %17;\n\t"
-        "addc.cc.u32 %5, %6, %18;\n\t"
-        "addc.cc.u32 %6, %7, %19;\n\t"
-        "addc.cc.u32 %7, %8, %20;\n\t"
-        "addc.cc.u32 %8, %9, %21;\n\t"
-        "addc.cc.u32 %9, %10, %22;\n\t"
-        "addc.cc.u32 %10, %11, %23;\n\t"
-        "addc.cc.u32 %11, %12, %24;\n\t"
-        "addc.u32 %12, %25, 0;"
-        : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]),
-          "+r"(e[8]), "+r"(e[9]), "+r"(e[10]), "+r"(e[11]), "+r"(e[12])
-        : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]),
-          "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]));
-}
-
 GB_D void fold8(uint32_t *e, const uint32_t *o)
 {
     asm("add.cc.u32 %0, %1, %9;\n\t"
@@ -302,21 +240,12 @@ GB_D void fold8(uint32_t *e, const uint32_t *o)
 template <int N>
 GB_D void fold(uint32_t *e, const uint32_t *o);
 template <>
-GB_D void fold<12>(uint32_t *e, const uint32_t *o) { fold12(e, o); }
-template <>
 GB_D void fold<8>(uint32_t *e, const uint32_t *o) { fold8(e, o); }
 
 // acc += x * y where x is given by its even (parity 0) or odd (parity 1)
 // limbs: x[parity + 2k] for k < N/2
 template <int N>
 GB_D void row_mac(uint32_t *acc, const uint32_t *x, int parity, uint32_t y);
-
-template <>
-GB_D void row_mac<12>(uint32_t *acc, const uint32_t *x, int parity, uint32_t y)
-{
-    if (parity == 0) row_mac12(acc, x[0], x[2], x[4], x[6], x[8], x[10], y);
-    else row_mac12(acc, x[1], x[3], x[5], x[7], x[9], x[11], y);
-}
 
 template <>
 GB_D void row_mac<8>(uint32_t *acc, const uint32_t *x, int parity, uint32_t y)
@@ -334,54 +263,30 @@ GB_D void mod_add_dev(uint32_t *r, const uint32_t *a, const uint32_t *b);
 template <class Cfg>
 GB_D void mod_sub_dev(uint32_t *r, const uint32_t *a, const uint32_t *b);
 
-// a + b mod m for a, b < m: one carry chain for the sum, one borrow chain
-// subtracting the modulus (immediates), then a select
+// a + b mod p for a, b < p: one carry chain for the sum (below 2^382, no
+// carry out), one borrow chain subtracting p (immediates), then a select
 template <>
 GB_D void mod_add_dev<FpCfg>(uint32_t *r, const uint32_t *a, const uint32_t *b)
 {
     typedef FpCfg C;
-    uint32_t s[12], t[12], c, br;
-    asm("add.cc.u32 %0, %13, %25;\n\t"
-        "addc.cc.u32 %1, %14, %26;\n\t"
-        "addc.cc.u32 %2, %15, %27;\n\t"
-        "addc.cc.u32 %3, %16, %28;\n\t"
-        "addc.cc.u32 %4, %17, %29;\n\t"
-        "addc.cc.u32 %5, %18, %30;\n\t"
-        "addc.cc.u32 %6, %19, %31;\n\t"
-        "addc.cc.u32 %7, %20, %32;\n\t"
-        "addc.cc.u32 %8, %21, %33;\n\t"
-        "addc.cc.u32 %9, %22, %34;\n\t"
-        "addc.cc.u32 %10, %23, %35;\n\t"
-        "addc.cc.u32 %11, %24, %36;\n\t"
-        "addc.u32 %12, 0, 0;"
-        : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(s[8]), "=r"(s[9]), "=r"(s[10]), "=r"(s[11]), "=r"(c)
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]));
-    asm("sub.cc.u32 %0, %13, %26;\n\t"
-        "subc.cc.u32 %1, %14, %27;\n\t"
-        "subc.cc.u32 %2, %15, %28;\n\t"
-        "subc.cc.u32 %3, %16, %29;\n\t"
-        "subc.cc.u32 %4, %17, %30;\n\t"
-        "subc.cc.u32 %5, %18, %31;\n\t"
-        "subc.cc.u32 %6, %19, %32;\n\t"
-        "subc.cc.u32 %7, %20, %33;\n\t"
-        "subc.cc.u32 %8, %21, %34;\n\t"
-        "subc.cc.u32 %9, %22, %35;\n\t"
-        "subc.cc.u32 %10, %23, %36;\n\t"
-        "subc.cc.u32 %11, %24, %37;\n\t"
-        "subc.u32 %12, %25, 0;"
-        : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "=r"(t[8]), "=r"(t[9]), "=r"(t[10]), "=r"(t[11]), "=r"(br)
-        : "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]), "r"(s[4]), "r"(s[5]), "r"(s[6]), "r"(s[7]), "r"(s[8]), "r"(s[9]), "r"(s[10]), "r"(s[11]), "r"(c), "n"(C::M0), "n"(C::M1), "n"(C::M2), "n"(C::M3), "n"(C::M4), "n"(C::M5), "n"(C::M6), "n"(C::M7), "n"(C::M8), "n"(C::M9), "n"(C::M10), "n"(C::M11));
-    // br = 0: s + c * 2^384 >= m, keep s - m
-#pragma unroll
-    for (int i = 0; i < 12; i++) r[i] = br ? s[i] : t[i];
-}
-
-// a - b mod m for a, b < m
-template <>
-GB_D void mod_sub_dev<FpCfg>(uint32_t *r, const uint32_t *a, const uint32_t *b)
-{
-    typedef FpCfg C;
-    uint32_t d[12], t[12], br;
+    uint32_t s[12], t[12], br;
+    asm("add.cc.u32 %0, %12, %24;\n\t"
+        "addc.cc.u32 %1, %13, %25;\n\t"
+        "addc.cc.u32 %2, %14, %26;\n\t"
+        "addc.cc.u32 %3, %15, %27;\n\t"
+        "addc.cc.u32 %4, %16, %28;\n\t"
+        "addc.cc.u32 %5, %17, %29;\n\t"
+        "addc.cc.u32 %6, %18, %30;\n\t"
+        "addc.cc.u32 %7, %19, %31;\n\t"
+        "addc.cc.u32 %8, %20, %32;\n\t"
+        "addc.cc.u32 %9, %21, %33;\n\t"
+        "addc.cc.u32 %10, %22, %34;\n\t"
+        "addc.u32 %11, %23, %35;"
+        : "=&r"(s[0]), "=&r"(s[1]), "=&r"(s[2]), "=&r"(s[3]), "=&r"(s[4]), "=&r"(s[5]), "=&r"(s[6]),
+          "=&r"(s[7]), "=&r"(s[8]), "=&r"(s[9]), "=&r"(s[10]), "=&r"(s[11])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]),
+          "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]),
+          "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]));
     asm("sub.cc.u32 %0, %13, %25;\n\t"
         "subc.cc.u32 %1, %14, %26;\n\t"
         "subc.cc.u32 %2, %15, %27;\n\t"
@@ -395,24 +300,62 @@ GB_D void mod_sub_dev<FpCfg>(uint32_t *r, const uint32_t *a, const uint32_t *b)
         "subc.cc.u32 %10, %23, %35;\n\t"
         "subc.cc.u32 %11, %24, %36;\n\t"
         "subc.u32 %12, 0, 0;"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(br)
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]));
-    asm("add.cc.u32 %0, %12, %24;\n\t"
-        "addc.cc.u32 %1, %13, %25;\n\t"
-        "addc.cc.u32 %2, %14, %26;\n\t"
-        "addc.cc.u32 %3, %15, %27;\n\t"
-        "addc.cc.u32 %4, %16, %28;\n\t"
-        "addc.cc.u32 %5, %17, %29;\n\t"
-        "addc.cc.u32 %6, %18, %30;\n\t"
-        "addc.cc.u32 %7, %19, %31;\n\t"
-        "addc.cc.u32 %8, %20, %32;\n\t"
-        "addc.cc.u32 %9, %21, %33;\n\t"
-        "addc.cc.u32 %10, %22, %34;\n\t"
-        "addc.u32 %11, %23, %35;\n\t"
-        : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "=r"(t[8]), "=r"(t[9]), "=r"(t[10]), "=r"(t[11])
-        : "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]), "r"(d[4]), "r"(d[5]), "r"(d[6]), "r"(d[7]), "r"(d[8]), "r"(d[9]), "r"(d[10]), "r"(d[11]), "n"(C::M0), "n"(C::M1), "n"(C::M2), "n"(C::M3), "n"(C::M4), "n"(C::M5), "n"(C::M6), "n"(C::M7), "n"(C::M8), "n"(C::M9), "n"(C::M10), "n"(C::M11));
+        : "=&r"(t[0]), "=&r"(t[1]), "=&r"(t[2]), "=&r"(t[3]), "=&r"(t[4]), "=&r"(t[5]), "=&r"(t[6]),
+          "=&r"(t[7]), "=&r"(t[8]), "=&r"(t[9]), "=&r"(t[10]), "=&r"(t[11]), "=r"(br)
+        : "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]), "r"(s[4]), "r"(s[5]), "r"(s[6]), "r"(s[7]), "r"(s[8]),
+          "r"(s[9]), "r"(s[10]), "r"(s[11]), "n"(C::M0), "n"(C::M1), "n"(C::M2), "n"(C::M3), "n"(C::M4),
+          "n"(C::M5), "n"(C::M6), "n"(C::M7), "n"(C::M8), "n"(C::M9), "n"(C::M10), "n"(C::M11));
 #pragma unroll
-    for (int i = 0; i < 12; i++) r[i] = br ? t[i] : d[i];
+    for (int i = 0; i < 12; i++) r[i] = br ? s[i] : t[i];
+}
+
+// a - b mod p for a, b < p: the addition of p is predicated on the borrow, so
+// there is no select (carry additions take 2 cycles a warp, and a mixed
+// addition has six subtractions)
+template <>
+GB_D void mod_sub_dev<FpCfg>(uint32_t *r, const uint32_t *a, const uint32_t *b)
+{
+    typedef FpCfg C;
+    uint32_t d[12];
+    asm("{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .u32 br;\n\t"
+        "sub.cc.u32 %0, %12, %24;\n\t"
+        "subc.cc.u32 %1, %13, %25;\n\t"
+        "subc.cc.u32 %2, %14, %26;\n\t"
+        "subc.cc.u32 %3, %15, %27;\n\t"
+        "subc.cc.u32 %4, %16, %28;\n\t"
+        "subc.cc.u32 %5, %17, %29;\n\t"
+        "subc.cc.u32 %6, %18, %30;\n\t"
+        "subc.cc.u32 %7, %19, %31;\n\t"
+        "subc.cc.u32 %8, %20, %32;\n\t"
+        "subc.cc.u32 %9, %21, %33;\n\t"
+        "subc.cc.u32 %10, %22, %34;\n\t"
+        "subc.cc.u32 %11, %23, %35;\n\t"
+        "subc.u32 br, 0, 0;\n\t"
+        "setp.ne.u32 p, br, 0;\n\t"
+        "@p add.cc.u32 %0, %0, %36;\n\t"
+        "@p addc.cc.u32 %1, %1, %37;\n\t"
+        "@p addc.cc.u32 %2, %2, %38;\n\t"
+        "@p addc.cc.u32 %3, %3, %39;\n\t"
+        "@p addc.cc.u32 %4, %4, %40;\n\t"
+        "@p addc.cc.u32 %5, %5, %41;\n\t"
+        "@p addc.cc.u32 %6, %6, %42;\n\t"
+        "@p addc.cc.u32 %7, %7, %43;\n\t"
+        "@p addc.cc.u32 %8, %8, %44;\n\t"
+        "@p addc.cc.u32 %9, %9, %45;\n\t"
+        "@p addc.cc.u32 %10, %10, %46;\n\t"
+        "@p addc.u32 %11, %11, %47;\n\t"
+        "}"
+        : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(d[4]), "=&r"(d[5]), "=&r"(d[6]),
+          "=&r"(d[7]), "=&r"(d[8]), "=&r"(d[9]), "=&r"(d[10]), "=&r"(d[11])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]),
+          "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]),
+          "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]), "n"(C::M0), "n"(C::M1),
+          "n"(C::M2), "n"(C::M3), "n"(C::M4), "n"(C::M5), "n"(C::M6), "n"(C::M7), "n"(C::M8), "n"(C::M9),
+          "n"(C::M10), "n"(C::M11));
+#pragma unroll
+    for (int i = 0; i < 12; i++) r[i] = d[i];
 }
 
 // a + b mod m for a, b < m: one carry chain for the sum, one borrow chain
@@ -592,7 +535,7 @@ struct mont_t {
     GB_HD mont_t &operator*=(const mont_t &o) { return *this = *this * o; }
     GB_HD mont_t sqr() const
     {
-#if defined(__CUDA_ARCH__) && !defined(GB_FP_MUL_INLINE) && !defined(GB_FP_SQR_OFF)
+#if defined(__CUDA_ARCH__) && !defined(GB_FP_MUL_INLINE)
         if constexpr (N == 12) return sqr_by_value(*this);
 #endif
         return *this * *this;
@@ -712,7 +655,10 @@ struct mont_t {
 };
 
 #if defined(__CUDA_ARCH__)
-// Device CIOS: for each limb b[i], accumulate a*b[i] and m*p into the running
+// Device CIOS of Fr (Fp's product and squaring are gb_fp_rows.cuh: measured
+// on GB300 with one out-of-line copy called by value, 28.4 -> 29.9 G products/s
+// and 33.6 -> 36.0 G squarings/s on all SMs, 1063 -> 982 and 893 -> 798 ns
+// for one dependent operation): for each limb b[i], accumulate a*b[i] and m*p into the running
 // sum held as two rows, `even` (products of even-indexed limbs) and `odd`
 // (products of odd-indexed limbs, stored one limb lower), so each row is a
 // single uninterrupted carry chain; the rows are folded once per iteration
@@ -739,37 +685,23 @@ GB_D void mont_step(uint32_t *even, uint32_t *odd, const uint32_t *a, uint32_t b
     fold<N>(even, odd);
 }
 
-// REDUCE = false skips the final conditional subtraction: the result is
-// then below m + a*b/R, i.e. below 2m whenever a*b < m*R
-template <class Cfg, bool REDUCE = true>
+template <class Cfg>
 GB_D void mont_mul_device(uint32_t *out, const uint32_t *a, const uint32_t *b)
 {
     constexpr int N = Cfg::N;
-    uint32_t even[N + 1], odd[N + 1];
+    if constexpr (N == 12) {
+        fp_mul_rows(out, a, b);
+    } else {
+        uint32_t even[N + 1], odd[N + 1];
 #pragma unroll
-    for (int i = 0; i < N + 1; i++) even[i] = 0;
-#if defined(GB_MUL_ROLLED)
-    // rolled outer loop: b's limbs are shifted down each step, so the code
-    // of one product stays a few hundred instructions (instruction-cache
-    // friendly when many products are inlined into one kernel)
-    uint32_t bb[N];
+        for (int i = 0; i < N + 1; i++) even[i] = 0;
 #pragma unroll
-    for (int i = 0; i < N; i++) bb[i] = b[i];
-#pragma unroll 1
-    for (int i = 0; i < N; i++) {
-        const uint32_t bi = bb[0];
+        for (int i = 0; i < N; i++) mont_step<Cfg>(even, odd, a, b[i]);
+        // even[0..N] < 2m; final conditional subtraction
+        mont_t<Cfg>::reduce_once(even, even[N]);
 #pragma unroll
-        for (int j = 0; j + 1 < N; j++) bb[j] = bb[j + 1];
-        mont_step<Cfg>(even, odd, a, bi);
+        for (int i = 0; i < N; i++) out[i] = even[i];
     }
-#else
-#pragma unroll
-    for (int i = 0; i < N; i++) mont_step<Cfg>(even, odd, a, b[i]);
-#endif
-    // even[0..N] < 2m; final conditional subtraction
-    if (REDUCE) mont_t<Cfg>::reduce_once(even, even[N]);
-#pragma unroll
-    for (int i = 0; i < N; i++) out[i] = even[i];
 }
 #endif
 
@@ -808,72 +740,12 @@ __device__ __noinline__ mont_t<Cfg> mont_t<Cfg>::mul_by_value(mont_t<Cfg> a, mon
 }
 #endif
 
-#if defined(__CUDA_ARCH__)
-// Fp Montgomery squaring: CIOS whose step i adds a_i times (a_i at word i,
-// then the words of 2 * sum_{j>i} a_j 2^(32 j)), so every cross product
-// a_i a_j is computed once, doubled: the a*a rows take 84 products instead
-// of 144 (the Montgomery rows are unchanged), 234 multiply-adds in all
-// against 300.  A step's multiplicand is below 2a < 2p, so the running sum
-// stays below 3p < 2^384 and the result below 2p, as in the product (the
-// rows are restated word by word and checked against a^2 R^-1 mod p in
-// tests/test_fp_sqr_rows.py).  Measured on GB300: the 2^20 MSM's
-// accumulation 3 % faster.  GB_FP_SQR_OFF selects the product form.
-template <int I>
-GB_D void sqr_step_fp(uint32_t *even, uint32_t *odd, const uint32_t *a, const uint32_t *d)
-{
-    typedef FpCfg C;
-    constexpr int J0 = (I + 1) & ~1;  // first even word at or above I
-    // multiplicand word j of step I: 0 below I, a_I at I, 2 a_{I+1} (without
-    // a_I's top bit) at I + 1, the words of 2a above
-    auto y = [&](int j) -> uint32_t {
-        return j < I ? 0u : j == I ? a[I] : j == I + 1 ? (a[(I + 1) % 12] << 1) : d[j % 12];
-    };
-    uint32_t ye[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++) ye[k] = J0 + 2 * k < 12 ? y(J0 + 2 * k) : 0u;
-    if constexpr (J0 < 12) sqr_row12<J0>(even, ye, a[I]);
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        const int j = 2 * k + 1;
-        const uint32_t yj = y(j);
-        odd[2 * k] = j < I ? 0u : yj * a[I];
-        odd[2 * k + 1] = j < I ? 0u : __umulhi(yj, a[I]);
-    }
-    odd[12] = 0;
-    const uint32_t m = even[0] * C::INV;
-    row_mac_mod<C>(even, 0, m);
-    row_mac_mod<C>(odd, 1, m);
-    fold<12>(even, odd);
-}
-
-template <int... I>
-GB_D void sqr_steps_fp(uint32_t *even, uint32_t *odd, const uint32_t *a, const uint32_t *d,
-                       std::integer_sequence<int, I...>)
-{
-    (sqr_step_fp<I>(even, odd, a, d), ...);
-}
-
-GB_D void mont_sqr_fp_device(uint32_t *out, const uint32_t *a)
-{
-    uint32_t d[12], even[13], odd[13];
-    d[0] = a[0] << 1;
-#pragma unroll
-    for (int j = 1; j < 12; j++) d[j] = (a[j] << 1) | (a[j - 1] >> 31);
-#pragma unroll
-    for (int i = 0; i < 13; i++) even[i] = 0;
-    sqr_steps_fp(even, odd, a, d, std::make_integer_sequence<int, 12>{});
-    mont_t<FpCfg>::reduce_once(even, even[12]);
-#pragma unroll
-    for (int i = 0; i < 12; i++) out[i] = even[i];
-}
-#endif
-
 #if defined(__CUDA_ARCH__) && !defined(GB_FP_MUL_INLINE)
 template <class Cfg>
 __device__ __noinline__ mont_t<Cfg> mont_t<Cfg>::sqr_by_value(mont_t<Cfg> a)
 {
     mont_t<Cfg> r;
-    if constexpr (Cfg::N == 12) mont_sqr_fp_device(r.v, a.v);
+    if constexpr (Cfg::N == 12) fp_sqr_rows(r.v, a.v);
     else mont_mul_device<Cfg>(r.v, a.v, a.v);
     return r;
 }

@@ -20,35 +20,11 @@ offsets in the other, so that a row of products is one carry chain.
 
     python gen_fr_shoup.py > gb_fr_shoup.cuh
 """
+from gen_rows import chain, emit
 
 R = 0x73EDA753299D7D483339D80809A1D80553BDA402FFFE5BFEFFFFFFFF00000001
 NEG_R = [((1 << 256) - R) >> (32 * i) & 0xFFFFFFFF for i in range(8)]
 assert NEG_R[0] == 0xFFFFFFFF and NEG_R[1] == 0
-
-
-def emit(ins):
-    """one asm statement for the (opcode, destination, sources...) list;
-    operands are C lvalues, '#...' immediates"""
-    outs, ins_only, read_first, written = [], [], set(), set()
-    for _, d, *_ in ins:
-        if d not in outs:
-            outs.append(d)
-    for _, d, *src in ins:
-        for o in src:
-            if o[0] == "#":
-                continue
-            if o in outs:
-                if o not in written:
-                    read_first.add(o)
-            elif o not in ins_only:
-                ins_only.append(o)
-        written.add(d)
-    num = {o: "%%%d" % i for i, o in enumerate(outs + ins_only)}
-    text = "\\n\\t\"\n        \"".join(
-        op + " " + ", ".join(o[1:] if o[0] == "#" else num[o] for o in ops) + ";" for op, *ops in ins)
-    res = ", ".join('"%s"(%s)' % ("+r" if o in read_first else "=&r", o) for o in outs)
-    arg = ", ".join('"r"(%s)' % o for o in ins_only)
-    return '    asm("%s"\n        : %s\n        : %s);\n' % (text, res, arg)
 
 
 class Rows:
@@ -94,12 +70,6 @@ class Rows:
             ins.append(("addc.u32", self.word(w), self.have(w), "#0"))
             self.live.add(w)
         return emit(ins) if ins else ""
-
-
-def chain(op, dst, a, b, head=()):
-    n = len(dst)
-    return emit(list(head) + [(op + ("" if k == 0 and not head else "c") + (".u32" if k == n - 1 else ".cc.u32"),
-                               dst[k], a[k], b[k]) for k in range(n)])
 
 
 def body():
