@@ -35,6 +35,7 @@
 #include <initializer_list>
 #include <vector>
 
+#include "gb_fp_inv.cuh"
 #include "gb_runtime.cuh"
 
 namespace gb {
@@ -242,9 +243,11 @@ __global__ void msm_hist_kernel(const uint32_t *__restrict__ digits, const seg_d
 }
 
 // 3. per global key g = seg * K + k: exclusive prefix over the segment's
-//    blocks (in place in hist) and the total into counts[g]
+//    blocks (in place in hist) and the total into counts[g], rounded up to a
+//    multiple of pad + 1 (a power of two; the places past the total hold
+//    kNoPoint)
 __global__ void msm_colscan_kernel(uint32_t *__restrict__ hist, const seg_desc *__restrict__ segs, uint32_t K,
-                                   uint32_t G, uint32_t *__restrict__ counts)
+                                   uint32_t G, uint32_t pad, uint32_t *__restrict__ counts)
 {
     uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= G) return;
@@ -269,7 +272,7 @@ __global__ void msm_colscan_kernel(uint32_t *__restrict__ hist, const seg_desc *
         col[(size_t)w * K] = run;
         run += v;
     }
-    counts[g] = run;
+    counts[g] = (run + pad) & ~pad;
 }
 
 // 4. exclusive scan of counts[0..G) into starts[0..G], starts[G] = total:
@@ -364,10 +367,308 @@ __global__ void msm_scatter_kernel(const uint32_t *__restrict__ digits, const se
     }
 }
 
+// 5b. affine rounds.  Adding two affine points takes one inversion, 2 products
+//     and 1 squaring, and Montgomery's trick shares one inversion among many
+//     additions for 3 products each: 5 products and a squaring against the 8
+//     and 2 of a mixed addition into XYZZ.  A round adds the entries 2i and
+//     2i + 1 of the bucket-ordered list and leaves a list of half the length:
+//     the buckets' starts are multiples of 2^rounds (kNoPoint fills them up),
+//     so no pair crosses a bucket.  A block's tile is 128 x per_thread pairs:
+//     each thread multiplies up its denominators, keeping the running products
+//     in `prefix`, the block's 128 totals go up a product tree, one warp
+//     inverts the root, the inverses come down, and each thread walks back
+//     through its pairs.
+//
+//     What bounds it: the multiply-add pipe, 82 % busy between inversions
+//     (about 8000 of its cycles a warp and pair, 6800 of them products), with
+//     four blocks an SM.  The first round of a 2^20-point MSM (8.4 M pairs)
+//     takes 2.2 ms, 0.27 ns a pair, against 0.33 ns a mixed addition.
+//     Measured and not kept: an inversion per warp instead of per block (no
+//     barriers, but four times the inversions' instructions: 0.6 ms more at
+//     2^20), tiles of different lengths so that an SM's blocks invert at
+//     different times (60 us more a round), 5 or 6 blocks an SM (spills).  The
+//     points come through shared memory by asynchronous copies that go
+//     through L1 (a 96-byte point is three sectors, each fetched by two 16-byte
+//     copies): two pairs ahead on the way up, one on the way back, 2 % better
+//     than plain loads; past L1 they were 8 % worse.
+static constexpr uint32_t kNoPoint = 0xffffffffu;
+static constexpr uint32_t kPairThreads = 128;
+static constexpr uint32_t kPairBlocks = 4;      // blocks an SM
+static constexpr uint32_t kPairsPerThread = 64;  // at most, in one tile
+
+__device__ __forceinline__ void store_words8(void *p, const uint32_t *w)
+{
+    asm volatile("st.global.v8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "l"(p)
+                 : "memory");
+}
+
+// the products of a pair, inlined: the two loops hold six copies in all
+// (45 KB), and the moves around a call cost more than fetching them
+__device__ __forceinline__ fp_t mul_here(const fp_t &a, const fp_t &b)
+{
+    fp_t r;
+#if defined(__CUDA_ARCH__)
+    fp_mul_rows(r.v, a.v, b.v);
+#endif
+    return r;
+}
+
+__device__ __forceinline__ fp_t sqr_here(const fp_t &a)
+{
+    fp_t r;
+#if defined(__CUDA_ARCH__)
+    fp_sqr_rows(r.v, a.v);
+#endif
+    return r;
+}
+
+// a thread's 16-byte slots in shared memory, one a 128-thread row
+struct pair_stage {
+    uint4 *slot;  // the thread's place in row 0
+    __device__ __forceinline__ void copy(uint32_t row, const void *src, uint32_t count) const
+    {
+#pragma unroll
+        for (uint32_t c = 0; c < count; c++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(slot + (row + c) * kPairThreads)),
+                         "l"((const uint4 *)src + c)
+                         : "memory");
+    }
+    __device__ __forceinline__ void copy_strided(uint32_t row, const uint4 *src) const
+    {
+#pragma unroll
+        for (uint32_t c = 0; c < 3; c++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(slot + (row + c) * kPairThreads)),
+                         "l"(src + c * kPairThreads)
+                         : "memory");
+    }
+    static __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+    template <int N>
+    static __device__ __forceinline__ void wait()
+    {
+        asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+    }
+    __device__ __forceinline__ fp_t value(uint32_t row) const
+    {
+        fp_t v;
+        uint4 *d = reinterpret_cast<uint4 *>(&v);
+#pragma unroll
+        for (int c = 0; c < 3; c++) d[c] = slot[(row + c) * kPairThreads];
+        return v;
+    }
+};
+
+// a list's pair i: signed references into the bases, or the points themselves
+template <bool REFS>
+struct pair_refs {
+    uint2 r;
+    __device__ __forceinline__ void load(const uint32_t *refs, uint64_t i, bool in)
+    {
+        if (REFS) r = in ? reinterpret_cast<const uint2 *>(refs)[i] : make_uint2(kNoPoint, kNoPoint);
+    }
+    __device__ __forceinline__ bool none(int side) const { return REFS && (side ? r.y : r.x) == kNoPoint; }
+    __device__ __forceinline__ bool neg(int side) const { return REFS && (side ? r.y : r.x) >> 31; }
+    __device__ __forceinline__ const affine_t *point(const affine_t *points, uint64_t i, int side) const
+    {
+        if (!REFS) return points + 2 * i + side;
+        return points + (none(side) ? 0u : (side ? r.y : r.x) & 0x7fffffffu);
+    }
+    __device__ __forceinline__ fp_t y(const affine_t *points, uint64_t i, int side) const
+    {
+        const fp_t v = point(points, i, side)->y;
+        return neg(side) ? -v : v;
+    }
+};
+
+enum { PAIR_ADD, PAIR_FIRST, PAIR_SECOND, PAIR_DOUBLE, PAIR_INF };
+
+// how the pair's points are added, and the denominator of the slope (one
+// where there is none); the point at infinity is all zero, so the second
+// coordinates are read only where a first one is zero or both are equal
+template <bool REFS>
+__device__ __forceinline__ int pair_kind(const pair_refs<REFS> &ref, const affine_t *points, uint64_t i,
+                                         const fp_t &xa, const fp_t &xb, fp_t &den)
+{
+    den = xb - xa;
+    int kind = PAIR_ADD;
+    if (ref.none(1) || (xb.is_zero() && ref.y(points, i, 1).is_zero())) {
+        kind = PAIR_FIRST;
+    } else if (ref.none(0) || (xa.is_zero() && ref.y(points, i, 0).is_zero())) {
+        kind = PAIR_SECOND;
+    } else if (den.is_zero()) {
+        const fp_t ya = ref.y(points, i, 0);
+        kind = ya == ref.y(points, i, 1) && !ya.is_zero() ? PAIR_DOUBLE : PAIR_INF;
+        den = ya.dbl();
+    }
+    if (kind != PAIR_ADD && kind != PAIR_DOUBLE) den = fp_t::one();
+    return kind;
+}
+
+template <bool REFS>
+__global__ void __launch_bounds__(kPairThreads, kPairBlocks)
+    msm_affine_pairs_kernel(const uint32_t *__restrict__ refs, const affine_t *__restrict__ points,
+                            affine_t *__restrict__ out, const uint32_t *__restrict__ entries, int round,
+                            uint32_t per_thread, uint4 *__restrict__ prefix)
+{
+    __shared__ fp_t node[2 * kPairThreads];  // product tree: root 1, leaves 128 ..
+    __shared__ uint4 stage_mem[15 * kPairThreads];
+    const uint32_t tid = threadIdx.x;
+    const pair_stage stage{stage_mem + tid};
+    const uint64_t pairs = *entries >> round, tile = (uint64_t)kPairThreads * per_thread;
+    uint4 *pre = prefix + (uint64_t)blockIdx.x * per_thread * 3 * kPairThreads + tid;
+    for (uint64_t base = blockIdx.x * tile + tid; base - tid < pairs; base += gridDim.x * tile) {
+        const int turns =
+            (int)min((uint64_t)per_thread, (pairs - (base - tid) + kPairThreads - 1) / kPairThreads);
+        auto at = [&](int k) { return base + (uint64_t)(uint32_t)k * kPairThreads; };
+        auto in = [&](int k) { return k >= 0 && k < turns && at(k) < pairs; };
+
+        // up: the running product before each pair, x coordinates two ahead
+        // (rows 0..5 and 6..11)
+        pair_refs<REFS> r0, r1, r2;
+        r0.load(refs, at(0), in(0));
+        r1.load(refs, at(1), in(1));
+        r2.load(refs, at(2), in(2));
+        auto fetch_x = [&](const pair_refs<REFS> &r, int k) {
+            if (in(k)) {
+                const uint32_t row = k & 1 ? 6 : 0;
+                stage.copy(row, r.point(points, at(k), 0), 3);
+                stage.copy(row + 3, r.point(points, at(k), 1), 3);
+            }
+            stage.commit();
+        };
+        fetch_x(r0, 0);
+        fetch_x(r1, 1);
+        fp_t run = fp_t::one();
+        for (int k = 0; k < turns; k++) {
+            const uint4 *w = reinterpret_cast<const uint4 *>(&run);
+#pragma unroll
+            for (int c = 0; c < 3; c++) pre[(k * 3 + c) * kPairThreads] = w[c];
+            stage.wait<1>();
+            fp_t den = fp_t::one();
+            if (in(k)) {
+                const uint32_t row = k & 1 ? 6 : 0;
+                pair_kind<REFS>(r0, points, at(k), stage.value(row), stage.value(row + 3), den);
+            }
+            r0 = r1, r1 = r2;
+            fetch_x(r1, k + 2);
+            r2.load(refs, at(k + 3), in(k + 3));
+            run = mul_here(run, den);
+        }
+        __threadfence();  // the prefixes are read back by asynchronous copies
+
+        // down: all of a pair but its sign, one ahead (a 0..5, b 6..11, its
+        // prefix 12..14)
+        auto fetch = [&](const pair_refs<REFS> &r, int k) {
+            if (in(k)) {
+                stage.copy(0, r.point(points, at(k), 0), 6);
+                stage.copy(6, r.point(points, at(k), 1), 6);
+                stage.copy_strided(12, pre + k * 3 * kPairThreads);
+            }
+            stage.commit();
+        };
+        stage.wait<0>();
+        r0.load(refs, at(turns - 1), in(turns - 1));
+        r1.load(refs, at(turns - 2), in(turns - 2));
+        fetch(r0, turns - 1);
+
+        __syncthreads();  // the previous tile's tree is read
+        node[kPairThreads + tid] = run;
+        __syncthreads();
+        if (tid < 64) node[64 + tid] = node[128 + 2 * tid] * node[129 + 2 * tid];
+        __syncthreads();
+        fp_t inv;
+        if (tid < 32) {
+            for (uint32_t n = 32; n > 0; n >>= 1) {
+                if (tid < n) inv = node[2 * (n + tid)] * node[2 * (n + tid) + 1];
+                if (tid < n) node[n + tid] = inv;
+                __syncwarp();
+            }
+            inv = fp_inverse_warp(node + 1);
+            __syncwarp();
+            if (tid == 0) node[1] = inv;
+            __syncwarp();
+            // a child's inverse: its parent's times its sibling
+            for (uint32_t n = 2; n <= 32; n <<= 1) {
+                if (tid < n) inv = node[(n + tid) >> 1] * node[(n + tid) ^ 1];
+                __syncwarp();
+                if (tid < n) node[n + tid] = inv;
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        if (tid < 64) inv = node[(64 + tid) >> 1] * node[(64 + tid) ^ 1];
+        __syncthreads();
+        if (tid < 64) node[64 + tid] = inv;
+        __syncthreads();
+        inv = node[(128 + tid) >> 1] * node[(128 + tid) ^ 1];
+
+        for (int k = turns; k-- > 0;) {
+            stage.wait<0>();
+            const uint64_t i = at(k);
+            fp_t xa = fp_t::zero(), num = xa, ya = xa, di = xa;
+            int kind = PAIR_INF;
+            if (in(k)) {
+                di = mul_here(inv, stage.value(12));
+                xa = stage.value(0);
+                const fp_t xb = stage.value(6);
+                fp_t den;
+                kind = pair_kind<REFS>(r0, points, i, xa, xb, den);
+                inv = mul_here(inv, den);
+                ya = stage.value(3);
+                if (r0.neg(0)) ya = -ya;
+                num = stage.value(9);
+                if (r0.neg(1)) num = -num;
+            }
+            affine_t r;
+            if (kind == PAIR_SECOND) {
+                r.x = stage.value(6), r.y = num;
+            } else if (kind == PAIR_FIRST && !r0.none(0)) {
+                r.x = xa, r.y = ya;
+            } else {
+                r = affine_t::inf();
+            }
+            if (kind == PAIR_ADD) {
+                num = num - ya;
+                r.x = stage.value(6);
+            } else if (kind == PAIR_DOUBLE) {
+                num = sqr_here(xa);
+                num = num.dbl() + num;
+                r.x = xa;
+            }
+            r0 = r1;
+            fetch(r0, k - 1);
+            r1.load(refs, at(k - 2), in(k - 2));
+            if (kind == PAIR_ADD || kind == PAIR_DOUBLE) {
+                const fp_t s = mul_here(num, di);
+                r.x = sqr_here(s) - xa - r.x;
+                r.y = mul_here(s, xa - r.x) - ya;
+            }
+            if (i < pairs) {
+                const uint32_t *o = reinterpret_cast<const uint32_t *>(&r);
+#pragma unroll
+                for (int c = 0; c < 3; c++) store_words8(reinterpret_cast<uint32_t *>(out + i) + 8 * c, o + 8 * c);
+            }
+        }
+        stage.wait<0>();
+    }
+}
+
+// starts of the lists after the affine rounds
+__global__ void msm_shift_starts_kernel(const uint32_t *__restrict__ starts, uint32_t n, int rounds,
+                                        uint32_t *__restrict__ out)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = starts[i] >> rounds;
+}
+
 // 6. accumulate L sorted entries per thread.  Instantiated for several
 //    (block size, min blocks per SM) pairs: the register cap trades
 //    occupancy against spills, and the plan picks one.
-template <int BLOCK, int MINB>
+//    With REFS the entries are references into the bases, without it (after
+//    affine rounds) the points themselves.
+template <int BLOCK, int MINB, bool REFS = true>
 __global__ void __launch_bounds__(BLOCK, MINB) msm_accumulate_kernel(
     const uint32_t *__restrict__ sorted, const uint32_t *__restrict__ starts, uint32_t G, uint32_t L,
     size_t nchunks, const affine_t *__restrict__ points, xyzz_t *__restrict__ buckets,
@@ -392,9 +693,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) msm_accumulate_kernel(
     bool open = false;
     xyzz_t acc = xyzz_t::inf();
     for (uint64_t pos = lo; pos < hi; pos++) {
-        uint32_t ref = sorted[pos];
-        affine_t p = load_affine(points, ref & 0x7fffffffu);
-        acc.add_affine(p, (ref >> 31) != 0);
+        if (REFS) {
+            uint32_t ref = sorted[pos];
+            affine_t p = load_affine(points, ref & 0x7fffffffu);
+            acc.add_affine(p, (ref >> 31) != 0);
+        } else {
+            acc.add_affine(load_affine(points, (uint32_t)pos), false);
+        }
         open = true;
         if (pos + 1 == gend) {
             if (started_here) buckets[g] = acc;
@@ -960,12 +1265,39 @@ static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int varian
     return (uint32_t)std::min<uint64_t>(L, std::max<uint64_t>(4, std::max(by_latency, by_load)));
 }
 
+// Affine rounds of a batch: as long as a round has pairs enough to fill the
+// GPU (a round costs about 55 us whatever its size: product trees and one
+// inversion a block), and buckets 3 entries or longer remain, as every bucket
+// is padded to a multiple of 2^rounds.  Measured on GB300, ms a call without
+// rounds and with 1, 2, 3, 4 (* chosen):
+//   1 x 2^16 points  0.86*  0.87   0.87   0.95   1.01
+//   2 x 2^16         1.31   1.26*  1.31   1.35   1.52
+//   3 x 2^16         1.89   1.78   1.74*  1.84   1.99
+//   2^17             1.21   1.16*  1.19   1.19   1.31
+//   2^18             1.94   1.79   1.71*  1.76   1.80
+//   2^20             6.33   5.66   5.25   5.05   5.00*
+//   64 uneven ones  19.4   18.4   17.9   17.5*  19.4
+// Plain MSMs take rounds sooner: their sparse top window leaves a few long
+// buckets, which a round halves (2^16 points from host buffers 3.26 ms without
+// rounds, 2.93, 2.86* and 2.91 with 1, 2 and 3).
+static int affine_rounds(uint64_t digits, double avg, uint32_t G, bool precomputed)
+{
+    const uint64_t least = precomputed ? 3u << 18 : 5u << 16;
+    int r = 0;
+    while (r < 4 && digits >> (r + 1) >= least && avg >= 3.0 * (2 << r) &&
+           digits + (uint64_t)G * ((2u << r) - 1) < 0x80000000ull)
+        r++;
+    return r;
+}
+
 // The host half of a batch: its descriptors and launch sizes.
 struct batch_plan {
     int c = 0, nwin = 0, variant = 1;
     bool precomputed = false, coop_reduce = false;
     size_t stride = 0;
     uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, S = 0, S_coop = 0;
+    int rounds = 0;          // affine rounds before the accumulation
+    uint64_t entries = 0;    // bound of the bucket-ordered list, padding included
     uint64_t points_total = 0, digits_total = 0, nchunks = 0;
     std::vector<item_desc> idesc;
     std::vector<seg_desc> sdesc;
@@ -1029,7 +1361,9 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     const uint32_t nblocks = (uint32_t)bdesc.size();
     const double avg = (double)digits_total / (double)G;
     const int variant = default_acc_variant();
-    const uint32_t L = chunk_length(digits_total, avg, G, variant);
+    const int rounds = affine_rounds(digits_total, avg, G, precomputed);
+    const uint64_t entries = digits_total + (uint64_t)G * ((1u << rounds) - 1);
+    const uint32_t L = chunk_length(entries >> rounds, avg / (1 << rounds), G, variant);
     // reduction sub-segments: ~64K threads over the batch, 32..8192 per segment
     uint32_t S = 32;
     while (S < 8192 && (uint64_t)S * 2 * nseg <= 65536) S *= 2;
@@ -1048,7 +1382,7 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     const uint64_t budget = K >= (1u << 15) ? kCoopGroupBudget : kCoopGroupBudgetSmall;
     uint32_t S_coop = kCoopGroups;
     while (S_coop < K && (uint64_t)S_coop * 2 * nseg <= budget) S_coop *= 2;
-    const uint64_t nchunks = std::max<uint64_t>(1, (digits_total + L - 1) / L);
+    const uint64_t nchunks = std::max<uint64_t>(1, ((entries >> rounds) + L - 1) / L);
 
     P.c = c;
     P.nwin = nwin;
@@ -1067,10 +1401,47 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     P.points_total = points_total;
     P.digits_total = digits_total;
     P.nchunks = nchunks;
+    P.rounds = rounds;
+    P.entries = entries;
     P.idesc = std::move(idesc);
     P.sdesc = std::move(sdesc);
     P.bdesc = std::move(bdesc);
     return P;
+}
+
+// The affine rounds: the bucket-ordered references through P.rounds pairwise
+// additions, to a list of points a 2^rounds-th as long.
+static const affine_t *run_affine_rounds(const batch_plan &P, const uint32_t *sorted, const uint32_t *starts,
+                                         const affine_t *points, dev_buf<affine_t> &list_a,
+                                         dev_buf<affine_t> &list_b, cudaStream_t s)
+{
+    int sms = 0;
+    GB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device()));
+    const uint64_t slots = (uint64_t)sms * kPairBlocks;
+    // pairs a thread: whole waves of tiles of at most 16 a thread
+    auto per_thread = [&](uint64_t pairs) {
+        const uint64_t per = std::max<uint64_t>(1, (pairs + slots * kPairThreads - 1) / (slots * kPairThreads));
+        const uint64_t waves = (per + kPairsPerThread - 1) / kPairsPerThread;
+        return (uint32_t)((per + waves - 1) / waves);
+    };
+    dev_buf<uint4> prefix(slots * per_thread(P.entries / 2) * 3 * kPairThreads, s);
+    list_a = dev_buf<affine_t>(P.entries / 2 + 1, s);
+    if (P.rounds > 1) list_b = dev_buf<affine_t>(P.entries / 4 + 1, s);
+    const affine_t *in = points;
+    for (int r = 1; r <= P.rounds; r++) {
+        affine_t *out = r & 1 ? list_a.get() : list_b.get();
+        const uint64_t pairs = P.entries >> r;
+        const uint32_t per = std::min(per_thread(pairs), per_thread(P.entries / 2));
+        const uint64_t tiles = (pairs + (uint64_t)per * kPairThreads - 1) / ((uint64_t)per * kPairThreads);
+        const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(slots, tiles));
+        if (r == 1)
+            msm_affine_pairs_kernel<true><<<grid, kPairThreads, 0, s>>>(sorted, in, out, starts + P.G, r, per, prefix);
+        else
+            msm_affine_pairs_kernel<false><<<grid, kPairThreads, 0, s>>>(nullptr, in, out, starts + P.G, r, per, prefix);
+        GB_CHECK_LAUNCH();
+        in = out;
+    }
+    return in;
 }
 
 // The device half: every launch of the batch, its scratch allocated and
@@ -1087,7 +1458,7 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     const uint32_t nblocks = P.nblocks, L = P.L, S = P.S, S_coop = P.S_coop;
     const uint64_t points_total = P.points_total, digits_total = P.digits_total, nchunks = P.nchunks;
     (void)precomputed;
-    dev_buf<uint32_t> digits(std::max<uint64_t>(digits_total, 1), s), sorted(std::max<uint64_t>(digits_total, 1), s);
+    dev_buf<uint32_t> digits(std::max<uint64_t>(digits_total, 1), s), sorted(std::max<uint64_t>(P.entries, 1), s);
     dev_buf<uint32_t> hist((size_t)nblocks * K, s), counts(G, s), starts((size_t)G + 1, s);
     dev_buf<xyzz_t> buckets(G, s), head(nchunks, s), tail(nchunks, s);
     dev_buf<xyzz_t> partial((size_t)nseg * (coop_reduce ? S_coop / kCoopGroups : S), s), segsum(nseg, s);
@@ -1100,15 +1471,27 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     const size_t smem = (size_t)K * 4;
     msm_hist_kernel<<<nblocks, 1024, smem, s>>>(digits, d_segs, d_blks, K, hist);
     GB_CHECK_LAUNCH();
-    msm_colscan_kernel<<<blocks_for(G, 256), 256, 0, s>>>(hist, d_segs, K, G, counts);
+    msm_colscan_kernel<<<blocks_for(G, 256), 256, 0, s>>>(hist, d_segs, K, G, (1u << P.rounds) - 1, counts);
     GB_CHECK_LAUNCH();
+    if (P.rounds) GB_CUDA_OK(cudaMemsetAsync(sorted.get(), 0xff, P.entries * sizeof(uint32_t), s));  // kNoPoint
     u32_exclusive_scan(counts, G, starts, s);
     msm_scatter_kernel<<<nblocks, 1024, smem, s>>>(digits, d_segs, d_blks, K, precomputed ? stride : 0, hist,
                                                    starts, sorted);
     GB_CHECK_LAUNCH();
     timed_end(tok_sort, s, GB_SLOT_MSM_SORT);
     int tok = timed_begin(s);
-    if (variant == 1) {
+    dev_buf<affine_t> list_a, list_b;
+    dev_buf<uint32_t> shifted;
+    const uint32_t *bounds = starts;
+    if (P.rounds) {
+        const affine_t *list = run_affine_rounds(P, sorted, starts, points, list_a, list_b, s);
+        shifted = dev_buf<uint32_t>((size_t)G + 1, s);
+        msm_shift_starts_kernel<<<blocks_for(G + 1, 256), 256, 0, s>>>(starts, G + 1, P.rounds, shifted);
+        GB_CHECK_LAUNCH();
+        bounds = shifted;
+        msm_accumulate_kernel<256, 2, false><<<(unsigned)((nchunks + 255) / 256), 256, 0, s>>>(
+            nullptr, bounds, G, L, nchunks, list, buckets, head, tail);
+    } else if (variant == 1) {
         msm_accumulate_kernel<256, 2><<<(unsigned)((nchunks + 255) / 256), 256, 0, s>>>(
             sorted, starts, G, L, nchunks, points, buckets, head, tail);
     } else if (variant == 2) {
@@ -1130,14 +1513,14 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         // bucket keeps more of the multiply-add pipe busy (2^16 points
         // 0.104 -> 0.136 ms with groups)
         if (G <= kCoopFixupMaxBuckets)
-            msm_fixup_coop_kernel<<<(G + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(starts, G, L, head, tail,
+            msm_fixup_coop_kernel<<<(G + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(bounds, G, L, head, tail,
                                                                                      buckets, longs, nlong);
         else
-            msm_fixup_kernel<<<blocks_for(G, 128), 128, 0, s>>>(starts, G, L, head, tail, buckets, longs, nlong);
+            msm_fixup_kernel<<<blocks_for(G, 128), 128, 0, s>>>(bounds, G, L, head, tail, buckets, longs, nlong);
         GB_CHECK_LAUNCH();
         int sms = 0;
         GB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device()));
-        msm_fixup_long_kernel<<<(unsigned)sms * 2, 256, 0, s>>>(starts, L, head, tail, longs, nlong, buckets);
+        msm_fixup_long_kernel<<<(unsigned)sms * 2, 256, 0, s>>>(bounds, L, head, tail, longs, nlong, buckets);
         GB_CHECK_LAUNCH();
     }
     timed_end(tok_fix, s, GB_SLOT_MSM_FIXUP);
@@ -1212,11 +1595,12 @@ struct graph_key {
     bool precomputed = false, coop_reduce = false;
     size_t stride = 0;
     uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, S = 0, S_coop = 0;
+    int rounds = 0;
     uint64_t points_total = 0, digits_total = 0, nchunks = 0;
     auto tie() const
     {
         return std::tie(device, stream, points, c, variant, precomputed, coop_reduce, stride, nitems, K,
-                        segs_per_item, nseg, G, nblocks, L, S, S_coop, points_total, digits_total, nchunks);
+                        segs_per_item, nseg, G, nblocks, L, S, S_coop, rounds, points_total, digits_total, nchunks);
     }
     bool operator<(const graph_key &o) const { return tie() < o.tie(); }
 };
@@ -1279,7 +1663,7 @@ static bool run_planned_graph(const batch_plan &P, const affine_t *points, jacob
     key.c = P.c, key.variant = P.variant, key.precomputed = P.precomputed, key.coop_reduce = P.coop_reduce;
     key.stride = P.stride, key.nitems = P.nitems, key.K = P.K, key.segs_per_item = P.segs_per_item;
     key.nseg = P.nseg, key.G = P.G, key.nblocks = P.nblocks, key.L = P.L, key.S = P.S, key.S_coop = P.S_coop;
-    key.points_total = P.points_total, key.digits_total = P.digits_total, key.nchunks = P.nchunks;
+    key.points_total = P.points_total, key.digits_total = P.digits_total, key.nchunks = P.nchunks, key.rounds = P.rounds;
 
     // a stream the caller is capturing gets the launches themselves
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;

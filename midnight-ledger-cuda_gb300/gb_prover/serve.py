@@ -40,7 +40,9 @@ def proof_footprint_bytes(circuit):
     L, m, sets = circuit.lookups, circuit.m, circuit.permutation_sets
     ext_cols = m + sets + 3 * L + 2
     n_cols = 3 * (m + sets + 3 * L) + 12
-    msm_scratch = n * max(m, 4) * 24 * 4
+    # 16 windows of at most max(m, 4) polynomials: digits and bucket-ordered
+    # references, the affine rounds' two lists and their prefix products
+    msm_scratch = n * max(m, 4) * 16 * (8 + 72 + 24)
     return 32 * (ext * ext_cols + n * n_cols) + msm_scratch
 
 

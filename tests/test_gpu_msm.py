@@ -467,3 +467,29 @@ def test_async_batch_reads_scalars_as_queued(gb, orc):
         for i in range(3):
             assert (affine_of(orc, got[i]) == want[i]).all(), (rep, i)
     ctx.close()
+
+
+@pytest.mark.parametrize("n,count", [(1 << 16, 2), (65537, 3), (1 << 17, 3), (99991, 1)])
+def test_affine_rounds_special_pairs(gb, orc, n, count):
+    """Batches long enough for 1 to 3 affine rounds over bases that repeat:
+    equal points (doublings), opposite points (sums at infinity) and points
+    at infinity meet in the same bucket, and buckets of odd lengths end in
+    padding.  Every second MSM has uniform scalars, the others three values."""
+    rng = np.random.default_rng(n + count)
+    some = gb.g1_generator_mul(orc.fr_random(7, rng))
+    some[3] = 0
+    some = np.concatenate([some, some])
+    for row in some[7:]:  # the second half negated: y -> p - y
+        y = orc.P_MOD - sum(int(w) << (64 * i) for i, w in enumerate(row[6:]))
+        if any(row[6:]):
+            row[6:] = [(y >> (64 * i)) & 0xFFFFFFFFFFFFFFFF for i in range(6)]
+    bases = some[rng.integers(0, len(some), size=n)]
+    scal = orc.fr_random(n * count, rng).reshape(count, n, 4)
+    few = orc.fr_random(3, rng)
+    for i in range(0, count, 2):
+        scal[i] = few[rng.integers(0, 3, size=n)]
+    ctx = gb.Bls12_381G1MsmContext(bases)
+    got = ctx.batch(scal)
+    for i in range(count):
+        assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
+    ctx.close()
