@@ -14,8 +14,11 @@
 //                   sizes), writing finished buckets directly and chunk-edge
 //                   partials aside
 //   7. fix-up     : buckets spanning chunks add their partials
-//   8. reduce     : sum_k (k+1) B_k per segment by segmented running sums and
-//                   a tree, then per MSM the window combination.
+//                   (large batches: affine rounds before it)
+//   8. reduce     : sum_k (k+1) B_k per segment, by line and bit sums (few
+//                   buckets) or segmented running sums and a tree, then per
+//                   MSM the window combination; a few MSMs' last dependent
+//                   steps are the host's.
 //
 // A "segment" owns 2^(c-1) buckets.  Two modes:
 //   * precomputed (MSM contexts, whose bases are fixed): context creation
@@ -36,6 +39,7 @@
 #include <vector>
 
 #include "gb_fp_inv.cuh"
+#include "gb_host_fp.h"
 #include "gb_runtime.cuh"
 
 namespace gb {
@@ -43,29 +47,39 @@ namespace gb {
 static constexpr uint32_t kZeroDigit = 0xffffffffu;
 static constexpr int kMaxWindowBits = 16;  // 2^15 u32 counters = 128 KB smem
 
-static int windows_for(int c) { return 255 / c + 1; }
+// A scalar's 255 bits in windows of c and c - 1 bits, the wider ones first, so
+// that no window is a remainder of a few bits whose digits would crowd a few
+// buckets.  A (c - 1)-bit digit is at most 2^(c - 1), carry included, so it
+// stays positive and fills all the buckets; the top window is always one of
+// these (scalars are below 2^255, and 255 < windows c), so no carry is left.
+__host__ __device__ constexpr int windows_for(int c) { return 255 / c + 1; }
+__host__ __device__ constexpr int window_bits(int c, int j) { return j < 255 - windows_for(c) * (c - 1) ? c : c - 1; }
+__host__ __device__ constexpr int window_offset(int c, int j)
+{
+    const int wide = 255 - windows_for(c) * (c - 1);
+    return j < wide ? j * c : wide * c + (j - wide) * (c - 1);
+}
 
-// Window size: minimise mixed additions plus bucket-reduction additions,
-// over the sizes whose top window keeps at least 5 of the scalar's 255 bits
-// (8, 10, 13, 16).  With fewer, nearly every point's top digit falls in a
-// handful of buckets, which then span thousands of accumulation chunks.
+// Window size for n points, measured on GB300.  With the precomputed table an
+// MSM has 2^(c - 1) buckets in all: ms a call for one and for three MSMs (*
+// chosen)
+//   2^8 points   c = 8 0.26 0.29, 11* 0.19 0.23, 13 0.22 0.28
+//   2^10         10 0.26 0.29, 11 0.23 0.27, 12* 0.22 0.28, 13 0.22 0.29
+//   2^12         11 0.32 0.39, 12 0.28 0.38, 13* 0.25 0.39, 14 0.29 0.43
+//   2^14         12 0.42 0.70, 13* 0.38 0.66, 15 0.39 0.74, 16 0.44 0.84
+//   2^16         13 0.76 1.47, 15* 0.74 1.47, 16 0.73 1.54
+//   2^17         13 1.13 2.44, 15 1.08 2.38, 16* 1.03 2.41
+// Without it every window has its own buckets:
+//   2^10 points  8* 0.46, 9 0.47, 10 0.51
+//   2^12         8 0.52, 9* 0.52, 10 0.54
+//   2^14         9 0.71, 10* 0.71, 11 0.75
+//   2^16         10 1.14, 11* 1.11, 12 1.13, 13 1.18
+//   2^18         11 2.31, 12* 2.25, 13 2.30
 static int choose_window(size_t n, bool precomputed)
 {
-    if (n <= 1) return 8;
-    int best = 8;
-    double best_cost = 1e300;
-    for (int c = 8; c <= kMaxWindowBits; c++) {
-        if (255 % c < 5) continue;
-        double w = windows_for(c);
-        double adds = (double)n * w;
-        double red = (precomputed ? 1.0 : w) * std::ldexp(1.0, c) * 1.4;
-        double cost = adds + red;
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = c;
-        }
-    }
-    return best;
+    auto upto = [&](int lg) { return n <= (size_t)1 << lg; };
+    if (precomputed) return upto(7) ? 8 : upto(9) ? 11 : upto(11) ? 12 : upto(15) ? 13 : upto(16) ? 15 : 16;
+    return upto(11) ? 8 : upto(13) ? 9 : upto(15) ? 10 : upto(17) ? 11 : upto(19) ? 12 : 13;
 }
 
 static int default_acc_variant()
@@ -165,9 +179,8 @@ template <int C>
 __global__ void msm_recode_kernel(const item_desc *__restrict__ items, uint32_t nitems, uint64_t total,
                                   uint32_t *__restrict__ digits)
 {
-    constexpr int NWIN = 255 / C + 1;
+    constexpr int NWIN = windows_for(C);
     constexpr uint32_t half = 1u << (C - 1);
-    constexpr uint32_t mask = (1u << C) - 1;
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
     uint32_t lo = 0, hi = nitems;  // last item with point_prefix <= t
@@ -183,7 +196,8 @@ __global__ void msm_recode_kernel(const item_desc *__restrict__ items, uint32_t 
     uint32_t *out = digits + it.digit_base + i;
 #pragma unroll
     for (int j = 0; j < NWIN; j++) {
-        const int bit = j * C;
+        const int bit = window_offset(C, j);
+        const uint32_t mask = (1u << window_bits(C, j)) - 1;
         const int limb = bit >> 5, off = bit & 31;
         const uint32_t l0 = limb < 8 ? s.v[limb < 8 ? limb : 7] : 0;
         const uint32_t l1 = limb + 1 < 8 ? s.v[limb + 1 < 8 ? limb + 1 : 7] : 0;
@@ -851,12 +865,7 @@ __global__ void __launch_bounds__(256) xyzz_tree_sum_kernel(const xyzz_t *__rest
 // values after a group barrier, so the 8 lanes always take the same path.
 static constexpr uint32_t kCoopLanes = 8;
 static constexpr uint32_t kCoopGroups = 16;  // groups per 128-thread block
-static constexpr uint64_t kCoopMaxBuckets = 8u << 15;  // cooperative reduction up to 8 x 2^15 buckets
-// groups of the cooperative reduction over a batch: 2^15 buckets a segment,
-// then fewer buckets (a shorter chain per group, so the groups' contention
-// for the SMs' issue slots weighs more)
-static constexpr uint64_t kCoopGroupBudget = 6144;
-static constexpr uint64_t kCoopGroupBudgetSmall = 2048;
+static constexpr uint64_t kLinesMaxBuckets = 8u << 15;  // line sums up to 8 x 2^15 buckets
 static constexpr uint32_t kCoopFixupMaxBuckets = 1u << 14;  // cooperative fix-up up to 2^14 buckets in all
 // slots of a group: RUN, SUM, OPD (operand), RES (4 each: X, Y, ZZ, ZZZ),
 // then 12 temporaries
@@ -1027,10 +1036,11 @@ __device__ void coop_add(const coop_t &c, int a, int q)
     c.sync();
 }
 
-// the 16 groups of a block add their SUM slots into group 0's (4 levels)
+// the GROUPS groups of a block add their SUM slots into group 0's
+template <uint32_t GROUPS>
 __device__ void coop_block_tree(fp_t *sh, const coop_t &c, uint32_t grp)
 {
-    for (uint32_t off = kCoopGroups / 2; off > 0; off >>= 1) {
+    for (uint32_t off = GROUPS / 2; off > 0; off >>= 1) {
         __syncthreads();
         if (grp < off) {
             coop_copy(c, c.s + CO_OPD, sh + (size_t)(grp + off) * CO_SLOTS + CO_SUM);
@@ -1077,81 +1087,139 @@ __global__ void __launch_bounds__(128) msm_fixup_coop_kernel(const uint32_t *__r
     coop_store(c, CO_SUM, buckets + g);
 }
 
-// 8a'. msm_reduce_partial_kernel with one 8-lane group per (segment,
-//      sub-segment) and the block's 16 groups summed at the end: `partial`
-//      holds nseg * S / 16 points.  S is a power of two >= 16.
-__global__ void __launch_bounds__(128) msm_reduce_coop_kernel(const xyzz_t *__restrict__ buckets, uint32_t K,
-                                                              uint32_t S, xyzz_t *__restrict__ partial)
+// 8'. The reduction of a single MSM or a small batch, whose time is the depth
+//     of its chain of dependent additions: no running sums and no
+//     multiplication by an offset.  A segment's K = rows x cols buckets, bucket
+//     k at row k / cols and column k mod cols, have
+//         sum (k + 1) B_k = cols sum_i i R_i + sum_j (j + 1) C_j
+//     with the sums R_i of the rows and C_j of the columns: 2 K additions in
+//     trees, as many as running sums take.  Each weighted sum of lines is
+//     split by the bits of the weights, T_b = sum of the lines whose weight has
+//     bit b, so that sum_b 2^b T_b over both is log2 K + 1 doublings and as
+//     many additions, done by the host for a few segments and by one group a
+//     segment beyond.  Measured against running sums over sub-segments, each
+//     with its offset's double-and-add: one MSM of 2^12 buckets 0.172 -> 0.066
+//     ms, of 2^15 0.299 -> 0.150, three of 2^15 0.53 -> 0.265 (with the host's
+//     share, 15 us an MSM, outside these).  What bounds it: about 20 dependent
+//     additions of 5 to 10 us.
+struct line_shape {
+    uint32_t lr, lc;  // log2 of rows and columns
+    __host__ __device__ uint32_t lines() const { return (1u << lr) + (1u << lc); }
+    __host__ __device__ uint32_t bits() const { return lr + lc + 1; }
+};
+
+// 8a'. partial line sums, 2^lm buckets a thread: a segment's 2 K / 2^lm
+//      partials are the rows' [row][cols / 2^lm], then the columns'
+//      [column][rows / 2^lm]
+__global__ void __launch_bounds__(128) msm_line_partial_kernel(const xyzz_t *__restrict__ buckets, line_shape sh,
+                                                               uint32_t lm, uint64_t total,
+                                                               xyzz_t *__restrict__ partial)
 {
-    __shared__ __align__(16) fp_t sh[kCoopGroups * CO_SLOTS];
-    const uint32_t grp = threadIdx.x / kCoopLanes;
-    const coop_t c{sh + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
-    const uint32_t gid = blockIdx.x * kCoopGroups + grp;
-    const uint32_t seg = gid / S, sub = gid % S, m = K / S, k0 = sub * m;
-    const xyzz_t *B = buckets + (size_t)seg * K;
-    coop_set_inf(c, CO_RUN);
-    coop_set_inf(c, CO_SUM);
-    for (uint32_t k = k0 + m; k-- > k0;) {
-        coop_load(c, CO_OPD, B + k);
-        coop_add(c, CO_RUN, CO_OPD);  // run += B[k]
-        coop_add(c, CO_SUM, CO_RUN);  // sum += run
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    const uint32_t lk = sh.lr + sh.lc, half = 1u << (lk - lm), m = 1u << lm;
+    const uint64_t seg = t >> (lk + 1 - lm);
+    const uint32_t u = (uint32_t)t & (2 * half - 1);
+    const xyzz_t *B = buckets + (seg << lk);
+    uint32_t first, step, to;
+    if (u < half) {
+        const uint32_t row = u >> (sh.lc - lm), q = u & ((1u << (sh.lc - lm)) - 1);
+        first = (row << sh.lc) + q, step = 1u << (sh.lc - lm), to = u;
+    } else {
+        const uint32_t col = (u - half) & ((1u << sh.lc) - 1), q = (u - half) >> sh.lc;
+        first = (q << sh.lc) + col, step = 1u << (lk - lm), to = half + (col << (sh.lr - lm)) + q;
     }
-    if (k0) {
-        // sum += k0 * run, double-and-add from the top bit
-        coop_copy(c, c.s + CO_RES, c.s + CO_RUN);
-        int top = 31;
-        while (!((k0 >> top) & 1u)) top--;
-        for (int i = top - 1; i >= 0; i--) {
-            coop_dbl(c, CO_RES);
-            if ((k0 >> i) & 1u) coop_add(c, CO_RES, CO_RUN);
-        }
-        coop_add(c, CO_SUM, CO_RES);
-    }
-    coop_block_tree(sh, c, grp);
-    if (grp == 0) coop_store(c, CO_SUM, partial + blockIdx.x);
+    xyzz_t acc = B[first];
+    for (uint32_t e = 1; e < m; e++) acc.add(B[first + e * step]);
+    partial[seg * 2 * half + to] = acc;
 }
 
-// 8b'. tree sum with groups: out[seg * gridDim.x + b] = sum of the 32-element
-//      slice b of in[seg * n .. seg * n + n)
-__global__ void __launch_bounds__(128) xyzz_tree_sum_coop_kernel(const xyzz_t *__restrict__ in, uint32_t n,
-                                                                 xyzz_t *__restrict__ out)
+// 8b'. whole line sums, a block a line, from the partials (lm > 0) or the
+//      buckets (lm = 0)
+__global__ void __launch_bounds__(128) msm_line_sum_kernel(const xyzz_t *__restrict__ src, line_shape sh, uint32_t lm,
+                                                           xyzz_t *__restrict__ lines)
 {
-    __shared__ __align__(16) fp_t sh[kCoopGroups * CO_SLOTS];
+    __shared__ __align__(16) fp_t mem[kCoopGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
-    const coop_t c{sh + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
-    const xyzz_t *src = in + (size_t)blockIdx.y * n;
-    const uint32_t i0 = blockIdx.x * 2 * kCoopGroups + grp, i1 = i0 + kCoopGroups;
-    if (i0 < n) coop_load(c, CO_SUM, src + i0);
-    else coop_set_inf(c, CO_SUM);
-    if (i1 < n) {
-        coop_load(c, CO_OPD, src + i1);
+    const coop_t c{mem + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const uint32_t lk = sh.lr + sh.lc, rows = 1u << sh.lr, line = blockIdx.x, seg = blockIdx.y;
+    const bool row = line < rows;
+    const uint32_t n = 1u << ((row ? sh.lc : sh.lr) - lm);
+    const xyzz_t *p = src + ((uint64_t)seg << (lm ? lk + 1 - lm : lk));
+    uint32_t step = 1;
+    if (row) p += (uint64_t)line * n;
+    else if (lm) p += ((uint64_t)1 << (lk - lm)) + (uint64_t)(line - rows) * n;
+    else p += line - rows, step = 1u << sh.lc;
+    coop_set_inf(c, CO_SUM);
+    for (uint32_t e = grp; e < n; e += kCoopGroups) {
+        c.sync();
+        coop_load(c, CO_OPD, p + (uint64_t)e * step);
         coop_add(c, CO_SUM, CO_OPD);
     }
-    coop_block_tree(sh, c, grp);
-    if (grp == 0) coop_store(c, CO_SUM, out + (size_t)blockIdx.y * gridDim.x + blockIdx.x);
+    coop_block_tree<kCoopGroups>(mem, c, grp);
+    if (grp == 0) coop_store(c, CO_SUM, lines + (uint64_t)seg * sh.lines() + line);
 }
 
-// 8c. per MSM: combine its window segments (Horner) and emit a Jacobian point
-__global__ void msm_combine_kernel(const xyzz_t *__restrict__ seg_sum, uint32_t nitems, uint32_t segs_per_item,
-                                   int c, jacobian_t *__restrict__ out)
+// 8c'. the sums by weight bit, a block a bit: rows weigh i (bits 0 .. lr - 1,
+//      in places 2^lc and up of the result), columns j + 1 (bits 0 .. lc)
+static constexpr uint32_t kBitGroups = 32;
+
+__global__ void __launch_bounds__(kBitGroups *kCoopLanes) msm_bit_sum_kernel(const xyzz_t *__restrict__ lines,
+                                                                             line_shape sh, xyzz_t *__restrict__ bits)
 {
-    uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= nitems) return;
-    const xyzz_t *ss = seg_sum + (size_t)m * segs_per_item;
-    xyzz_t acc = xyzz_t::inf();
-    for (int w = (int)segs_per_item - 1; w >= 0; w--) {
-        if (w != (int)segs_per_item - 1)
-            for (int k = 0; k < c; k++) acc = acc.GB_DBL_LAT();
-        acc.GB_ADD_LAT(ss[w]);
+    __shared__ __align__(16) fp_t mem[kBitGroups * CO_SLOTS];
+    const uint32_t grp = threadIdx.x / kCoopLanes;
+    const coop_t c{mem + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const uint32_t seg = blockIdx.y, rows = 1u << sh.lr;
+    const bool row = blockIdx.x < sh.lr;
+    const uint32_t b = row ? blockIdx.x : blockIdx.x - sh.lr, lw = row ? sh.lr : sh.lc;
+    const xyzz_t *p = lines + (uint64_t)seg * sh.lines() + (row ? 0 : rows);
+    // weights below 2^lw with bit b, or 2^lc itself for the columns' last bit
+    const uint32_t n = b < lw ? 1u << (lw - 1) : 1u;
+    coop_set_inf(c, CO_SUM);
+    for (uint32_t e = grp; e < n; e += kBitGroups) {
+        const uint32_t w = b < lw ? (e >> b) << (b + 1) | 1u << b | (e & ((1u << b) - 1)) : 1u << b;
+        c.sync();
+        coop_load(c, CO_OPD, p + (row ? w : w - 1));
+        coop_add(c, CO_SUM, CO_OPD);
     }
-    out[m] = acc.to_jacobian();
+    coop_block_tree<kBitGroups>(mem, c, grp);
+    if (grp == 0) coop_store(c, CO_SUM, bits + (uint64_t)seg * sh.bits() + blockIdx.x);
 }
 
-// 8c'. msm_combine_kernel with one 8-lane group per MSM (16 MSMs a block):
-//       the Horner chain of a plain MSM is (windows - 1) * c doublings long
+// 8d'. the bit sums of a segment to one point: an 8-lane group a segment
+__global__ void __launch_bounds__(128) msm_bit_combine_kernel(const xyzz_t *__restrict__ bits, line_shape sh,
+                                                              uint32_t nseg, xyzz_t *__restrict__ seg_sum)
+{
+    __shared__ __align__(16) fp_t mem[kCoopGroups * CO_SLOTS];
+    const uint32_t grp = threadIdx.x / kCoopLanes;
+    const coop_t c{mem + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const uint32_t seg = blockIdx.x * kCoopGroups + grp;
+    if (seg >= nseg) return;  // whole groups leave together; no block barrier follows
+    const xyzz_t *p = bits + (uint64_t)seg * sh.bits();
+    coop_set_inf(c, CO_SUM);
+    for (int b = (int)(sh.lr + sh.lc); b >= 0; b--) {
+        coop_dbl(c, CO_SUM);
+        if (b >= (int)sh.lc && b < (int)(sh.lr + sh.lc)) {
+            c.sync();
+            coop_load(c, CO_OPD, p + b - sh.lc);
+            coop_add(c, CO_SUM, CO_OPD);
+        }
+        if (b <= (int)sh.lc) {
+            c.sync();
+            coop_load(c, CO_OPD, p + sh.lr + b);
+            coop_add(c, CO_SUM, CO_OPD);
+        }
+    }
+    c.sync();
+    coop_store(c, CO_SUM, seg_sum + seg);
+}
+
+// 8e. plain MSMs beyond a few: combine an MSM's window segments by Horner's
+//     rule, an 8-lane group an MSM ((windows - 1) * c doublings)
 __global__ void __launch_bounds__(128) msm_combine_coop_kernel(const xyzz_t *__restrict__ seg_sum, uint32_t nitems,
                                                                uint32_t segs_per_item, int c,
-                                                               jacobian_t *__restrict__ out)
+                                                               xyzz_t *__restrict__ out)
 {
     __shared__ __align__(16) fp_t sh[kCoopGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
@@ -1162,15 +1230,12 @@ __global__ void __launch_bounds__(128) msm_combine_coop_kernel(const xyzz_t *__r
     coop_set_inf(cp, CO_SUM);
     for (int w = (int)segs_per_item - 1; w >= 0; w--) {
         if (w != (int)segs_per_item - 1)
-            for (int k = 0; k < c; k++) coop_dbl(cp, CO_SUM);
+            for (int k = 0; k < window_bits(c, w); k++) coop_dbl(cp, CO_SUM);
         coop_load(cp, CO_OPD, ss + w);
         coop_add(cp, CO_SUM, CO_OPD);
     }
-    if (cp.lane == 0) {
-        xyzz_t acc;
-        acc.x = cp.s[CO_SUM], acc.y = cp.s[CO_SUM + 1], acc.zz = cp.s[CO_SUM + 2], acc.zzz = cp.s[CO_SUM + 3];
-        out[m] = acc.to_jacobian();
-    }
+    cp.sync();
+    coop_store(cp, CO_SUM, out + m);
 }
 
 // precompute: table[j * n + i] = 2^(c*j) P_i
@@ -1181,7 +1246,7 @@ __global__ void msm_precompute_kernel(affine_t *table, size_t n, int c, int nwin
     affine_t p = table[i];
     xyzz_t acc = xyzz_t::from_affine(p);
     for (int j = 1; j < nwin; j++) {
-        for (int k = 0; k < c; k++) acc = acc.dbl();
+        for (int k = 0; k < window_bits(c, j - 1); k++) acc = acc.dbl();
         table[(size_t)j * n + i] = acc.to_affine();
     }
 }
@@ -1277,12 +1342,9 @@ static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int varian
 //   2^18             1.94   1.79   1.71*  1.76   1.80
 //   2^20             6.33   5.66   5.25   5.05   5.00*
 //   64 uneven ones  19.4   18.4   17.9   17.5*  19.4
-// Plain MSMs take rounds sooner: their sparse top window leaves a few long
-// buckets, which a round halves (2^16 points from host buffers 3.26 ms without
-// rounds, 2.93, 2.86* and 2.91 with 1, 2 and 3).
-static int affine_rounds(uint64_t digits, double avg, uint32_t G, bool precomputed)
+static int affine_rounds(uint64_t digits, double avg, uint32_t G)
 {
-    const uint64_t least = precomputed ? 3u << 18 : 5u << 16;
+    const uint64_t least = 3u << 18;
     int r = 0;
     while (r < 4 && digits >> (r + 1) >= least && avg >= 3.0 * (2 << r) &&
            digits + (uint64_t)G * ((2u << r) - 1) < 0x80000000ull)
@@ -1290,12 +1352,65 @@ static int affine_rounds(uint64_t digits, double avg, uint32_t G, bool precomput
     return r;
 }
 
+// What the device leaves of each MSM and the host finishes once it is copied:
+// one point; the bit sums of its buckets (a context's MSM); or its window
+// sums (a plain MSM).  The last two are one chain of dependent doublings and
+// additions, which a host core runs 7 times faster than a group of GPU lanes
+// (about 25 us for 16 bit sums, 0.2 ms for 20 windows, against 0.13 and
+// 1.1 ms); the GPU runs them for batches of more than a few MSMs.
+static constexpr uint32_t kHostTailBits = 8, kHostTailWindows = 4;  // MSMs at most
+
+struct msm_tail {
+    enum { POINT, BITS, WINDOWS } kind = POINT;
+    uint32_t points = 1;  // of an MSM
+    int c = 0;
+    line_shape shape{0, 0};
+    jacobian_t finish(const xyzz_t *p) const;
+};
+
+jacobian_t msm_tail::finish(const xyzz_t *dev) const
+{
+    using namespace hostfp;
+    static_assert(sizeof(xyzz64) == sizeof(xyzz_t), "one memory image");
+    const xyzz64 *p = reinterpret_cast<const xyzz64 *>(dev);
+    xyzz64 acc = infinity();
+    if (kind == POINT) {
+        acc = p[0];
+    } else if (kind == WINDOWS) {
+        for (int w = (int)points - 1; w >= 0; w--) {
+            if (w != (int)points - 1)
+                for (int k = 0; k < window_bits(c, w); k++) acc = dbl(acc);
+            acc = add(acc, p[w]);
+        }
+    } else {
+        const int lr = (int)shape.lr, lc = (int)shape.lc;
+        for (int b = lr + lc; b >= 0; b--) {
+            acc = dbl(acc);
+            if (b >= lc && b < lr + lc) acc = add(acc, p[b - lc]);
+            if (b <= lc) acc = add(acc, p[lr + b]);
+        }
+    }
+    // (X ZZ^2, Y ZZZ^2, ZZZ) is a Jacobian form of the point
+    xyzz64 r{kOne, kOne, acc.zzz, acc.zzz};
+    if (!is_zero(acc.zz)) {
+        r.x = mont_mul(acc.x, mont_mul(acc.zz, acc.zz));
+        r.y = mont_mul(acc.y, mont_mul(acc.zzz, acc.zzz));
+    } else {
+        r.zz = acc.zz;
+    }
+    jacobian_t j;
+    memcpy(&j, &r, sizeof(j));  // x, y and z in place of zz
+    return j;
+}
+
 // The host half of a batch: its descriptors and launch sizes.
 struct batch_plan {
     int c = 0, nwin = 0, variant = 1;
-    bool precomputed = false, coop_reduce = false;
+    bool precomputed = false, by_lines = false;
     size_t stride = 0;
-    uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, S = 0, S_coop = 0;
+    uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, S = 0;
+    line_shape shape{0, 0};
+    msm_tail tail;
     int rounds = 0;          // affine rounds before the accumulation
     uint64_t entries = 0;    // bound of the bucket-ordered list, padding included
     uint64_t points_total = 0, digits_total = 0, nchunks = 0;
@@ -1361,34 +1476,24 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     const uint32_t nblocks = (uint32_t)bdesc.size();
     const double avg = (double)digits_total / (double)G;
     const int variant = default_acc_variant();
-    const int rounds = affine_rounds(digits_total, avg, G, precomputed);
+    const int rounds = affine_rounds(digits_total, avg, G);
     const uint64_t entries = digits_total + (uint64_t)G * ((1u << rounds) - 1);
     const uint32_t L = chunk_length(entries >> rounds, avg / (1 << rounds), G, variant);
     // reduction sub-segments: ~64K threads over the batch, 32..8192 per segment
     uint32_t S = 32;
     while (S < 8192 && (uint64_t)S * 2 * nseg <= 65536) S *= 2;
     S = std::min<uint32_t>(K, S);
-    // Few buckets in all (a single MSM or a small batch): the reduction is a
-    // chain per sub-segment, run by cooperative 8-lane groups.  More groups
-    // shorten the running sums, but each adds a double-and-add, and the
-    // groups share the SMs' issue slots: one operation took about 5 us up to
-    // 2048 groups, 6.5 us at 4096, 9 us at 6144 and 11 us at 8192 (GB300).
-    // Measured best: at most 6144 groups over the batch with 2^15 buckets a
-    // segment (4096 groups for one MSM, 6144 for three), 2048 with 2^12
-    // (three 2^14-point MSMs 0.274 -> 0.225 ms).  Many buckets (large
-    // batches): the one-thread-per-chain kernel keeps the multiply-add pipe
-    // busier.
-    const bool coop_reduce = (uint64_t)nseg * K <= kCoopMaxBuckets && K >= kCoopGroups;
-    const uint64_t budget = K >= (1u << 15) ? kCoopGroupBudget : kCoopGroupBudgetSmall;
-    uint32_t S_coop = kCoopGroups;
-    while (S_coop < K && (uint64_t)S_coop * 2 * nseg <= budget) S_coop *= 2;
+    // Few buckets in all (a single MSM or a small batch): line and bit sums,
+    // a short chain.  Many buckets (large batches): one running sum a thread
+    // keeps the multiply-add pipe busier.
+    const bool by_lines = (uint64_t)nseg * K <= kLinesMaxBuckets;
     const uint64_t nchunks = std::max<uint64_t>(1, ((entries >> rounds) + L - 1) / L);
 
     P.c = c;
     P.nwin = nwin;
     P.variant = variant;
     P.precomputed = precomputed;
-    P.coop_reduce = coop_reduce;
+    P.by_lines = by_lines;
     P.stride = stride;
     P.K = K;
     P.segs_per_item = segs_per_item;
@@ -1397,7 +1502,18 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     P.nblocks = nblocks;
     P.L = L;
     P.S = S;
-    P.S_coop = S_coop;
+    P.shape.lr = (uint32_t)(c - 1) / 2;
+    P.shape.lc = (uint32_t)(c - 1) - P.shape.lr;
+    // the steps left to the host: see msm_tail
+    P.tail.c = c;
+    if (precomputed && by_lines && nseg <= kHostTailBits) {
+        P.tail.kind = msm_tail::BITS;
+        P.tail.shape = P.shape;
+        P.tail.points = P.shape.bits();
+    } else if (!precomputed && nitems <= kHostTailWindows) {
+        P.tail.kind = msm_tail::WINDOWS;
+        P.tail.points = segs_per_item;
+    }
     P.points_total = points_total;
     P.digits_total = digits_total;
     P.nchunks = nchunks;
@@ -1449,19 +1565,17 @@ static const affine_t *run_affine_rounds(const batch_plan &P, const uint32_t *so
 // Queues device work only (no host synchronisation, no copy from host
 // memory), so a CUDA graph can capture it.
 static void run_planned(const batch_plan &P, const item_desc *d_items, const seg_desc *d_segs,
-                        const blk_desc *d_blks, const affine_t *points, jacobian_t *d_out, cudaStream_t s)
+                        const blk_desc *d_blks, const affine_t *points, xyzz_t *d_out, cudaStream_t s)
 {
     const int c = P.c, variant = P.variant;
-    const bool precomputed = P.precomputed, coop_reduce = P.coop_reduce;
+    const bool precomputed = P.precomputed;
     const size_t stride = P.stride;
     const uint32_t nitems = P.nitems, K = P.K, segs_per_item = P.segs_per_item, nseg = P.nseg, G = P.G;
-    const uint32_t nblocks = P.nblocks, L = P.L, S = P.S, S_coop = P.S_coop;
+    const uint32_t nblocks = P.nblocks, L = P.L, S = P.S;
     const uint64_t points_total = P.points_total, digits_total = P.digits_total, nchunks = P.nchunks;
-    (void)precomputed;
     dev_buf<uint32_t> digits(std::max<uint64_t>(digits_total, 1), s), sorted(std::max<uint64_t>(P.entries, 1), s);
     dev_buf<uint32_t> hist((size_t)nblocks * K, s), counts(G, s), starts((size_t)G + 1, s);
     dev_buf<xyzz_t> buckets(G, s), head(nchunks, s), tail(nchunks, s);
-    dev_buf<xyzz_t> partial((size_t)nseg * (coop_reduce ? S_coop / kCoopGroups : S), s), segsum(nseg, s);
 
     int tok_all = timed_begin(s);
     int tok_sort = timed_begin(s);
@@ -1525,29 +1639,49 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     }
     timed_end(tok_fix, s, GB_SLOT_MSM_FIXUP);
     int tok_red = timed_begin(s);
-    if (coop_reduce) {
-        // latency-bound: one 8-lane group per sub-segment, 16 groups a block
-        msm_reduce_coop_kernel<<<nseg * S_coop / kCoopGroups, 128, 0, s>>>(buckets, K, S_coop, partial);
-        GB_CHECK_LAUNCH();
-        const xyzz_t *src = partial;
-        uint32_t len = S_coop / kCoopGroups;
-        dev_buf<xyzz_t> tmp_a, tmp_b;
-        bool use_a = true;
-        while (len > 1) {
-            const uint32_t blocks = (len + 2 * kCoopGroups - 1) / (2 * kCoopGroups);
-            dev_buf<xyzz_t> &dst = use_a ? tmp_a : tmp_b;
-            dst = dev_buf<xyzz_t>((size_t)nseg * blocks, s);
-            xyzz_tree_sum_coop_kernel<<<dim3(blocks, nseg), 128, 0, s>>>(src, len, dst);
+    // an MSM's one point goes to d_out, its segments' sums elsewhere first
+    dev_buf<xyzz_t> sums;
+    xyzz_t *seg_sum = d_out;
+    if (segs_per_item > 1 && P.tail.kind == msm_tail::POINT) {
+        sums = dev_buf<xyzz_t>(nseg, s);
+        seg_sum = sums;
+    }
+    if (P.by_lines) {
+        const line_shape sh = P.shape;
+        const uint64_t total = (uint64_t)nseg * K;
+        // 2^lm buckets a thread adds before the lines' blocks take over: none
+        // where these are few, else as many as leave the blocks little to do
+        // (one-thread additions take 14 us each but fill all lanes; measured,
+        // us for lm = 0, 1, 2, 3, 4: 4096 buckets 67* 83 106 159 269, 2^14
+        // 105* 106 124 173 282, 2^15 178 159 151* 193 302, 3 x 2^15 311 289
+        // 265* 264 323, 4 x 2^15 398 371 313 277* 334)
+        const uint32_t lm = total <= (1u << 14) ? 0 : total <= 3u << 15 ? 2 : 3;
+        dev_buf<xyzz_t> partial, lines((size_t)nseg * sh.lines(), s), bits;
+        const xyzz_t *src = buckets;
+        if (lm) {
+            const uint64_t n = total * 2 >> lm;
+            partial = dev_buf<xyzz_t>(n, s);
+            msm_line_partial_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(buckets, sh, lm, n, partial);
             GB_CHECK_LAUNCH();
-            src = dst;
-            len = blocks;
-            use_a = !use_a;
+            src = partial;
         }
-        GB_CUDA_OK(cudaMemcpyAsync(segsum, src, (size_t)nseg * sizeof(xyzz_t), cudaMemcpyDeviceToDevice, s));
+        msm_line_sum_kernel<<<dim3(sh.lines(), nseg), 128, 0, s>>>(src, sh, lm, lines);
+        GB_CHECK_LAUNCH();
+        xyzz_t *bit_sum = d_out;
+        if (P.tail.kind != msm_tail::BITS) {
+            bits = dev_buf<xyzz_t>((size_t)nseg * sh.bits(), s);
+            bit_sum = bits;
+        }
+        msm_bit_sum_kernel<<<dim3(sh.bits(), nseg), kBitGroups * kCoopLanes, 0, s>>>(lines, sh, bit_sum);
+        GB_CHECK_LAUNCH();
+        if (P.tail.kind != msm_tail::BITS) {
+            msm_bit_combine_kernel<<<(nseg + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(bits, sh, nseg, seg_sum);
+            GB_CHECK_LAUNCH();
+        }
     } else {
-    msm_reduce_partial_kernel<<<blocks_for((size_t)nseg * S, 128), 128, 0, s>>>(buckets, K, S, nseg, partial);
-    GB_CHECK_LAUNCH();
-    {
+        dev_buf<xyzz_t> partial((size_t)nseg * S, s);
+        msm_reduce_partial_kernel<<<blocks_for((size_t)nseg * S, 128), 128, 0, s>>>(buckets, K, S, nseg, partial);
+        GB_CHECK_LAUNCH();
         // tree-sum each segment's S / group partials down to one point
         const xyzz_t *src = partial;
         uint32_t len = S / std::min<uint32_t>(S, 128);
@@ -1563,17 +1697,13 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
             len = blocks;
             use_a = !use_a;
         }
-        GB_CUDA_OK(cudaMemcpyAsync(segsum, src, (size_t)nseg * sizeof(xyzz_t), cudaMemcpyDeviceToDevice, s));
+        GB_CUDA_OK(cudaMemcpyAsync(seg_sum, src, (size_t)nseg * sizeof(xyzz_t), cudaMemcpyDeviceToDevice, s));
     }
-    }
-    if (segs_per_item > 1) {
-        // plain MSMs: a Horner chain per MSM, cooperative groups
-        msm_combine_coop_kernel<<<(nitems + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(segsum, nitems,
+    if (segs_per_item > 1 && P.tail.kind == msm_tail::POINT) {
+        msm_combine_coop_kernel<<<(nitems + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(seg_sum, nitems,
                                                                                           segs_per_item, c, d_out);
-    } else {
-        msm_combine_kernel<<<blocks_for(nitems, 32), 32, 0, s>>>(segsum, nitems, segs_per_item, c, d_out);
+        GB_CHECK_LAUNCH();
     }
-    GB_CHECK_LAUNCH();
     timed_end(tok_red, s, GB_SLOT_MSM_REDUCE);
     timed_end(tok_all, s, GB_SLOT_MSM_TOTAL);
 }
@@ -1592,15 +1722,15 @@ struct graph_key {
     cudaStream_t stream = nullptr;
     const affine_t *points = nullptr;
     int c = 0, variant = 0;
-    bool precomputed = false, coop_reduce = false;
+    bool precomputed = false, by_lines = false;
     size_t stride = 0;
-    uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, S = 0, S_coop = 0;
+    uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, S = 0;
     int rounds = 0;
     uint64_t points_total = 0, digits_total = 0, nchunks = 0;
     auto tie() const
     {
-        return std::tie(device, stream, points, c, variant, precomputed, coop_reduce, stride, nitems, K,
-                        segs_per_item, nseg, G, nblocks, L, S, S_coop, rounds, points_total, digits_total, nchunks);
+        return std::tie(device, stream, points, c, variant, precomputed, by_lines, stride, nitems, K, segs_per_item,
+                        nseg, G, nblocks, L, S, rounds, points_total, digits_total, nchunks);
     }
     bool operator<(const graph_key &o) const { return tie() < o.tie(); }
 };
@@ -1614,7 +1744,7 @@ struct graph_entry {
     item_desc *d_items = nullptr;
     seg_desc *d_segs = nullptr;
     blk_desc *d_blks = nullptr;
-    jacobian_t *d_out = nullptr;
+    xyzz_t *d_out = nullptr;
     uint64_t last_use = 0;
     std::mutex mu;  // descriptor upload, launch and result copy stay together
     ~graph_entry()
@@ -1654,15 +1784,15 @@ static bool graphs_enabled()
 
 // Runs the planned batch through a cached graph; false when this shape
 // cannot be captured (the caller then launches it directly).
-static bool run_planned_graph(const batch_plan &P, const affine_t *points, jacobian_t *d_out, cudaStream_t s)
+static bool run_planned_graph(const batch_plan &P, const affine_t *points, xyzz_t *d_out, cudaStream_t s)
 {
     graph_key key;
     key.device = current_device();
     key.stream = s;
     key.points = points;
-    key.c = P.c, key.variant = P.variant, key.precomputed = P.precomputed, key.coop_reduce = P.coop_reduce;
+    key.c = P.c, key.variant = P.variant, key.precomputed = P.precomputed, key.by_lines = P.by_lines;
     key.stride = P.stride, key.nitems = P.nitems, key.K = P.K, key.segs_per_item = P.segs_per_item;
-    key.nseg = P.nseg, key.G = P.G, key.nblocks = P.nblocks, key.L = P.L, key.S = P.S, key.S_coop = P.S_coop;
+    key.nseg = P.nseg, key.G = P.G, key.nblocks = P.nblocks, key.L = P.L, key.S = P.S;
     key.points_total = P.points_total, key.digits_total = P.digits_total, key.nchunks = P.nchunks, key.rounds = P.rounds;
 
     // a stream the caller is capturing gets the launches themselves
@@ -1686,7 +1816,7 @@ static bool run_planned_graph(const batch_plan &P, const affine_t *points, jacob
             e->d_items = (item_desc *)dev_alloc(P.nitems * sizeof(item_desc), s);
             e->d_segs = (seg_desc *)dev_alloc(P.nseg * sizeof(seg_desc), s);
             e->d_blks = (blk_desc *)dev_alloc(P.nblocks * sizeof(blk_desc), s);
-            e->d_out = (jacobian_t *)dev_alloc(P.nitems * sizeof(jacobian_t), s);
+            e->d_out = (xyzz_t *)dev_alloc((size_t)P.nitems * P.tail.points * sizeof(xyzz_t), s);
             cudaGraph_t g = nullptr;
             if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
                 (void)cudaGetLastError();
@@ -1727,30 +1857,41 @@ static bool run_planned_graph(const batch_plan &P, const affine_t *points, jacob
     h2d(e->d_segs, P.sdesc.data(), P.nseg * sizeof(seg_desc), s);
     h2d(e->d_blks, P.bdesc.data(), P.nblocks * sizeof(blk_desc), s);
     GB_CUDA_OK(cudaGraphLaunch(e->exec, s));
-    GB_CUDA_OK(cudaMemcpyAsync(d_out, e->d_out, P.nitems * sizeof(jacobian_t), cudaMemcpyDeviceToDevice, s));
+    GB_CUDA_OK(cudaMemcpyAsync(d_out, e->d_out, (size_t)P.nitems * P.tail.points * sizeof(xyzz_t),
+                               cudaMemcpyDeviceToDevice, s));
     g_graph_launches++;
     return true;
 }
 
+// A batch's results: tail.points XYZZ points per MSM, in device memory of the
+// stream the batch ran on.
+struct batch_result {
+    msm_tail tail;
+    dev_buf<xyzz_t> points;
+};
+
 // Run a batch of MSMs.  precomputed: `points` is a table of nwin rows of
 // `stride` bases (row j = 2^(c*j) P); plain: `points` holds the bases.
-// Results (one Jacobian point per item) are written to d_out (device).
 // use_graph: the bases pointer is stable across calls (a context's), so
 // the batch may replay a captured graph.
-static void msm_run_batch(const std::vector<msm_item> &items, int c, bool precomputed, const affine_t *points,
-                          size_t stride, jacobian_t *d_out, cudaStream_t s, bool use_graph = false)
+static batch_result msm_run_batch(const std::vector<msm_item> &items, int c, bool precomputed, const affine_t *points,
+                                  size_t stride, cudaStream_t s, bool use_graph = false)
 {
     set_smem_attrs();
-    if (items.empty()) return;
+    batch_result r;
+    if (items.empty()) return r;
     const batch_plan P = plan_batch(items, c, precomputed, stride);
-    if (use_graph && graphs_enabled() && run_planned_graph(P, points, d_out, s)) return;
+    r.tail = P.tail;
+    r.points = dev_buf<xyzz_t>((size_t)P.nitems * P.tail.points, s);
+    if (use_graph && graphs_enabled() && run_planned_graph(P, points, r.points, s)) return r;
     dev_buf<item_desc> d_items(P.nitems, s);
     dev_buf<seg_desc> d_segs(P.nseg, s);
     dev_buf<blk_desc> d_blks(P.nblocks, s);
     h2d(d_items, P.idesc.data(), P.nitems * sizeof(item_desc), s);
     h2d(d_segs, P.sdesc.data(), P.nseg * sizeof(seg_desc), s);
     h2d(d_blks, P.bdesc.data(), P.nblocks * sizeof(blk_desc), s);
-    run_planned(P, d_items, d_segs, d_blks, points, d_out, s);
+    run_planned(P, d_items, d_segs, d_blks, points, r.points, s);
+    return r;
 }
 
 }  // namespace gb
@@ -1851,11 +1992,10 @@ static int tuned_window(const std::vector<msm_item> &items, const affine_t *poin
     const std::string key = "msm:2^" + std::to_string(lg) + ":b" + std::to_string(bclass) + ":z" +
                             std::to_string(cls(h[0])) + ":s" + std::to_string(cls(h[1]));
     if (autotune_lookup(key, &c)) return c;
-    dev_buf<jacobian_t> scratch(nitems, s);
     float best = 1e30f;
     for (int cand : {8, 10, 13, 16}) {
         if (cand > kMaxWindowBits || ((size_t)1 << (cand - 1)) > 8 * total) continue;
-        float ms = time_on_stream(s, [&] { msm_run_batch(items, cand, false, points, stride, scratch, s); });
+        float ms = time_on_stream(s, [&] { msm_run_batch(items, cand, false, points, stride, s); });
         if (ms < best) {
             best = ms;
             c = cand;
@@ -1865,75 +2005,45 @@ static int tuned_window(const std::vector<msm_item> &items, const affine_t *poin
     return c;
 }
 
+// A plain batch over bases in device memory, results to the host.
+static void plain_run_items(jacobian_t *out, const affine_t *d_points, const std::vector<msm_item> &items,
+                            cudaStream_t s)
+{
+    const batch_result r = msm_run_batch(items, tuned_window(items, d_points, 0, s), false, d_points, 0, s);
+    std::vector<xyzz_t> staging(items.size() * r.tail.points);
+    d2h(staging.data(), r.points, staging.size() * sizeof(xyzz_t), s);
+    lane_sync(s);
+    for (size_t i = 0; i < items.size(); i++) out[i] = r.tail.finish(staging.data() + i * r.tail.points);
+    timed_collect();
+}
+
 static void msm_host_plain(jacobian_t *out, const affine_t *points, const fr_t *scalars, size_t n, size_t nmsms)
 {
     cudaStream_t s = lane_stream();
     dev_buf<affine_t> d_points(n, s);
     dev_buf<fr_t> d_scalars(n * nmsms, s);
-    dev_buf<jacobian_t> d_out(std::max<size_t>(nmsms, 1), s);
     h2d(d_points, points, n * sizeof(affine_t), s);
     h2d(d_scalars, scalars, n * nmsms * sizeof(fr_t), s);
     std::vector<msm_item> items;
     for (size_t m = 0; m < nmsms; m++) items.push_back(msm_item{d_scalars.get() + m * n, n, 0});
-    msm_run_batch(items, tuned_window(items, d_points, 0, s), false, d_points, 0, d_out, s);
-    d2h(out, d_out, nmsms * sizeof(jacobian_t), s);
-    lane_sync(s);
-    timed_collect();
+    plain_run_items(out, d_points, items, s);
 }
 
 // An MSM far smaller than the context's bucket count (2^(c-1)) skips the
-// precomputed windows: a precomputed MSM always pays for all the buckets,
-// while a small plain MSM with its own small window pays far less.  Below
-// this ratio of points to buckets the plain path is taken.
-static constexpr size_t kPrecomputedMinRatio = 8;
-
-// A batch against the context, queued on stream s.  Large items use the
-// precomputed table; small ones run as one plain batch over table row 0 (the
-// bases themselves) with a window sized for them.  The results (one Jacobian
-// point per item) are copied to `staging` on s, large items first; the
-// returned vector gives the item index of each staging slot.  `staging` must
-// be page-locked when the caller does not synchronise s before reading it.
-static std::vector<size_t> context_enqueue_items(msm_context_t *ctx, jacobian_t *staging,
-                                                 const std::vector<msm_item> &items, cudaStream_t s)
-{
-    std::vector<msm_item> big, small;
-    std::vector<size_t> big_idx, small_idx;
-    for (size_t i = 0; i < items.size(); i++) {
-        if (items[i].n * kPrecomputedMinRatio >= ((size_t)1 << (ctx->c - 1)) || items.size() == 1) {
-            big.push_back(items[i]);
-            big_idx.push_back(i);
-        } else {
-            small.push_back(items[i]);
-            small_idx.push_back(i);
-        }
-    }
-    dev_buf<jacobian_t> d_big(std::max<size_t>(big.size(), 1), s), d_small(std::max<size_t>(small.size(), 1), s);
-    if (!big.empty()) msm_run_batch(big, ctx->c, true, ctx->table, ctx->npoints, d_big, s, true);
-    if (!small.empty())
-        msm_run_batch(small, tuned_window(small, ctx->table, 0, s), false, ctx->table, 0, d_small, s, true);
-    d2h(staging, d_big, big.size() * sizeof(jacobian_t), s);
-    d2h(staging + big.size(), d_small, small.size() * sizeof(jacobian_t), s);
-    big_idx.insert(big_idx.end(), small_idx.begin(), small_idx.end());
-    return big_idx;
-}
-
-// The same, results to the host when it returns.
-static void context_run_items(msm_context_t *ctx, jacobian_t *out_host, const std::vector<msm_item> &items,
-                              cudaStream_t s)
-{
-    std::vector<jacobian_t> staging(items.size());
-    const std::vector<size_t> order = context_enqueue_items(ctx, staging.data(), items, s);
-    lane_sync(s);
-    for (size_t i = 0; i < order.size(); i++) out_host[order[i]] = staging[i];
-    timed_collect();
-}
+// precomputed windows: with the table it pays for all the buckets (about 30 us
+// for 2^15 of them), as a plain MSM with its own small window far less.  But
+// the plain MSMs are a batch of their own behind the other one (1 to 2 ms), so
+// the line lies well below where the two cost the same alone.  Measured: 64
+// MSMs of 2^10 .. 2^18 points on a 2^18 context, 9 of them below 2^11, 17.8 ms
+// with a ratio of 16 (two batches) and 15.8 ms with 32 and 64 (one).
+static constexpr size_t kPrecomputedMinRatio = 64;  // buckets / points
 
 // Page-locked staging buffers of the asynchronous MSM calls, reused: a
 // cudaFreeHost would synchronise the device, so buffers are kept until exit.
 static std::mutex g_pinned_mu;
-static std::multimap<size_t, jacobian_t *> g_pinned_free;
+static std::multimap<size_t, xyzz_t *> g_pinned_free;
 
-static jacobian_t *pinned_take(size_t n, size_t *cap)
+static xyzz_t *pinned_take(size_t n, size_t *cap)
 {
     n = std::max<size_t>(n, 64);
     {
@@ -1941,40 +2051,99 @@ static jacobian_t *pinned_take(size_t n, size_t *cap)
         auto it = g_pinned_free.lower_bound(n);
         if (it != g_pinned_free.end()) {
             *cap = it->first;
-            jacobian_t *p = it->second;
+            xyzz_t *p = it->second;
             g_pinned_free.erase(it);
             return p;
         }
     }
-    jacobian_t *p = nullptr;
-    GB_CUDA_OK(cudaHostAlloc((void **)&p, n * sizeof(jacobian_t), cudaHostAllocPortable));
+    xyzz_t *p = nullptr;
+    GB_CUDA_OK(cudaHostAlloc((void **)&p, n * sizeof(xyzz_t), cudaHostAllocPortable));
     *cap = n;
     return p;
 }
 
-static void pinned_give(jacobian_t *p, size_t cap)
+static void pinned_give(xyzz_t *p, size_t cap)
 {
     if (!p) return;
     std::lock_guard<std::mutex> lk(g_pinned_mu);
     g_pinned_free.emplace(cap, p);
 }
 
-// An MSM batch in flight: its completion event, the page-locked buffer its
-// results land in and the item order of that buffer.
+// A context batch's results on their way to the host: the page-locked buffer
+// they land in, and per part (the items with the precomputed table, then the
+// others) what is left to do and the items' places in the batch.
+struct pending_points {
+    xyzz_t *staging = nullptr;
+    size_t cap = 0;
+    struct part {
+        msm_tail tail;
+        std::vector<size_t> order;
+    };
+    std::vector<part> parts;
+    pending_points() = default;
+    pending_points(const pending_points &) = delete;
+    pending_points &operator=(const pending_points &) = delete;
+    ~pending_points() { pinned_give(staging, cap); }
+    // once the copies have landed
+    void finish(jacobian_t *out) const
+    {
+        const xyzz_t *p = staging;
+        for (const part &q : parts)
+            for (size_t i : q.order) {
+                out[i] = q.tail.finish(p);
+                p += q.tail.points;
+            }
+    }
+};
+
+// A batch against the context, queued on stream s.  Large items use the
+// precomputed table; small ones run as one plain batch over table row 0 (the
+// bases themselves) with a window sized for them.  The results are copied to
+// page-locked memory on s.
+static void context_enqueue_items(msm_context_t *ctx, pending_points &pending, const std::vector<msm_item> &items,
+                                  cudaStream_t s)
+{
+    std::vector<msm_item> sub[2];
+    std::vector<size_t> idx[2];
+    for (size_t i = 0; i < items.size(); i++) {
+        const bool big = items[i].n * kPrecomputedMinRatio >= ((size_t)1 << (ctx->c - 1)) || items.size() == 1;
+        sub[!big].push_back(items[i]);
+        idx[!big].push_back(i);
+    }
+    batch_result r[2];
+    if (!sub[0].empty()) r[0] = msm_run_batch(sub[0], ctx->c, true, ctx->table, ctx->npoints, s, true);
+    if (!sub[1].empty())
+        r[1] = msm_run_batch(sub[1], tuned_window(sub[1], ctx->table, 0, s), false, ctx->table, 0, s, true);
+    const size_t n0 = sub[0].size() * r[0].tail.points, n1 = sub[1].size() * r[1].tail.points;
+    pending.staging = pinned_take(n0 + n1, &pending.cap);
+    d2h(pending.staging, r[0].points, n0 * sizeof(xyzz_t), s);
+    d2h(pending.staging + n0, r[1].points, n1 * sizeof(xyzz_t), s);
+    for (int k = 0; k < 2; k++) pending.parts.push_back({r[k].tail, std::move(idx[k])});
+}
+
+// The same, results to the host when it returns.
+static void context_run_items(msm_context_t *ctx, jacobian_t *out_host, const std::vector<msm_item> &items,
+                              cudaStream_t s)
+{
+    pending_points pending;
+    context_enqueue_items(ctx, pending, items, s);
+    lane_sync(s);
+    pending.finish(out_host);
+    timed_collect();
+}
+
+// An MSM batch in flight: its completion event and its results.
 struct msm_ticket_t {
     int device = 0;
     uint32_t lane = 0;
     cudaEvent_t done = nullptr;
-    jacobian_t *staging = nullptr;
-    size_t cap = 0;
-    std::vector<size_t> order;
+    pending_points pending;
 };
 
 static void ticket_release(msm_ticket_t *t)
 {
     if (!t) return;
     if (t->done) cudaEventDestroy(t->done);
-    pinned_give(t->staging, t->cap);
     delete t;
 }
 
@@ -2035,12 +2204,7 @@ RustError gb_g1_msm_device(RawG1Projective *out_raw, const RawG1Affine *d_points
     if (!out || (n && (!d_points || !d_scalars)))
         return make_error((int)cudaErrorInvalidValue, "invalid device MSM arguments");
     cudaStream_t s = lane_stream();
-    dev_buf<jacobian_t> d_out(1, s);
-    std::vector<msm_item> items{msm_item{d_scalars, n, 0}};
-    msm_run_batch(items, tuned_window(items, d_points, 0, s), false, d_points, 0, d_out, s);
-    d2h(out, d_out, sizeof(jacobian_t), s);
-    lane_sync(s);
-    timed_collect();
+    plain_run_items(out, d_points, {msm_item{d_scalars, n, 0}}, s);
     return ok();
     GB_ENTRY_END
 }
@@ -2194,14 +2358,13 @@ RustError gb_g1_msm_context_device_batch_async(void **ticket, void *context, con
     try {
         t->device = current_device();
         t->lane = current_lane();
-        t->staging = pinned_take(nmsms, &t->cap);
         GB_CUDA_OK(cudaEventCreateWithFlags(&t->done, cudaEventDisableTiming));
         if (nmsms) {
             device_vec_wait(dv, s);
             std::vector<msm_item> items;
             for (size_t m = 0; m < nmsms; m++)
                 items.push_back(msm_item{dv->values + scalar_offset + m * npoints, npoints, 0});
-            t->order = context_enqueue_items(ctx, t->staging, items, s);
+            context_enqueue_items(ctx, t->pending, items, s);
         }
         GB_CUDA_OK(cudaEventRecord(t->done, s));
     } catch (...) {
@@ -2260,8 +2423,7 @@ RustError gb_msm_ticket_wait(void *ticket, RawG1Projective *out_raw)
     }
     set_lane(prev_lane);
     if (prev_dev != t->device) GB_CUDA_OK(cudaSetDevice(prev_dev));
-    if (out)
-        for (size_t i = 0; i < t->order.size(); i++) out[t->order[i]] = t->staging[i];
+    if (out) t->pending.finish(out);
     ticket_release(t);
     timed_collect();
     return ok();

@@ -493,3 +493,37 @@ def test_affine_rounds_special_pairs(gb, orc, n, count):
     for i in range(count):
         assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
     ctx.close()
+
+
+@pytest.mark.parametrize("bits", range(8, 17))
+@pytest.mark.parametrize("count", [1, 8, 9])
+def test_reduction_forms(gb, orc, bits, count):
+    """Every window size with one MSM, with the most the host finishes and
+    with one more (combined on the device): uniform scalars, one MSM of zeros
+    and one with a single nonzero scalar among them."""
+    rng = np.random.default_rng(bits * 16 + count)
+    n = 700
+    bases = gb.g1_generator_mul(orc.fr_random(n, rng))
+    from gb_prover._lib import RawMsmConfig
+    ctx = gb.Bls12_381G1MsmContext(bases, RawMsmConfig.default(n, bits))
+    scal = orc.fr_random(n * count, rng).reshape(count, n, 4)
+    if count > 2:
+        scal[1] = 0
+        scal[2, 1:] = 0
+    got = ctx.batch(scal)
+    for i in range(count):
+        assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
+    ctx.close()
+
+
+@pytest.mark.parametrize("count", [1, 4, 5])
+def test_plain_batches_host_and_device_combination(gb, orc, count):
+    """Plain batches on both sides of the line where the windows' Horner chain
+    moves from the host to the device."""
+    rng = np.random.default_rng(count)
+    n = 3000
+    bases = gb.g1_generator_mul(orc.fr_random(n, rng))
+    scal = orc.fr_random(n * count, rng).reshape(count, n, 4)
+    got = gb.bls12_381_g1_msm_batch(bases, scal)
+    for i in range(count):
+        assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
