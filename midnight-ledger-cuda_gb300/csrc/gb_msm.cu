@@ -686,7 +686,7 @@ template <int BLOCK, int MINB, bool REFS = true>
 __global__ void __launch_bounds__(BLOCK, MINB) msm_accumulate_kernel(
     const uint32_t *__restrict__ sorted, const uint32_t *__restrict__ starts, uint32_t G, uint32_t L,
     size_t nchunks, const affine_t *__restrict__ points, xyzz_t *__restrict__ buckets,
-    xyzz_t *__restrict__ head, xyzz_t *__restrict__ tail)
+    xyzz_t *__restrict__ head, xyzz_t *__restrict__ tail, uint32_t *__restrict__ open_bucket)
 {
     size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nchunks) return;
@@ -726,30 +726,41 @@ __global__ void __launch_bounds__(BLOCK, MINB) msm_accumulate_kernel(
             gend = g < G ? starts[g + 1] : T;
         }
     }
-    if (open) tail[t] = acc;
+    if (open) {
+        tail[t] = acc;
+        if (open_bucket && started_here) open_bucket[t] = g;
+    }
 }
 
-// 7. buckets spanning several chunks; empty buckets become infinity.  A
-//    bucket spanning up to kShortSpan chunks is summed by its own thread;
-//    longer ones (skewed digit distributions: a sparse top window,
-//    structured scalars) are appended to `longs` for msm_fixup_long_kernel.
-static constexpr uint32_t kShortSpan = 32;
+// 7. buckets spanning several chunks (empty buckets are infinity already: all
+//    zero, as they were before the accumulation).  A bucket spanning a few
+//    chunks is summed by its own thread; longer ones (skewed digits: structured
+//    scalars, the carry out of scalars below 2^64) are appended to `longs` for
+//    msm_fixup_long_kernel.  One thread a bucket, or, where buckets are shorter
+//    than chunks and most span none, one a chunk, so that the lanes that add
+//    lie closer together.  Measured, 64 MSMs of 2^10 .. 2^18 points with 2^15
+//    buckets each 1.60 -> 0.47 ms (chunks of 8 waves at most among it), 20 of
+//    2^10 .. 2^13 0.77 -> 0.10 ms (long buckets out of the threads' hands
+//    among it: one thread's 30 additions took 0.45 ms).
+static constexpr uint32_t kShortSpan = 32;  // chunks at most
+static constexpr uint32_t kNoBucket = 0xffffffffu;
 
-__global__ void msm_fixup_kernel(const uint32_t *__restrict__ starts, uint32_t G, uint32_t L,
+__global__ void msm_fixup_kernel(const uint32_t *__restrict__ starts, const uint32_t *__restrict__ open_bucket,
+                                 uint32_t n, uint32_t L, uint32_t short_span,
                                  const xyzz_t *__restrict__ head, const xyzz_t *__restrict__ tail,
                                  xyzz_t *__restrict__ buckets, uint32_t *__restrict__ longs,
                                  uint32_t *__restrict__ nlong)
 {
     uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G) return;
+    if (g >= n) return;
+    // a thread a chunk: the bucket that starts in it and runs on past its end
+    if (open_bucket) g = open_bucket[g];
+    if (g == kNoBucket) return;
     uint32_t s = starts[g], e = starts[g + 1];
-    if (s == e) {
-        buckets[g] = xyzz_t::inf();
-        return;
-    }
+    if (s == e) return;
     uint32_t cs = s / L, ce = (e - 1) / L;
     if (cs == ce) return;
-    if (ce - cs > kShortSpan) {
+    if (ce - cs > short_span) {
         longs[atomicAdd(nlong, 1u)] = g;
         return;
     }
@@ -757,99 +768,6 @@ __global__ void msm_fixup_kernel(const uint32_t *__restrict__ starts, uint32_t G
     for (uint32_t c = cs + 1; c < ce; c++) acc.GB_ADD_LAT(tail[c]);
     acc.GB_ADD_LAT(head[ce]);
     buckets[g] = acc;
-}
-
-// 7b. long buckets, one block each (grid-stride over the list): every
-//     thread sums a strided share of the bucket's chunk partials, then a
-//     shared-memory tree adds the 256 shares
-__global__ void __launch_bounds__(256) msm_fixup_long_kernel(const uint32_t *__restrict__ starts, uint32_t L,
-                                                            const xyzz_t *__restrict__ head,
-                                                            const xyzz_t *__restrict__ tail,
-                                                            const uint32_t *__restrict__ longs,
-                                                            const uint32_t *__restrict__ nlong,
-                                                            xyzz_t *__restrict__ buckets)
-{
-    __shared__ xyzz_t sh[256];
-    const uint32_t count = *nlong;
-    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
-        const uint32_t g = longs[i];
-        const uint32_t cs = starts[g] / L, ce = (starts[g + 1] - 1) / L;
-        // partials: tail[cs], tail[cs+1 .. ce-1], head[ce]
-        xyzz_t acc = xyzz_t::inf();
-        for (uint32_t c = cs + threadIdx.x; c <= ce; c += blockDim.x) acc.GB_ADD_LAT(c == ce ? head[c] : tail[c]);
-        sh[threadIdx.x] = acc;
-        __syncthreads();
-        for (uint32_t off = 128; off > 0; off >>= 1) {
-            if (threadIdx.x < off) {
-                xyzz_t v = sh[threadIdx.x];
-                v.GB_ADD_LAT(sh[threadIdx.x + off]);
-                sh[threadIdx.x] = v;
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) buckets[g] = sh[0];
-        __syncthreads();
-    }
-}
-
-// 8a. per (segment, sub-segment): U = sum_{k in sub} (k+1) B_k; then each
-//     aligned group of min(S, 128) sub-segments of a block is summed in
-//     shared memory, so `partial` holds nseg * S / group points
-__global__ void __launch_bounds__(128) msm_reduce_partial_kernel(const xyzz_t *__restrict__ buckets, uint32_t K,
-                                                                 uint32_t S, uint32_t nseg,
-                                                                 xyzz_t *__restrict__ partial)
-{
-    __shared__ xyzz_t sh[128];
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    xyzz_t sum = xyzz_t::inf();
-    if (t < nseg * S) {
-        uint32_t seg = t / S, s = t % S;
-        uint32_t m = K / S;
-        uint32_t k0 = s * m;
-        const xyzz_t *B = buckets + (size_t)seg * K;
-        xyzz_t run = xyzz_t::inf();
-        for (uint32_t k = k0 + m; k-- > k0;) {
-            run.GB_ADD_LAT(B[k]);
-            sum.GB_ADD_LAT(run);
-        }
-        if (k0) sum.GB_ADD_LAT(xyzz_mul_small(run, k0));
-    }
-    sh[threadIdx.x] = sum;
-    __syncthreads();
-    const uint32_t group = S < 128 ? S : 128;
-    for (uint32_t off = group / 2; off > 0; off >>= 1) {
-        if ((threadIdx.x & (group - 1)) < off) {
-            xyzz_t v = sh[threadIdx.x];
-            v.GB_ADD_LAT(sh[threadIdx.x + off]);
-            sh[threadIdx.x] = v;
-        }
-        __syncthreads();
-    }
-    if ((threadIdx.x & (group - 1)) == 0 && t < nseg * S) partial[t / group] = sh[threadIdx.x];
-}
-
-// 8b. tree sum: out[seg * gridDim.x + b] = sum of the 512-element slice b of
-//     in[seg * n .. seg * n + n), one block of 256 threads per slice
-__global__ void __launch_bounds__(256) xyzz_tree_sum_kernel(const xyzz_t *__restrict__ in, uint32_t n,
-                                                            xyzz_t *__restrict__ out)
-{
-    __shared__ xyzz_t sh[256];
-    const uint32_t seg = blockIdx.y;
-    const xyzz_t *src = in + (size_t)seg * n;
-    uint32_t i0 = blockIdx.x * 512 + threadIdx.x, i1 = i0 + 256;
-    xyzz_t acc = i0 < n ? src[i0] : xyzz_t::inf();
-    if (i1 < n) acc.GB_ADD_LAT(src[i1]);
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (uint32_t off = 128; off > 0; off >>= 1) {
-        if (threadIdx.x < off) {
-            xyzz_t v = sh[threadIdx.x];
-            v.GB_ADD_LAT(sh[threadIdx.x + off]);
-            sh[threadIdx.x] = v;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[(size_t)seg * gridDim.x + blockIdx.x] = sh[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -865,7 +783,6 @@ __global__ void __launch_bounds__(256) xyzz_tree_sum_kernel(const xyzz_t *__rest
 // values after a group barrier, so the 8 lanes always take the same path.
 static constexpr uint32_t kCoopLanes = 8;
 static constexpr uint32_t kCoopGroups = 16;  // groups per 128-thread block
-static constexpr uint64_t kLinesMaxBuckets = 8u << 15;  // line sums up to 8 x 2^15 buckets
 static constexpr uint32_t kCoopFixupMaxBuckets = 1u << 14;  // cooperative fix-up up to 2^14 buckets in all
 // slots of a group: RUN, SUM, OPD (operand), RES (4 each: X, Y, ZZ, ZZZ),
 // then 12 temporaries
@@ -1067,11 +984,7 @@ __global__ void __launch_bounds__(128) msm_fixup_coop_kernel(const uint32_t *__r
     const uint32_t g = blockIdx.x * kCoopGroups + grp;
     if (g >= G) return;  // whole groups leave together; no block barrier follows
     const uint32_t s = starts[g], e = starts[g + 1];
-    if (s == e) {
-        coop_set_inf(c, CO_SUM);
-        coop_store(c, CO_SUM, buckets + g);
-        return;
-    }
+    if (s == e) return;
     const uint32_t cs = s / L, ce = (e - 1) / L;
     if (cs == ce) return;
     if (ce - cs > kShortSpan) {
@@ -1085,6 +998,49 @@ __global__ void __launch_bounds__(128) msm_fixup_coop_kernel(const uint32_t *__r
         coop_add(c, CO_SUM, CO_OPD);
     }
     coop_store(c, CO_SUM, buckets + g);
+}
+
+// 7b. long buckets, one block each (grid-stride over the list): up to
+//     kLongDirect partials are shared out to the block's 32 groups and the
+//     groups' sums added in a tree (about 10 additions of 5 us); of more,
+//     every thread first sums a strided share (14 us an addition, but 256 at
+//     once), and the groups add the 256 shares.
+static constexpr uint32_t kLongGroups = 32, kLongDirect = 512;
+static constexpr size_t kLongSmem = kLongGroups * CO_SLOTS * sizeof(fp_t) + kLongGroups * kCoopLanes * sizeof(xyzz_t);
+
+__global__ void __launch_bounds__(kLongGroups *kCoopLanes)
+    msm_fixup_long_kernel(const uint32_t *__restrict__ starts, uint32_t L, const xyzz_t *__restrict__ head,
+                          const xyzz_t *__restrict__ tail, const uint32_t *__restrict__ longs,
+                          const uint32_t *__restrict__ nlong, xyzz_t *__restrict__ buckets)
+{
+    extern __shared__ __align__(16) unsigned char long_mem[];
+    fp_t *mem = reinterpret_cast<fp_t *>(long_mem);
+    xyzz_t *share = reinterpret_cast<xyzz_t *>(mem + kLongGroups * CO_SLOTS);
+    const uint32_t grp = threadIdx.x / kCoopLanes;
+    const coop_t c{mem + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const uint32_t count = *nlong;
+    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+        const uint32_t g = longs[i];
+        // partials: tail[cs], tail[cs+1 .. ce-1], head[ce]
+        const uint32_t cs = starts[g] / L, ce = (starts[g + 1] - 1) / L;
+        const bool direct = ce - cs < kLongDirect;
+        if (!direct) {
+            xyzz_t acc = xyzz_t::inf();
+            for (uint32_t k = cs + threadIdx.x; k <= ce; k += blockDim.x) acc.add(k == ce ? head[k] : tail[k]);
+            share[threadIdx.x] = acc;
+        }
+        __syncthreads();
+        const uint32_t n = direct ? ce - cs + 1 : kLongGroups * kCoopLanes;
+        coop_set_inf(c, CO_SUM);
+        for (uint32_t k = grp; k < n; k += kLongGroups) {
+            c.sync();
+            coop_load(c, CO_OPD, !direct ? share + k : cs + k == ce ? head + ce : tail + cs + k);
+            coop_add(c, CO_SUM, CO_OPD);
+        }
+        coop_block_tree<kLongGroups>(mem, c, grp);
+        if (grp == 0) coop_store(c, CO_SUM, buckets + g);
+        __syncthreads();
+    }
 }
 
 // 8'. The reduction of a single MSM or a small batch, whose time is the depth
@@ -1270,6 +1226,7 @@ static void set_smem_attrs()
         int bytes = (1 << (kMaxWindowBits - 1)) * 4;
         cudaFuncSetAttribute(msm_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         cudaFuncSetAttribute(msm_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaFuncSetAttribute(msm_fixup_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongSmem);
     });
 }
 
@@ -1309,6 +1266,9 @@ static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int varian
         per_sm[v] = std::max(1, b) * (v == 2 ? 128 : 256);
     }
     const uint64_t wave = (uint64_t)sms * (uint64_t)per_sm[v];  // chunks resident at once
+    // short buckets, large batches: chunks long enough for 8 waves, as every
+    // chunk's edge costs a fix-up
+    if (wave) L = std::max<uint32_t>(L, (uint32_t)std::min<uint64_t>(64, digits / (8 * wave)));
     if (!wave || !digits) return L;
     // whole waves, rounded down (longer chunks: shorter fix-up chains) when
     // there are several, up when there is less than one
@@ -1406,9 +1366,9 @@ jacobian_t msm_tail::finish(const xyzz_t *dev) const
 // The host half of a batch: its descriptors and launch sizes.
 struct batch_plan {
     int c = 0, nwin = 0, variant = 1;
-    bool precomputed = false, by_lines = false;
+    bool precomputed = false, fix_by_chunk = false;
     size_t stride = 0;
-    uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, S = 0;
+    uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, short_span = kShortSpan;
     line_shape shape{0, 0};
     msm_tail tail;
     int rounds = 0;          // affine rounds before the accumulation
@@ -1479,21 +1439,12 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     const int rounds = affine_rounds(digits_total, avg, G);
     const uint64_t entries = digits_total + (uint64_t)G * ((1u << rounds) - 1);
     const uint32_t L = chunk_length(entries >> rounds, avg / (1 << rounds), G, variant);
-    // reduction sub-segments: ~64K threads over the batch, 32..8192 per segment
-    uint32_t S = 32;
-    while (S < 8192 && (uint64_t)S * 2 * nseg <= 65536) S *= 2;
-    S = std::min<uint32_t>(K, S);
-    // Few buckets in all (a single MSM or a small batch): line and bit sums,
-    // a short chain.  Many buckets (large batches): one running sum a thread
-    // keeps the multiply-add pipe busier.
-    const bool by_lines = (uint64_t)nseg * K <= kLinesMaxBuckets;
     const uint64_t nchunks = std::max<uint64_t>(1, ((entries >> rounds) + L - 1) / L);
 
     P.c = c;
     P.nwin = nwin;
     P.variant = variant;
     P.precomputed = precomputed;
-    P.by_lines = by_lines;
     P.stride = stride;
     P.K = K;
     P.segs_per_item = segs_per_item;
@@ -1501,12 +1452,11 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     P.G = G;
     P.nblocks = nblocks;
     P.L = L;
-    P.S = S;
     P.shape.lr = (uint32_t)(c - 1) / 2;
     P.shape.lc = (uint32_t)(c - 1) - P.shape.lr;
     // the steps left to the host: see msm_tail
     P.tail.c = c;
-    if (precomputed && by_lines && nseg <= kHostTailBits) {
+    if (precomputed && nseg <= kHostTailBits) {
         P.tail.kind = msm_tail::BITS;
         P.tail.shape = P.shape;
         P.tail.points = P.shape.bits();
@@ -1517,6 +1467,10 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     P.points_total = points_total;
     P.digits_total = digits_total;
     P.nchunks = nchunks;
+    P.fix_by_chunk = G > kCoopFixupMaxBuckets && avg / (1 << rounds) < L;
+    // a thread adds spans of some 3 times the mean, as a longer chain holds up
+    // the launch (14 us an addition)
+    P.short_span = std::min<uint32_t>(kShortSpan, 6 + (uint32_t)(3.0 * avg / (1 << rounds) / L));
     P.rounds = rounds;
     P.entries = entries;
     P.idesc = std::move(idesc);
@@ -1571,11 +1525,12 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     const bool precomputed = P.precomputed;
     const size_t stride = P.stride;
     const uint32_t nitems = P.nitems, K = P.K, segs_per_item = P.segs_per_item, nseg = P.nseg, G = P.G;
-    const uint32_t nblocks = P.nblocks, L = P.L, S = P.S;
+    const uint32_t nblocks = P.nblocks, L = P.L;
     const uint64_t points_total = P.points_total, digits_total = P.digits_total, nchunks = P.nchunks;
     dev_buf<uint32_t> digits(std::max<uint64_t>(digits_total, 1), s), sorted(std::max<uint64_t>(P.entries, 1), s);
     dev_buf<uint32_t> hist((size_t)nblocks * K, s), counts(G, s), starts((size_t)G + 1, s);
     dev_buf<xyzz_t> buckets(G, s), head(nchunks, s), tail(nchunks, s);
+    dev_buf<uint32_t> open_bucket(P.fix_by_chunk ? nchunks : 0, s);
 
     int tok_all = timed_begin(s);
     int tok_sort = timed_begin(s);
@@ -1594,6 +1549,9 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     GB_CHECK_LAUNCH();
     timed_end(tok_sort, s, GB_SLOT_MSM_SORT);
     int tok = timed_begin(s);
+    // empty buckets: all zero, a point at infinity (ZZ = 0)
+    GB_CUDA_OK(cudaMemsetAsync(buckets.get(), 0, (size_t)G * sizeof(xyzz_t), s));
+    if (P.fix_by_chunk) GB_CUDA_OK(cudaMemsetAsync(open_bucket.get(), 0xff, nchunks * sizeof(uint32_t), s));
     dev_buf<affine_t> list_a, list_b;
     dev_buf<uint32_t> shifted;
     const uint32_t *bounds = starts;
@@ -1604,16 +1562,16 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         GB_CHECK_LAUNCH();
         bounds = shifted;
         msm_accumulate_kernel<256, 2, false><<<(unsigned)((nchunks + 255) / 256), 256, 0, s>>>(
-            nullptr, bounds, G, L, nchunks, list, buckets, head, tail);
+            nullptr, bounds, G, L, nchunks, list, buckets, head, tail, open_bucket);
     } else if (variant == 1) {
         msm_accumulate_kernel<256, 2><<<(unsigned)((nchunks + 255) / 256), 256, 0, s>>>(
-            sorted, starts, G, L, nchunks, points, buckets, head, tail);
+            sorted, starts, G, L, nchunks, points, buckets, head, tail, open_bucket);
     } else if (variant == 2) {
         msm_accumulate_kernel<128, 3><<<(unsigned)((nchunks + 127) / 128), 128, 0, s>>>(
-            sorted, starts, G, L, nchunks, points, buckets, head, tail);
+            sorted, starts, G, L, nchunks, points, buckets, head, tail, open_bucket);
     } else {
         msm_accumulate_kernel<256, 1><<<(unsigned)((nchunks + 255) / 256), 256, 0, s>>>(
-            sorted, starts, G, L, nchunks, points, buckets, head, tail);
+            sorted, starts, G, L, nchunks, points, buckets, head, tail, open_bucket);
     }
     GB_CHECK_LAUNCH();
     timed_end(tok, s, GB_SLOT_MSM_ACCUMULATE);
@@ -1629,12 +1587,15 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         if (G <= kCoopFixupMaxBuckets)
             msm_fixup_coop_kernel<<<(G + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(bounds, G, L, head, tail,
                                                                                      buckets, longs, nlong);
-        else
-            msm_fixup_kernel<<<blocks_for(G, 128), 128, 0, s>>>(bounds, G, L, head, tail, buckets, longs, nlong);
+        else {
+            const uint32_t n = P.fix_by_chunk ? (uint32_t)nchunks : G;
+            msm_fixup_kernel<<<blocks_for(n, 128), 128, 0, s>>>(bounds, open_bucket, n, L, P.short_span, head, tail, buckets, longs,
+                                                                nlong);
+        }
         GB_CHECK_LAUNCH();
         int sms = 0;
         GB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device()));
-        msm_fixup_long_kernel<<<(unsigned)sms * 2, 256, 0, s>>>(bounds, L, head, tail, longs, nlong, buckets);
+        msm_fixup_long_kernel<<<(unsigned)sms * 2, kLongGroups * kCoopLanes, kLongSmem, s>>>(bounds, L, head, tail, longs, nlong, buckets);
         GB_CHECK_LAUNCH();
     }
     timed_end(tok_fix, s, GB_SLOT_MSM_FIXUP);
@@ -1646,7 +1607,7 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         sums = dev_buf<xyzz_t>(nseg, s);
         seg_sum = sums;
     }
-    if (P.by_lines) {
+    {
         const line_shape sh = P.shape;
         const uint64_t total = (uint64_t)nseg * K;
         // 2^lm buckets a thread adds before the lines' blocks take over: none
@@ -1654,8 +1615,9 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         // (one-thread additions take 14 us each but fill all lanes; measured,
         // us for lm = 0, 1, 2, 3, 4: 4096 buckets 67* 83 106 159 269, 2^14
         // 105* 106 124 173 282, 2^15 178 159 151* 193 302, 3 x 2^15 311 289
-        // 265* 264 323, 4 x 2^15 398 371 313 277* 334)
-        const uint32_t lm = total <= (1u << 14) ? 0 : total <= 3u << 15 ? 2 : 3;
+        // 265* 264 323, 4 x 2^15 398 371 313 277* 334; 64 x 2^15 ms 3.23, 2.99*
+        // and 3.10 for 3, 4 and 5, and 3.45 by running sums over sub-segments)
+        const uint32_t lm = total <= (1u << 14) ? 0 : total <= 3u << 15 ? 2 : total <= 1u << 18 ? 3 : 4;
         dev_buf<xyzz_t> partial, lines((size_t)nseg * sh.lines(), s), bits;
         const xyzz_t *src = buckets;
         if (lm) {
@@ -1678,26 +1640,6 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
             msm_bit_combine_kernel<<<(nseg + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(bits, sh, nseg, seg_sum);
             GB_CHECK_LAUNCH();
         }
-    } else {
-        dev_buf<xyzz_t> partial((size_t)nseg * S, s);
-        msm_reduce_partial_kernel<<<blocks_for((size_t)nseg * S, 128), 128, 0, s>>>(buckets, K, S, nseg, partial);
-        GB_CHECK_LAUNCH();
-        // tree-sum each segment's S / group partials down to one point
-        const xyzz_t *src = partial;
-        uint32_t len = S / std::min<uint32_t>(S, 128);
-        dev_buf<xyzz_t> tmp_a, tmp_b;
-        bool use_a = true;
-        while (len > 1) {
-            uint32_t blocks = (len + 511) / 512;
-            dev_buf<xyzz_t> &dst = use_a ? tmp_a : tmp_b;
-            dst = dev_buf<xyzz_t>((size_t)nseg * blocks, s);
-            xyzz_tree_sum_kernel<<<dim3(blocks, nseg), 256, 0, s>>>(src, len, dst);
-            GB_CHECK_LAUNCH();
-            src = dst;
-            len = blocks;
-            use_a = !use_a;
-        }
-        GB_CUDA_OK(cudaMemcpyAsync(seg_sum, src, (size_t)nseg * sizeof(xyzz_t), cudaMemcpyDeviceToDevice, s));
     }
     if (segs_per_item > 1 && P.tail.kind == msm_tail::POINT) {
         msm_combine_coop_kernel<<<(nitems + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(seg_sum, nitems,
@@ -1722,15 +1664,15 @@ struct graph_key {
     cudaStream_t stream = nullptr;
     const affine_t *points = nullptr;
     int c = 0, variant = 0;
-    bool precomputed = false, by_lines = false;
+    bool precomputed = false, fix_by_chunk = false;
     size_t stride = 0;
-    uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, S = 0;
+    uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, short_span = 0;
     int rounds = 0;
     uint64_t points_total = 0, digits_total = 0, nchunks = 0;
     auto tie() const
     {
-        return std::tie(device, stream, points, c, variant, precomputed, by_lines, stride, nitems, K, segs_per_item,
-                        nseg, G, nblocks, L, S, rounds, points_total, digits_total, nchunks);
+        return std::tie(device, stream, points, c, variant, precomputed, fix_by_chunk, stride, nitems, K, segs_per_item,
+                        nseg, G, nblocks, L, short_span, rounds, points_total, digits_total, nchunks);
     }
     bool operator<(const graph_key &o) const { return tie() < o.tie(); }
 };
@@ -1790,9 +1732,9 @@ static bool run_planned_graph(const batch_plan &P, const affine_t *points, xyzz_
     key.device = current_device();
     key.stream = s;
     key.points = points;
-    key.c = P.c, key.variant = P.variant, key.precomputed = P.precomputed, key.by_lines = P.by_lines;
+    key.c = P.c, key.variant = P.variant, key.precomputed = P.precomputed, key.fix_by_chunk = P.fix_by_chunk;
     key.stride = P.stride, key.nitems = P.nitems, key.K = P.K, key.segs_per_item = P.segs_per_item;
-    key.nseg = P.nseg, key.G = P.G, key.nblocks = P.nblocks, key.L = P.L, key.S = P.S;
+    key.nseg = P.nseg, key.G = P.G, key.nblocks = P.nblocks, key.L = P.L, key.short_span = P.short_span;
     key.points_total = P.points_total, key.digits_total = P.digits_total, key.nchunks = P.nchunks, key.rounds = P.rounds;
 
     // a stream the caller is capturing gets the launches themselves
