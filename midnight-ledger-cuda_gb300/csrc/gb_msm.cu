@@ -38,7 +38,7 @@
 #include <initializer_list>
 #include <vector>
 
-#include "gb_fp_inv.cuh"
+#include "gb_inv_warp.cuh"
 #include "gb_host_fp.h"
 #include "gb_runtime.cuh"
 
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairBlocks)
                 if (tid < n) node[n + tid] = inv;
                 __syncwarp();
             }
-            inv = fp_inverse_warp(node + 1);
+            inv = inverse_warp<FpCfg>(node + 1);
             __syncwarp();
             if (tid == 0) node[1] = inv;
             __syncwarp();

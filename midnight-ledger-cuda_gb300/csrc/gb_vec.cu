@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "gb_inv_warp.cuh"
 #include "gb_ntt.cuh"
 #include "gb_vec.cuh"
 
@@ -195,54 +196,91 @@ void suffix_sum(fr_t *out, const fr_t *in, size_t n, cudaStream_t s)
 
 // ------------------------------------------------------------ batch inversion
 
-// Montgomery's trick per tile: one binary-GCD inversion per tile of 2048
-// elements; zeros stay zero (the field inverse the reference applies maps
-// 0 to 0).  out may alias in.  If `mul` is given, out[i] = mul[i] / in[i].
-__global__ void __launch_bounds__(kScanThreads) batch_invert_kernel(const fr_t *in, size_t n,
-                                                                    const fr_t *mul,
+// 1 / p for the nonzero p of each of the block's 256 threads: a product tree
+// in shared memory (root 1, leaves 256 ..), the root inverted by one warp, the
+// inverses coming down (a child's is its parent's times its sibling).
+__device__ fr_t block_inverses(fr_t p, fr_t *node)
+{
+    const unsigned t = threadIdx.x;
+    node[kScanThreads + t] = p;
+    __syncthreads();
+    for (unsigned n = kScanThreads / 2; n >= 32; n >>= 1) {
+        if (t < n) node[n + t] = node[2 * (n + t)] * node[2 * (n + t) + 1];
+        __syncthreads();
+    }
+    if (t < 32) {
+        fr_t v;
+        for (unsigned n = 16; n > 0; n >>= 1) {
+            if (t < n) v = node[2 * (n + t)] * node[2 * (n + t) + 1];
+            if (t < n) node[n + t] = v;
+            __syncwarp();
+        }
+        v = inverse_warp<FrCfg>(node + 1);
+        __syncwarp();
+        if (t == 0) node[1] = v;
+        __syncwarp();
+        for (unsigned n = 2; n <= 32; n <<= 1) {
+            if (t < n) v = node[(n + t) >> 1] * node[(n + t) ^ 1];
+            __syncwarp();
+            if (t < n) node[n + t] = v;
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    for (unsigned n = 64; n < kScanThreads; n <<= 1) {
+        fr_t v;
+        if (t < n) v = node[(n + t) >> 1] * node[(n + t) ^ 1];
+        __syncthreads();
+        if (t < n) node[n + t] = v;
+        __syncthreads();
+    }
+    return node[(kScanThreads + t) >> 1] * node[(kScanThreads + t) ^ 1];
+}
+
+// Montgomery's trick per tile of 256 x PER elements, one inversion a tile;
+// zeros stay zero (the field inverse the reference applies maps 0 to 0).  out
+// may alias in.  If `mul` is given, out[i] = mul[i] / in[i].
+template <int PER>
+__global__ void __launch_bounds__(kScanThreads) batch_invert_kernel(const fr_t *in, size_t n, const fr_t *mul,
                                                                     fr_t *out)
 {
-    __shared__ fr_t sh[kScanThreads];
-    __shared__ fr_t total_inv;
-    size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanPer;
-    fr_t x[kScanPer], q[kScanPer];
+    __shared__ fr_t node[2 * kScanThreads];
+    const size_t base = (size_t)blockIdx.x * (kScanThreads * PER) + threadIdx.x;
+    fr_t x[PER], q[PER];
     fr_t p = fr_t::one();
 #pragma unroll
-    for (int e = 0; e < kScanPer; e++) {
-        fr_t v = base + e < n ? in[base + e] : fr_t::zero();
-        x[e] = v;
+    for (int e = 0; e < PER; e++) {
+        const size_t i = base + (size_t)e * kScanThreads;
+        x[e] = i < n ? in[i] : fr_t::zero();
         q[e] = p;  // product of this thread's earlier nonzero elements
-        if (!v.is_zero()) p = p * v;
+        if (!x[e].is_zero()) p = p * x[e];
     }
-    fr_t incl = block_scan_mul(p, sh);
-    __syncthreads();
-    fr_t excl = threadIdx.x ? sh[threadIdx.x - 1] : fr_t::one();
-    if (threadIdx.x == blockDim.x - 1) total_inv = incl.inverse_binary();
-    __syncthreads();
-    fr_t suffix_incl = block_suffix_scan_mul(p, sh);
-    __syncthreads();
-    fr_t suffix_excl = threadIdx.x + 1 < blockDim.x ? sh[threadIdx.x + 1] : fr_t::one();
-    (void)suffix_incl;
-    // 1/p = total^-1 * (product of every other thread's p)
-    fr_t J = total_inv * excl * suffix_excl;
+    fr_t J = block_inverses(p, node);
 #pragma unroll
-    for (int e = kScanPer - 1; e >= 0; e--) {
-        if (base + e >= n) continue;
-        if (x[e].is_zero()) {
-            out[base + e] = fr_t::zero();
-            continue;
+    for (int e = PER - 1; e >= 0; e--) {
+        const size_t i = base + (size_t)e * kScanThreads;
+        if (i >= n) continue;
+        fr_t r = fr_t::zero();
+        if (!x[e].is_zero()) {
+            r = J * q[e];
+            J = J * x[e];
+            if (mul) r = mul[i] * r;
         }
-        fr_t inv = J * q[e];
-        J = J * x[e];
-        out[base + e] = mul ? mul[base + e] * inv : inv;
+        out[i] = r;
     }
 }
+
+// Elements a thread: 4 until the tiles fill the GPU (a tile is one chain: its
+// inversion, about 12 us, and 16 tree levels), then 8
+static int tile_per(size_t n) { return n <= (size_t)1 << 18 ? 4 : 8; }
 
 void batch_invert(fr_t *out, const fr_t *in, size_t n, const fr_t *mul, cudaStream_t s)
 {
     if (!n) return;
-    size_t tiles = (n + kScanTile - 1) / kScanTile;
-    batch_invert_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, mul, out);
+    const int per = tile_per(n);
+    const size_t tiles = (n + kScanThreads * per - 1) / (kScanThreads * per);
+    if (per == 4) batch_invert_kernel<4><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, mul, out);
+    else batch_invert_kernel<8><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, mul, out);
     GB_CHECK_LAUNCH();
 }
 
@@ -348,106 +386,213 @@ __global__ void shifted_apply_kernel(fr_t *__restrict__ out, const fr_t *__restr
     out[i] = i ? a * prefix[i - 1] : a;
 }
 
-__global__ void blind_tail_kernel(fr_t *__restrict__ values, const fr_t *__restrict__ blinds, size_t len, size_t bf)
-{
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < bf) values[len - bf + i] = blinds[i];
-}
+// A grand product z is two launches: the fractions num / den of every row with
+// their tiles' products, then each tile's share of z, which multiplies the
+// tiles before it itself.  Neither numerators nor denominators touch memory.
+// Both are a few chains on few warps, bound by the latency of a product (0.45
+// us) and of the tile's inversion (12 us, by a warp; 100 us by one thread).
+// Measured, the permutation products of 3 columns of 2^16 rows 0.297 -> 0.100
+// ms, of 2^10 0.22 -> 0.073 ms.
 
-__global__ void copy_one_kernel(fr_t *dst, const fr_t *src) { *dst = *src; }
+static __device__ __noinline__ fr_t fr_mul_called(fr_t a, fr_t b) { return a * b; }
 
-__global__ void set_scalar_kernel(fr_t *dst, fr_t v) { *dst = v; }
-
-// Permutation fraction numerator / denominator per row (prover.rs:392-460):
+// Permutation fraction of row i, set `set` (prover.rs:392-460):
 // num = prod_j (v_j + delta^j w^i beta + gamma), den = prod_j (v_j + beta s_j + gamma).
 // Column c is columns[c * len ..] or, with a pointer table, col_ptrs[c][..].
-__global__ void perm_num_den_kernel(const fr_t *__restrict__ columns, const fr_t *const *__restrict__ col_ptrs,
-                                    const fr_t *__restrict__ perms, const fr_t *__restrict__ delta_powers,
-                                    fr_t omega, fr_t beta, fr_t gamma, size_t len, size_t c0, size_t ncols,
-                                    fr_t *__restrict__ num, fr_t *__restrict__ den)
-{
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= len) return;
-    fr_t wi = omega.pow_u64(i);
-    fr_t bw = beta * wi;
-    fr_t nn = fr_t::one(), dd = fr_t::one();
-    for (size_t j = 0; j < ncols; j++) {
-        size_t c = c0 + j;
-        fr_t v = col_ptrs ? col_ptrs[c][i] : columns[c * len + i];
-        nn = nn * (v + delta_powers[c] * bw + gamma);
-        dd = dd * (v + beta * perms[c * len + i] + gamma);
+struct perm_fraction {
+    const fr_t *columns;
+    const fr_t *const *col_ptrs;
+    const fr_t *perms, *delta_powers;
+    fr_t beta, gamma;
+    size_t len, column_count, chunk_len;
+    fr_t w2[32];  // omega^(2^b)
+    typedef fr_t state;  // beta w^i
+    __device__ state begin(size_t i) const
+    {
+        fr_t v = beta;
+        for (int b = 0; b < 32 && (i >> b); b++)
+            if ((i >> b) & 1) v = fr_mul_called(v, w2[b]);
+        if (i >> 32) v = fr_mul_called(v, fr_mul_called(w2[31], w2[31]).pow_u64(i >> 32));
+        return v;
     }
-    num[i] = nn;
-    den[i] = dd;
-}
+    // kScanThreads = 2^8 rows on
+    __device__ void next(state &v) const { v = fr_mul_called(v, w2[8]); }
+    __device__ void at(size_t set, size_t i, const state &bw, fr_t &num, fr_t &den) const
+    {
+        const size_t c0 = set * chunk_len, c1 = min(c0 + chunk_len, column_count);
+        num = fr_t::one(), den = fr_t::one();
+        for (size_t c = c0; c < c1; c++) {
+            const fr_t v = (col_ptrs ? col_ptrs[c][i] : columns[c * len + i]) + gamma;
+            num = fr_mul_called(num, v + fr_mul_called(delta_powers[c], bw));
+            den = fr_mul_called(den, v + fr_mul_called(beta, perms[c * len + i]));
+        }
+    }
+};
 
-// Lookup fraction numerator / denominator (lookup/prover.rs:1075-1240):
+// Lookup fraction (lookup/prover.rs:1075-1240):
 // num = (A + beta)(S + gamma), den = (A' + beta)(S' + gamma)
-__global__ void lookup_num_den_kernel(const fr_t *__restrict__ ci, const fr_t *__restrict__ ct,
-                                      const fr_t *__restrict__ pi, const fr_t *__restrict__ pt, fr_t beta,
-                                      fr_t gamma, size_t total, fr_t *__restrict__ num, fr_t *__restrict__ den)
+struct lookup_fraction {
+    const fr_t *ci, *ct, *pi, *pt;
+    fr_t beta, gamma;
+    size_t len;
+    typedef int state;
+    __device__ state begin(size_t) const { return 0; }
+    __device__ void next(state &) const {}
+    __device__ void at(size_t set, size_t i, const state &, fr_t &num, fr_t &den) const
+    {
+        const size_t f = set * len + i;
+        num = fr_mul_called(ci[f] + beta, ct[f] + gamma);
+        den = fr_mul_called(pi[f] + beta, pt[f] + gamma);
+    }
+};
+
+// frac[set][i] = num / den (0 where den is 0) and tile_products[set][tile]
+template <class F, int PER>
+__global__ void __launch_bounds__(kScanThreads) fraction_kernel(const __grid_constant__ F f, size_t len, size_t set0,
+                                                                fr_t *__restrict__ frac,
+                                                                fr_t *__restrict__ tile_products)
 {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    num[i] = (ci[i] + beta) * (ct[i] + gamma);
-    den[i] = (pi[i] + beta) * (pt[i] + gamma);
+    __shared__ fr_t node[2 * kScanThreads];
+    const size_t base = (size_t)blockIdx.x * kScanThreads * PER + threadIdx.x, set = set0 + blockIdx.y;
+    fr_t num[PER], den[PER], q[PER];
+    fr_t p = fr_t::one();
+    typename F::state st = f.begin(base);
+#pragma unroll
+    for (int e = 0; e < PER; e++) {
+        const size_t i = base + (size_t)e * kScanThreads;
+        num[e] = fr_t::one(), den[e] = fr_t::one();
+        if (i < len) f.at(set, i, st, num[e], den[e]);
+        if (e + 1 < PER) f.next(st);
+        q[e] = p;
+        if (!den[e].is_zero()) p = fr_mul_called(p, den[e]);
+    }
+    fr_t J = block_inverses(p, node), prod = fr_t::one();
+#pragma unroll
+    for (int e = PER - 1; e >= 0; e--) {
+        const size_t i = base + (size_t)e * kScanThreads;
+        fr_t r = fr_t::zero();
+        if (!den[e].is_zero()) {
+            r = fr_mul_called(num[e], fr_mul_called(J, q[e]));
+            J = fr_mul_called(J, den[e]);
+        }
+        if (i < len) frac[set * len + i] = r;
+        prod = fr_mul_called(prod, r);  // one past the end
+    }
+    __syncthreads();
+    node[threadIdx.x] = prod;
+    __syncthreads();
+    for (unsigned off = kScanThreads / 2; off > 0; off >>= 1) {
+        if (threadIdx.x < off) node[threadIdx.x] = node[threadIdx.x] * node[threadIdx.x + off];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) tile_products[set * gridDim.x + blockIdx.x] = node[0];
 }
 
-// grand product of fractions with chained initial value; `out` gets z
-static void grand_product(fr_t *out, fr_t *num, fr_t *den, size_t len, const fr_t *d_init, fr_t *scratch,
-                          cudaStream_t s)
+// z[i] = init * (product of the fractions before i) for i < len - bf, the
+// blinds after; `tiles` are the tiles' products, or with `scanned` their
+// inclusive prefix products
+template <int PER>
+__global__ void __launch_bounds__(kScanThreads) grand_product_kernel(const fr_t *__restrict__ frac,
+                                                                     const fr_t *__restrict__ tiles, bool scanned,
+                                                                     size_t len, size_t set0, const fr_t *init,
+                                                                     const fr_t *__restrict__ blinds, size_t bf,
+                                                                     fr_t *z)
 {
-    // fraction = num / den (batch inversion), prefix product, shift by init
-    batch_invert(num, den, len, num, s);
-    prefix_product(scratch, num, len, s);
-    shifted_apply_kernel<<<blocks_for(len, 256), 256, 0, s>>>(out, scratch, d_init, len);
-    GB_CHECK_LAUNCH();
+    __shared__ fr_t sh[kScanThreads];
+    const size_t set = set0 + blockIdx.y, b = blockIdx.x;
+    frac += set * len;
+    tiles += set * gridDim.x;
+    z += set * len;
+    fr_t carry = init ? *init : fr_t::one();
+    if (scanned) {
+        if (b) carry = carry * tiles[b - 1];
+    } else if (b) {
+        fr_t p = fr_t::one();
+        for (size_t t = threadIdx.x; t < b; t += kScanThreads) p = p * tiles[t];
+        sh[threadIdx.x] = p;
+        __syncthreads();
+        for (unsigned off = kScanThreads / 2; off > 0; off >>= 1) {
+            if (threadIdx.x < off && threadIdx.x + off < b) sh[threadIdx.x] = sh[threadIdx.x] * sh[threadIdx.x + off];
+            __syncthreads();
+        }
+        carry = carry * sh[0];
+        __syncthreads();
+    }
+    const size_t base = (b * kScanThreads + threadIdx.x) * PER;
+    fr_t v[PER], p = fr_t::one();
+#pragma unroll
+    for (int e = 0; e < PER; e++) {
+        v[e] = base + e < len ? frac[base + e] : fr_t::one();
+        p = p * v[e];
+    }
+    block_scan_mul(p, sh);
+    __syncthreads();
+    fr_t run = threadIdx.x ? carry * sh[threadIdx.x - 1] : carry;
+#pragma unroll
+    for (int e = 0; e < PER; e++) {
+        const size_t i = base + e;
+        if (i < len) z[i] = i < len - bf ? run : blinds[set * bf + i - (len - bf)];
+        run = run * v[e];
+    }
+}
+
+// z of `sets` products into out [sets][len]; chained: a set starts from the
+// last unblinded value of the one before
+template <int PER, class F>
+static void grand_products_tiled(fr_t *out, const F &f, size_t len, size_t sets, bool chained, const fr_t *d_blinds,
+                           size_t bf, cudaStream_t s)
+{
+    const size_t tile = (size_t)kScanThreads * PER, tiles = (len + tile - 1) / tile;
+    if (tiles > 0x7fffffff) throw cuda_error((int)cudaErrorInvalidValue, "grand product too large");
+    dev_buf<fr_t> frac(len * sets, s), products(tiles * sets, s);
+    constexpr size_t kMaxY = 65535;
+    for (size_t k = 0; k < sets; k += kMaxY) {
+        const dim3 grid((unsigned)tiles, (unsigned)std::min(kMaxY, sets - k));
+        fraction_kernel<F, PER><<<grid, kScanThreads, 0, s>>>(f, len, k, frac, products);
+        GB_CHECK_LAUNCH();
+    }
+    // beyond 2^20 rows a tile's own walk over the tiles before it costs more
+    // than a scan of their products
+    const bool scanned = tiles > 1024;
+    if (scanned)
+        for (size_t k = 0; k < sets; k++) prefix_product(products + k * tiles, products + k * tiles, tiles, s);
+    for (size_t k = 0; k < sets; k += chained ? 1 : kMaxY) {
+        const dim3 grid((unsigned)tiles, chained ? 1u : (unsigned)std::min(kMaxY, sets - k));
+        const fr_t *init = chained && k ? out + (k - 1) * len + (len - (bf + 1)) : nullptr;
+        grand_product_kernel<PER><<<grid, kScanThreads, 0, s>>>(frac, products, scanned, len, k, init, d_blinds, bf, out);
+        GB_CHECK_LAUNCH();
+    }
+}
+
+template <class F>
+static void grand_products(fr_t *out, const F &f, size_t len, size_t sets, bool chained, const fr_t *d_blinds,
+                           size_t bf, cudaStream_t s)
+{
+    if (!len || !sets) return;
+    // rows a thread: a tile is one chain, so short products take short tiles.
+    // Measured, us a call with 1, 2 and 4: 2^12 rows 78* 94 129, 2^15 82* 98
+    // 137, 2^16 113 99* 137, 2^17 202 144 137*, 2^18 355 264 251*.
+    if (len <= (size_t)1 << 15) grand_products_tiled<1>(out, f, len, sets, chained, d_blinds, bf, s);
+    else if (len <= (size_t)1 << 16) grand_products_tiled<2>(out, f, len, sets, chained, d_blinds, bf, s);
+    else grand_products_tiled<4>(out, f, len, sets, chained, d_blinds, bf, s);
 }
 
 void permutation_products(fr_t *out, const fr_t *d_columns, const fr_t *const *d_col_ptrs, const fr_t *d_perms,
                           size_t len, size_t column_count, size_t chunk_len, const fr_t &beta, const fr_t &gamma,
                           const fr_t &omega, const fr_t *d_delta, const fr_t *d_blinds, size_t bf, cudaStream_t s)
 {
-    const size_t sets = (column_count + chunk_len - 1) / chunk_len;
-    dev_buf<fr_t> num(len, s), den(len, s), scratch(len, s), init(1, s);
-    set_scalar_kernel<<<1, 1, 0, s>>>(init, fr_t::one());
-    GB_CHECK_LAUNCH();
-    for (size_t set = 0; set < sets; set++) {
-        size_t c0 = set * chunk_len;
-        size_t nc = std::min(chunk_len, column_count - c0);
-        fr_t *z = out + set * len;
-        perm_num_den_kernel<<<blocks_for(len, 256), 256, 0, s>>>(d_columns, d_col_ptrs, d_perms, d_delta, omega, beta,
-                                                                 gamma, len, c0, nc, num, den);
-        GB_CHECK_LAUNCH();
-        grand_product(z, num, den, len, init, scratch, s);
-        // next set starts from this set's last unblinded value
-        copy_one_kernel<<<1, 1, 0, s>>>(init, z + (len - (bf + 1)));
-        GB_CHECK_LAUNCH();
-        if (bf) {
-            blind_tail_kernel<<<blocks_for(bf, 256), 256, 0, s>>>(z, d_blinds + set * bf, len, bf);
-            GB_CHECK_LAUNCH();
-        }
-    }
+    perm_fraction f{d_columns, d_col_ptrs, d_perms, d_delta, beta, gamma, len, column_count, chunk_len, {}};
+    f.w2[0] = omega;
+    for (int b = 1; b < 32; b++) f.w2[b] = b <= 8 || (len >> b) ? f.w2[b - 1].sqr() : fr_t::one();
+    grand_products(out, f, len, (column_count + chunk_len - 1) / chunk_len, true, d_blinds, bf, s);
 }
 
 void lookup_products(fr_t *out, const fr_t *ci, const fr_t *ct, const fr_t *pi, const fr_t *pt, size_t len,
                      size_t lookup_count, const fr_t &beta, const fr_t &gamma, const fr_t *d_blinds, size_t bf,
                      cudaStream_t s)
 {
-    size_t total = len * lookup_count;
-    dev_buf<fr_t> num(total, s), den(total, s), scratch(len, s), init(1, s);
-    set_scalar_kernel<<<1, 1, 0, s>>>(init, fr_t::one());
-    GB_CHECK_LAUNCH();
-    lookup_num_den_kernel<<<blocks_for(total, 256), 256, 0, s>>>(ci, ct, pi, pt, beta, gamma, total, num, den);
-    GB_CHECK_LAUNCH();
-    for (size_t l = 0; l < lookup_count; l++) {
-        fr_t *z = out + l * len;
-        grand_product(z, num.get() + l * len, den.get() + l * len, len, init, scratch, s);
-        if (bf) {
-            blind_tail_kernel<<<blocks_for(bf, 256), 256, 0, s>>>(z, d_blinds + l * bf, len, bf);
-            GB_CHECK_LAUNCH();
-        }
-    }
+    const lookup_fraction f{ci, ct, pi, pt, beta, gamma, len};
+    grand_products(out, f, len, lookup_count, false, d_blinds, bf, s);
 }
 
 // ------------------------------------------------------------ misc kernels
