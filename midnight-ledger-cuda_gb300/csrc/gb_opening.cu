@@ -4,10 +4,12 @@
 // (f(X) - f(z)) / (X - z) of every polynomial of a batch (the division the
 // reference's multi-open computes with its kate scan, .cu:1923-1959).
 //
-// Evaluation: z^i is tabulated by a multiplicative scan, each block sums a
-// slice of c_i z^i, a second pass adds the slices.  Kate quotient: with
-// S_k = sum_{j >= k} f_j z^j (an additive suffix scan), q_i = S_{i+1} z^-(i+1)
-// for i < n-1 and q_{n-1} = 0; z = 0 is the shift q_i = f_{i+1}.
+// Evaluation and division are Horner's rule in blocks: every thread runs it
+// over a few coefficients, and the threads' values meet in log steps with the
+// powers z^(2^s), which are squarings.  No power of z is tabulated and 1 / z
+// is not needed.  With tables and a suffix sum, a quotient of 2^12 coefficients
+// was ten launches of 80 us together; now it is two.  A proof of 2^12 rows
+// takes 3.32 ms instead of 3.94 with that, one of 2^16 rows 9.96.
 #include <algorithm>
 #include <vector>
 
@@ -16,159 +18,271 @@
 namespace gb {
 
 static constexpr int kEvalThreads = 256;
-static constexpr size_t kEvalSlice = 8192;
 
-__global__ void __launch_bounds__(kEvalThreads) eval_slices_kernel(const fr_t *__restrict__ polys, size_t len,
-                                                                   const fr_t *__restrict__ pw, uint32_t slices,
-                                                                   fr_t *__restrict__ partial)
-{
-    __shared__ fr_t sh[kEvalThreads];
-    const size_t p = blockIdx.y, sl = blockIdx.x;
-    const fr_t *c = polys + p * len;
-    size_t lo = sl * kEvalSlice, hi = min(lo + kEvalSlice, len);
-    fr_t acc = fr_t::zero();
-    for (size_t i = lo + threadIdx.x; i < hi; i += blockDim.x) acc = acc + c[i] * pw[i];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (unsigned off = blockDim.x / 2; off; off >>= 1) {
-        if (threadIdx.x < off) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + off];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) partial[p * slices + sl] = sh[0];
-}
-
-__global__ void sum_slices_kernel(const fr_t *__restrict__ partial, uint32_t slices, size_t count,
-                                  fr_t *__restrict__ out)
-{
-    size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= count) return;
-    fr_t acc = fr_t::zero();
-    for (uint32_t s = 0; s < slices; s++) acc = acc + partial[p * slices + s];
-    out[p] = acc;
-}
-
-void eval_polys(fr_t *d_out, const fr_t *polys, size_t len, size_t count, const fr_t &z, cudaStream_t s)
-{
-    dev_buf<fr_t> pw(len, s);
-    omega_powers(pw, z, len, s);
-    uint32_t slices = (uint32_t)((len + kEvalSlice - 1) / kEvalSlice);
-    dev_buf<fr_t> partial(count * slices, s);
-    eval_slices_kernel<<<dim3(slices, (unsigned)count), kEvalThreads, 0, s>>>(polys, len, pw, slices, partial);
-    GB_CHECK_LAUNCH();
-    sum_slices_kernel<<<blocks_for(count, 128), 128, 0, s>>>(partial, slices, count, d_out);
-    GB_CHECK_LAUNCH();
-}
-
-// evaluations of a batch of (polynomial, point) pairs: pair p reads the
-// coefficients at polys[p] and the power row pw + row[p] * len
+// an evaluation: len coefficients at polys, at points[row]
 struct eval_pair {
     const fr_t *polys;
     uint32_t row;
 };
 
-__global__ void __launch_bounds__(kEvalThreads) eval_slices_many_kernel(const eval_pair *__restrict__ pairs, size_t len,
-                                                                        const fr_t *__restrict__ pw, uint32_t slices,
-                                                                        fr_t *__restrict__ partial)
+// One slice of 256 * per coefficients of one polynomial a block: out[p *
+// slices + slice] = its value at y = points[row]^(2^squarings).  Thread t runs
+// Horner's rule in y^256 over the coefficients t, t + 256, .. of the slice,
+// then the threads are folded by y^128, y^64, .. y.  A chain of 16 + per
+// dependent products and what they wait for bounds it at per = 16.
+__global__ void __launch_bounds__(kEvalThreads) eval_slices_kernel(const eval_pair *__restrict__ pairs, size_t len,
+                                                                   const fr_t *__restrict__ points, int squarings,
+                                                                   int per, uint32_t slices, fr_t *__restrict__ out)
 {
     __shared__ fr_t sh[kEvalThreads];
-    const size_t p = blockIdx.y, sl = blockIdx.x;
+    const size_t p = blockIdx.y, lo = (size_t)blockIdx.x * per * kEvalThreads, t = threadIdx.x;
     const eval_pair e = pairs[p];
-    const fr_t *c = e.polys;
-    const fr_t *z = pw + (size_t)e.row * len;
-    size_t lo = sl * kEvalSlice, hi = min(lo + kEvalSlice, len);
-    fr_t acc = fr_t::zero();
-    for (size_t i = lo + threadIdx.x; i < hi; i += blockDim.x) acc = acc + c[i] * z[i];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (unsigned off = blockDim.x / 2; off; off >>= 1) {
-        if (threadIdx.x < off) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + off];
-        __syncthreads();
+    fr_t y = points[e.row];
+    for (int k = 0; k < squarings; k++) y = y.sqr();
+    fr_t pw[8];  // y^(2^s)
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        pw[k] = y;
+        y = y.sqr();
     }
-    if (threadIdx.x == 0) partial[p * slices + sl] = sh[0];
+    fr_t acc = fr_t::zero();
+    for (int k = per - 1; k >= 0; k--) {
+        const size_t i = lo + (size_t)k * kEvalThreads;
+        if (i >= len) continue;  // the whole block
+        acc = acc * y;
+        if (i + t < len) acc = acc + e.polys[i + t];
+    }
+    sh[t] = acc;
+#pragma unroll
+    for (int k = 7; k >= 0; k--) {
+        __syncthreads();
+        if (t < (1u << k)) sh[t] = sh[t] + sh[t + (1u << k)] * pw[k];
+    }
+    if (t == 0) out[p * slices + blockIdx.x] = sh[0];
 }
 
-// evaluations of pairs (pair p: coefficients at pairs[p].polys of len
-// values, at the host point points[pairs[p].row]) into d_out; the powers of
-// every point tabulated once
+// evaluations of pairs (pair p: len coefficients at pairs[p].polys, at the host
+// point points[pairs[p].row]) into d_out; the slices' values are the
+// coefficients of a polynomial in point^slice, evaluated the same way
 static void eval_pairs(fr_t *d_out, const std::vector<eval_pair> &pairs, const RawFr *points, size_t npoints,
                        size_t len, cudaStream_t s)
 {
-    const size_t total = pairs.size();
+    const size_t total = pairs.size(), chunk = 65535;  // grid.y limit
     if (!total) return;
-    dev_buf<fr_t> d_points(npoints, s), pw(npoints * len, s);
-    dev_buf<eval_pair> d_pairs(total, s);
+    if (npoints > 65535 && len <= ((size_t)1 << 24))
+        throw cuda_error((int)cudaErrorInvalidValue, "too many evaluation points");
+    dev_buf<fr_t> d_points(npoints, s);
     h2d(d_points, points, npoints * sizeof(fr_t), s);
-    h2d(d_pairs, pairs.data(), total * sizeof(eval_pair), s);
-    if (len <= ((size_t)1 << 24)) {
-        omega_powers_many(pw, d_points, npoints, len, s);
-    } else {
-        for (size_t q = 0; q < npoints; q++) omega_powers(pw.get() + q * len, from_raw(points[q]), len, s);
+    std::vector<eval_pair> now = pairs;
+    dev_buf<fr_t> values;
+    // 64 coefficients a thread where that leaves two waves of blocks, which
+    // spares the products of the squarings and folds; else 16, to be short
+    const int log_per = total * (len >> 14) >= 608 ? 6 : 4;
+    for (int squarings = 0;; squarings += 8 + log_per) {
+        const size_t slice = (size_t)kEvalThreads << log_per;
+        const uint32_t slices = (uint32_t)((len + slice - 1) / slice);
+        dev_buf<eval_pair> d_pairs(total, s);
+        h2d(d_pairs, now.data(), total * sizeof(eval_pair), s);
+        dev_buf<fr_t> next(slices > 1 ? total * slices : 0, s);
+        fr_t *out = slices > 1 ? next.get() : d_out;
+        for (size_t b = 0; b < total; b += chunk) {
+            eval_slices_kernel<<<dim3(slices, (unsigned)std::min(chunk, total - b)), kEvalThreads, 0, s>>>(
+                d_pairs.get() + b, len, d_points, squarings, 1 << log_per, slices, out + b * slices);
+            GB_CHECK_LAUNCH();
+        }
+        if (slices == 1) return;
+        for (size_t p = 0; p < total; p++) now[p].polys = out + p * slices;
+        len = slices;
+        values = std::move(next);
     }
-    const uint32_t slices = (uint32_t)((len + kEvalSlice - 1) / kEvalSlice);
-    const size_t chunk = 65535;  // grid.y limit
-    dev_buf<fr_t> partial(std::min(total, chunk) * slices, s);
-    for (size_t b = 0; b < total; b += chunk) {
-        const size_t m = std::min(chunk, total - b);
-        eval_slices_many_kernel<<<dim3(slices, (unsigned)m), kEvalThreads, 0, s>>>(d_pairs.get() + b, len, pw, slices,
-                                                                                   partial);
+}
+
+static void eval_polys(fr_t *d_out, const fr_t *polys, size_t len, size_t count, const RawFr &z, cudaStream_t s)
+{
+    std::vector<eval_pair> pairs(count);
+    for (size_t p = 0; p < count; p++) pairs[p] = eval_pair{polys + p * len, 0};
+    eval_pairs(d_out, pairs, &z, 1, len, s);
+}
+
+// Kate quotient.  With the coefficients taken from the top, a_t =
+// f_(len-1-t), Horner's values H_t = a_t + z H_(t-1) are the quotient:
+// q_(len-2-t) = H_t, and q_(len-1) = 0.  A tile is 256 threads of PER
+// coefficients; a first launch leaves every tile's last H, as if the tile were
+// the first one, a second launch adds what the tiles before bring and writes q.
+// grid.y divisions in a launch, each with its own polynomial and point.
+struct kate_item {
+    const fr_t *f;
+    fr_t *q;
+    const fr_t *z;  // z^(2^s) for s < kKatePowers
+};
+static constexpr int kKatePowers = 48;
+static constexpr int kKateLog = 8;  // log2 of the threads
+static constexpr int kKateThreads = 1 << kKateLog;
+
+// Horner's rule over a thread's coefficients from v on
+template <int LOG_PER>
+__device__ __forceinline__ fr_t kate_thread(const fr_t *f, size_t len, size_t base, const fr_t &z, fr_t v)
+{
+#pragma unroll
+    for (int e = 0; e < 1 << LOG_PER; e++) {
+        v = v * z;
+        if (base + e < len) v = v + f[len - 1 - (base + e)];
+    }
+    return v;
+}
+
+template <int LOG_PER>
+__global__ void __launch_bounds__(kKateThreads) kate_tile_kernel(const kate_item *__restrict__ items, size_t len,
+                                                                 fr_t *__restrict__ totals)
+{
+    __shared__ fr_t sh[kKateThreads];
+    const unsigned t = threadIdx.x;
+    const kate_item it = items[blockIdx.y];
+    const size_t base = ((size_t)blockIdx.x * kKateThreads + t) << LOG_PER;
+    sh[t] = kate_thread<LOG_PER>(it.f, len, base, it.z[0], fr_t::zero());
+    for (int k = 0; k < kKateLog; k++) {
+        const unsigned off = 1u << k;
+        __syncthreads();
+        if ((t & (2 * off - 1)) == 2 * off - 1) sh[t] = sh[t] + sh[t - off] * it.z[LOG_PER + k];
+    }
+    if (t == kKateThreads - 1) totals[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = sh[t];
+}
+
+// inclusive scan of the recurrence over a block: thread t's value is left as
+// sum_u z^(2^log_step u) sh[t - u]
+__device__ __forceinline__ void kate_block_scan(fr_t *sh, const fr_t *z, int log_step)
+{
+    const unsigned t = threadIdx.x;
+    for (int k = 0; k < kKateLog; k++) {
+        const unsigned off = 1u << k;
+        __syncthreads();
+        const fr_t other = t >= off ? sh[t - off] * z[log_step + k] : fr_t::zero();
+        __syncthreads();
+        if (t >= off) sh[t] = sh[t] + other;
+    }
+    __syncthreads();
+}
+
+// what the tiles before each one bring to it, in place of the totals; one
+// block a division, 2^log_m tiles a thread
+__global__ void __launch_bounds__(kKateThreads) kate_carry_kernel(const kate_item *__restrict__ items,
+                                                                  fr_t *__restrict__ totals, size_t tiles,
+                                                                  int log_tile, int log_m)
+{
+    __shared__ fr_t sh[kKateThreads];
+    fr_t *T = totals + (size_t)blockIdx.x * tiles;
+    const fr_t *z = items[blockIdx.x].z;
+    const unsigned t = threadIdx.x;
+    const size_t lo = (size_t)t << log_m, end = lo + ((size_t)1 << log_m);
+    fr_t v = fr_t::zero();
+    for (size_t b = lo; b < end; b++) {
+        v = v * z[log_tile];
+        if (b < tiles) v = v + T[b];
+    }
+    sh[t] = v;
+    kate_block_scan(sh, z, log_tile + log_m);
+    v = t ? sh[t - 1] : fr_t::zero();
+    for (size_t b = lo; b < end && b < tiles; b++) {
+        const fr_t own = T[b];
+        T[b] = v;
+        v = v * z[log_tile] + own;
+    }
+}
+
+template <int LOG_PER>
+__global__ void __launch_bounds__(kKateThreads) kate_apply_kernel(const kate_item *__restrict__ items, size_t len,
+                                                                  const fr_t *__restrict__ totals, bool carried)
+{
+    __shared__ fr_t sh[kKateThreads];
+    const unsigned t = threadIdx.x, b = blockIdx.x;
+    const kate_item it = items[blockIdx.y];
+    const fr_t *T = totals + (size_t)blockIdx.y * gridDim.x;
+    const size_t base = ((size_t)b * kKateThreads + t) << LOG_PER;
+    fr_t carry = fr_t::zero();
+    if (carried) {
+        carry = T[b];
+    } else if (b) {
+        // the at most 255 tiles before: sum_u z^(tile u) T[b - 1 - u]
+        sh[t] = t < b ? T[b - 1 - t] : fr_t::zero();
+        for (int k = kKateLog - 1; k >= 0; k--) {
+            __syncthreads();
+            if (t < (1u << k)) sh[t] = sh[t] + sh[t + (1u << k)] * it.z[kKateLog + LOG_PER + k];
+        }
+        __syncthreads();
+        carry = sh[0];
+        __syncthreads();
+    }
+    sh[t] = kate_thread<LOG_PER>(it.f, len, base, it.z[0], t ? fr_t::zero() : carry);
+    kate_block_scan(sh, it.z, LOG_PER);
+    fr_t h = t ? sh[t - 1] : carry;  // Horner's value before the thread's coefficients
+#pragma unroll
+    for (int e = 0; e < 1 << LOG_PER; e++) {
+        const size_t i = base + e;
+        if (i >= len) break;
+        h = h * it.z[0] + it.f[len - 1 - i];
+        if (i + 1 < len) it.q[len - 2 - i] = h;
+        else it.q[len - 1] = fr_t::zero();
+    }
+}
+
+static std::vector<fr_t> kate_powers(const fr_t *points, size_t n)
+{
+    std::vector<fr_t> z(n * kKatePowers);
+    for (size_t p = 0; p < n; p++) {
+        z[p * kKatePowers] = points[p];
+        for (int k = 1; k < kKatePowers; k++) z[p * kKatePowers + k] = z[p * kKatePowers + k - 1].sqr();
+    }
+    return z;
+}
+
+template <int LOG_PER>
+static void kate_divide_tiled(const kate_item *d_items, size_t count, size_t len, cudaStream_t s)
+{
+    constexpr int log_tile = kKateLog + LOG_PER;
+    const size_t tiles = (len + ((size_t)1 << log_tile) - 1) >> log_tile;
+    int log_m = 0;
+    while (((size_t)kKateThreads << log_m) < tiles) log_m++;
+    if (tiles > 0x7fffffff || log_tile + log_m + kKateLog > kKatePowers)
+        throw cuda_error((int)cudaErrorInvalidValue, "Kate division too long");
+    constexpr size_t kMaxY = 65535;
+    dev_buf<fr_t> totals(tiles * std::min(count, kMaxY), s);
+    for (size_t p = 0; p < count; p += kMaxY, d_items += kMaxY) {
+        const unsigned m = (unsigned)std::min(kMaxY, count - p);
+        if (tiles > 1) {
+            kate_tile_kernel<LOG_PER><<<dim3((unsigned)tiles, m), kKateThreads, 0, s>>>(d_items, len, totals);
+            GB_CHECK_LAUNCH();
+        }
+        if (log_m) {
+            kate_carry_kernel<<<m, kKateThreads, 0, s>>>(d_items, totals, tiles, log_tile, log_m);
+            GB_CHECK_LAUNCH();
+        }
+        kate_apply_kernel<LOG_PER><<<dim3((unsigned)tiles, m), kKateThreads, 0, s>>>(d_items, len, totals, log_m > 0);
         GB_CHECK_LAUNCH();
-        sum_slices_kernel<<<blocks_for(m, 128), 128, 0, s>>>(partial, slices, m, d_out + b);
-        GB_CHECK_LAUNCH();
     }
 }
 
-// g[p][j] = f[p][j] * z^j
-__global__ void scale_by_powers_kernel(const fr_t *__restrict__ f, const fr_t *__restrict__ pw, size_t len,
-                                       size_t total, fr_t *__restrict__ g)
+// divisions of polynomials of len coefficients; an item's q and f don't overlap
+static void kate_divide_items(const kate_item *d_items, size_t count, size_t len, cudaStream_t s)
 {
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < total) g[t] = f[t] * pw[t % len];
+    if (!len || !count) return;
+    // one coefficient a thread as long as 256 tiles hold the polynomial, which
+    // is the shortest chain; above, 8, so that the scan's 8 steps cost no more
+    // than the coefficients
+    if (len <= (size_t)1 << 16) kate_divide_tiled<0>(d_items, count, len, s);
+    else kate_divide_tiled<3>(d_items, count, len, s);
 }
 
-// q[p][i] = S[p][i+1] * zinv^(i+1), q[p][len-1] = 0, where S is the suffix sum
-__global__ void kate_finish_kernel(const fr_t *__restrict__ S, const fr_t *__restrict__ zinv_pw, size_t len,
-                                   size_t total, fr_t *__restrict__ q)
+// count polynomials in a row, divided by X - z; d_out and f don't overlap
+static void kate_divide(fr_t *d_out, const fr_t *f, size_t len, size_t count, const fr_t &z, cudaStream_t s)
 {
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    size_t i = t % len;
-    q[t] = i + 1 < len ? S[t + 1] * zinv_pw[i + 1] : fr_t::zero();
-}
-
-__global__ void shift_down_kernel(const fr_t *__restrict__ f, size_t len, size_t total, fr_t *__restrict__ q)
-{
-    size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    size_t i = t % len;
-    q[t] = i + 1 < len ? f[t + 1] : fr_t::zero();
-}
-
-void kate_divide(fr_t *d_out, const fr_t *f, size_t len, size_t count, const fr_t &z, cudaStream_t s)
-{
-    const size_t total = len * count;
-    if (!total) return;
-    if (z.is_zero()) {
-        shift_down_kernel<<<blocks_for(total, 256), 256, 0, s>>>(f, len, total, d_out);
-        GB_CHECK_LAUNCH();
-        return;
-    }
-    // powers of z and of 1/z (rows 0 and 1 of pws), in one launch pair up
-    // to 2^24 coefficients
-    dev_buf<fr_t> zs(2, s), pws(2 * len, s), g(total, s);
-    const fr_t hz[2] = {z, z.inverse()};
-    if (len <= ((size_t)1 << 24)) {
-        h2d(zs, hz, sizeof(hz), s);
-        omega_powers_many(pws, zs, 2, len, s);
-    } else {
-        omega_powers(pws, hz[0], len, s);
-        omega_powers(pws.get() + len, hz[1], len, s);
-    }
-    const fr_t *pw = pws.get(), *ipw = pws.get() + len;
-    scale_by_powers_kernel<<<blocks_for(total, 256), 256, 0, s>>>(f, pw, len, total, g);
-    GB_CHECK_LAUNCH();
-    for (size_t p = 0; p < count; p++) suffix_sum(g.get() + p * len, g.get() + p * len, len, s);
-    kate_finish_kernel<<<blocks_for(total, 256), 256, 0, s>>>(g, ipw, len, total, d_out);
-    GB_CHECK_LAUNCH();
+    const std::vector<fr_t> powers = kate_powers(&z, 1);
+    dev_buf<fr_t> d_powers(powers.size(), s);
+    h2d(d_powers, powers.data(), powers.size() * sizeof(fr_t), s);
+    std::vector<kate_item> items(count);
+    for (size_t p = 0; p < count; p++) items[p] = kate_item{f + p * len, d_out + p * len, d_powers.get()};
+    dev_buf<kate_item> d_items(count, s);
+    h2d(d_items, items.data(), count * sizeof(kate_item), s);
+    kate_divide_items(d_items, count, len, s);
 }
 
 // q[k][i] = sum over the items t of q k (q_offsets[k] <= t < q_offsets[k+1])
@@ -258,7 +372,7 @@ RustError midnight_sppark_bls12_381_fr_device_eval_polys(RawFr *out_raw, const v
     cudaStream_t s = lane_stream();
     device_vec_wait(v, s);
     dev_buf<fr_t> d(poly_count, s);
-    eval_polys(d, v->values, poly_len, poly_count, from_raw(point_raw), s);
+    eval_polys(d, v->values, poly_len, poly_count, point_raw, s);
     d2h(out_raw, d, poly_count * sizeof(fr_t), s);
     lane_sync(s);
     return ok();
@@ -435,18 +549,33 @@ RustError midnight_sppark_bls12_381_fr_multiopen_f_poly_device(void **out, const
     GB_ENTRY_BEGIN
     cudaStream_t s = lane_stream();
     device_vec_wait(qv, s);
-    dev_buf<fr_t> divided(q_count * poly_len, s), work(2 * poly_len, s);
+    // round j divides every q that has more than j points by X - its j-th
+    // one, into one half of work and the other in turn
+    size_t rounds = 0;
+    for (size_t k = 0; k < q_count; k++) rounds = std::max<size_t>(rounds, point_offsets[k + 1] - point_offsets[k]);
+    dev_buf<fr_t> work(std::min<size_t>(rounds, 2) * q_count * poly_len, s);
+    std::vector<fr_t> zs(point_count);
+    for (size_t j = 0; j < point_count; j++) zs[j] = from_raw(points[j]);
+    const std::vector<fr_t> powers = kate_powers(zs.data(), point_count);
+    dev_buf<fr_t> d_powers(powers.size(), s);
+    h2d(d_powers, powers.data(), powers.size() * sizeof(fr_t), s);
     std::vector<const fr_t *> table(q_count);
-    for (size_t k = 0; k < q_count; k++) {
-        const fr_t *cur = qv->values + k * poly_len;
-        const uint32_t p0 = point_offsets[k], p1 = point_offsets[k + 1];
-        for (uint32_t j = p0; j < p1; j++) {
-            fr_t *dst = j + 1 == p1 ? divided.get() + k * poly_len : work.get() + ((j - p0) & 1) * poly_len;
-            kate_divide(dst, cur, poly_len, 1, from_raw(points[j]), s);
-            cur = dst;
+    for (size_t k = 0; k < q_count; k++) table[k] = qv->values + k * poly_len;
+    std::vector<kate_item> items;
+    std::vector<size_t> starts(1, 0);
+    for (size_t j = 0; j < rounds; j++) {
+        for (size_t k = 0; k < q_count; k++) {
+            if (j >= point_offsets[k + 1] - point_offsets[k]) continue;
+            fr_t *dst = work.get() + ((j & 1) * q_count + k) * poly_len;
+            items.push_back(kate_item{table[k], dst, d_powers.get() + (point_offsets[k] + j) * kKatePowers});
+            table[k] = dst;
         }
-        table[k] = cur;
+        starts.push_back(items.size());
     }
+    dev_buf<kate_item> d_items(items.size(), s);
+    h2d(d_items, items.data(), items.size() * sizeof(kate_item), s);
+    for (size_t j = 0; j < rounds; j++)
+        kate_divide_items(d_items.get() + starts[j], starts[j + 1] - starts[j], poly_len, s);
     dev_buf<const fr_t *> d_table(q_count, s);
     h2d(d_table, table.data(), q_count * sizeof(const fr_t *), s);
     dev_buf<fr_t> d_scalars(scalar_count, s);

@@ -35,20 +35,6 @@ __device__ fr_t block_scan_mul(fr_t v, fr_t *sh)
     return sh[threadIdx.x];
 }
 
-// Inclusive multiplicative suffix scan (thread t gets prod_{t' >= t}).
-__device__ fr_t block_suffix_scan_mul(fr_t v, fr_t *sh)
-{
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (unsigned off = 1; off < blockDim.x; off <<= 1) {
-        fr_t other = threadIdx.x + off < blockDim.x ? sh[threadIdx.x + off] : fr_t::one();
-        __syncthreads();
-        if (threadIdx.x + off < blockDim.x) sh[threadIdx.x] = sh[threadIdx.x] * other;
-        __syncthreads();
-    }
-    return sh[threadIdx.x];
-}
-
 // ------------------------------------------------------------ prefix product
 
 // phase 1: per tile product -> aux[tile]
@@ -102,95 +88,6 @@ void prefix_product(fr_t *out, const fr_t *in, size_t n, cudaStream_t s)
     GB_CHECK_LAUNCH();
     if (tiles > 1) prefix_product(aux, aux, tiles, s);
     scan_tile_apply_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, aux, out);
-    GB_CHECK_LAUNCH();
-}
-
-// ------------------------------------------------------------ additive suffix scan
-
-// out[i] = sum_{j >= i} in[j], by tiles of 2048 counted from the top end
-__global__ void __launch_bounds__(kScanThreads) sfx_tile_sum_kernel(const fr_t *__restrict__ in, size_t n,
-                                                                    fr_t *__restrict__ aux)
-{
-    __shared__ fr_t sh[kScanThreads];
-    // tile t covers reversed positions [t*2048, (t+1)*2048), element n-1-r
-    size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanPer;
-    fr_t acc = fr_t::zero();
-#pragma unroll
-    for (int e = 0; e < kScanPer; e++)
-        if (base + e < n) acc = acc + in[n - 1 - (base + e)];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (unsigned off = blockDim.x / 2; off; off >>= 1) {
-        if (threadIdx.x < off) sh[threadIdx.x] = sh[threadIdx.x] + sh[threadIdx.x + off];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) aux[blockIdx.x] = sh[0];
-}
-
-__global__ void __launch_bounds__(kScanThreads) sfx_tile_apply_kernel(const fr_t *in, size_t n,
-                                                                      const fr_t *__restrict__ aux_incl, fr_t *out)
-{
-    __shared__ fr_t sh[kScanThreads];
-    size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanPer;
-    fr_t v[kScanPer];
-    fr_t acc = fr_t::zero();
-#pragma unroll
-    for (int e = 0; e < kScanPer; e++) {
-        v[e] = base + e < n ? in[n - 1 - (base + e)] : fr_t::zero();
-        acc = acc + v[e];
-    }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (unsigned off = 1; off < blockDim.x; off <<= 1) {
-        fr_t other = threadIdx.x >= off ? sh[threadIdx.x - off] : fr_t::zero();
-        __syncthreads();
-        if (threadIdx.x >= off) sh[threadIdx.x] = sh[threadIdx.x] + other;
-        __syncthreads();
-    }
-    fr_t run = threadIdx.x ? sh[threadIdx.x - 1] : fr_t::zero();
-    if (blockIdx.x) run = run + aux_incl[blockIdx.x - 1];
-#pragma unroll
-    for (int e = 0; e < kScanPer; e++) {
-        run = run + v[e];
-        if (base + e < n) out[n - 1 - (base + e)] = run;
-    }
-}
-
-// inclusive prefix sum of tile totals, in place (reuses the suffix machinery
-// on the reversed view of a reversed array: a plain forward scan)
-__global__ void __launch_bounds__(kScanThreads) fwd_sum_scan_small_kernel(fr_t *a, size_t n)
-{
-    // single block, n <= kScanTile * kScanTile handled by recursion on the host
-    __shared__ fr_t sh[kScanThreads];
-    const size_t per = (n + blockDim.x - 1) / blockDim.x;
-    const size_t lo = threadIdx.x * per, hi = min(lo + per, n);
-    fr_t acc = fr_t::zero();
-    for (size_t i = lo; i < hi; i++) acc = acc + a[i];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (unsigned off = 1; off < blockDim.x; off <<= 1) {
-        fr_t other = threadIdx.x >= off ? sh[threadIdx.x - off] : fr_t::zero();
-        __syncthreads();
-        if (threadIdx.x >= off) sh[threadIdx.x] = sh[threadIdx.x] + other;
-        __syncthreads();
-    }
-    fr_t run = threadIdx.x ? sh[threadIdx.x - 1] : fr_t::zero();
-    for (size_t i = lo; i < hi; i++) {
-        run = run + a[i];
-        a[i] = run;
-    }
-}
-
-void suffix_sum(fr_t *out, const fr_t *in, size_t n, cudaStream_t s)
-{
-    if (!n) return;
-    size_t tiles = (n + kScanTile - 1) / kScanTile;
-    dev_buf<fr_t> aux(tiles, s);
-    sfx_tile_sum_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, aux);
-    GB_CHECK_LAUNCH();
-    fwd_sum_scan_small_kernel<<<1, kScanThreads, 0, s>>>(aux, tiles);
-    GB_CHECK_LAUNCH();
-    sfx_tile_apply_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, aux, out);
     GB_CHECK_LAUNCH();
 }
 
@@ -291,21 +188,19 @@ __global__ void power_factors_kernel(fr_t *d, fr_t w, size_t n)
 }
 
 // Power tables up to 2^24 entries: w^i = T0[i & 255] * T1[(i >> 8) & 255] *
-// T2[i >> 16], where T0[j] = w^j, T1[j] = w^(256 j), T2[j] = w^(65536 j).
-// One block builds the three 256-entry tables with block scans (exclusive:
-// T[j] = base^j); the apply kernel spends two products per element.
+// T2[i >> 16], where T0[j] = w^j, T1[j] = w^(256 j), T2[j] = w^(65536 j); a
+// block a table.  Every thread squares its way to its entry's bits (at most 32
+// dependent products, 13 us; block scans took 24 us for the three tables).  The
+// apply kernel spends two products per element.
 __global__ void __launch_bounds__(256) power_tables_kernel(fr_t w, fr_t *__restrict__ tables)
 {
-    __shared__ fr_t sh[256];
-    fr_t base = w;
-    for (int level = 0; level < 3; level++) {
-        fr_t incl = block_scan_mul(base, sh);  // base^(t+1)
-        __syncthreads();
-        tables[level * 256 + threadIdx.x] = threadIdx.x ? sh[threadIdx.x - 1] : fr_t::one();
-        base = sh[255];  // base^256, the next level's base
-        __syncthreads();
-        (void)incl;
+    for (unsigned k = 0; k < 8 * blockIdx.x; k++) w = w.sqr();
+    fr_t v = fr_t::one();
+    for (unsigned b = 0; b < 8; b++) {
+        if ((threadIdx.x >> b) & 1u) v = v * w;
+        w = w.sqr();
     }
+    tables[blockIdx.x * 256 + threadIdx.x] = v;
 }
 
 __global__ void power_apply_kernel(const fr_t *__restrict__ tables, size_t n, fr_t *__restrict__ d)
@@ -318,46 +213,6 @@ __global__ void power_apply_kernel(const fr_t *__restrict__ tables, size_t n, fr
     d[i] = v;
 }
 
-// the tables of power_tables_kernel for several points: block q reads
-// points[q] and writes tables[q * 768 ..]
-__global__ void __launch_bounds__(256) power_tables_many_kernel(const fr_t *__restrict__ points,
-                                                                fr_t *__restrict__ tables)
-{
-    __shared__ fr_t sh[256];
-    fr_t base = points[blockIdx.x];
-    fr_t *t = tables + (size_t)blockIdx.x * 768;
-    for (int level = 0; level < 3; level++) {
-        block_scan_mul(base, sh);  // sh[t] = base^(t+1)
-        __syncthreads();
-        t[level * 256 + threadIdx.x] = threadIdx.x ? sh[threadIdx.x - 1] : fr_t::one();
-        base = sh[255];
-        __syncthreads();
-    }
-}
-
-// d[q * n + i] = tables_q-powers, i < n <= 2^24, one grid row per point
-__global__ void power_apply_many_kernel(const fr_t *__restrict__ tables, size_t n, fr_t *__restrict__ d)
-{
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const fr_t *t = tables + (size_t)blockIdx.y * 768;
-    fr_t v = t[i & 255];
-    if (i >> 8) v = v * t[256 + ((i >> 8) & 255)];
-    if (i >> 16) v = v * t[512 + (i >> 16)];
-    d[(size_t)blockIdx.y * n + i] = v;
-}
-
-void omega_powers_many(fr_t *d, const fr_t *d_points, size_t npoints, size_t n, cudaStream_t s)
-{
-    if (!n || !npoints) return;
-    if (n > ((size_t)1 << 24) || npoints > 65535) throw cuda_error((int)cudaErrorInvalidValue, "power table too large");
-    dev_buf<fr_t> tables(768 * npoints, s);
-    power_tables_many_kernel<<<(unsigned)npoints, 256, 0, s>>>(d_points, tables);
-    GB_CHECK_LAUNCH();
-    power_apply_many_kernel<<<dim3(blocks_for(n, 256), (unsigned)npoints), 256, 0, s>>>(tables, n, d);
-    GB_CHECK_LAUNCH();
-}
-
 void omega_powers(fr_t *d, const fr_t &w, size_t n, cudaStream_t s)
 {
     if (!n) return;
@@ -368,7 +223,7 @@ void omega_powers(fr_t *d, const fr_t &w, size_t n, cudaStream_t s)
         return;
     }
     dev_buf<fr_t> tables(3 * 256, s);
-    power_tables_kernel<<<1, 256, 0, s>>>(w, tables);
+    power_tables_kernel<<<n > 65536 ? 3 : n > 256 ? 2 : 1, 256, 0, s>>>(w, tables);
     GB_CHECK_LAUNCH();
     power_apply_kernel<<<blocks_for(n, 256), 256, 0, s>>>(tables, n, d);
     GB_CHECK_LAUNCH();

@@ -77,3 +77,38 @@ def test_eval_many_matches_single_evaluations(gb, orc):
         assert (g == gb.bls12_381_fr_device_eval_polys(v, n, c, p)).all()
     want0 = orc.fr_eval_poly(vecs[1].download()[:n], pts[1])
     assert (got[1][0] == want0).all()
+
+
+@pytest.mark.parametrize("ln,count", [(1, 2), (2, 1), (255, 1), (256, 3), (257, 2), (513, 1), (1 << 16, 1),
+                                      ((1 << 16) + 1, 2), (1 << 19, 1), ((1 << 19) + 1, 1), ((1 << 20) + 2049, 1)])
+@pytest.mark.parametrize("point", ["random", "zero", "one"])
+def test_kate_divide_tile_edges(gb, orc, ln, count, point):
+    """Around the block's scan (256), the change of coefficients a thread
+    (2^16) and the carry pass (above 256 tiles of 2048)."""
+    rng = np.random.default_rng(ln + count)
+    polys = orc.fr_random(ln * count, rng)
+    z = orc.fr_random(1, rng)[0] if point == "random" else orc.fr_from_ints([int(point == "one")])[0]
+    dv = gb.Bls12_381FrDeviceVec.upload(polys)
+    q = gb.fr_device_kate_divide(dv, ln, count, z)
+    got = q.download().reshape(count, ln, 4)
+    for p in range(count):
+        if ln > 1:
+            assert (got[p, :ln - 1] == orc.fr_kate_division(polys[p * ln:(p + 1) * ln], z)).all()
+        assert (got[p, ln - 1] == 0).all()
+    q.free()
+    dv.free()
+
+
+@pytest.mark.parametrize("ln,requests", [(1, 1), (255, 2), (256, 1), (257, 1), (4096, 3), (4097, 3),
+                                         ((1 << 20) + 5, 1), ((1 << 14) + 1, 608), ((1 << 14) - 1, 608)])
+def test_eval_many_slice_edges(gb, orc, ln, requests):
+    """Around a slice of 4096, with more than one level of slices, and with
+    slices of 16384 (many requests)."""
+    rng = np.random.default_rng(ln + requests)
+    coeffs = orc.fr_random(ln, rng)
+    points = orc.fr_random(requests, rng)
+    dv = gb.Bls12_381FrDeviceVec.upload(coeffs)
+    got = gb.fr_device_eval_many([(dv, 1, z) for z in points], ln)
+    for r in range(0, requests, 101):
+        assert (got[r][0] == orc.fr_eval_poly(coeffs, points[r])).all()
+    dv.free()
