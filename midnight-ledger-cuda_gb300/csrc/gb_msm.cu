@@ -238,11 +238,16 @@ static void launch_recode(const item_desc *items, uint32_t nitems, uint64_t tota
     GB_CHECK_LAUNCH();
 }
 
+// control words of a batch, zeroed by its first kernel that has them
+enum { CTL_LONGS = 0, CTL_DONE = 1, CTL_WORDS = 2 };  // long buckets so far; column blocks done
+
 // 2. per-block histograms: hist[b][k]
 __global__ void msm_hist_kernel(const uint32_t *__restrict__ digits, const seg_desc *__restrict__ segs,
-                                const blk_desc *__restrict__ blks, uint32_t K, uint32_t *__restrict__ hist)
+                                const blk_desc *__restrict__ blks, uint32_t K, uint32_t *__restrict__ hist,
+                                uint32_t *__restrict__ ctl)
 {
     extern __shared__ uint32_t sh[];
+    if (blockIdx.x == 0 && threadIdx.x < CTL_WORDS) ctl[threadIdx.x] = 0;
     const blk_desc bd = blks[blockIdx.x];
     for (uint32_t k = threadIdx.x; k < K; k += blockDim.x) sh[k] = 0;
     __syncthreads();
@@ -259,34 +264,100 @@ __global__ void msm_hist_kernel(const uint32_t *__restrict__ digits, const seg_d
 // 3. per global key g = seg * K + k: exclusive prefix over the segment's
 //    blocks (in place in hist) and the total into counts[g], rounded up to a
 //    multiple of pad + 1 (a power of two; the places past the total hold
-//    kNoPoint)
-__global__ void msm_colscan_kernel(uint32_t *__restrict__ hist, const seg_desc *__restrict__ segs, uint32_t K,
-                                   uint32_t G, uint32_t pad, uint32_t *__restrict__ counts)
+//    kNoPoint).  The sum of a key without entries is infinity (all zero) here;
+//    the accumulation writes all others.  With few keys (starts given, blocks
+//    of 1024 threads), the last block to finish also scans the counts: one
+//    launch in place of four and two copies, 12 us of the 2^10-point MSM's
+//    200.
+static constexpr uint32_t kScanHere = 16 * 1024;  // keys at most
+
+__global__ void __launch_bounds__(1024)
+    msm_colscan_kernel(uint32_t *__restrict__ hist, const seg_desc *__restrict__ segs, uint32_t K, uint32_t G,
+                       uint32_t pad, uint32_t *counts, xyzz_t *__restrict__ buckets, uint32_t *__restrict__ starts,
+                       uint32_t *ctl)
 {
-    uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    const seg_desc sd = segs[g / K];
-    const uint32_t k = g % K;
-    uint32_t run = 0;
-    uint32_t *col = hist + (size_t)sd.blk0 * K + k;
-    uint32_t w = 0;
-    // batches of 16 independent loads keep the column walk off the latency path
-    for (; w + 16 <= sd.nblk; w += 16) {
-        uint32_t v[16];
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < G) {
+        const seg_desc sd = segs[g / K];
+        const uint32_t k = g % K;
+        uint32_t run = 0;
+        uint32_t *col = hist + (size_t)sd.blk0 * K + k;
+        uint32_t w = 0;
+        // batches of 16 independent loads keep the column walk off the latency path
+        for (; w + 16 <= sd.nblk; w += 16) {
+            uint32_t v[16];
 #pragma unroll
-        for (int u = 0; u < 16; u++) v[u] = col[(size_t)(w + u) * K];
+            for (int u = 0; u < 16; u++) v[u] = col[(size_t)(w + u) * K];
 #pragma unroll
-        for (int u = 0; u < 16; u++) {
-            col[(size_t)(w + u) * K] = run;
-            run += v[u];
+            for (int u = 0; u < 16; u++) {
+                col[(size_t)(w + u) * K] = run;
+                run += v[u];
+            }
+        }
+        for (; w < sd.nblk; w++) {
+            uint32_t v = col[(size_t)w * K];
+            col[(size_t)w * K] = run;
+            run += v;
+        }
+        counts[g] = (run + pad) & ~pad;
+        if (!run) buckets[g] = xyzz_t::inf();
+    }
+    if (!starts) return;
+    __shared__ uint32_t part[16 * 32];
+    __shared__ bool last;
+    __threadfence();  // this thread's count before the block's arrival
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&ctl[CTL_DONE], 1u) + 1 == gridDim.x;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // strip j holds keys 1024 j ..: a warp's scan, the warps' totals, the strips'
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t v[16], incl[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        const uint32_t i = j * 1024u + threadIdx.x;
+        v[j] = i < G ? __ldcg(counts + i) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        incl[j] = v[j];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, incl[j], off);
+            if (lane >= (uint32_t)off) incl[j] += x;
+        }
+        if (lane == 31) part[j * 32 + warp] = incl[j];
+    }
+    __syncthreads();
+    if (warp == 0) {
+        // lane l: the 16 totals 16 l .. 16 l + 15, in key order
+        uint32_t sum = 0, own[16];
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            own[j] = part[lane * 16 + j];
+            sum += own[j];
+        }
+        uint32_t run = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, run, off);
+            if (lane >= (uint32_t)off) run += x;
+        }
+        if (lane == 31) starts[G] = run;
+        run -= sum;
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            part[lane * 16 + j] = run;
+            run += own[j];
         }
     }
-    for (; w < sd.nblk; w++) {
-        uint32_t v = col[(size_t)w * K];
-        col[(size_t)w * K] = run;
-        run += v;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        const uint32_t i = j * 1024u + threadIdx.x;
+        if (i < G) starts[i] = part[j * 32 + warp] + incl[j] - v[j];
     }
-    counts[g] = (run + pad) & ~pad;
 }
 
 // 4. exclusive scan of counts[0..G) into starts[0..G], starts[G] = total:
@@ -732,8 +803,144 @@ __global__ void __launch_bounds__(BLOCK, MINB) msm_accumulate_kernel(
     }
 }
 
-// 7. buckets spanning several chunks (empty buckets are infinity already: all
-//    zero, as they were before the accumulation).  A bucket spanning a few
+// 6'. The same with two lanes a chunk, for batches too small to fill the GPU
+//     with a thread a chunk: the 10 products of a mixed addition are 5 levels of
+//     two that do not depend on each other, so an addition takes half as long
+//     and its products cost the same.  Of the running point the even lane has
+//     X (and a copy of Y) and ZZ, the odd one Y (and X) and ZZZ; of an entry the
+//     even lane reads x, the odd one y.  A warp's lanes go through all L steps
+//     together, so that the exchanges have all of them; what does not hold for
+//     a pair (no entry left, nothing summed yet) is selected away.
+__device__ __forceinline__ fp_t pair_swap(const fp_t &a)
+{
+    fp_t r;
+#pragma unroll
+    for (int i = 0; i < 12; i++) r.v[i] = __shfl_xor_sync(0xffffffffu, a.v[i], 1);
+    return r;
+}
+
+__device__ __forceinline__ fp_t pair_pick(bool odd, const fp_t &o, const fp_t &e)
+{
+    fp_t r;
+#pragma unroll
+    for (int i = 0; i < 12; i++) r.v[i] = odd ? o.v[i] : e.v[i];
+    return r;
+}
+
+static constexpr uint32_t kPairChunks = 64, kPairSm = 3;  // a block's chunks, an SM's blocks
+
+__global__ void __launch_bounds__(2 * kPairChunks, kPairSm) msm_accumulate_pair_kernel(
+    const uint32_t *__restrict__ sorted, const uint32_t *__restrict__ starts, uint32_t G, uint32_t L,
+    size_t nchunks, const affine_t *__restrict__ points, xyzz_t *__restrict__ buckets,
+    xyzz_t *__restrict__ head, xyzz_t *__restrict__ tail, uint32_t *__restrict__ open_bucket)
+{
+    const size_t t = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 2;
+    const bool odd = threadIdx.x & 1u;
+    const uint32_t T = starts[G];
+    uint64_t lo = (uint64_t)t * L, hi = lo + L;
+    if (t >= nchunks || lo >= T) lo = hi = 0;
+    hi = min((uint64_t)T, hi);
+    uint32_t g = 0, gend = 0;
+    bool started_here = false;
+    if (lo < hi) {
+        // largest g with starts[g] <= lo; starts[G] = T > lo
+        uint32_t b = G;
+        while (b - g > 1) {
+            const uint32_t mid = (g + b) >> 1;
+            if (starts[mid] <= lo) g = mid;
+            else b = mid;
+        }
+        gend = starts[g + 1];
+        started_here = starts[g] >= lo;
+    }
+    auto load = [&](uint64_t pos) {
+        fp_t q = fp_t::zero();
+        if (pos >= hi) return q;
+        const uint32_t ref = sorted[pos];
+        const uint4 *src = reinterpret_cast<const uint4 *>(points + (ref & 0x7fffffffu)) + (odd ? 3 : 0);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const uint4 w = __ldg(src + i);
+            q.v[4 * i] = w.x, q.v[4 * i + 1] = w.y, q.v[4 * i + 2] = w.z, q.v[4 * i + 3] = w.w;
+        }
+        if (odd && (ref >> 31)) q = -q;
+        return q;
+    };
+    // the lane's coordinate, the other lane's, and its denominator (ZZ or ZZZ)
+    fp_t own = fp_t::zero(), other = fp_t::zero(), den = fp_t::zero();
+    bool empty = true, open = false;
+    auto store = [&](xyzz_t *to) {
+        fp_t *f = reinterpret_cast<fp_t *>(to) + (odd ? 1 : 0);
+        f[0] = empty ? fp_t::zero() : own;
+        f[2] = empty ? fp_t::zero() : den;
+    };
+    fp_t next = load(lo);
+    for (uint32_t i = 0; i < L; i++) {
+        const uint64_t pos = lo + i;
+        const fp_t q = next;
+        next = load(pos + 1);
+        const bool valid = pos < hi, zero = q.is_zero();
+        // every lane of the warp takes part in an exchange: none stands behind
+        // a condition of its own
+        const bool zero2 = __shfl_xor_sync(0xffffffffu, (int)zero, 1);
+        const bool take = valid && !(zero && zero2);  // a base at infinity adds nothing
+        const fp_t q2 = pair_swap(q);
+        if (__any_sync(0xffffffffu, take && !empty)) {
+            const fp_t d = q * den - own;  // P | R
+            const bool dz = d.is_zero(), dz2 = __shfl_xor_sync(0xffffffffu, (int)dz, 1);
+            const fp_t e = d.sqr(), f = pair_swap(e);                               // PP | RR and the other
+            const fp_t h = pair_pick(odd, other, d) * pair_pick(odd, f, e);         // P PP | X PP
+            const fp_t h2 = pair_swap(h);
+            const fp_t ppp = pair_pick(odd, h2, h), xpp = pair_pick(odd, h, h2);
+            const fp_t x3 = pair_pick(odd, e, f) - ppp - xpp.dbl();
+            const fp_t k = pair_pick(odd, d, other) * pair_pick(odd, xpp - x3, ppp);  // Y PPP | R (X PP - X3)
+            const fp_t k2 = pair_swap(k);
+            const fp_t y3 = pair_pick(odd, k, k2) - pair_pick(odd, k2, k);
+            const fp_t den3 = den * pair_pick(odd, ppp, e);
+            const bool same_x = odd ? dz2 : dz, same_y = odd ? dz : dz2;
+            if (take && !empty) {
+                if (!same_x) {
+                    own = pair_pick(odd, y3, x3);
+                    other = pair_pick(odd, x3, y3);
+                    den = den3;
+                } else if (same_y) {
+                    const xyzz_t v = xyzz_t::dbl_affine(pair_pick(odd, q2, q), pair_pick(odd, q, q2));
+                    own = pair_pick(odd, v.y, v.x);
+                    other = pair_pick(odd, v.x, v.y);
+                    den = pair_pick(odd, v.zzz, v.zz);
+                    empty = v.zz.is_zero();
+                } else {
+                    empty = true;
+                }
+            } else if (take) {
+                own = q, other = q2, den = fp_t::one();
+                empty = false;
+            }
+        } else if (take) {
+            own = q, other = q2, den = fp_t::one();
+            empty = false;
+        }
+        if (valid) {
+            open = true;
+            if (pos + 1 == gend) {
+                store(started_here ? buckets + g : head + t);
+                empty = true;
+                open = false;
+                started_here = true;
+                g++;
+                while (g < G && starts[g + 1] == starts[g]) g++;
+                gend = g < G ? starts[g + 1] : T;
+            }
+        }
+        __syncwarp();
+    }
+    if (open) {
+        store(tail + t);
+        if (open_bucket && started_here && !odd) open_bucket[t] = g;
+    }
+}
+
+// 7. buckets spanning several chunks.  A bucket spanning a few
 //    chunks is summed by its own thread; longer ones (skewed digits: structured
 //    scalars, the carry out of scalars below 2^64) are appended to `longs` for
 //    msm_fixup_long_kernel.  One thread a bucket, or, where buckets are shorter
@@ -774,24 +981,32 @@ __global__ void msm_fixup_kernel(const uint32_t *__restrict__ starts, const uint
 // Cooperative point arithmetic for the latency-bound reduction.  The bucket
 // reduction is a few chains of dependent XYZZ operations per segment, run on
 // few warps, so its time is the latency of one operation times the chain
-// length.  Here a group of 8 lanes (a quarter warp) runs one chain: the
-// products of a point operation that do not depend on each other are
-// computed by different lanes at the same time, with the operands and
-// results in the group's shared-memory slots.  An addition is then 4 product
-// levels deep (instead of 14 products in sequence) and a doubling 3 (instead
-// of 10).  Every decision (infinity, equal or opposite points) reads shared
-// values after a group barrier, so the 8 lanes always take the same path.
-static constexpr uint32_t kCoopLanes = 8;
-static constexpr uint32_t kCoopGroups = 16;  // groups per 128-thread block
-static constexpr uint32_t kCoopFixupMaxBuckets = 1u << 14;  // cooperative fix-up up to 2^14 buckets in all
-// slots of a group: RUN, SUM, OPD (operand), RES (4 each: X, Y, ZZ, ZZZ),
-// then 12 temporaries
-enum { CO_RUN = 0, CO_SUM = 4, CO_OPD = 8, CO_RES = 12, CO_TMP = 16, CO_SLOTS = 28 };
+// length.  Here a group of 4 lanes runs one chain: the products of a point
+// operation that do not depend on each other are computed by different lanes
+// at the same time, with the operands and results in the group's
+// shared-memory slots.  An addition is then 4 product levels deep (instead of
+// 14 products in sequence) and a doubling 3 (instead of 10); with 8 lanes it is
+// as deep, and half of them idle (4 x 2^16 points, fix-up and reduction with 8
+// lanes 289 us, with 4 245).  Every decision (infinity, equal or opposite points) reads shared
+// values after a group barrier, so the lanes always take the same path.
+static constexpr uint32_t kCoopLanes = 4;
+static constexpr uint32_t kCoopGroups = 32;  // groups per 128-thread block
+// buckets up to which groups do the fix-up, and up to which they do so also
+// where chunks are longer than buckets
+static constexpr uint32_t kCoopFixupMaxBuckets = 1u << 16, kCoopFixupSmall = 1u << 14;
+// slots of a group: SUM, OPD (operand; 4 each: X, Y, ZZ, ZZZ), then 12
+// temporaries; an odd number, so that a warp's groups lie in different banks
+enum { CO_SUM = 0, CO_OPD = 4, CO_TMP = 8, CO_SLOTS = 21 };
 
 struct coop_t {
     fp_t *s;        // the group's slots
-    uint32_t lane;  // 0..7
+    uint32_t lane;  // 0..3
     uint32_t mask;  // the group's lanes in the warp
+    __device__ coop_t(fp_t *mem)
+        : s(mem + (size_t)(threadIdx.x / kCoopLanes) * CO_SLOTS), lane(threadIdx.x % kCoopLanes),
+          mask(0xfu << (threadIdx.x & 28u))
+    {
+    }
     __device__ void sync() const { __syncwarp(mask); }
 };
 
@@ -804,31 +1019,45 @@ __device__ __forceinline__ void coop_set_inf(const coop_t &c, int a)
     c.sync();
 }
 
-// 4 slots (48 words) from src to dst, 6 words per lane
+// a point (4 field elements, one a lane), read and written 16 bytes at a time
+__device__ __forceinline__ fp_t load16(const void *p)
+{
+    const uint4 *f = reinterpret_cast<const uint4 *>(p);
+    fp_t r;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const uint4 w = f[i];
+        r.v[4 * i] = w.x, r.v[4 * i + 1] = w.y, r.v[4 * i + 2] = w.z, r.v[4 * i + 3] = w.w;
+    }
+    return r;
+}
+
+__device__ __forceinline__ void store16(void *p, const fp_t &v)
+{
+    uint4 *t = reinterpret_cast<uint4 *>(p);
+#pragma unroll
+    for (int i = 0; i < 3; i++) t[i] = make_uint4(v.v[4 * i], v.v[4 * i + 1], v.v[4 * i + 2], v.v[4 * i + 3]);
+}
+
+__device__ __forceinline__ fp_t coop_get(const coop_t &c, const void *p) { return load16((const fp_t *)p + c.lane); }
+__device__ __forceinline__ void coop_put(const coop_t &c, void *p, const fp_t &v) { store16((fp_t *)p + c.lane, v); }
+
+// 4 slots from src to dst
 __device__ __forceinline__ void coop_copy(const coop_t &c, fp_t *dst, const fp_t *src)
 {
-    const uint2 *f = reinterpret_cast<const uint2 *>(src);
-    uint2 *t = reinterpret_cast<uint2 *>(dst);
-    const uint2 a = f[c.lane * 3], b = f[c.lane * 3 + 1], d = f[c.lane * 3 + 2];
+    const fp_t v = coop_get(c, src);
     c.sync();
-    t[c.lane * 3] = a, t[c.lane * 3 + 1] = b, t[c.lane * 3 + 2] = d;
+    coop_put(c, dst, v);
     c.sync();
 }
 
 __device__ __forceinline__ void coop_load(const coop_t &c, int a, const xyzz_t *g)
 {
-    const uint2 *f = reinterpret_cast<const uint2 *>(g);
-    uint2 *t = reinterpret_cast<uint2 *>(c.s + a);
-    t[c.lane * 3] = f[c.lane * 3], t[c.lane * 3 + 1] = f[c.lane * 3 + 1], t[c.lane * 3 + 2] = f[c.lane * 3 + 2];
+    coop_put(c, c.s + a, coop_get(c, g));
     c.sync();
 }
 
-__device__ __forceinline__ void coop_store(const coop_t &c, int a, xyzz_t *g)
-{
-    const uint2 *f = reinterpret_cast<const uint2 *>(c.s + a);
-    uint2 *t = reinterpret_cast<uint2 *>(g);
-    t[c.lane * 3] = f[c.lane * 3], t[c.lane * 3 + 1] = f[c.lane * 3 + 1], t[c.lane * 3 + 2] = f[c.lane * 3 + 2];
-}
+__device__ __forceinline__ void coop_store(const coop_t &c, int a, xyzz_t *g) { coop_put(c, g, coop_get(c, c.s + a)); }
 
 // One level of products: lane l < n computes s[xi[l]] * s[yi[l]] into
 // s[oi[l]].  All lanes run the same call with their own operands, so the
@@ -847,10 +1076,10 @@ __device__ __forceinline__ uint32_t coop_pack(std::initializer_list<int> v)
 __device__ __forceinline__ void coop_level(const coop_t &c, uint32_t n, uint32_t x, uint32_t y, uint32_t o)
 {
     const uint32_t sh = 5u * (c.lane < n ? c.lane : 0u);
-    const fp_t a = c.s[(x >> sh) & 31u], b = c.s[(y >> sh) & 31u];
+    const fp_t a = load16(c.s + ((x >> sh) & 31u)), b = load16(c.s + ((y >> sh) & 31u));
     const fp_t r = a * b;
     c.sync();
-    if (c.lane < n) c.s[(o >> sh) & 31u] = r;
+    if (c.lane < n) store16(c.s + ((o >> sh) & 31u), r);
     c.sync();
 }
 
@@ -859,9 +1088,9 @@ __device__ __forceinline__ void coop_level(const coop_t &c, uint32_t n, uint32_t
 __device__ __forceinline__ void coop_level_sqr(const coop_t &c, uint32_t n, uint32_t x, uint32_t o)
 {
     const uint32_t sh = 5u * (c.lane < n ? c.lane : 0u);
-    const fp_t r = c.s[(x >> sh) & 31u].sqr();
+    const fp_t r = load16(c.s + ((x >> sh) & 31u)).sqr();
     c.sync();
-    if (c.lane < n) c.s[(o >> sh) & 31u] = r;
+    if (c.lane < n) store16(c.s + ((o >> sh) & 31u), r);
     c.sync();
 }
 
@@ -916,39 +1145,43 @@ __device__ void coop_add(const coop_t &c, int a, int q)
     }
     enum { U1 = CO_TMP, U2, S1, S2, Z12, W12, P, R, PP, RR, PPP, QQ };
     {
-        // U1 = X1 ZZ2, U2 = X2 ZZ1, S1 = Y1 ZZZ2, S2 = Y2 ZZZ1, ZZ1 ZZ2, ZZZ1 ZZZ2
-        coop_level(c, 6, coop_pack({a, q, a + 1, q + 1, a + 2, a + 3}), coop_pack({q + 2, a + 2, q + 3, a + 3, q + 2, q + 3}), coop_pack({U1, U2, S1, S2, Z12, W12}));
+        // U1 = X1 ZZ2, U2 = X2 ZZ1, S1 = Y1 ZZZ2, S2 = Y2 ZZZ1
+        coop_level(c, 4, coop_pack({a, q, a + 1, q + 1}), coop_pack({q + 2, a + 2, q + 3, a + 3}),
+                   coop_pack({U1, U2, S1, S2}));
     }
     {
-        const fp_t p = s[U2] - s[U1];
-        const fp_t r = s[S2] - s[S1];
+        const fp_t p = load16(s + U2) - load16(s + U1);
+        const fp_t r = load16(s + S2) - load16(s + S1);
         if (p.is_zero()) {
             if (r.is_zero()) coop_dbl(c, a);
             else coop_set_inf(c, a);
             return;
         }
         c.sync();
-        if (c.lane == 0) s[P] = p;
-        if (c.lane == 1) s[R] = r;
+        if (c.lane == 0) store16(s + P, p);
+        if (c.lane == 1) store16(s + R, r);
         c.sync();
     }
     {
-        coop_level_sqr(c, 2, coop_pack({P, R}), coop_pack({PP, RR}));  // PP = P^2, RR = R^2
+        // PP = P^2, RR = R^2, ZZ1 ZZ2, ZZZ1 ZZZ2
+        coop_level(c, 4, coop_pack({P, R, a + 2, a + 3}), coop_pack({P, R, q + 2, q + 3}),
+                   coop_pack({PP, RR, Z12, W12}));
     }
     {
         // PPP = P PP, Q = U1 PP, ZZ3 = ZZ1 ZZ2 PP
         coop_level(c, 3, coop_pack({P, U1, Z12}), coop_pack({PP, PP, PP}), coop_pack({PPP, QQ, a + 2}));
     }
-    const fp_t X3 = s[RR] - s[PPP] - s[QQ].dbl();
-    if (c.lane == 0) s[U2] = s[QQ] - X3;  // U2 is free from here on
+    const fp_t qq = load16(s + QQ);
+    const fp_t X3 = load16(s + RR) - load16(s + PPP) - qq.dbl();
+    if (c.lane == 0) store16(s + U2, qq - X3);  // U2 is free from here on
     c.sync();
     {
         // R (Q - X3) -> S2, S1 PPP -> U1, ZZZ3 = ZZZ1 ZZZ2 PPP
         coop_level(c, 3, coop_pack({R, S1, W12}), coop_pack({U2, PPP, PPP}), coop_pack({S2, U1, a + 3}));
     }
     if (c.lane == 0) {
-        s[a] = X3;
-        s[a + 1] = s[S2] - s[U1];
+        store16(s + a, X3);
+        store16(s + a + 1, load16(s + S2) - load16(s + U1));
     }
     c.sync();
 }
@@ -966,13 +1199,15 @@ __device__ void coop_block_tree(fp_t *sh, const coop_t &c, uint32_t grp)
     }
 }
 
-// 7'. msm_fixup_kernel with one 8-lane group per bucket: the partials of a
-//     bucket spanning several chunks are added by cooperative additions.
-//     The kernel's time is the longest span's chain (bucket sizes vary), so
-//     the shorter cooperative additions shorten it most where there are few
-//     buckets and short chunks (proof-size MSMs).
+// 7'. msm_fixup_kernel with 2^log_parts groups of lanes a bucket: the partials
+//     of a bucket are shared out to its groups, whose sums meet in a tree.  The
+//     time is the longest bucket's chain of 5 us an addition.  A group takes as
+//     many products as a thread (an addition's 14 and 2 idle ones), so it also
+//     does up to 2^16 buckets (4 x 2^16 points 111 -> 88 us, 2^16 points 118 ->
+//     82); several groups a bucket where there are few (2^10 points 51 -> 32
+//     us with 4, 2^12 53 -> 41 with 2).
 __global__ void __launch_bounds__(128) msm_fixup_coop_kernel(const uint32_t *__restrict__ starts, uint32_t G,
-                                                             uint32_t L, const xyzz_t *__restrict__ head,
+                                                             uint32_t L, uint32_t log_parts, const xyzz_t *__restrict__ head,
                                                              const xyzz_t *__restrict__ tail,
                                                              xyzz_t *__restrict__ buckets,
                                                              uint32_t *__restrict__ longs,
@@ -980,32 +1215,43 @@ __global__ void __launch_bounds__(128) msm_fixup_coop_kernel(const uint32_t *__r
 {
     __shared__ __align__(16) fp_t sh[kCoopGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
-    const coop_t c{sh + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
-    const uint32_t g = blockIdx.x * kCoopGroups + grp;
-    if (g >= G) return;  // whole groups leave together; no block barrier follows
+    const coop_t c(sh);
+    const uint32_t parts = 1u << log_parts, g = (blockIdx.x * kCoopGroups + grp) >> log_parts, part = grp & (parts - 1);
+    // a bucket's groups, side by side in a warp, go together everywhere
+    if (g >= G) return;
     const uint32_t s = starts[g], e = starts[g + 1];
     if (s == e) return;
     const uint32_t cs = s / L, ce = (e - 1) / L;
     if (cs == ce) return;
     if (ce - cs > kShortSpan) {
-        if (c.lane == 0) longs[atomicAdd(nlong, 1u)] = g;
+        if (c.lane == 0 && part == 0) longs[atomicAdd(nlong, 1u)] = g;
         return;
     }
-    coop_load(c, CO_SUM, tail + cs);
-    for (uint32_t k = cs + 1; k <= ce; k++) {
+    if (cs + part <= ce) coop_load(c, CO_SUM, cs + part == ce ? head + ce : tail + cs + part);
+    else coop_set_inf(c, CO_SUM);
+    for (uint32_t k = cs + part + parts; k <= ce; k += parts) {
         c.sync();
         coop_load(c, CO_OPD, k == ce ? head + k : tail + k);
         coop_add(c, CO_SUM, CO_OPD);
     }
-    coop_store(c, CO_SUM, buckets + g);
+    const uint32_t lanes = parts * kCoopLanes;
+    const uint32_t bucket_mask = (lanes == 32 ? 0xffffffffu : (1u << lanes) - 1) << (threadIdx.x & 31u & ~(lanes - 1));
+    for (uint32_t off = parts / 2; off > 0; off >>= 1) {
+        __syncwarp(bucket_mask);
+        if (part < off) {
+            coop_copy(c, c.s + CO_OPD, c.s + off * CO_SLOTS + CO_SUM);
+            coop_add(c, CO_SUM, CO_OPD);
+        }
+    }
+    if (part == 0) coop_store(c, CO_SUM, buckets + g);
 }
 
 // 7b. long buckets, one block each (grid-stride over the list): up to
-//     kLongDirect partials are shared out to the block's 32 groups and the
+//     kLongDirect partials are shared out to the block's 64 groups and the
 //     groups' sums added in a tree (about 10 additions of 5 us); of more,
 //     every thread first sums a strided share (14 us an addition, but 256 at
 //     once), and the groups add the 256 shares.
-static constexpr uint32_t kLongGroups = 32, kLongDirect = 512;
+static constexpr uint32_t kLongGroups = 64, kLongDirect = 512;
 static constexpr size_t kLongSmem = kLongGroups * CO_SLOTS * sizeof(fp_t) + kLongGroups * kCoopLanes * sizeof(xyzz_t);
 
 __global__ void __launch_bounds__(kLongGroups *kCoopLanes)
@@ -1017,7 +1263,7 @@ __global__ void __launch_bounds__(kLongGroups *kCoopLanes)
     fp_t *mem = reinterpret_cast<fp_t *>(long_mem);
     xyzz_t *share = reinterpret_cast<xyzz_t *>(mem + kLongGroups * CO_SLOTS);
     const uint32_t grp = threadIdx.x / kCoopLanes;
-    const coop_t c{mem + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const coop_t c(mem);
     const uint32_t count = *nlong;
     for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
         const uint32_t g = longs[i];
@@ -1055,9 +1301,9 @@ __global__ void __launch_bounds__(kLongGroups *kCoopLanes)
 //     many additions, done by the host for a few segments and by one group a
 //     segment beyond.  Measured against running sums over sub-segments, each
 //     with its offset's double-and-add: one MSM of 2^12 buckets 0.172 -> 0.066
-//     ms, of 2^15 0.299 -> 0.150, three of 2^15 0.53 -> 0.265 (with the host's
+//     ms, of 2^15 0.299 -> 0.128, three of 2^15 0.53 -> 0.211 (with the host's
 //     share, 15 us an MSM, outside these).  What bounds it: about 20 dependent
-//     additions of 5 to 10 us.
+//     additions of 5 us.
 struct line_shape {
     uint32_t lr, lc;  // log2 of rows and columns
     __host__ __device__ uint32_t lines() const { return (1u << lr) + (1u << lc); }
@@ -1097,7 +1343,7 @@ __global__ void __launch_bounds__(128) msm_line_sum_kernel(const xyzz_t *__restr
 {
     __shared__ __align__(16) fp_t mem[kCoopGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
-    const coop_t c{mem + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const coop_t c(mem);
     const uint32_t lk = sh.lr + sh.lc, rows = 1u << sh.lr, line = blockIdx.x, seg = blockIdx.y;
     const bool row = line < rows;
     const uint32_t n = 1u << ((row ? sh.lc : sh.lr) - lm);
@@ -1125,7 +1371,7 @@ __global__ void __launch_bounds__(kBitGroups *kCoopLanes) msm_bit_sum_kernel(con
 {
     __shared__ __align__(16) fp_t mem[kBitGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
-    const coop_t c{mem + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const coop_t c(mem);
     const uint32_t seg = blockIdx.y, rows = 1u << sh.lr;
     const bool row = blockIdx.x < sh.lr;
     const uint32_t b = row ? blockIdx.x : blockIdx.x - sh.lr, lw = row ? sh.lr : sh.lc;
@@ -1143,13 +1389,13 @@ __global__ void __launch_bounds__(kBitGroups *kCoopLanes) msm_bit_sum_kernel(con
     if (grp == 0) coop_store(c, CO_SUM, bits + (uint64_t)seg * sh.bits() + blockIdx.x);
 }
 
-// 8d'. the bit sums of a segment to one point: an 8-lane group a segment
+// 8d'. the bit sums of a segment to one point, a group a segment
 __global__ void __launch_bounds__(128) msm_bit_combine_kernel(const xyzz_t *__restrict__ bits, line_shape sh,
                                                               uint32_t nseg, xyzz_t *__restrict__ seg_sum)
 {
     __shared__ __align__(16) fp_t mem[kCoopGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
-    const coop_t c{mem + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const coop_t c(mem);
     const uint32_t seg = blockIdx.x * kCoopGroups + grp;
     if (seg >= nseg) return;  // whole groups leave together; no block barrier follows
     const xyzz_t *p = bits + (uint64_t)seg * sh.bits();
@@ -1172,14 +1418,14 @@ __global__ void __launch_bounds__(128) msm_bit_combine_kernel(const xyzz_t *__re
 }
 
 // 8e. plain MSMs beyond a few: combine an MSM's window segments by Horner's
-//     rule, an 8-lane group an MSM ((windows - 1) * c doublings)
+//     rule, a group an MSM ((windows - 1) * c doublings)
 __global__ void __launch_bounds__(128) msm_combine_coop_kernel(const xyzz_t *__restrict__ seg_sum, uint32_t nitems,
                                                                uint32_t segs_per_item, int c,
                                                                xyzz_t *__restrict__ out)
 {
     __shared__ __align__(16) fp_t sh[kCoopGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
-    const coop_t cp{sh + (size_t)grp * CO_SLOTS, threadIdx.x % kCoopLanes, 0xffu << (threadIdx.x & 24u)};
+    const coop_t cp(sh);
     const uint32_t m = blockIdx.x * kCoopGroups + grp;
     if (m >= nitems) return;  // whole groups leave together; no block barrier follows
     const xyzz_t *ss = seg_sum + (size_t)m * segs_per_item;
@@ -1276,18 +1522,42 @@ static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int varian
     const uint64_t L2 = (digits + waves * wave - 1) / (waves * wave);
     if (L2 >= 8 && L2 <= 2 * (uint64_t)L) return (uint32_t)L2;
     if (L2 >= 8) return L;
-    // Less than one wave of 8-digit chunks (small MSMs): the accumulation
-    // takes about L dependent additions per thread and the fix-up about
-    // avg / L (the chunks a bucket spans; cooperative groups up to
-    // kCoopFixupMaxBuckets buckets, single threads, ~1.6x slower, beyond),
-    // so L ~ sqrt(avg x their latency ratio); and at least 3 digits per
-    // resident chunk slot, where the additions start to queue on the
-    // multiply-add pipe.  Measured on GB300 (one MSM, resident bases):
-    // 2^10 points 0.65 -> 0.41 ms, 2^12 0.50 -> 0.45 ms, 2^14 0.97 -> 0.59 ms.
+    // Less than one wave of 8-digit chunks (small MSMs, where two lanes a chunk
+    // are not chosen): the accumulation takes about L dependent additions per
+    // thread and the fix-up about avg / L (the chunks a bucket spans; groups of
+    // lanes up to kCoopFixupMaxBuckets buckets, single threads, ~1.6x slower,
+    // beyond), so L ~ sqrt(avg x their latency ratio); and at least 3 digits
+    // per resident chunk slot, where the additions start to queue on the
+    // multiply-add pipe.
     const double ratio = G <= kCoopFixupMaxBuckets ? 0.8 : 1.3;
     const uint64_t by_latency = (uint64_t)std::lround(std::sqrt(avg * ratio));
     const uint64_t by_load = (3 * digits + wave - 1) / wave;
     return (uint32_t)std::min<uint64_t>(L, std::max<uint64_t>(4, std::max(by_latency, by_load)));
+}
+
+static uint32_t sm_count()
+{
+    int sms = 0;
+    GB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device()));
+    return (uint32_t)sms;
+}
+
+// Entries per pair of lanes: the accumulation takes about L dependent
+// additions of 5 us and the fix-up avg / L, so L ~ sqrt(avg); and the chunks
+// fill whole waves of resident ones, one wave unless that takes more than twice
+// that (measured, call in us for L = 3, 4, 5, 6, 8: 2^10 points, 11 entries a
+// bucket, 176* 181 186 190 197; 2^12, 20 entries, 220 220 210* 214 224; 2 x
+// 2^12 268 259 268 249* 264).
+static uint32_t pair_chunk_length(uint64_t digits, double avg)
+{
+    const uint64_t wave = (uint64_t)sm_count() * kPairSm * kPairChunks;
+    const double by_latency = std::max(3.0, std::sqrt(avg * 1.1));
+    uint64_t L = 1;
+    for (uint64_t waves = 1;; waves++) {
+        L = (digits + waves * wave - 1) / (waves * wave);
+        if ((double)L <= 2 * by_latency) break;
+    }
+    return (uint32_t)std::max<uint64_t>(L, (uint64_t)by_latency);
 }
 
 // Affine rounds of a batch: as long as a round has pairs enough to fill the
@@ -1365,6 +1635,8 @@ jacobian_t msm_tail::finish(const xyzz_t *dev) const
 
 // The host half of a batch: its descriptors and launch sizes.
 struct batch_plan {
+    bool pair = false, fix_coop = false;  // two lanes a chunk; groups of lanes in the fix-up
+    uint32_t log_parts = 0;               // log2 of the groups a bucket in it
     int c = 0, nwin = 0, variant = 1;
     bool precomputed = false, fix_by_chunk = false;
     size_t stride = 0;
@@ -1438,9 +1710,17 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     const int variant = default_acc_variant();
     const int rounds = affine_rounds(digits_total, avg, G);
     const uint64_t entries = digits_total + (uint64_t)G * ((1u << rounds) - 1);
-    const uint32_t L = chunk_length(entries >> rounds, avg / (1 << rounds), G, variant);
+    // a batch of less than 6 entries a resident thread: two lanes a chunk
+    // (measured, accumulation in us with a thread and with two lanes a chunk:
+    // 2^10 points 63 -> 25, 2^12 64 -> 44, 2 x 2^12 107 -> 72, 4 x 2^12 151 ->
+    // 129, 2^14 189 -> 149; 2 x 2^14, 8 entries a thread, 243 and 243, and 2^16
+    // 432 and 450)
+    const bool pair = variant == 1 && !rounds && digits_total < 6 * (uint64_t)sm_count() * 512;
+    const uint32_t L = pair ? pair_chunk_length(digits_total, avg)
+                            : chunk_length(entries >> rounds, avg / (1 << rounds), G, variant);
     const uint64_t nchunks = std::max<uint64_t>(1, ((entries >> rounds) + L - 1) / L);
 
+    P.pair = pair;
     P.c = c;
     P.nwin = nwin;
     P.variant = variant;
@@ -1467,7 +1747,9 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     P.points_total = points_total;
     P.digits_total = digits_total;
     P.nchunks = nchunks;
-    P.fix_by_chunk = G > kCoopFixupMaxBuckets && avg / (1 << rounds) < L;
+    P.fix_by_chunk = G > kCoopFixupSmall && avg / (1 << rounds) < L;
+    P.fix_coop = !P.fix_by_chunk && G <= kCoopFixupMaxBuckets;
+    P.log_parts = G <= 2048 ? 2 : G <= 8192 ? 1 : 0;
     // a thread adds spans of some 3 times the mean, as a longer chain holds up
     // the launch (14 us an addition)
     P.short_span = std::min<uint32_t>(kShortSpan, 6 + (uint32_t)(3.0 * avg / (1 << rounds) / L));
@@ -1528,7 +1810,7 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     const uint32_t nblocks = P.nblocks, L = P.L;
     const uint64_t points_total = P.points_total, digits_total = P.digits_total, nchunks = P.nchunks;
     dev_buf<uint32_t> digits(std::max<uint64_t>(digits_total, 1), s), sorted(std::max<uint64_t>(P.entries, 1), s);
-    dev_buf<uint32_t> hist((size_t)nblocks * K, s), counts(G, s), starts((size_t)G + 1, s);
+    dev_buf<uint32_t> hist((size_t)nblocks * K, s), counts(G, s), starts((size_t)G + 1, s), ctl(CTL_WORDS, s);
     dev_buf<xyzz_t> buckets(G, s), head(nchunks, s), tail(nchunks, s);
     dev_buf<uint32_t> open_bucket(P.fix_by_chunk ? nchunks : 0, s);
 
@@ -1538,19 +1820,20 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         launch_recode(d_items, nitems, points_total, c, digits, s);
     }
     const size_t smem = (size_t)K * 4;
-    msm_hist_kernel<<<nblocks, 1024, smem, s>>>(digits, d_segs, d_blks, K, hist);
+    msm_hist_kernel<<<nblocks, 1024, smem, s>>>(digits, d_segs, d_blks, K, hist, ctl);
     GB_CHECK_LAUNCH();
-    msm_colscan_kernel<<<blocks_for(G, 256), 256, 0, s>>>(hist, d_segs, K, G, (1u << P.rounds) - 1, counts);
+    const bool scan_here = G <= kScanHere;
+    const uint32_t col_threads = scan_here ? 1024 : 256;
+    msm_colscan_kernel<<<blocks_for(G, col_threads), col_threads, 0, s>>>(
+        hist, d_segs, K, G, (1u << P.rounds) - 1, counts, buckets, scan_here ? starts.get() : nullptr, ctl);
     GB_CHECK_LAUNCH();
     if (P.rounds) GB_CUDA_OK(cudaMemsetAsync(sorted.get(), 0xff, P.entries * sizeof(uint32_t), s));  // kNoPoint
-    u32_exclusive_scan(counts, G, starts, s);
+    if (!scan_here) u32_exclusive_scan(counts, G, starts, s);
     msm_scatter_kernel<<<nblocks, 1024, smem, s>>>(digits, d_segs, d_blks, K, precomputed ? stride : 0, hist,
                                                    starts, sorted);
     GB_CHECK_LAUNCH();
     timed_end(tok_sort, s, GB_SLOT_MSM_SORT);
     int tok = timed_begin(s);
-    // empty buckets: all zero, a point at infinity (ZZ = 0)
-    GB_CUDA_OK(cudaMemsetAsync(buckets.get(), 0, (size_t)G * sizeof(xyzz_t), s));
     if (P.fix_by_chunk) GB_CUDA_OK(cudaMemsetAsync(open_bucket.get(), 0xff, nchunks * sizeof(uint32_t), s));
     dev_buf<affine_t> list_a, list_b;
     dev_buf<uint32_t> shifted;
@@ -1563,6 +1846,9 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         bounds = shifted;
         msm_accumulate_kernel<256, 2, false><<<(unsigned)((nchunks + 255) / 256), 256, 0, s>>>(
             nullptr, bounds, G, L, nchunks, list, buckets, head, tail, open_bucket);
+    } else if (P.pair) {
+        msm_accumulate_pair_kernel<<<(unsigned)((nchunks + kPairChunks - 1) / kPairChunks), 2 * kPairChunks, 0, s>>>(
+            sorted, starts, G, L, nchunks, points, buckets, head, tail, open_bucket);
     } else if (variant == 1) {
         msm_accumulate_kernel<256, 2><<<(unsigned)((nchunks + 255) / 256), 256, 0, s>>>(
             sorted, starts, G, L, nchunks, points, buckets, head, tail, open_bucket);
@@ -1577,25 +1863,20 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     timed_end(tok, s, GB_SLOT_MSM_ACCUMULATE);
     int tok_fix = timed_begin(s);
     {
-        dev_buf<uint32_t> longs(G, s), nlong(1, s);
-        GB_CUDA_OK(cudaMemsetAsync(nlong.get(), 0, sizeof(uint32_t), s));
-        // few buckets: cooperative groups shorten the longest chain (measured
-        // on GB300: 2^12 points, 4096 buckets 0.121 -> 0.051 ms; 3 x 4096
-        // buckets 0.108 -> 0.071 ms); 2^15 buckets and more: one thread per
-        // bucket keeps more of the multiply-add pipe busy (2^16 points
-        // 0.104 -> 0.136 ms with groups)
-        if (G <= kCoopFixupMaxBuckets)
-            msm_fixup_coop_kernel<<<(G + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(bounds, G, L, head, tail,
-                                                                                     buckets, longs, nlong);
-        else {
+        dev_buf<uint32_t> longs(G, s);
+        uint32_t *nlong = ctl.get() + CTL_LONGS;
+        if (P.fix_coop) {
+            const uint32_t groups = G << P.log_parts;
+            msm_fixup_coop_kernel<<<(groups + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(
+                bounds, G, L, P.log_parts, head, tail, buckets, longs, nlong);
+        } else {
             const uint32_t n = P.fix_by_chunk ? (uint32_t)nchunks : G;
-            msm_fixup_kernel<<<blocks_for(n, 128), 128, 0, s>>>(bounds, open_bucket, n, L, P.short_span, head, tail, buckets, longs,
-                                                                nlong);
+            msm_fixup_kernel<<<blocks_for(n, 128), 128, 0, s>>>(bounds, open_bucket, n, L, P.short_span, head, tail,
+                                                                buckets, longs, nlong);
         }
         GB_CHECK_LAUNCH();
-        int sms = 0;
-        GB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device()));
-        msm_fixup_long_kernel<<<(unsigned)sms * 2, kLongGroups * kCoopLanes, kLongSmem, s>>>(bounds, L, head, tail, longs, nlong, buckets);
+        msm_fixup_long_kernel<<<sm_count() * 2, kLongGroups * kCoopLanes, kLongSmem, s>>>(bounds, L, head, tail, longs,
+                                                                                          nlong, buckets);
         GB_CHECK_LAUNCH();
     }
     timed_end(tok_fix, s, GB_SLOT_MSM_FIXUP);
@@ -1610,14 +1891,14 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     {
         const line_shape sh = P.shape;
         const uint64_t total = (uint64_t)nseg * K;
-        // 2^lm buckets a thread adds before the lines' blocks take over: none
-        // where these are few, else as many as leave the blocks little to do
-        // (one-thread additions take 14 us each but fill all lanes; measured,
-        // us for lm = 0, 1, 2, 3, 4: 4096 buckets 67* 83 106 159 269, 2^14
-        // 105* 106 124 173 282, 2^15 178 159 151* 193 302, 3 x 2^15 311 289
-        // 265* 264 323, 4 x 2^15 398 371 313 277* 334; 64 x 2^15 ms 3.23, 2.99*
-        // and 3.10 for 3, 4 and 5, and 3.45 by running sums over sub-segments)
-        const uint32_t lm = total <= (1u << 14) ? 0 : total <= 3u << 15 ? 2 : total <= 1u << 18 ? 3 : 4;
+        // 2^lm buckets a thread adds before the lines' blocks take over: none up
+        // to 2^17 buckets, beyond as many as leave the blocks little to do
+        // (one-thread additions take 14 us each, a group's 5; measured, us for
+        // lm = 0, 1, 2, 3, 4: 4096 buckets 66* 87 110 162 271, 2^14 89* 100 123
+        // 175 283, 2^15 128* 136 140 191 300, 3 x 2^15 211* 249 250 255 322, 4 x
+        // 2^15 272* 310 284 271 334; 64 x 2^15 ms 3.23, 2.99* and 3.10 for 3, 4
+        // and 5, and 3.45 by running sums over sub-segments)
+        const uint32_t lm = total <= 1u << 17 ? 0 : total <= 1u << 18 ? 3 : 4;
         dev_buf<xyzz_t> partial, lines((size_t)nseg * sh.lines(), s), bits;
         const xyzz_t *src = buckets;
         if (lm) {

@@ -527,3 +527,31 @@ def test_plain_batches_host_and_device_combination(gb, orc, count):
     got = gb.bls12_381_g1_msm_batch(bases, scal)
     for i in range(count):
         assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
+
+
+@pytest.mark.parametrize("n,count", [(1, 1), (1, 3), (33, 1), (1024, 1), (2000, 5), (4096, 4), (4096, 5), (23000, 1),
+                                     (25000, 1)])
+def test_two_lane_accumulation_special_bases(gb, orc, n, count):
+    """Small batches, on both sides of the lines for two lanes a chunk (about
+    23300 points), for the groups a bucket in the fix-up and for the scan in the
+    column kernel (16384 buckets), over bases that repeat: doublings, opposite
+    points and points at infinity inside a chunk and at its edges.  Every second
+    MSM has uniform scalars, the others three values."""
+    rng = np.random.default_rng(7 * n + count)
+    some = gb.g1_generator_mul(orc.fr_random(5, rng))
+    some[3] = 0
+    some = np.concatenate([some, some])
+    for row in some[5:]:  # the second half negated: y -> p - y
+        y = orc.P_MOD - sum(int(w) << (64 * i) for i, w in enumerate(row[6:]))
+        if any(row[6:]):
+            row[6:] = [(y >> (64 * i)) & 0xFFFFFFFFFFFFFFFF for i in range(6)]
+    bases = some[rng.integers(0, len(some), size=n)]
+    scal = orc.fr_random(n * count, rng).reshape(count, n, 4)
+    few = orc.fr_random(3, rng)
+    for i in range(1, count, 2):
+        scal[i] = few[rng.integers(0, 3, size=n)]
+    ctx = gb.Bls12_381G1MsmContext(bases)
+    got = ctx.batch(scal)
+    for i in range(count):
+        assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
+    ctx.close()
