@@ -63,11 +63,11 @@ __host__ __device__ constexpr int window_offset(int c, int j)
 // Window size for n points, measured on GB300.  With the precomputed table an
 // MSM has 2^(c - 1) buckets in all: ms a call for one and for three MSMs (*
 // chosen)
-//   2^8 points   c = 8 0.26 0.29, 11* 0.19 0.23, 13 0.22 0.28
-//   2^10         10 0.26 0.29, 11 0.23 0.27, 12* 0.22 0.28, 13 0.22 0.29
-//   2^12         11 0.32 0.39, 12 0.28 0.38, 13* 0.25 0.39, 14 0.29 0.43
-//   2^14         12 0.42 0.70, 13* 0.38 0.66, 15 0.39 0.74, 16 0.44 0.84
-//   2^16         13 0.76 1.47, 15* 0.74 1.47, 16 0.73 1.54
+//   2^8 points   c = 8 0.16 0.19, 10 0.15 0.18, 11* 0.14 0.18, 12 0.15 0.20
+//   2^10         10 0.17 0.21, 11* 0.16 0.21, 12 0.16 0.23, 13 0.17 0.24
+//   2^12         11 0.21 0.31, 12* 0.20 0.31, 13 0.20 0.31, 14 0.23 0.38
+//   2^14         12 0.31 0.63, 13* 0.30 0.61, 14 0.32 0.63, 15 0.35 0.67
+//   2^16         13 0.70 1.42, 14 0.67 1.43, 15* 0.67 1.41, 16 0.68 1.47
 //   2^17         13 1.13 2.44, 15 1.08 2.38, 16* 1.03 2.41
 // Without it every window has its own buckets:
 //   2^10 points  8* 0.46, 9 0.47, 10 0.51
@@ -78,7 +78,7 @@ __host__ __device__ constexpr int window_offset(int c, int j)
 static int choose_window(size_t n, bool precomputed)
 {
     auto upto = [&](int lg) { return n <= (size_t)1 << lg; };
-    if (precomputed) return upto(7) ? 8 : upto(9) ? 11 : upto(11) ? 12 : upto(15) ? 13 : upto(16) ? 15 : 16;
+    if (precomputed) return upto(7) ? 8 : upto(11) ? 11 : upto(12) ? 12 : upto(15) ? 13 : upto(16) ? 15 : 16;
     return upto(11) ? 8 : upto(13) ? 9 : upto(15) ? 10 : upto(17) ? 11 : upto(19) ? 12 : 13;
 }
 
