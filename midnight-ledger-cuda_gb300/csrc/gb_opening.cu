@@ -19,6 +19,19 @@ namespace gb {
 
 static constexpr int kEvalThreads = 256;
 
+// The loops around products stay loops (unroll 1): these kernels run for
+// microseconds from a cold instruction cache, and a product is 5 KB of code
+// (40 polynomials of 2^12 coefficients: 37 us unrolled, 26 as loops).
+
+// the value of the lane `off` further up in a full warp
+__device__ __forceinline__ fr_t lane_down(const fr_t &a, unsigned off)
+{
+    fr_t r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = __shfl_down_sync(0xffffffffu, a.v[i], off);
+    return r;
+}
+
 // an evaluation: len coefficients at polys, at points[row]
 struct eval_pair {
     const fr_t *polys;
@@ -29,36 +42,58 @@ struct eval_pair {
 // slices + slice] = its value at y = points[row]^(2^squarings).  Thread t runs
 // Horner's rule in y^256 over the coefficients t, t + 256, .. of the slice,
 // then the threads are folded by y^128, y^64, .. y.  A chain of 16 + per
-// dependent products and what they wait for bounds it at per = 16.
+// dependent products bounds it at per = 16, so the coefficients are read 4
+// ahead and one warp has the powers ready (40 polynomials of 2^12 coefficients
+// 48 -> 26 us, of 2^16 87 -> 45).
 __global__ void __launch_bounds__(kEvalThreads) eval_slices_kernel(const eval_pair *__restrict__ pairs, size_t len,
                                                                    const fr_t *__restrict__ points, int squarings,
                                                                    int per, uint32_t slices, fr_t *__restrict__ out)
 {
-    __shared__ fr_t sh[kEvalThreads];
+    __shared__ fr_t sh[kEvalThreads], pw[9];  // pw[s] = y^(2^s)
     const size_t p = blockIdx.y, lo = (size_t)blockIdx.x * per * kEvalThreads, t = threadIdx.x;
     const eval_pair e = pairs[p];
-    fr_t y = points[e.row];
-    for (int k = 0; k < squarings; k++) y = y.sqr();
-    fr_t pw[8];  // y^(2^s)
+    const fr_t *c = e.polys + lo + t;
+    const size_t left = lo + t < len ? len - (lo + t) : 0;
+    auto load = [&](fr_t *v, int k) {  // coefficients k .. k + 3 of the thread
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        pw[k] = y;
-        y = y.sqr();
+        for (int u = 0; u < 4; u++)
+            v[u] = (size_t)(k + u) * kEvalThreads < left ? c[(size_t)(k + u) * kEvalThreads] : fr_t::zero();
+    };
+    fr_t now[4], next[4];
+    load(now, per - 4);
+    if (t < 32) {
+        fr_t y = points[e.row];
+#pragma unroll 1
+        for (int k = 0; k < squarings; k++) y = y.sqr();
+#pragma unroll 1
+        for (int k = 0; k < 9; k++) {
+            if (t == 0) pw[k] = y;
+            if (k < 8) y = y.sqr();
+        }
     }
+    __syncthreads();
+    const fr_t y = pw[8];
     fr_t acc = fr_t::zero();
-    for (int k = per - 1; k >= 0; k--) {
-        const size_t i = lo + (size_t)k * kEvalThreads;
-        if (i >= len) continue;  // the whole block
-        acc = acc * y;
-        if (i + t < len) acc = acc + e.polys[i + t];
+    for (int k = per - 4; k >= 0; k -= 4) {
+        if (k) load(next, k - 4);
+        if (lo + (size_t)k * kEvalThreads < len) {  // the same for the block
+#pragma unroll
+            for (int u = 3; u >= 0; u--) acc = acc * y + now[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) now[u] = next[u];
     }
     sh[t] = acc;
-#pragma unroll
-    for (int k = 7; k >= 0; k--) {
+#pragma unroll 1
+    for (int k = 7; k >= 5; k--) {
         __syncthreads();
         if (t < (1u << k)) sh[t] = sh[t] + sh[t + (1u << k)] * pw[k];
     }
-    if (t == 0) out[p * slices + blockIdx.x] = sh[0];
+    if (t >= 32) return;
+    acc = sh[t];
+#pragma unroll 1
+    for (int k = 4; k >= 0; k--) acc = acc + lane_down(acc, 1u << k) * pw[k];
+    if (t == 0) out[p * slices + blockIdx.x] = acc;
 }
 
 // evaluations of pairs (pair p: len coefficients at pairs[p].polys, at the host
@@ -265,10 +300,14 @@ static void kate_divide_tiled(const kate_item *d_items, size_t count, size_t len
 static void kate_divide_items(const kate_item *d_items, size_t count, size_t len, cudaStream_t s)
 {
     if (!len || !count) return;
-    // one coefficient a thread as long as 256 tiles hold the polynomial, which
-    // is the shortest chain; above, 8, so that the scan's 8 steps cost no more
-    // than the coefficients
-    if (len <= (size_t)1 << 16) kate_divide_tiled<0>(d_items, count, len, s);
+    // a coefficient a thread is the shortest chain and most products (the scan's
+    // 12 a warp); more coefficients share the scan (measured, us a call with 1,
+    // 2, 4, 8: 2^12 coefficients 40* 40 40 40, 3 x 2^14 52 45* 58 74, 2^16 51
+    // 46* 58 74, 3 x 2^16 105 74* 82 74, 2^18 133 100 82 75*, 3 x 2^20 1060 655
+    // 561 504*)
+    const size_t total = len * count;
+    if (total <= (size_t)1 << 14) kate_divide_tiled<0>(d_items, count, len, s);
+    else if (total <= (size_t)3 << 16) kate_divide_tiled<1>(d_items, count, len, s);
     else kate_divide_tiled<3>(d_items, count, len, s);
 }
 

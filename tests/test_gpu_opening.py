@@ -79,12 +79,13 @@ def test_eval_many_matches_single_evaluations(gb, orc):
     assert (got[1][0] == want0).all()
 
 
-@pytest.mark.parametrize("ln,count", [(1, 2), (2, 1), (255, 1), (256, 3), (257, 2), (513, 1), (1 << 16, 1),
-                                      ((1 << 16) + 1, 2), (1 << 19, 1), ((1 << 19) + 1, 1), ((1 << 20) + 2049, 1)])
+@pytest.mark.parametrize("ln,count", [(1, 2), (2, 1), (255, 1), (256, 3), (257, 2), (513, 1), (1 << 14, 1),
+                                      ((1 << 14) + 1, 1), (1 << 17, 1), ((1 << 17) + 1, 1), (3 << 16, 1),
+                                      ((3 << 16) + 1, 1), (1 << 19, 1), ((1 << 19) + 1, 1), ((1 << 20) + 2049, 1)])
 @pytest.mark.parametrize("point", ["random", "zero", "one"])
 def test_kate_divide_tile_edges(gb, orc, ln, count, point):
-    """Around the block's scan (256), the change of coefficients a thread
-    (2^16) and the carry pass (above 256 tiles of 2048)."""
+    """Around the block's scan (256), the changes of coefficients a thread (2^14
+    and 3 * 2^16 in all) and the carry pass (above 256 tiles of 512 and 2048)."""
     rng = np.random.default_rng(ln + count)
     polys = orc.fr_random(ln * count, rng)
     z = orc.fr_random(1, rng)[0] if point == "random" else orc.fr_from_ints([int(point == "one")])[0]
