@@ -11,7 +11,7 @@ KZG commitments use).
   e2e   : Mpts/s through the host-buffer context entry point; every step
           copies its 32 MiB of scalars host->device and the 144-byte result back
 
-Also reported: the roofline of the dominant kernel (bucket accumulation)
+Also reported: the roofline of the dominant kernels (bucket accumulation)
 against the measured 32x32->64 multiply-add peak, the whole-MSM roofline,
 the plain (non-resident) MSM, NTT/LDE timings of the same configuration, and
 the oracle's CPU multiexp on this host as the CPU baseline.
@@ -39,10 +39,11 @@ for _p in (REPO, PKG):
 R_MOD = 0x73EDA753299D7D483339D80809A1D80553BDA402FFFE5BFEFFFFFFFF00000001
 R_LIMBS = np.array([(R_MOD >> (64 * i)) & 0xFFFFFFFFFFFFFFFF for i in range(4)], dtype=np.uint64)
 METRIC = "G1 MSM Mpts/s at 2^20"
-FP_MULS_PER_MADD = 10    # XYZZ mixed addition: 8M + 2S
+FP_MULS_PER_ENTRY = 6    # affine addition with a shared inversion: 5M + 1S (an XYZZ mixed one: 8M + 2S)
 FP_MULS_PER_ADD = 14     # XYZZ addition: 12M + 2S
 MADDS_PER_FP_MUL = 300   # 2 * 12^2 + 12 32x32->64 multiply-adds per Fp product
-ACC_DRAM_BYTES_PER_ENTRY = 801.33e6 / ((1 << 18) * 16)  # ncu, n = 2^18 launch (c = 16: 16 windows)
+MADDS_PER_TWIDDLE = 89.5  # Fr product by a prepared constant: 79 of them and 21 32-bit ones at twice the rate
+ACC_DRAM_BYTES_PER_ENTRY = 2410.0e6 / ((1 << 18) * 16)  # ncu, n = 2^18: two affine rounds, then XYZZ (c = 16)
 
 
 def fr_uniform(n, rng):
@@ -71,16 +72,16 @@ def windows(c):
 
 def f_msm(n):
     """Algorithmic Fp products of an n-point MSM with uniform scalars:
-    min over c in [8, 20] of 10 n W(c) + 14 W(c) 2^c, W(c) = floor(254/c)+1.
-    Returns (total, mixed-addition term, c)."""
-    best = None
-    for c in range(8, 21):
-        w = windows(c)
-        madd = FP_MULS_PER_MADD * n * w
-        tot = madd + FP_MULS_PER_ADD * w * (1 << c)
-        if best is None or tot < best[0]:
-            best = (tot, madd, c)
-    return best
+    min over c in [8, 20] of 6 n W(c) + 14 W(c) 2^c, W(c) = floor(254/c)+1."""
+    return min(FP_MULS_PER_ENTRY * n * windows(c) + FP_MULS_PER_ADD * windows(c) * (1 << c) for c in range(8, 21))
+
+
+def table_bits(n):
+    """The window size the resident-bases context picks for n points."""
+    for lg, c in ((7, 8), (11, 11), (12, 12), (15, 13), (16, 15)):
+        if n <= 1 << lg:
+            return c
+    return 16
 
 
 _MAX_MHZ = []
@@ -348,27 +349,27 @@ def main():
     e2e = world * n * args.steps / e2e_s / 1e6
 
     # ---- roofline
-    total_fp, madd_fp, c_star = f_msm(n)
+    total_fp, c_table = f_msm(n), table_bits(n)
     acc_avg_s = acc_ms / max(acc_n, 1) * 1e-3
     msm_avg_s = msm_ms / max(msm_n, 1) * 1e-3
-    acc_ops = madd_fp * MADDS_PER_FP_MUL
+    acc_ops = FP_MULS_PER_ENTRY * n * windows(c_table) * MADDS_PER_FP_MUL
     achieved = acc_ops / acc_avg_s / 1e12 if acc_avg_s else None
     roofline = {
         "bound": "imad", "unit": "Tmadd/s",
-        "kernel": "msm_accumulate_kernel",
+        "kernel": "msm_affine_pairs_kernel rounds and msm_accumulate_kernel (one timed span)",
         "achieved": achieved, "peak": peak / 1e12, "frac": achieved / (peak / 1e12) if achieved else None,
         "peak_source": "measured live: gb_imad_probe, the fastest of mad.wide.u32 chains and carry-chained 12-limb "
                        "rows (1, 2, 4 accumulator sets per thread) with operands that change every iteration, all SMs; "
                        "unit = one 32x32->64 product",
         "peak_forms": {"wide": probe_forms[0] / 1e12, "rows1": probe_forms[1] / 1e12,
                        "rows2": probe_forms[2] / 1e12, "rows4": probe_forms[3] / 1e12},
-        "algorithmic_per_launch": "10 Fp-mul x n x W(c*) mixed additions, c*=%d, W=%d, 300 madd per Fp-mul"
-                                  % (c_star, windows(c_star)),
+        "algorithmic_per_launch": "6 Fp-mul x n x W(c): one affine addition with a shared inversion per digit, "
+                                  "c=%d, W=%d, 300 madd per Fp-mul" % (c_table, windows(c_table)),
         "avg_launch_ms": acc_avg_s * 1e3, "launches": acc_n,
-        # DRAM bytes of one accumulate launch: the ncu capture of the n=2^18
-        # launch (dram__bytes_read.sum + dram__bytes_write.sum = 801.33 MB over
-        # 2^18 x 16 digit entries) scaled by this launch's n x W entries
-        "traffic": ACC_DRAM_BYTES_PER_ENTRY * n * windows(c_star),
+        # DRAM bytes of the span: the ncu capture of the n=2^18 launches
+        # (dram__bytes_read.sum + dram__bytes_write.sum over 2^18 x 16 digit
+        # entries) scaled by this launch's n x W entries
+        "traffic": ACC_DRAM_BYTES_PER_ENTRY * n * windows(c_table),
         "traffic_source": "ncu capture at n=2^18, scaled per digit entry",
     }
     roofline_msm = {
@@ -410,9 +411,9 @@ def main():
                                    % args.log_n,
                        "n": n, "l2": "inputs larger than L2: 2^20 x 16-window base table (1.5 GiB) and 8 "
                                      "rotating 32 MiB scalar sets", "parallelism": "replicas" if world > 1 else "1gpu",
-                       "table_bytes": n * windows(c_star) * 96,
+                       "table_bytes": n * windows(c_table) * 96,
                        "table": "the context keeps 2^(16 j) P_i for the 16 windows j (fixed-base precomputation "
-                                "over the resident SRS; every digit still costs one mixed addition); "
+                                "over the resident SRS; every digit still costs one addition); "
                                 "extra.msm_2p20_resident_no_table_ms is the same MSM without it"},
             "e2e": {"value": e2e, "unit": "Mpts/s", "h2d_bytes_per_step": n * 32, "d2h_bytes_per_step": 144},
             "gpu_launches": launches,
@@ -836,13 +837,13 @@ def extras(gb, torch, n, rng, bases, args, peak):
     dv = gb.Bls12_381FrDeviceVec.upload(polys)
     for name, inverse in (("ntt_2p20_x16_fwd_ms", False), ("ntt_2p20_x16_inv_ms", True)):
         out[name] = median_ms(torch, stream, lambda: dv.ntt_zeta_batch(log_n, count, inverse, one, one, one))
-    # (n/2) log n Fr products per transform, 136 multiply-adds each
-    ntt_madd = count * (1 << (log_n - 1)) * log_n * 136
+    # (n/2) log n Fr products by prepared twiddles per transform
+    ntt_madd = count * (1 << (log_n - 1)) * log_n * MADDS_PER_TWIDDLE
     achieved = ntt_madd / (out["ntt_2p20_x16_fwd_ms"] * 1e-3) / 1e12
     out["roofline_ntt"] = {"bound": "imad", "unit": "Tmadd/s", "kernel": "16 x NTT 2^20, all passes",
                            "achieved": achieved, "peak": peak / 1e12, "frac": achieved / (peak / 1e12),
                            "frac_issue_ceiling": achieved / issue_ceiling_tmadd(),
-                           "algorithmic": "(n/2) log2 n Fr products x 136 madd per transform"}
+                           "algorithmic": "(n/2) log2 n prepared Fr products x 89.5 madd per transform"}
     del dv
     src = gb.Bls12_381FrDeviceVec.upload(polys)
 
@@ -860,7 +861,7 @@ def extras(gb, torch, n, rng, bases, args, peak):
     out["lde_2p20_to_2p22_x16_resident_ms"] = median_ms(torch, stream, lde_zeta)
     out["lde_gen7_2p20_to_2p22_x16_resident_ms"] = median_ms(torch, stream, lde_gen)
     # butterflies (N/2) log2 N Fr products per output transform + the input factors
-    lde_madd = count * ((1 << 21) * 22) * 136
+    lde_madd = count * ((1 << 21) * 22) * MADDS_PER_TWIDDLE
     out["roofline_lde"] = {"bound": "imad", "unit": "Tmadd/s", "kernel": "16 x coset LDE 2^20 -> 2^22",
                            "achieved": lde_madd / (out["lde_2p20_to_2p22_x16_resident_ms"] * 1e-3) / 1e12,
                            "peak": peak / 1e12}

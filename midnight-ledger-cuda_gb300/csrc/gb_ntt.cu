@@ -256,9 +256,10 @@ __device__ __forceinline__ void ntt_st(uint4 *s, uint32_t t, uint32_t x, const f
 // of the former and about 140 carry additions; the prepared product
 // (gb_fr_shoup.cuh) 79 and 21 of the latter and 50 additions, for a second
 // 32-byte word per twiddle.  Measured alone on all SMs, 65.8 -> 96.8 G
-// products/s; 16 transforms of 2^20, 3.53 -> 2.34 ms with the register paths
-// of ntt_tw_piece (2.37 ms of 3.15 came from those), 8 coset extensions
-// 2^18 -> 2^20 1.80 -> 1.08 ms.
+// products/s; 16 transforms of 2^20 take 3.53 ms with Montgomery products, 3.15
+// with prepared ones, 2.37 with the register paths of ntt_tw_piece, which make
+// room for a third CTA, and 2.34 with the predicated subtraction; 8 coset
+// extensions 2^18 -> 2^20 1.80 -> 1.08 ms.
 __device__ __forceinline__ fr_t bfly_add(const fr_t &a, const fr_t &b)
 {
     fr_t r;

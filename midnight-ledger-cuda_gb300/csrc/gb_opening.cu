@@ -45,14 +45,16 @@ struct eval_pair {
 // dependent products bounds it at per = 16, so the coefficients are read 4
 // ahead and one warp has the powers ready (40 polynomials of 2^12 coefficients
 // 48 -> 26 us, of 2^16 87 -> 45).
-__global__ void __launch_bounds__(kEvalThreads) eval_slices_kernel(const eval_pair *__restrict__ pairs, size_t len,
+// Given flat, polynomial p lies at flat + p * len.
+__global__ void __launch_bounds__(kEvalThreads) eval_slices_kernel(const eval_pair *__restrict__ pairs,
+                                                                   const fr_t *__restrict__ flat, size_t len,
                                                                    const fr_t *__restrict__ points, int squarings,
                                                                    int per, uint32_t slices, fr_t *__restrict__ out)
 {
     __shared__ fr_t sh[kEvalThreads], pw[9];  // pw[s] = y^(2^s)
     const size_t p = blockIdx.y, lo = (size_t)blockIdx.x * per * kEvalThreads, t = threadIdx.x;
     const eval_pair e = pairs[p];
-    const fr_t *c = e.polys + lo + t;
+    const fr_t *c = (flat ? flat + p * len : e.polys) + lo + t;
     const size_t left = lo + t < len ? len - (lo + t) : 0;
     auto load = [&](fr_t *v, int k) {  // coefficients k .. k + 3 of the thread
 #pragma unroll
@@ -108,7 +110,8 @@ static void eval_pairs(fr_t *d_out, const std::vector<eval_pair> &pairs, const R
         throw cuda_error((int)cudaErrorInvalidValue, "too many evaluation points");
     dev_buf<fr_t> d_points(npoints, s);
     h2d(d_points, points, npoints * sizeof(fr_t), s);
-    std::vector<eval_pair> now = pairs;
+    dev_buf<eval_pair> d_pairs(total, s);
+    h2d(d_pairs, pairs.data(), total * sizeof(eval_pair), s);
     dev_buf<fr_t> values;
     // 64 coefficients a thread where that leaves two waves of blocks, which
     // spares the products of the squarings and folds; else 16, to be short
@@ -116,17 +119,15 @@ static void eval_pairs(fr_t *d_out, const std::vector<eval_pair> &pairs, const R
     for (int squarings = 0;; squarings += 8 + log_per) {
         const size_t slice = (size_t)kEvalThreads << log_per;
         const uint32_t slices = (uint32_t)((len + slice - 1) / slice);
-        dev_buf<eval_pair> d_pairs(total, s);
-        h2d(d_pairs, now.data(), total * sizeof(eval_pair), s);
         dev_buf<fr_t> next(slices > 1 ? total * slices : 0, s);
         fr_t *out = slices > 1 ? next.get() : d_out;
         for (size_t b = 0; b < total; b += chunk) {
             eval_slices_kernel<<<dim3(slices, (unsigned)std::min(chunk, total - b)), kEvalThreads, 0, s>>>(
-                d_pairs.get() + b, len, d_points, squarings, 1 << log_per, slices, out + b * slices);
+                d_pairs.get() + b, values ? values.get() + b * len : nullptr, len, d_points, squarings, 1 << log_per,
+                slices, out + b * slices);
             GB_CHECK_LAUNCH();
         }
         if (slices == 1) return;
-        for (size_t p = 0; p < total; p++) now[p].polys = out + p * slices;
         len = slices;
         values = std::move(next);
     }
