@@ -1389,32 +1389,30 @@ __global__ void __launch_bounds__(kBitGroups *kCoopLanes) msm_bit_sum_kernel(con
     if (grp == 0) coop_store(c, CO_SUM, bits + (uint64_t)seg * sh.bits() + blockIdx.x);
 }
 
-// 8d'. the bit sums of a segment to one point, a group a segment
-__global__ void __launch_bounds__(128) msm_bit_combine_kernel(const xyzz_t *__restrict__ bits, line_shape sh,
-                                                              uint32_t nseg, xyzz_t *__restrict__ seg_sum)
+// 8d'. the bit sums of a segment to one point, a block a segment: a group
+//      doubles a bit's sum up to its place, and the groups' points meet in a
+//      tree (at most 15 doublings and 4 additions in a row, where Horner's rule
+//      by one group takes as many doublings and 16 additions: a plain MSM of
+//      2^16 points, 24 segments of 2^10 buckets, reduction 205 -> 168 us)
+static constexpr uint32_t kCombineGroups = 16;
+
+__global__ void __launch_bounds__(kCombineGroups *kCoopLanes) msm_bit_combine_kernel(const xyzz_t *__restrict__ bits,
+                                                                                    line_shape sh,
+                                                                                    xyzz_t *__restrict__ seg_sum)
 {
-    __shared__ __align__(16) fp_t mem[kCoopGroups * CO_SLOTS];
+    __shared__ __align__(16) fp_t mem[kCombineGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
     const coop_t c(mem);
-    const uint32_t seg = blockIdx.x * kCoopGroups + grp;
-    if (seg >= nseg) return;  // whole groups leave together; no block barrier follows
-    const xyzz_t *p = bits + (uint64_t)seg * sh.bits();
-    coop_set_inf(c, CO_SUM);
-    for (int b = (int)(sh.lr + sh.lc); b >= 0; b--) {
-        coop_dbl(c, CO_SUM);
-        if (b >= (int)sh.lc && b < (int)(sh.lr + sh.lc)) {
-            c.sync();
-            coop_load(c, CO_OPD, p + b - sh.lc);
-            coop_add(c, CO_SUM, CO_OPD);
-        }
-        if (b <= (int)sh.lc) {
-            c.sync();
-            coop_load(c, CO_OPD, p + sh.lr + b);
-            coop_add(c, CO_SUM, CO_OPD);
-        }
+    const xyzz_t *p = bits + (uint64_t)blockIdx.x * sh.bits();
+    if (grp < sh.bits()) {
+        coop_load(c, CO_SUM, p + grp);
+        const uint32_t place = grp < sh.lr ? sh.lc + grp : grp - sh.lr;
+        for (uint32_t k = 0; k < place; k++) coop_dbl(c, CO_SUM);
+    } else {
+        coop_set_inf(c, CO_SUM);
     }
-    c.sync();
-    coop_store(c, CO_SUM, seg_sum + seg);
+    coop_block_tree<kCombineGroups>(mem, c, grp);
+    if (grp == 0) coop_store(c, CO_SUM, seg_sum + blockIdx.x);
 }
 
 // 8e. plain MSMs beyond a few: combine an MSM's window segments by Horner's
@@ -1586,9 +1584,11 @@ static int affine_rounds(uint64_t digits, double avg, uint32_t G)
 // one point; the bit sums of its buckets (a context's MSM); or its window
 // sums (a plain MSM).  The last two are one chain of dependent doublings and
 // additions, which a host core runs 7 times faster than a group of GPU lanes
-// (about 25 us for 16 bit sums, 0.2 ms for 20 windows, against 0.13 and
-// 1.1 ms); the GPU runs them for batches of more than a few MSMs.
-static constexpr uint32_t kHostTailBits = 8, kHostTailWindows = 4;  // MSMs at most
+// (about 25 us for 16 bit sums, 0.15 to 0.2 ms for 20 windows, against 0.13
+// and 1.1 ms); the GPU runs them for batches of more than a few MSMs (plain,
+// 2^16 points, ms finished by the host and by the GPU: 5 3.82 4.00, 6 4.50
+// 4.53, 7 5.25 5.14).
+static constexpr uint32_t kHostTailBits = 8, kHostTailWindows = 6;  // MSMs at most
 
 struct msm_tail {
     enum { POINT, BITS, WINDOWS } kind = POINT;
@@ -1918,7 +1918,7 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         msm_bit_sum_kernel<<<dim3(sh.bits(), nseg), kBitGroups * kCoopLanes, 0, s>>>(lines, sh, bit_sum);
         GB_CHECK_LAUNCH();
         if (P.tail.kind != msm_tail::BITS) {
-            msm_bit_combine_kernel<<<(nseg + kCoopGroups - 1) / kCoopGroups, 128, 0, s>>>(bits, sh, nseg, seg_sum);
+            msm_bit_combine_kernel<<<nseg, kCombineGroups * kCoopLanes, 0, s>>>(bits, sh, seg_sum);
             GB_CHECK_LAUNCH();
         }
     }

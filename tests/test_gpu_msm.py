@@ -516,7 +516,7 @@ def test_reduction_forms(gb, orc, bits, count):
     ctx.close()
 
 
-@pytest.mark.parametrize("count", [1, 4, 5])
+@pytest.mark.parametrize("count", [1, 4, 5, 6, 7])
 def test_plain_batches_host_and_device_combination(gb, orc, count):
     """Plain batches on both sides of the line where the windows' Horner chain
     moves from the host to the device."""
