@@ -1344,7 +1344,8 @@ __global__ void __launch_bounds__(128) msm_line_sum_kernel(const xyzz_t *__restr
     __shared__ __align__(16) fp_t mem[kCoopGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
     const coop_t c(mem);
-    const uint32_t lk = sh.lr + sh.lc, rows = 1u << sh.lr, line = blockIdx.x, seg = blockIdx.y;
+    const uint32_t lk = sh.lr + sh.lc, rows = 1u << sh.lr;
+    const uint32_t seg = blockIdx.x / sh.lines(), line = blockIdx.x % sh.lines();
     const bool row = line < rows;
     const uint32_t n = 1u << ((row ? sh.lc : sh.lr) - lm);
     const xyzz_t *p = src + ((uint64_t)seg << (lm ? lk + 1 - lm : lk));
@@ -1359,7 +1360,7 @@ __global__ void __launch_bounds__(128) msm_line_sum_kernel(const xyzz_t *__restr
         coop_add(c, CO_SUM, CO_OPD);
     }
     coop_block_tree<kCoopGroups>(mem, c, grp);
-    if (grp == 0) coop_store(c, CO_SUM, lines + (uint64_t)seg * sh.lines() + line);
+    if (grp == 0) coop_store(c, CO_SUM, lines + blockIdx.x);
 }
 
 // 8c'. the sums by weight bit, a block a bit: rows weigh i (bits 0 .. lr - 1,
@@ -1372,9 +1373,9 @@ __global__ void __launch_bounds__(kBitGroups *kCoopLanes) msm_bit_sum_kernel(con
     __shared__ __align__(16) fp_t mem[kBitGroups * CO_SLOTS];
     const uint32_t grp = threadIdx.x / kCoopLanes;
     const coop_t c(mem);
-    const uint32_t seg = blockIdx.y, rows = 1u << sh.lr;
-    const bool row = blockIdx.x < sh.lr;
-    const uint32_t b = row ? blockIdx.x : blockIdx.x - sh.lr, lw = row ? sh.lr : sh.lc;
+    const uint32_t seg = blockIdx.x / sh.bits(), place = blockIdx.x % sh.bits(), rows = 1u << sh.lr;
+    const bool row = place < sh.lr;
+    const uint32_t b = row ? place : place - sh.lr, lw = row ? sh.lr : sh.lc;
     const xyzz_t *p = lines + (uint64_t)seg * sh.lines() + (row ? 0 : rows);
     // weights below 2^lw with bit b, or 2^lc itself for the columns' last bit
     const uint32_t n = b < lw ? 1u << (lw - 1) : 1u;
@@ -1386,7 +1387,7 @@ __global__ void __launch_bounds__(kBitGroups *kCoopLanes) msm_bit_sum_kernel(con
         coop_add(c, CO_SUM, CO_OPD);
     }
     coop_block_tree<kBitGroups>(mem, c, grp);
-    if (grp == 0) coop_store(c, CO_SUM, bits + (uint64_t)seg * sh.bits() + blockIdx.x);
+    if (grp == 0) coop_store(c, CO_SUM, bits + blockIdx.x);
 }
 
 // 8d'. the bit sums of a segment to one point, a block a segment: a group
@@ -1892,13 +1893,14 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
         const line_shape sh = P.shape;
         const uint64_t total = (uint64_t)nseg * K;
         // 2^lm buckets a thread adds before the lines' blocks take over: none up
-        // to 2^17 buckets, beyond as many as leave the blocks little to do
-        // (one-thread additions take 14 us each, a group's 5; measured, us for
-        // lm = 0, 1, 2, 3, 4: 4096 buckets 66* 87 110 162 271, 2^14 89* 100 123
-        // 175 283, 2^15 128* 136 140 191 300, 3 x 2^15 211* 249 250 255 322, 4 x
-        // 2^15 272* 310 284 271 334; 64 x 2^15 ms 3.23, 2.99* and 3.10 for 3, 4
-        // and 5, and 3.45 by running sums over sub-segments)
-        const uint32_t lm = total <= 1u << 17 ? 0 : total <= 1u << 18 ? 3 : 4;
+        // to 2^20 buckets, where chains are what costs (one-thread additions
+        // take 14 us each, a group's 5), and 16 beyond, where a thread's 14
+        // products an addition beat a group's 16 slots (measured, us for lm =
+        // 0, 1, 2, 3, 4: 4096 buckets 66* 87 110 162 271, 2^15 128* 136 140 191
+        // 300, 4 x 2^15 272* 310 284 271 334, 8 x 2^15 428* 505 487 461 442, 12
+        // x 2^15 669* 792 751 730 844; 64 x 2^15 ms 2.89 3.53 3.21 3.04 2.88*);
+        // but no more than a column has (8 with windows of 8 bits).
+        const uint32_t lm = total <= 1u << 20 ? 0 : std::min(4u, sh.lr);
         dev_buf<xyzz_t> partial, lines((size_t)nseg * sh.lines(), s), bits;
         const xyzz_t *src = buckets;
         if (lm) {
@@ -1908,14 +1910,14 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
             GB_CHECK_LAUNCH();
             src = partial;
         }
-        msm_line_sum_kernel<<<dim3(sh.lines(), nseg), 128, 0, s>>>(src, sh, lm, lines);
+        msm_line_sum_kernel<<<sh.lines() * nseg, 128, 0, s>>>(src, sh, lm, lines);
         GB_CHECK_LAUNCH();
         xyzz_t *bit_sum = d_out;
         if (P.tail.kind != msm_tail::BITS) {
             bits = dev_buf<xyzz_t>((size_t)nseg * sh.bits(), s);
             bit_sum = bits;
         }
-        msm_bit_sum_kernel<<<dim3(sh.bits(), nseg), kBitGroups * kCoopLanes, 0, s>>>(lines, sh, bit_sum);
+        msm_bit_sum_kernel<<<sh.bits() * nseg, kBitGroups * kCoopLanes, 0, s>>>(lines, sh, bit_sum);
         GB_CHECK_LAUNCH();
         if (P.tail.kind != msm_tail::BITS) {
             msm_bit_combine_kernel<<<nseg, kCombineGroups * kCoopLanes, 0, s>>>(bits, sh, seg_sum);

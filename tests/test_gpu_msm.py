@@ -555,3 +555,16 @@ def test_two_lane_accumulation_special_bases(gb, orc, n, count):
     for i in range(count):
         assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
     ctx.close()
+
+
+@pytest.mark.parametrize("n,count", [(40, 250), (40, 260), (2049, 145), (3, 2100)])
+def test_plain_batches_of_many_buckets(gb, orc, n, count):
+    """Below and above the 2^20 buckets from which threads add buckets before
+    the line sums, with windows of 8 bits (8 rows of 16 buckets) and of 9, and
+    more than 65535 segments."""
+    rng = np.random.default_rng(n + count)
+    bases = gb.g1_generator_mul(orc.fr_random(n, rng))
+    scal = orc.fr_random(n * count, rng).reshape(count, n, 4)
+    got = gb.bls12_381_g1_msm_batch(bases, scal)
+    for i in list(range(0, count, 24)) + [count - 1]:
+        assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
