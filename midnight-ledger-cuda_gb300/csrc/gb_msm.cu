@@ -1561,21 +1561,28 @@ static uint32_t pair_chunk_length(uint64_t digits, double avg)
 
 // Affine rounds of a batch: as long as a round has pairs enough to fill the
 // GPU (a round costs about 55 us whatever its size: product trees and one
-// inversion a block), and buckets 3 entries or longer remain, as every bucket
-// is padded to a multiple of 2^rounds.  Measured on GB300, ms a call without
-// rounds and with 1, 2, 3, 4 (* chosen):
-//   1 x 2^16 points  0.86*  0.87   0.87   0.95   1.01
-//   2 x 2^16         1.31   1.26*  1.31   1.35   1.52
-//   3 x 2^16         1.89   1.78   1.74*  1.84   1.99
-//   2^17             1.21   1.16*  1.19   1.19   1.31
-//   2^18             1.94   1.79   1.71*  1.76   1.80
-//   2^20             6.33   5.66   5.25   5.05   5.00*
-//   64 uneven ones  19.4   18.4   17.9   17.5*  19.4
+// inversion a block) and buckets are long enough, as every bucket is padded to
+// a multiple of 2^rounds.  Measured on GB300, entries and entries a bucket, and
+// ms a call without rounds and with 1, 2, 3, 4 (* chosen):
+//    1.0 M   80   0.61*  0.68   0.65
+//    1.2 M   72   0.68   0.66*  0.66   0.74   0.79
+//    2.0 M   80   1.04   0.99*  1.05
+//    2.4 M   72   1.14   1.07   1.04*  1.08   1.20
+//    4.7 M   72   2.07   1.84   1.77*  1.82   2.01
+//    5.9 M   72                 2.20   2.19*  2.35
+//   12.6 M  128   4.95   4.41   4.15   4.10*  4.16
+//   16.8 M  128                 5.41   5.28*  5.37
+//   16.8 M  512                 5.08   4.88   4.83*
+//    4.2 M  7.8          2.48*  2.66   3.07   3.45
+//    6.3 M   12          3.21   3.12*  3.59   4.01
+//    7.2 M   27          3.25   3.06*  3.12   3.51
+//   48 M     23         14.78  14.36* 14.94  17.18
 static int affine_rounds(uint64_t digits, double avg, uint32_t G)
 {
-    const uint64_t least = 3u << 18;
+    static constexpr uint64_t pairs[4] = {9 << 16, 9 << 16, 11 << 16, 1 << 20};
+    static constexpr double bucket[4] = {6, 11, 40, 192};
     int r = 0;
-    while (r < 4 && digits >> (r + 1) >= least && avg >= 3.0 * (2 << r) &&
+    while (r < 4 && digits >> (r + 1) >= pairs[r] && avg >= bucket[r] &&
            digits + (uint64_t)G * ((2u << r) - 1) < 0x80000000ull)
         r++;
     return r;

@@ -469,7 +469,7 @@ def test_async_batch_reads_scalars_as_queued(gb, orc):
     ctx.close()
 
 
-@pytest.mark.parametrize("n,count", [(1 << 16, 2), (65537, 3), (1 << 17, 3), (99991, 1)])
+@pytest.mark.parametrize("n,count", [(1 << 16, 1), (1 << 16, 2), (65537, 3), (1 << 17, 3), (99991, 1)])
 def test_affine_rounds_special_pairs(gb, orc, n, count):
     """Batches long enough for 1 to 3 affine rounds over bases that repeat:
     equal points (doublings), opposite points (sums at infinity) and points
