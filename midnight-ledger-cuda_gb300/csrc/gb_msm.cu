@@ -2179,7 +2179,7 @@ static int plan_window(size_t n, bool precomputed, uint32_t requested)
 // Autotuner for the plain path: the key is the size class of the largest
 // item, the batch-size class and the sparsity of a sample of the scalars
 // (zero scalars, scalars below 2^64: both empty the high windows); a new key
-// times every window size with a populated top window on this batch.
+// times the cost model's window and a few others on this batch.
 __global__ void scalar_sample_kernel(const fr_t *__restrict__ scalars, size_t n, unsigned *counts)
 {
     unsigned zero = 0, small = 0;
@@ -2225,7 +2225,9 @@ static int tuned_window(const std::vector<msm_item> &items, const affine_t *poin
                             std::to_string(cls(h[0])) + ":s" + std::to_string(cls(h[1]));
     if (autotune_lookup(key, &c)) return c;
     float best = 1e30f;
-    for (int cand : {8, 10, 13, 16}) {
+    const int model = c;
+    for (int cand : {model, 8, 10, 13, 16}) {
+        if (cand == model && best < 1e30f) continue;  // timed first
         if (cand > kMaxWindowBits || ((size_t)1 << (cand - 1)) > 8 * total) continue;
         float ms = time_on_stream(s, [&] { msm_run_batch(items, cand, false, points, stride, s); });
         if (ms < best) {
