@@ -1207,7 +1207,8 @@ __device__ void coop_block_tree(fp_t *sh, const coop_t &c, uint32_t grp)
 //     82); several groups a bucket where there are few (2^10 points 51 -> 32
 //     us with 4, 2^12 53 -> 41 with 2).
 __global__ void __launch_bounds__(128) msm_fixup_coop_kernel(const uint32_t *__restrict__ starts, uint32_t G,
-                                                             uint32_t L, uint32_t log_parts, const xyzz_t *__restrict__ head,
+                                                             uint32_t L, uint32_t log_parts,
+                                                             const xyzz_t *__restrict__ head,
                                                              const xyzz_t *__restrict__ tail,
                                                              xyzz_t *__restrict__ buckets,
                                                              uint32_t *__restrict__ longs,
@@ -1800,7 +1801,8 @@ static const affine_t *run_affine_rounds(const batch_plan &P, const uint32_t *so
         if (r == 1)
             msm_affine_pairs_kernel<true><<<grid, kPairThreads, 0, s>>>(sorted, in, out, starts + P.G, r, per, prefix);
         else
-            msm_affine_pairs_kernel<false><<<grid, kPairThreads, 0, s>>>(nullptr, in, out, starts + P.G, r, per, prefix);
+            msm_affine_pairs_kernel<false><<<grid, kPairThreads, 0, s>>>(nullptr, in, out, starts + P.G, r, per,
+                                                                         prefix);
         GB_CHECK_LAUNCH();
         in = out;
     }
@@ -2028,7 +2030,8 @@ static bool run_planned_graph(const batch_plan &P, const affine_t *points, xyzz_
     key.c = P.c, key.variant = P.variant, key.precomputed = P.precomputed, key.fix_by_chunk = P.fix_by_chunk;
     key.stride = P.stride, key.nitems = P.nitems, key.K = P.K, key.segs_per_item = P.segs_per_item;
     key.nseg = P.nseg, key.G = P.G, key.nblocks = P.nblocks, key.L = P.L, key.short_span = P.short_span;
-    key.points_total = P.points_total, key.digits_total = P.digits_total, key.nchunks = P.nchunks, key.rounds = P.rounds;
+    key.points_total = P.points_total, key.digits_total = P.digits_total, key.nchunks = P.nchunks;
+    key.rounds = P.rounds;
 
     // a stream the caller is capturing gets the launches themselves
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;

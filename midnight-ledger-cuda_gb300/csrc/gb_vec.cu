@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kScanThreads) grand_product_kernel(const fr_t 
 // last unblinded value of the one before
 template <int PER, class F>
 static void grand_products_tiled(fr_t *out, const F &f, size_t len, size_t sets, bool chained, const fr_t *d_blinds,
-                           size_t bf, cudaStream_t s)
+                                 size_t bf, cudaStream_t s)
 {
     const size_t tile = (size_t)kScanThreads * PER, tiles = (len + tile - 1) / tile;
     if (tiles > 0x7fffffff) throw cuda_error((int)cudaErrorInvalidValue, "grand product too large");
