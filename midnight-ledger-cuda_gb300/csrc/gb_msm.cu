@@ -1467,12 +1467,12 @@ __global__ void add_mask_kernel(fr_t *__restrict__ out, const fr_t *__restrict__
 
 static void set_smem_attrs()
 {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        int bytes = (1 << (kMaxWindowBits - 1)) * 4;
-        cudaFuncSetAttribute(msm_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(msm_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(msm_fixup_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLongSmem);
+    static device_once once;
+    once.run(current_device(), [] {
+        const size_t bytes = ((size_t)1 << (kMaxWindowBits - 1)) * 4;
+        allow_dynamic_smem(msm_hist_kernel, bytes);
+        allow_dynamic_smem(msm_scatter_kernel, bytes);
+        allow_dynamic_smem(msm_fixup_long_kernel, kLongSmem);
     });
 }
 
@@ -1501,17 +1501,17 @@ static void u32_exclusive_scan(const uint32_t *in, uint32_t n, uint32_t *out, cu
 static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int variant)
 {
     uint32_t L = (uint32_t)std::max(8.0, std::min(64.0, avg * 0.5));
-    static int per_sm[3] = {0, 0, 0}, sms = 0;
-    const int v = variant < 0 || variant > 2 ? 1 : variant;
-    if (!per_sm[v]) {
-        int dev = current_device(), b = 0;
-        GB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        if (v == 1) GB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, msm_accumulate_kernel<256, 2>, 256, 0));
-        else if (v == 2) GB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, msm_accumulate_kernel<128, 3>, 128, 0));
-        else GB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, msm_accumulate_kernel<256, 1>, 256, 0));
-        per_sm[v] = std::max(1, b) * (v == 2 ? 128 : 256);
-    }
-    const uint64_t wave = (uint64_t)sms * (uint64_t)per_sm[v];  // chunks resident at once
+    static device_once once;
+    static int per_sm[kMaxDevices][3];
+    const int v = variant < 0 || variant > 2 ? 1 : variant, dev = current_device();
+    once.run(dev, [&] {
+        int b[3];
+        GB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[0], msm_accumulate_kernel<256, 1>, 256, 0));
+        GB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[1], msm_accumulate_kernel<256, 2>, 256, 0));
+        GB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[2], msm_accumulate_kernel<128, 3>, 128, 0));
+        for (int k = 0; k < 3; k++) per_sm[dev][k] = std::max(1, b[k]) * (k == 2 ? 128 : 256);
+    });
+    const uint64_t wave = (uint64_t)sm_count() * (uint64_t)per_sm[dev][v];  // chunks resident at once
     // short buckets, large batches: chunks long enough for 8 waves, as every
     // chunk's edge costs a fix-up
     if (wave) L = std::max<uint32_t>(L, (uint32_t)std::min<uint64_t>(64, digits / (8 * wave)));
@@ -1533,13 +1533,6 @@ static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int varian
     const uint64_t by_latency = (uint64_t)std::lround(std::sqrt(avg * ratio));
     const uint64_t by_load = (3 * digits + wave - 1) / wave;
     return (uint32_t)std::min<uint64_t>(L, std::max<uint64_t>(4, std::max(by_latency, by_load)));
-}
-
-static uint32_t sm_count()
-{
-    int sms = 0;
-    GB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device()));
-    return (uint32_t)sms;
 }
 
 // Entries per pair of lanes: the accumulation takes about L dependent
@@ -1779,9 +1772,7 @@ static const affine_t *run_affine_rounds(const batch_plan &P, const uint32_t *so
                                          const affine_t *points, dev_buf<affine_t> &list_a,
                                          dev_buf<affine_t> &list_b, cudaStream_t s)
 {
-    int sms = 0;
-    GB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device()));
-    const uint64_t slots = (uint64_t)sms * kPairBlocks;
+    const uint64_t slots = (uint64_t)sm_count() * kPairBlocks;
     // pairs a thread: whole waves of tiles of at most 16 a thread
     auto per_thread = [&](uint64_t pairs) {
         const uint64_t per = std::max<uint64_t>(1, (pairs + slots * kPairThreads - 1) / (slots * kPairThreads));

@@ -1068,32 +1068,20 @@ const fr_t *twiddles(uint32_t log_n, bool inverse, cudaStream_t s)
 
 void set_ntt_smem()
 {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        cudaFuncSetAttribute(ntt_dif_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (1 << kPassBits) * (int)sizeof(fr_t));
-        cudaFuncSetAttribute(ntt_dif_pass_reg_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (1 << kPassBits) / 8 * 9 * (int)sizeof(fr_t));
-        cudaFuncSetAttribute(ntt_dif_pass_reg_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (1 << kPassBits) / 8 * 9 * (int)sizeof(fr_t));
-        const int staged = 2 * (1 << kPassBits) * (int)sizeof(fr_t);
-        cudaFuncSetAttribute(ntt_dif_pass_tw_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged);
-        cudaFuncSetAttribute(ntt_dif_pass_tw_kernel<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged);
-        cudaFuncSetAttribute(ntt_dif_pass_tw_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged);
-        cudaFuncSetAttribute(ntt_dif_pass_tw_kernel<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged);
-        cudaFuncSetAttribute(ntt_dif_pass_tw_kernel<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             staged);
-        cudaFuncSetAttribute(ntt_dif_pass_tw_kernel<3, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             staged);
-        cudaFuncSetAttribute(ntt_queue_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, staged);
+    static device_once once;
+    once.run(current_device(), [] {
+        allow_dynamic_smem(ntt_dif_pass_kernel, (1 << kPassBits) * sizeof(fr_t));
+        allow_dynamic_smem(ntt_dif_pass_reg_kernel<2>, (1 << kPassBits) / 8 * 9 * sizeof(fr_t));
+        allow_dynamic_smem(ntt_dif_pass_reg_kernel<3>, (1 << kPassBits) / 8 * 9 * sizeof(fr_t));
+        const size_t staged = 2 * (1 << kPassBits) * sizeof(fr_t);
+        allow_dynamic_smem(ntt_dif_pass_tw_kernel<2, false>, staged);
+        allow_dynamic_smem(ntt_dif_pass_tw_kernel<3, false>, staged);
+        allow_dynamic_smem(ntt_dif_pass_tw_kernel<2, true>, staged);
+        allow_dynamic_smem(ntt_dif_pass_tw_kernel<3, true>, staged);
+        allow_dynamic_smem(ntt_dif_pass_tw_kernel<2, false, true>, staged);
+        allow_dynamic_smem(ntt_dif_pass_tw_kernel<3, false, true>, staged);
+        allow_dynamic_smem(ntt_queue_kernel<2>, staged);
     });
-}
-
-static int sm_count()
-{
-    static int n = 0;
-    if (!n) GB_CUDA_OK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, current_device()));
-    return n;
 }
 
 // (s_hi, g) of each pass: ceil(log_n / 10) passes of near-equal size, the

@@ -10,7 +10,6 @@
 // per-thread local array sized to the graph.
 #include <algorithm>
 #include <functional>
-#include <mutex>
 #include <memory>
 #include <vector>
 
@@ -556,11 +555,11 @@ static uint32_t slots_for(uint32_t acc, const dgraph &g)
 
 static void set_slot_smem()
 {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        const int bytes = (int)(kNumThreads * kMaxSlots * sizeof(fr_t));
-        cudaFuncSetAttribute(numerator_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(graph_batch_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    static device_once once;
+    once.run(current_device(), [] {
+        const size_t bytes = kNumThreads * kMaxSlots * sizeof(fr_t);
+        allow_dynamic_smem(numerator_kernel<16, true>, bytes);
+        allow_dynamic_smem(graph_batch_kernel<16, true>, bytes);
     });
 }
 

@@ -27,8 +27,16 @@ int current_device()
     return d;
 }
 
+int sm_count()
+{
+    static device_once once;
+    static int sms[kMaxDevices];
+    const int dev = current_device();
+    once.run(dev, [&] { GB_CUDA_OK(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev)); });
+    return sms[dev];
+}
+
 namespace {
-constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
 cudaStream_t g_streams[kMaxDevices][GB_MAX_LANES + 1];
 // lane status words: host view and device view of 2 words per lane

@@ -20,6 +20,7 @@
 #include <string>
 
 #include "gb_curve.cuh"
+#include "gb_device_once.h"
 #include "gb_prover.h"
 
 namespace gb {
@@ -93,6 +94,7 @@ void set_lane(uint32_t lane);
 // The calling thread's lane stream on the current device (created lazily).
 cudaStream_t lane_stream();
 int current_device();
+int sm_count();  // of the current device
 
 // Status words of the bounded device waits (NTT twiddle copies, work-queue
 // dependencies), two per (device, lane), in mapped page-locked host memory:
@@ -208,6 +210,13 @@ float time_on_stream(cudaStream_t s, F fn)
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     return ms;
+}
+
+// the dynamic shared memory a kernel may ask for on the current device
+template <class K>
+void allow_dynamic_smem(K *kernel, size_t bytes)
+{
+    GB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
 inline unsigned blocks_for(size_t n, unsigned threads)
