@@ -566,6 +566,9 @@ GB_API RustError gb_ntt_wait_timeouts(uint32_t *out);
  * up at once and the error is reported as above, while the copy still lands
  * in a second, longer wait before the CTA moves on) */
 GB_API void gb_ntt_wait_limit_set(int64_t spins);
+/* test hook: device allocations of more than `bytes` fail as on a full device
+ * (cudaErrorMemoryAllocation), process-wide; 0 = none do (the default) */
+GB_API void gb_alloc_limit_set(size_t bytes);
 /* ---- coset by the powers of a shift: sppark's coset NTT and LDE form
  * (vendor/sppark-0.1.15/sppark/ntt/ntt.cuh:78-97,196-209,283-342; kernels.cu
  * LDE_distribute_powers / LDE_spread_distribute_powers), which the

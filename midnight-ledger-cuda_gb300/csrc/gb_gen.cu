@@ -82,10 +82,8 @@ const affine_t *generator_table(cudaStream_t s)
     int dev = current_device();
     std::lock_guard<std::mutex> lk(g_gen_mu);
     if (g_gen_table[dev]) return g_gen_table[dev];
-    affine_t *table = nullptr;
-    xyzz_t *bases = nullptr;
-    GB_CUDA_OK(cudaMalloc(&table, 32 * 256 * sizeof(affine_t)));
-    GB_CUDA_OK(cudaMalloc(&bases, 32 * sizeof(xyzz_t)));
+    affine_t *table = (affine_t *)dev_malloc(32 * 256 * sizeof(affine_t));
+    xyzz_t *bases = (xyzz_t *)dev_malloc(32 * sizeof(xyzz_t));
     gen_table_bases_kernel<<<1, 32, 0, s>>>(host_generator_canonical(), bases);
     GB_CHECK_LAUNCH();
     gen_table_fill_kernel<<<32, 256, 0, s>>>(bases, table);

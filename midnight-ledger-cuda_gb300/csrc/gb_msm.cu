@@ -2476,7 +2476,7 @@ RustError midnight_sppark_bls12_381_g1_msm_context_create_with_config(void **out
     try {
         size_t total = npoints * (size_t)ctx->nwin;
         if (total) {
-            GB_CUDA_OK(cudaMalloc(&ctx->table, total * sizeof(affine_t)));
+            ctx->table = (affine_t *)dev_malloc(total * sizeof(affine_t));
             h2d(ctx->table, points, npoints * sizeof(affine_t), s);
             msm_precompute_kernel<<<blocks_for(npoints, 128), 128, 0, s>>>(ctx->table, npoints, ctx->c,
                                                                            ctx->nwin);

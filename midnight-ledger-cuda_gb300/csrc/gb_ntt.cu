@@ -1057,8 +1057,7 @@ const fr_t *twiddles(uint32_t log_n, bool inverse, cudaStream_t s)
     auto it = g_tw.find(key);
     if (it != g_tw.end()) return it->second;
     size_t half = log_n ? ((size_t)1 << (log_n - 1)) : 1;
-    fr_t *tw = nullptr;
-    GB_CUDA_OK(cudaMalloc(&tw, half * sizeof(fr_t)));
+    fr_t *tw = (fr_t *)dev_malloc(half * sizeof(fr_t));
     twiddle_kernel<<<blocks_for(half, 256), 256, 0, s>>>(tw, half, host_omega(log_n, inverse));
     GB_CHECK_LAUNCH();
     GB_CUDA_OK(cudaStreamSynchronize(s));
@@ -1112,8 +1111,7 @@ const fr_t *pass_twiddles(uint32_t log_n, bool inverse, int s_hi, int g, const f
     const int s_lo = s_hi - g + 1;
     const size_t chunks = s_lo > 0 ? (size_t)1 << s_lo : 1;
     const size_t entries = chunks << g;
-    fr_t *t = nullptr;
-    GB_CUDA_OK(cudaMalloc(&t, 2 * entries * sizeof(fr_t)));
+    fr_t *t = (fr_t *)dev_malloc(2 * entries * sizeof(fr_t));
     pass_twiddle_kernel<<<blocks_for(entries, 256), 256, 0, s>>>(t, tw, log_n, s_lo, g, chunks);
     GB_CHECK_LAUNCH();
     GB_CUDA_OK(cudaStreamSynchronize(s));
@@ -1428,9 +1426,7 @@ static ntt_factors power_factors(const fr_t &shift, const fr_t &scale, size_t le
     std::lock_guard<std::mutex> lk(g_pw_mu);
     auto it = g_pw.find(key);
     if (it == g_pw.end()) {
-        fr_t *lo = nullptr, *hi = nullptr;
-        GB_CUDA_OK(cudaMalloc(&lo, n_lo * sizeof(fr_t)));
-        GB_CUDA_OK(cudaMalloc(&hi, n_hi * sizeof(fr_t)));
+        fr_t *lo = (fr_t *)dev_malloc(n_lo * sizeof(fr_t)), *hi = (fr_t *)dev_malloc(n_hi * sizeof(fr_t));
         fr_t step = shift;  // shift^(2^lo_bits)
         for (uint32_t b = 0; b < lo_bits; b++) step = step.sqr();
         powers_table_kernel<<<blocks_for(n_lo, 256), 256, 0, s>>>(lo, shift, fr_t::one(), n_lo);

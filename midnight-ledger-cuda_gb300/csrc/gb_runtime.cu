@@ -121,11 +121,44 @@ void lane_sync(cudaStream_t s)
 
 unsigned long long lane_timeouts_take() { return g_timeouts.exchange(0); }
 
+static std::atomic<size_t> g_alloc_limit{0};  // 0: none
+
+bool alloc_refused(size_t bytes)
+{
+    const size_t limit = g_alloc_limit.load(std::memory_order_relaxed);
+    return limit && bytes > limit;
+}
+
+// alloc() once, and again when the idle memory of the device's graphs is back
+template <class F>
+static void alloc_or_trim(size_t bytes, F alloc)
+{
+    cudaError_t e = alloc_refused(bytes) ? cudaErrorMemoryAllocation : alloc();
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        if (cudaDeviceGraphMemTrim(current_device()) != cudaSuccess) (void)cudaGetLastError();
+        if (!alloc_refused(bytes)) e = alloc();
+    }
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        throw cuda_error((int)e, "allocating " + std::to_string(bytes) + " bytes on the device failed: " +
+                                     cudaGetErrorString(e));
+    }
+}
+
 void *dev_alloc(size_t bytes, cudaStream_t s)
 {
     void *p = nullptr;
     if (bytes == 0) return nullptr;
-    GB_CUDA_OK(cudaMallocAsync(&p, bytes, s));
+    alloc_or_trim(bytes, [&] { return cudaMallocAsync(&p, bytes, s); });
+    return p;
+}
+
+void *dev_malloc(size_t bytes)
+{
+    void *p = nullptr;
+    if (bytes == 0) return nullptr;
+    alloc_or_trim(bytes, [&] { return cudaMalloc(&p, bytes); });
     return p;
 }
 
@@ -354,6 +387,10 @@ void gb_transfer_counters_reset(void)
     g_h2d.store(0);
     g_d2h.store(0);
 }
+
+// Test hook: device allocations of more than `bytes` fail as on a full device
+// (0: none do).
+void gb_alloc_limit_set(size_t bytes) { g_alloc_limit.store(bytes, std::memory_order_relaxed); }
 
 // Kernel launches issued by the library since load.
 uint64_t gb_launch_counter(void) { return g_launches.load(); }

@@ -47,10 +47,13 @@ inline RustError make_error(int code, const char *msg)
     return RustError{code, msg ? strdup(msg) : nullptr};
 }
 
+// a failed call also sets the error that cudaGetLastError returns, which the
+// next launch check would take for its own: it is taken here
 #define GB_CUDA_OK(expr)                                                               \
     do {                                                                               \
         cudaError_t gb_e_ = (expr);                                                    \
         if (gb_e_ != cudaSuccess) {                                                    \
+            (void)cudaGetLastError();                                                  \
             throw ::gb::cuda_error((int)gb_e_, std::string(#expr " failed: ") +        \
                                                    cudaGetErrorString(gb_e_));         \
         }                                                                              \
@@ -115,8 +118,16 @@ unsigned long long lane_timeouts_take();
 
 // Stream-ordered device memory from the device's default memory pool, whose
 // release threshold is raised once so freed blocks are reused, not returned.
+// What the pool holds and nobody uses, the driver takes back when another
+// allocation needs it; the memory that captured graphs keep between launches
+// it does not, so an allocation that fails gives that back and tries once more.
 void *dev_alloc(size_t bytes, cudaStream_t s);
 void dev_free(void *p, cudaStream_t s);
+// the same for memory that stays (cudaMalloc): tables, contexts
+void *dev_malloc(size_t bytes);
+// test hook (gb_alloc_limit_set): true for sizes that are to fail as they do on
+// a full device
+bool alloc_refused(size_t bytes);
 
 template <class T>
 struct dev_buf {

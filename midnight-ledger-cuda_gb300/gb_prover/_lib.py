@@ -177,6 +177,7 @@ def _declare(L):
         "gb_ntt_wait_timeouts": (E, [ctypes.POINTER(ctypes.c_uint32)]),
         "gb_fr_device_vec_ntt_ragged": (E, [vp, vp, vp, sz, b, fr, fr, fr]),
         "gb_ntt_wait_limit_set": (None, [ctypes.c_int64]),
+        "gb_alloc_limit_set": (None, [sz]),
         "gb_g1_msm_device": (E, [vp, vp, vp, sz]),
         "gb_g1_msm_context_device_batch_async": (E, [vp, vp, vp, sz, sz, sz]),
         "gb_msm_ticket_wait": (E, [vp, vp]),

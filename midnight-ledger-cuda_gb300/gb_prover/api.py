@@ -31,6 +31,7 @@ __all__ = [
     "bls12_381_fr_multiopen_pi_device", "bls12_381_fr_lookup_permute_batch", "hook_mask_delay",
     "bls12_381_fr_poseidon_hash_chain", "bls12_381_fr_poseidon_advice_from_witness",
     "hook_delayed_scale", "autotune_set", "autotune_reset", "autotune_report", "ntt_wait_limit_set",
+    "alloc_limit_set",
     "FR_GENERATOR", "fr_coeff_to_extended_coset_batch", "fr_device_coeff_to_extended_coset_batch", "fr_ntt_coset",
     "fr_lde_coset", "g1_msm_device",
 ]
@@ -946,6 +947,12 @@ def ntt_wait_limit_set(spins):
     """test hook (gb_ntt_wait_limit_set): poll limit of the first twiddle-copy
     wait; None or negative restores the default"""
     lib().gb_ntt_wait_limit_set(-1 if spins is None else int(spins))
+
+
+def alloc_limit_set(limit):
+    """test hook (gb_alloc_limit_set): device allocations of more than `limit`
+    bytes fail as on a full device; None or 0 restores the default"""
+    lib().gb_alloc_limit_set(int(limit or 0))
 
 
 def ntt_wait_timeouts():
