@@ -40,47 +40,12 @@
 
 #include "gb_inv_warp.cuh"
 #include "gb_host_fp.h"
+#include "gb_msm_rules.h"
 #include "gb_runtime.cuh"
 
 namespace gb {
 
 static constexpr uint32_t kZeroDigit = 0xffffffffu;
-static constexpr int kMaxWindowBits = 16;  // 2^15 u32 counters = 128 KB smem
-
-// A scalar's 255 bits in windows of c and c - 1 bits, the wider ones first, so
-// that no window is a remainder of a few bits whose digits would crowd a few
-// buckets.  A (c - 1)-bit digit is at most 2^(c - 1), carry included, so it
-// stays positive and fills all the buckets; the top window is always one of
-// these (scalars are below 2^255, and 255 < windows c), so no carry is left.
-__host__ __device__ constexpr int windows_for(int c) { return 255 / c + 1; }
-__host__ __device__ constexpr int window_bits(int c, int j) { return j < 255 - windows_for(c) * (c - 1) ? c : c - 1; }
-__host__ __device__ constexpr int window_offset(int c, int j)
-{
-    const int wide = 255 - windows_for(c) * (c - 1);
-    return j < wide ? j * c : wide * c + (j - wide) * (c - 1);
-}
-
-// Window size for n points, measured on GB300.  With the precomputed table an
-// MSM has 2^(c - 1) buckets in all: ms a call for one and for three MSMs (*
-// chosen)
-//   2^8 points   c = 8 0.16 0.19, 10 0.15 0.18, 11* 0.14 0.18, 12 0.15 0.20
-//   2^10         10 0.17 0.21, 11* 0.16 0.21, 12 0.16 0.23, 13 0.17 0.24
-//   2^12         11 0.21 0.31, 12* 0.20 0.31, 13 0.20 0.31, 14 0.23 0.38
-//   2^14         12 0.31 0.63, 13* 0.30 0.61, 14 0.32 0.63, 15 0.35 0.67
-//   2^16         13 0.70 1.42, 14 0.67 1.43, 15* 0.67 1.41, 16 0.68 1.47
-//   2^17         13 1.13 2.44, 15 1.08 2.38, 16* 1.03 2.41
-// Without it every window has its own buckets:
-//   2^10 points  8* 0.46, 9 0.47, 10 0.51
-//   2^12         8 0.52, 9* 0.52, 10 0.54
-//   2^14         9 0.71, 10* 0.71, 11 0.75
-//   2^16         10 1.14, 11* 1.11, 12 1.13, 13 1.18
-//   2^18         11 2.31, 12* 2.25, 13 2.30
-static int choose_window(size_t n, bool precomputed)
-{
-    auto upto = [&](int lg) { return n <= (size_t)1 << lg; };
-    if (precomputed) return upto(7) ? 8 : upto(11) ? 11 : upto(12) ? 12 : upto(15) ? 13 : upto(16) ? 15 : 16;
-    return upto(11) ? 8 : upto(13) ? 9 : upto(15) ? 10 : upto(17) ? 11 : upto(19) ? 12 : 13;
-}
 
 static int default_acc_variant()
 {
@@ -477,9 +442,6 @@ __global__ void msm_scatter_kernel(const uint32_t *__restrict__ digits, const se
 //     copies): two pairs ahead on the way up, one on the way back, 2 % better
 //     than plain loads; past L1 they were 8 % worse.
 static constexpr uint32_t kNoPoint = 0xffffffffu;
-static constexpr uint32_t kPairThreads = 128;
-static constexpr uint32_t kPairBlocks = 4;      // blocks an SM
-static constexpr uint32_t kPairsPerThread = 64;  // at most, in one tile
 
 __device__ __forceinline__ void store_words8(void *p, const uint32_t *w)
 {
@@ -1556,35 +1518,6 @@ static uint32_t pair_chunk_length(uint64_t digits, double avg, uint32_t G)
     return (uint32_t)std::max<uint64_t>(L, (uint64_t)by_latency);
 }
 
-// Affine rounds of a batch: as long as a round has pairs enough to fill the
-// GPU (a round costs about 55 us whatever its size: product trees and one
-// inversion a block) and buckets are long enough, as every bucket is padded to
-// a multiple of 2^rounds.  Measured on GB300, entries and entries a bucket, and
-// ms a call without rounds and with 1, 2, 3, 4 (* chosen):
-//    1.0 M   80   0.61*  0.68   0.65
-//    1.2 M   72   0.68   0.66*  0.66   0.74   0.79
-//    2.0 M   80   1.04   0.99*  1.05
-//    2.4 M   72   1.14   1.07   1.04*  1.08   1.20
-//    4.7 M   72   2.07   1.84   1.77*  1.82   2.01
-//    5.9 M   72                 2.20   2.19*  2.35
-//   12.6 M  128   4.95   4.41   4.15   4.10*  4.16
-//   16.8 M  128                 5.41   5.28*  5.37
-//   16.8 M  512                 5.08   4.88   4.83*
-//    4.2 M  7.8          2.48*  2.66   3.07   3.45
-//    6.3 M   12          3.21   3.12*  3.59   4.01
-//    7.2 M   27          3.25   3.06*  3.12   3.51
-//   48 M     23         14.78  14.36* 14.94  17.18
-static int affine_rounds(uint64_t digits, double avg, uint32_t G)
-{
-    static constexpr uint64_t pairs[4] = {9 << 16, 9 << 16, 11 << 16, 1 << 20};
-    static constexpr double bucket[4] = {6, 11, 40, 192};
-    int r = 0;
-    while (r < 4 && digits >> (r + 1) >= pairs[r] && avg >= bucket[r] &&
-           digits + (uint64_t)G * ((2u << r) - 1) < 0x80000000ull)
-        r++;
-    return r;
-}
-
 // What the device leaves of each MSM and the host finishes once it is copied:
 // one point; the bit sums of its buckets (a context's MSM); or its window
 // sums (a plain MSM).  The last two are one chain of dependent doublings and
@@ -1650,18 +1583,20 @@ struct batch_plan {
     msm_tail tail;
     int rounds = 0;          // affine rounds before the accumulation
     uint64_t entries = 0;    // bound of the bucket-ordered list, padding included
+    uint64_t scratch = 0;    // bytes of the affine rounds' lists and prefixes
     uint64_t points_total = 0, digits_total = 0, nchunks = 0;
     std::vector<item_desc> idesc;
     std::vector<seg_desc> sdesc;
     std::vector<blk_desc> bdesc;
 };
 
-static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool precomputed, size_t stride)
+// The plan of `nitems` items, a group of a batch of batch_items (all of them,
+// mostly); most_scratch bounds the affine rounds' scratch.
+static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batch_items, int c, bool precomputed,
+                             size_t stride, uint64_t most_scratch)
 {
     batch_plan P;
-    const uint32_t nitems = (uint32_t)items.size();
     P.nitems = nitems;
-    if (!nitems) return P;
     const int nwin = windows_for(c);
     const uint32_t K = 1u << (c - 1);
     const uint32_t segs_per_item = precomputed ? 1u : (uint32_t)nwin;
@@ -1713,8 +1648,9 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     const uint32_t nblocks = (uint32_t)bdesc.size();
     const double avg = (double)digits_total / (double)G;
     const int variant = default_acc_variant();
-    const int rounds = affine_rounds(digits_total, avg, G);
-    const uint64_t entries = digits_total + (uint64_t)G * ((1u << rounds) - 1);
+    const uint64_t slots = (uint64_t)sm_count() * kPairBlocks;
+    const int rounds = affine_rounds(digits_total, avg, G, slots, most_scratch);
+    const uint64_t entries = padded_entries(digits_total, G, rounds);
     // a batch of less than 6 entries a resident thread: two lanes a chunk
     // (measured, accumulation in us with a thread and with two lanes a chunk:
     // 2^10 points 63 -> 25, 2^12 64 -> 44, 2 x 2^12 107 -> 72, 4 x 2^12 151 ->
@@ -1741,11 +1677,11 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     P.shape.lc = (uint32_t)(c - 1) - P.shape.lr;
     // the steps left to the host: see msm_tail
     P.tail.c = c;
-    if (precomputed && nseg <= kHostTailBits) {
+    if (precomputed && batch_items <= kHostTailBits) {
         P.tail.kind = msm_tail::BITS;
         P.tail.shape = P.shape;
         P.tail.points = P.shape.bits();
-    } else if (!precomputed && nitems <= kHostTailWindows) {
+    } else if (!precomputed && batch_items <= kHostTailWindows) {
         P.tail.kind = msm_tail::WINDOWS;
         P.tail.points = segs_per_item;
     }
@@ -1760,40 +1696,47 @@ static batch_plan plan_batch(const std::vector<msm_item> &items, int c, bool pre
     P.short_span = std::min<uint32_t>(kShortSpan, 6 + (uint32_t)(3.0 * avg / (1 << rounds) / L));
     P.rounds = rounds;
     P.entries = entries;
+    P.scratch = rounds_scratch(entries, rounds, slots);
     P.idesc = std::move(idesc);
     P.sdesc = std::move(sdesc);
     P.bdesc = std::move(bdesc);
     return P;
 }
 
+// Buffers of the affine rounds, allocated before a batch's first launch, so
+// that a device without room for them fails before any work is queued.
+struct round_buffers {
+    dev_buf<uint4> prefix;
+    dev_buf<affine_t> list_a, list_b;
+    round_buffers(const batch_plan &P, cudaStream_t s)
+    {
+        if (!P.rounds) return;
+        const uint64_t slots = (uint64_t)sm_count() * kPairBlocks;
+        prefix = dev_buf<uint4>(slots * pairs_per_thread(P.entries / 2, slots) * 3 * kPairThreads, s);
+        list_a = dev_buf<affine_t>(P.entries / 2 + 1, s);
+        if (P.rounds > 1) list_b = dev_buf<affine_t>(P.entries / 4 + 1, s);
+    }
+};
+
 // The affine rounds: the bucket-ordered references through P.rounds pairwise
 // additions, to a list of points a 2^rounds-th as long.
 static const affine_t *run_affine_rounds(const batch_plan &P, const uint32_t *sorted, const uint32_t *starts,
-                                         const affine_t *points, dev_buf<affine_t> &list_a,
-                                         dev_buf<affine_t> &list_b, cudaStream_t s)
+                                         const affine_t *points, const round_buffers &buf, cudaStream_t s)
 {
     const uint64_t slots = (uint64_t)sm_count() * kPairBlocks;
-    // pairs a thread: whole waves of tiles of at most 16 a thread
-    auto per_thread = [&](uint64_t pairs) {
-        const uint64_t per = std::max<uint64_t>(1, (pairs + slots * kPairThreads - 1) / (slots * kPairThreads));
-        const uint64_t waves = (per + kPairsPerThread - 1) / kPairsPerThread;
-        return (uint32_t)((per + waves - 1) / waves);
-    };
-    dev_buf<uint4> prefix(slots * per_thread(P.entries / 2) * 3 * kPairThreads, s);
-    list_a = dev_buf<affine_t>(P.entries / 2 + 1, s);
-    if (P.rounds > 1) list_b = dev_buf<affine_t>(P.entries / 4 + 1, s);
     const affine_t *in = points;
     for (int r = 1; r <= P.rounds; r++) {
-        affine_t *out = r & 1 ? list_a.get() : list_b.get();
+        affine_t *out = r & 1 ? buf.list_a.get() : buf.list_b.get();
         const uint64_t pairs = P.entries >> r;
-        const uint32_t per = std::min(per_thread(pairs), per_thread(P.entries / 2));
+        const uint32_t per = std::min(pairs_per_thread(pairs, slots), pairs_per_thread(P.entries / 2, slots));
         const uint64_t tiles = (pairs + (uint64_t)per * kPairThreads - 1) / ((uint64_t)per * kPairThreads);
         const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(slots, tiles));
         if (r == 1)
-            msm_affine_pairs_kernel<true><<<grid, kPairThreads, 0, s>>>(sorted, in, out, starts + P.G, r, per, prefix);
+            msm_affine_pairs_kernel<true><<<grid, kPairThreads, 0, s>>>(sorted, in, out, starts + P.G, r, per,
+                                                                        buf.prefix);
         else
             msm_affine_pairs_kernel<false><<<grid, kPairThreads, 0, s>>>(nullptr, in, out, starts + P.G, r, per,
-                                                                         prefix);
+                                                                         buf.prefix);
         GB_CHECK_LAUNCH();
         in = out;
     }
@@ -1813,6 +1756,7 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     const uint32_t nitems = P.nitems, K = P.K, segs_per_item = P.segs_per_item, nseg = P.nseg, G = P.G;
     const uint32_t nblocks = P.nblocks, L = P.L;
     const uint64_t points_total = P.points_total, digits_total = P.digits_total, nchunks = P.nchunks;
+    const round_buffers round_buf(P, s);
     dev_buf<uint32_t> digits(std::max<uint64_t>(digits_total, 1), s), sorted(std::max<uint64_t>(P.entries, 1), s);
     dev_buf<uint32_t> hist((size_t)nblocks * K, s), counts(G, s), starts((size_t)G + 1, s), ctl(CTL_WORDS, s);
     dev_buf<xyzz_t> buckets(G, s), head(nchunks, s), tail(nchunks, s);
@@ -1839,11 +1783,10 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
     timed_end(tok_sort, s, GB_SLOT_MSM_SORT);
     int tok = timed_begin(s);
     if (P.fix_by_chunk) GB_CUDA_OK(cudaMemsetAsync(open_bucket.get(), 0xff, nchunks * sizeof(uint32_t), s));
-    dev_buf<affine_t> list_a, list_b;
     dev_buf<uint32_t> shifted;
     const uint32_t *bounds = starts;
     if (P.rounds) {
-        const affine_t *list = run_affine_rounds(P, sorted, starts, points, list_a, list_b, s);
+        const affine_t *list = run_affine_rounds(P, sorted, starts, points, round_buf, s);
         shifted = dev_buf<uint32_t>((size_t)G + 1, s);
         msm_shift_starts_kernel<<<blocks_for(G + 1, 256), 256, 0, s>>>(starts, G + 1, P.rounds, shifted);
         GB_CHECK_LAUNCH();
@@ -1951,13 +1894,14 @@ struct graph_key {
     const affine_t *points = nullptr;
     int c = 0, variant = 0;
     bool precomputed = false, fix_by_chunk = false;
+    int tail = 0;
     size_t stride = 0;
     uint32_t nitems = 0, K = 0, segs_per_item = 0, nseg = 0, G = 0, nblocks = 0, L = 0, short_span = 0;
     int rounds = 0;
     uint64_t points_total = 0, digits_total = 0, nchunks = 0;
     auto tie() const
     {
-        return std::tie(device, stream, points, c, variant, precomputed, fix_by_chunk, stride, nitems, K, segs_per_item,
+        return std::tie(device, stream, points, c, variant, precomputed, fix_by_chunk, tail, stride, nitems, K, segs_per_item,
                         nseg, G, nblocks, L, short_span, rounds, points_total, digits_total, nchunks);
     }
     bool operator<(const graph_key &o) const { return tie() < o.tie(); }
@@ -2022,7 +1966,7 @@ static bool run_planned_graph(const batch_plan &P, const affine_t *points, xyzz_
     key.stride = P.stride, key.nitems = P.nitems, key.K = P.K, key.segs_per_item = P.segs_per_item;
     key.nseg = P.nseg, key.G = P.G, key.nblocks = P.nblocks, key.L = P.L, key.short_span = P.short_span;
     key.points_total = P.points_total, key.digits_total = P.digits_total, key.nchunks = P.nchunks;
-    key.rounds = P.rounds;
+    key.rounds = P.rounds, key.tail = P.tail.kind;
 
     // a stream the caller is capturing gets the launches themselves
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -2099,27 +2043,52 @@ struct batch_result {
     dev_buf<xyzz_t> points;
 };
 
-// Run a batch of MSMs.  precomputed: `points` is a table of nwin rows of
-// `stride` bases (row j = 2^(c*j) P); plain: `points` holds the bases.
-// use_graph: the bases pointer is stable across calls (a context's), so
-// the batch may replay a captured graph.
-static batch_result msm_run_batch(const std::vector<msm_item> &items, int c, bool precomputed, const affine_t *points,
-                                  size_t stride, cudaStream_t s, bool use_graph = false)
+// A planned batch, or group of one, queued on s; d_out: its tail.points points
+// per MSM.
+static void launch_planned(const batch_plan &P, const affine_t *points, xyzz_t *d_out, cudaStream_t s, bool use_graph)
 {
-    set_smem_attrs();
-    batch_result r;
-    if (items.empty()) return r;
-    const batch_plan P = plan_batch(items, c, precomputed, stride);
-    r.tail = P.tail;
-    r.points = dev_buf<xyzz_t>((size_t)P.nitems * P.tail.points, s);
-    if (use_graph && graphs_enabled() && run_planned_graph(P, points, r.points, s)) return r;
+    if (use_graph && graphs_enabled() && run_planned_graph(P, points, d_out, s)) return;
     dev_buf<item_desc> d_items(P.nitems, s);
     dev_buf<seg_desc> d_segs(P.nseg, s);
     dev_buf<blk_desc> d_blks(P.nblocks, s);
     h2d(d_items, P.idesc.data(), P.nitems * sizeof(item_desc), s);
     h2d(d_segs, P.sdesc.data(), P.nseg * sizeof(seg_desc), s);
     h2d(d_blks, P.bdesc.data(), P.nblocks * sizeof(blk_desc), s);
-    run_planned(P, d_items, d_segs, d_blks, points, r.points, s);
+    run_planned(P, d_items, d_segs, d_blks, points, d_out, s);
+}
+
+// Run a batch of MSMs, in groups if it is very large.  precomputed: `points`
+// is a table of nwin rows of `stride` bases (row j = 2^(c*j) P); plain:
+// `points` holds the bases.  use_graph: the bases pointer is stable across
+// calls (a context's), so the batch may replay a captured graph.  A device
+// without room for the affine rounds' scratch runs the batch without rounds,
+// as it takes a ninth of the memory then.
+static batch_result msm_run_batch(const std::vector<msm_item> &items, int c, bool precomputed, const affine_t *points,
+                                  size_t stride, cudaStream_t s, bool use_graph = false)
+{
+    set_smem_attrs();
+    batch_result r;
+    std::vector<size_t> sizes;
+    for (const msm_item &it : items) sizes.push_back(it.n);
+    const std::vector<size_t> first = batch_groups(sizes, c, precomputed);
+    for (size_t g = 0; g + 1 < first.size() && !items.empty(); g++) {
+        auto plan = [&](uint64_t most_scratch) {
+            return plan_batch(items.data() + first[g], (uint32_t)(first[g + 1] - first[g]), items.size(), c,
+                              precomputed, stride, most_scratch);
+        };
+        batch_plan P = plan(kRoundsScratch);
+        if (!g) {
+            r.tail = P.tail;
+            r.points = dev_buf<xyzz_t>(items.size() * P.tail.points, s);
+        }
+        xyzz_t *out = r.points.get() + first[g] * P.tail.points;
+        try {
+            launch_planned(P, points, out, s, use_graph);
+        } catch (const cuda_error &e) {
+            if (e.code() != (int)cudaErrorMemoryAllocation || !P.rounds) throw;
+            launch_planned(plan(0), points, out, s, false);
+        }
+    }
     return r;
 }
 

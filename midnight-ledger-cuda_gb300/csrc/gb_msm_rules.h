@@ -1,0 +1,145 @@
+// The rules that plan an MSM batch from its sizes alone: windows, affine
+// rounds and their scratch, and how large batches are divided.  Host code
+// without CUDA, so that they can be checked over their whole range on the CPU.
+#pragma once
+
+#include <stddef.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <vector>
+
+#if defined(__CUDACC__)
+#define GB_RULE __host__ __device__ constexpr
+#else
+#define GB_RULE constexpr
+#endif
+
+namespace gb {
+
+static constexpr int kMaxWindowBits = 16;  // 2^15 u32 counters = 128 KB smem
+
+// A scalar's 255 bits in windows of c and c - 1 bits, the wider ones first, so
+// that no window is a remainder of a few bits whose digits would crowd a few
+// buckets.  A (c - 1)-bit digit is at most 2^(c - 1), carry included, so it
+// stays positive and fills all the buckets; the top window is always one of
+// these (scalars are below 2^255, and 255 < windows c), so no carry is left.
+GB_RULE int windows_for(int c) { return 255 / c + 1; }
+GB_RULE int window_bits(int c, int j) { return j < 255 - windows_for(c) * (c - 1) ? c : c - 1; }
+GB_RULE int window_offset(int c, int j)
+{
+    const int wide = 255 - windows_for(c) * (c - 1);
+    return j < wide ? j * c : wide * c + (j - wide) * (c - 1);
+}
+
+// Window size for n points, measured on GB300.  With the precomputed table an
+// MSM has 2^(c - 1) buckets in all: ms a call for one and for three MSMs (*
+// chosen)
+//   2^8 points   c = 8 0.16 0.19, 10 0.15 0.18, 11* 0.14 0.18, 12 0.15 0.20
+//   2^10         10 0.17 0.21, 11* 0.16 0.21, 12 0.16 0.23, 13 0.17 0.24
+//   2^12         11 0.21 0.31, 12* 0.20 0.31, 13 0.20 0.31, 14 0.23 0.38
+//   2^14         12 0.31 0.63, 13* 0.30 0.61, 14 0.32 0.63, 15 0.35 0.67
+//   2^16         13 0.70 1.42, 14 0.67 1.43, 15* 0.67 1.41, 16 0.68 1.47
+//   2^17         13 1.13 2.44, 15 1.08 2.38, 16* 1.03 2.41
+// Without it every window has its own buckets:
+//   2^10 points  8* 0.46, 9 0.47, 10 0.51
+//   2^12         8 0.52, 9* 0.52, 10 0.54
+//   2^14         9 0.71, 10* 0.71, 11 0.75
+//   2^16         10 1.14, 11* 1.11, 12 1.13, 13 1.18
+//   2^18         11 2.31, 12* 2.25, 13 2.30
+inline int choose_window(size_t n, bool precomputed)
+{
+    auto upto = [&](int lg) { return n <= (size_t)1 << lg; };
+    if (precomputed) return upto(7) ? 8 : upto(11) ? 11 : upto(12) ? 12 : upto(15) ? 13 : upto(16) ? 15 : 16;
+    return upto(11) ? 8 : upto(13) ? 9 : upto(15) ? 10 : upto(17) ? 11 : upto(19) ? 12 : 13;
+}
+
+// Affine rounds (see msm_affine_pairs_kernel): tiles of kPairThreads x up to
+// kPairsPerThread pairs, kPairBlocks blocks an SM.
+static constexpr uint32_t kPairThreads = 128;
+static constexpr uint32_t kPairBlocks = 4;
+static constexpr uint32_t kPairsPerThread = 64;
+
+// pairs a thread: whole waves of `slots` tiles of at most kPairsPerThread
+inline uint32_t pairs_per_thread(uint64_t pairs, uint64_t slots)
+{
+    const uint64_t per = std::max<uint64_t>(1, (pairs + slots * kPairThreads - 1) / (slots * kPairThreads));
+    const uint64_t waves = (per + kPairsPerThread - 1) / kPairsPerThread;
+    return (uint32_t)((per + waves - 1) / waves);
+}
+
+// the bucket-ordered list's length when buckets are padded for the rounds
+inline uint64_t padded_entries(uint64_t digits, uint64_t G, int rounds) { return digits + G * ((1u << rounds) - 1); }
+
+// Scratch of the rounds: the two lists of 96-byte points that they go between
+// (half and a quarter of the entries) and 48-byte prefix products.  Digits and
+// references are 8 bytes an entry, so this is 6 (one round) to 9 times the rest.
+inline uint64_t rounds_scratch(uint64_t entries, int rounds, uint64_t slots)
+{
+    if (!rounds) return 0;
+    return 96 * (entries / 2 + 1) + (rounds > 1 ? 96 * (entries / 4 + 1) : 0) +
+           48ull * kPairThreads * slots * pairs_per_thread(entries / 2, slots);
+}
+
+// Rounds are taken while their scratch is below kRoundsScratch, and a batch
+// that would take more than kGroupScratch is run as several, one after the
+// other on the same scratch (7 MSMs of 2^20 points with 16 windows, 35 ms of
+// work, against about 0.3 ms that a batch of its own costs).
+static constexpr uint64_t kRoundsScratch = 16ull << 30, kGroupScratch = 8ull << 30;
+// 72 bytes an entry of rounds' scratch, 192 a bucket
+static constexpr uint64_t kGroupDigits = kGroupScratch / 72, kGroupBuckets = 1ull << 25;
+
+// Affine rounds of a batch: as long as a round has pairs enough to fill the
+// GPU (a round costs about 55 us whatever its size: product trees and one
+// inversion a block) and buckets are long enough, as every bucket is padded to
+// a multiple of 2^rounds; and while their scratch is no more than
+// most_scratch.  Measured on GB300, entries and entries a bucket, and
+// ms a call without rounds and with 1, 2, 3, 4 (* chosen):
+//    1.0 M   80   0.61*  0.68   0.65
+//    1.2 M   72   0.68   0.66*  0.66   0.74   0.79
+//    2.0 M   80   1.04   0.99*  1.05
+//    2.4 M   72   1.14   1.07   1.04*  1.08   1.20
+//    4.7 M   72   2.07   1.84   1.77*  1.82   2.01
+//    5.9 M   72                 2.20   2.19*  2.35
+//   12.6 M  128   4.95   4.41   4.15   4.10*  4.16
+//   16.8 M  128                 5.41   5.28*  5.37
+//   16.8 M  512                 5.08   4.88   4.83*
+//    4.2 M  7.8          2.48*  2.66   3.07   3.45
+//    6.3 M   12          3.21   3.12*  3.59   4.01
+//    7.2 M   27          3.25   3.06*  3.12   3.51
+//   48 M     23         14.78  14.36* 14.94  17.18
+inline int affine_rounds(uint64_t digits, double avg, uint64_t G, uint64_t slots, uint64_t most_scratch)
+{
+    static constexpr uint64_t pairs[4] = {9 << 16, 9 << 16, 11 << 16, 1 << 20};
+    static constexpr double bucket[4] = {6, 11, 40, 192};
+    int r = 0;
+    while (r < 4 && digits >> (r + 1) >= pairs[r] && avg >= bucket[r] &&
+           padded_entries(digits, G, r + 1) < 0x80000000ull &&
+           rounds_scratch(padded_entries(digits, G, r + 1), r + 1, slots) <= most_scratch)
+        r++;
+    return r;
+}
+
+// The batch in groups of consecutive items: their first items, and the end.
+// A group holds as many as fit kGroupDigits digits and kGroupBuckets buckets,
+// one at least.
+inline std::vector<size_t> batch_groups(const std::vector<size_t> &sizes, int c, bool precomputed)
+{
+    const uint64_t nwin = (uint64_t)windows_for(c), K = (uint64_t)1 << (c - 1);
+    const uint64_t buckets = precomputed ? K : K * nwin;  // an item's
+    std::vector<size_t> first(1, 0);
+    uint64_t digits = 0, items = 0;
+    for (size_t i = 0; i < sizes.size(); i++) {
+        const uint64_t d = sizes[i] * nwin;
+        if (items && (digits + d > kGroupDigits || (items + 1) * buckets > kGroupBuckets)) {
+            first.push_back(i);
+            digits = items = 0;
+        }
+        digits += d;
+        items++;
+    }
+    first.push_back(sizes.size());
+    return first;
+}
+
+}  // namespace gb

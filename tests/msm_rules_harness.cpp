@@ -1,0 +1,23 @@
+// gb_msm_rules.h as host code, for test_msm_rules.py
+#include "gb_msm_rules.h"
+
+extern "C" {
+int r_choose_window(size_t n, int precomputed) { return gb::choose_window(n, precomputed != 0); }
+int r_windows(int c) { return gb::windows_for(c); }
+int r_rounds(uint64_t digits, uint64_t G, uint64_t slots, uint64_t most)
+{
+    return gb::affine_rounds(digits, (double)digits / (double)G, G, slots, most);
+}
+uint64_t r_scratch(uint64_t digits, uint64_t G, int rounds, uint64_t slots)
+{
+    return gb::rounds_scratch(gb::padded_entries(digits, G, rounds), rounds, slots);
+}
+uint64_t r_rounds_limit() { return gb::kRoundsScratch; }
+// the groups' first items and the end into out (n + 1 places at most); how many
+size_t r_groups(const size_t *sizes, size_t n, int c, int precomputed, size_t *out)
+{
+    const std::vector<size_t> g = gb::batch_groups(std::vector<size_t>(sizes, sizes + n), c, precomputed != 0);
+    std::copy(g.begin(), g.end(), out);
+    return g.size();
+}
+}

@@ -64,3 +64,47 @@ def test_a_failed_allocation_takes_back_what_graphs_keep(gb, orc):
     assert _graph_bytes(gb) < held
     assert (affine_of(orc, ctx.msm(scal)) == want).all()
     ctx.close()
+
+
+@pytest.mark.parametrize("kind", ["context", "plain"])
+def test_batches_without_room_for_the_affine_rounds(gb, orc, limit, kind):
+    """3 x 2^16 points take 170 MB and more for their affine rounds and no other buffer
+    of more than 40 MB: with less than that at hand they run without rounds."""
+    rng = np.random.default_rng(3)
+    n, count = 1 << 16, 3
+    bases = gb.g1_generator_mul(orc.fr_random(n, rng))
+    scal = orc.fr_random(n * count, rng).reshape(count, n, 4)
+    want = [affine_of(orc, orc.g1_msm(bases, scal[i])) for i in range(count)]
+    ctx = gb.Bls12_381G1MsmContext(bases)
+    gb.msm_graphs_enable(False)
+    try:
+        for most in (0, 64 << 20, 0):
+            limit(most)
+            got = ctx.batch(scal) if kind == "context" else gb.bls12_381_g1_msm_batch(bases, scal)
+            for i in range(count):
+                assert (affine_of(orc, got[i]) == want[i]).all(), (most, i)
+    finally:
+        gb.msm_graphs_enable(True)
+    limit(1 << 20)
+    with pytest.raises(gb.MsmError) as e:
+        ctx.batch(scal)
+    assert e.value.code == OUT_OF_MEMORY
+    limit(0)
+    assert (affine_of(orc, ctx.batch(scal)[0]) == want[0]).all()
+    ctx.close()
+
+
+def test_batch_divided_into_groups(gb, orc):
+    """5000 MSMs of 1024 points are 123 M digits, more than a group of a batch
+    holds; their results come in order."""
+    rng = np.random.default_rng(4)
+    n, count = 1024, 5000
+    bases = gb.g1_generator_mul(orc.fr_random(n, rng))
+    dv = gb.fr_random_chacha20(bytes(range(32)), 0, n * count)[0]
+    ctx = gb.Bls12_381G1MsmContext(bases)
+    got = ctx.device_batch(dv, 0, n, count)
+    scal = dv.download().reshape(count, n, 4)
+    for i in list(range(0, count, 500)) + list(range(4840, 4880, 5)) + [count - 1]:
+        assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all(), i
+    ctx.close()
+    dv.free()

@@ -1,0 +1,83 @@
+"""The rules that plan an MSM batch from its sizes (csrc/gb_msm_rules.h), over
+their range: the affine rounds' scratch stays below its bound, and large
+batches are divided into groups that stay below theirs and leave no item out."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import PKG, REPO
+
+SLOTS = 152 * 4  # blocks resident at once
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("rules") / "msm_rules.so")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(PKG, "csrc"), "-o", so,
+                           os.path.join(REPO, "tests", "msm_rules_harness.cpp")])
+    L = ctypes.CDLL(so)
+    u64 = ctypes.c_uint64
+    L.r_choose_window.argtypes = [ctypes.c_size_t, ctypes.c_int]
+    L.r_rounds.argtypes = [u64, u64, u64, u64]
+    L.r_scratch.argtypes = [u64, u64, ctypes.c_int, u64]
+    L.r_scratch.restype = L.r_rounds_limit.restype = u64
+    L.r_groups.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
+    L.r_groups.restype = ctypes.c_size_t
+    return L
+
+
+@pytest.mark.parametrize("buckets", [1 << 10, 1 << 15, 1 << 20, 1 << 25])
+def test_rounds_scratch_is_bounded(rules, buckets):
+    limit = rules.r_rounds_limit()
+    assert limit <= 16 << 30  # a sixteenth of the device
+    for lg in np.arange(10, 31, 0.25):
+        digits = int(2 ** lg)
+        r = rules.r_rounds(digits, buckets, SLOTS, limit)
+        assert rules.r_scratch(digits, buckets, r, SLOTS) <= limit
+        assert rules.r_rounds(digits, buckets, SLOTS, 0) == 0
+        # less room, fewer rounds
+        for most in (limit >> 2, limit >> 6):
+            less = rules.r_rounds(digits, buckets, SLOTS, most)
+            assert less <= r and rules.r_scratch(digits, buckets, less, SLOTS) <= most
+
+
+def test_rounds_of_ordinary_batches(rules):
+    """The bound does not touch what is measured in the rule's table."""
+    for digits, avg, want in ((1 << 20, 80, 0), (4_700_000, 72, 2), (16_800_000, 512, 4), (48_000_000, 23, 2)):
+        assert rules.r_rounds(digits, digits // avg, SLOTS, rules.r_rounds_limit()) == want
+
+
+def groups(rules, sizes, c, precomputed):
+    sizes = np.asarray(sizes, dtype=np.uint64)
+    out = np.zeros(len(sizes) + 2, dtype=np.uint64)
+    n = rules.r_groups(sizes.ctypes.data, len(sizes), c, precomputed, out.ctypes.data)
+    return [int(x) for x in out[:n]]
+
+
+@pytest.mark.parametrize("c,precomputed", [(8, 0), (11, 1), (13, 0), (16, 1), (16, 0)])
+@pytest.mark.parametrize("sizes", [[0], [5], [1 << 20] * 3, [1 << 20] * 100, [700] * 70000, [1 << 24] * 3 + [9] * 50,
+                                   [1 << 26, 1, 1 << 26, 0, 1 << 26], [0] * 5000])
+def test_groups(rules, sizes, c, precomputed):
+    first = groups(rules, sizes, c, precomputed)
+    assert first[0] == 0 and first[-1] == len(sizes) and all(a < b for a, b in zip(first, first[1:]))
+    nwin = rules.r_windows(c)
+    per_item = (1 << (c - 1)) * (1 if precomputed else nwin)
+    parts = [(sum(sizes[a:b]) * nwin, (b - a) * per_item, b - a) for a, b in zip(first, first[1:])]
+    for digits, buckets, items in parts:
+        if items > 1:
+            assert digits * 72 <= 8 << 30 and buckets <= 1 << 25
+        assert buckets < 1 << 28  # the count scan's range
+        r = rules.r_rounds(digits, buckets, SLOTS, rules.r_rounds_limit())
+        assert rules.r_scratch(digits, buckets, r, SLOTS) <= rules.r_rounds_limit()
+    # no more groups than needed: the next item does not fit
+    for (digits, _, items), nxt in zip(parts, first[1:-1]):
+        assert (digits + sizes[nxt] * nwin) * 72 > 8 << 30 or (items + 1) * per_item > 1 << 25
+
+
+def test_ordinary_batches_are_one_group(rules):
+    assert len(groups(rules, [1 << 18] * 20, 16, 1)) == 2
+    assert len(groups(rules, [1 << 20] * 7, 16, 1)) == 2
+    assert len(groups(rules, [2049] * 145, 9, 0)) == 2
