@@ -1955,9 +1955,11 @@ static bool graphs_enabled()
 }
 
 // Runs the planned batch through a cached graph; false when this shape
-// cannot be captured (the caller then launches it directly).
+// cannot be captured, or the device has no memory for the graph's scratch (the
+// caller then launches it directly).
 static bool run_planned_graph(const batch_plan &P, const affine_t *points, xyzz_t *d_out, cudaStream_t s)
 {
+    if (P.scratch > kGraphScratch) return false;
     graph_key key;
     key.device = current_device();
     key.stream = s;
@@ -2029,7 +2031,17 @@ static bool run_planned_graph(const batch_plan &P, const affine_t *points, xyzz_
     h2d(e->d_items, P.idesc.data(), P.nitems * sizeof(item_desc), s);
     h2d(e->d_segs, P.sdesc.data(), P.nseg * sizeof(seg_desc), s);
     h2d(e->d_blks, P.bdesc.data(), P.nblocks * sizeof(blk_desc), s);
-    GB_CUDA_OK(cudaGraphLaunch(e->exec, s));
+    // a graph's scratch is allocated when it is launched
+    const cudaError_t el = alloc_refused(P.scratch) ? cudaErrorMemoryAllocation : cudaGraphLaunch(e->exec, s);
+    if (el == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        std::lock_guard<std::mutex> lg(g_graph_mu);
+        auto it = g_graphs.find(key);
+        if (it != g_graphs.end() && it->second == e) g_graphs.erase(it);
+        g_graph_seen.erase(key);
+        return false;
+    }
+    GB_CUDA_OK(el);
     GB_CUDA_OK(cudaMemcpyAsync(d_out, e->d_out, (size_t)P.nitems * P.tail.points * sizeof(xyzz_t),
                                cudaMemcpyDeviceToDevice, s));
     g_graph_launches++;

@@ -86,6 +86,10 @@ inline uint64_t rounds_scratch(uint64_t entries, int rounds, uint64_t slots)
 // other on the same scratch (7 MSMs of 2^20 points with 16 windows, 35 ms of
 // work, against about 0.3 ms that a batch of its own costs).
 static constexpr uint64_t kRoundsScratch = 16ull << 30, kGroupScratch = 8ull << 30;
+// Batches with more scratch are not captured as graphs: a graph's memory stays
+// with it between launches, and the gaps between the launches that it spares,
+// 0.1 ms, do not show beside the 8 ms that such a batch takes.
+static constexpr uint64_t kGraphScratch = 2ull << 30;
 // 72 bytes an entry of rounds' scratch, 192 a bucket
 static constexpr uint64_t kGroupDigits = kGroupScratch / 72, kGroupBuckets = 1ull << 25;
 

@@ -108,3 +108,50 @@ def test_batch_divided_into_groups(gb, orc):
         assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all(), i
     ctx.close()
     dv.free()
+
+
+def test_graph_without_room_for_its_scratch(gb, orc, limit):
+    """A captured batch whose launch finds no memory runs launch by launch (and
+    without rounds), and is captured again once there is room."""
+    rng = np.random.default_rng(5)
+    n, count = 1 << 16, 2
+    bases = gb.g1_generator_mul(orc.fr_random(n, rng))
+    scal = orc.fr_random(n * count, rng).reshape(count, n, 4)
+    want = [affine_of(orc, orc.g1_msm(bases, scal[i])) for i in range(count)]
+    ctx = gb.Bls12_381G1MsmContext(bases)
+
+    def check():
+        got = ctx.batch(scal)
+        for i in range(count):
+            assert (affine_of(orc, got[i]) == want[i]).all()
+
+    captures, launches = gb.msm_graph_stats()
+    for _ in range(3):
+        check()
+    assert gb.msm_graph_stats() == (captures + 1, launches + 2)
+    limit(64 << 20)
+    for _ in range(2):
+        check()
+    assert gb.msm_graph_stats()[1] == launches + 2
+    limit(0)
+    for _ in range(3):
+        check()
+    assert gb.msm_graph_stats()[1] > launches + 2
+    ctx.close()
+
+
+def test_batches_with_much_scratch_are_not_captured(gb, orc):
+    rng = np.random.default_rng(6)
+    n, count = 1 << 18, 8
+    ctx = gb.Bls12_381G1MsmContext(gb.g1_generator_mul(orc.fr_random(n, rng)))
+    dv = gb.fr_random_chacha20(bytes(range(32)), 0, n * count)[0]
+    captures = gb.msm_graph_stats()[0]
+    first = ctx.device_batch(dv, 0, n, count)
+    for _ in range(2):
+        assert (affine_of(orc, ctx.device_batch(dv, 0, n, count)) == affine_of(orc, first)).all()
+    assert gb.msm_graph_stats()[0] == captures
+    ctx.device_batch(dv, 0, n, 1)
+    ctx.device_batch(dv, 0, n, 1)
+    assert gb.msm_graph_stats()[0] == captures + 1
+    ctx.close()
+    dv.free()
