@@ -911,7 +911,6 @@ __global__ void __launch_bounds__(2 * kPairChunks, kPairSm) msm_accumulate_pair_
 //    buckets each 1.60 -> 0.47 ms (chunks of 8 waves at most among it), 20 of
 //    2^10 .. 2^13 0.77 -> 0.10 ms (long buckets out of the threads' hands
 //    among it: one thread's 30 additions took 0.45 ms).
-static constexpr uint32_t kShortSpan = 32;  // chunks at most
 static constexpr uint32_t kNoBucket = 0xffffffffu;
 
 __global__ void msm_fixup_kernel(const uint32_t *__restrict__ starts, const uint32_t *__restrict__ open_bucket,
@@ -1657,8 +1656,11 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
     // 129, 2^14 189 -> 149; 2 x 2^14, 8 entries a thread, 243 and 243, and 2^16
     // 432 and 450)
     const bool pair = variant == 1 && !rounds && digits_total < 6 * (uint64_t)sm_count() * 512;
-    const uint32_t L = pair ? pair_chunk_length(digits_total, avg, G)
-                            : chunk_length(entries >> rounds, avg / (1 << rounds), G, variant);
+    std::vector<size_t> sizes;
+    for (uint32_t m = 0; m < nitems; m++) sizes.push_back(items[m].n);
+    const double typical = typical_bucket(sizes, c, precomputed) / (1 << rounds);
+    const uint32_t L = pair ? pair_chunk_length(digits_total, typical, G)
+                            : chunk_length(entries >> rounds, typical, G, variant);
     const uint64_t nchunks = std::max<uint64_t>(1, ((entries >> rounds) + L - 1) / L);
 
     P.pair = pair;
@@ -1691,9 +1693,7 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
     P.fix_by_chunk = G > kCoopFixupSmall && avg / (1 << rounds) < L;
     P.fix_coop = !P.fix_by_chunk && G <= kCoopFixupMaxBuckets;
     P.log_parts = G <= 2048 ? 2 : G <= 8192 ? 1 : 0;
-    // a thread adds spans of some 3 times the mean, as a longer chain holds up
-    // the launch (14 us an addition)
-    P.short_span = std::min<uint32_t>(kShortSpan, 6 + (uint32_t)(3.0 * avg / (1 << rounds) / L));
+    P.short_span = short_span(avg / (1 << rounds), typical, L);
     P.rounds = rounds;
     P.entries = entries;
     P.scratch = rounds_scratch(entries, rounds, slots);

@@ -12,6 +12,11 @@ uint64_t r_scratch(uint64_t digits, uint64_t G, int rounds, uint64_t slots)
 {
     return gb::rounds_scratch(gb::padded_entries(digits, G, rounds), rounds, slots);
 }
+double r_typical(const size_t *sizes, size_t n, int c, int precomputed)
+{
+    return gb::typical_bucket(std::vector<size_t>(sizes, sizes + n), c, precomputed != 0);
+}
+uint32_t r_short_span(double mean, double typical, uint32_t L) { return gb::short_span(mean, typical, L); }
 uint64_t r_rounds_limit() { return gb::kRoundsScratch; }
 // the groups' first items and the end into out (n + 1 places at most); how many
 size_t r_groups(const size_t *sizes, size_t n, int c, int precomputed, size_t *out)

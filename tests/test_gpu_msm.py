@@ -568,3 +568,22 @@ def test_plain_batches_of_many_buckets(gb, orc, n, count):
     got = gb.bls12_381_g1_msm_batch(bases, scal)
     for i in list(range(0, count, 24)) + [count - 1]:
         assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
+
+
+@pytest.mark.parametrize("sizes", [[1 << 16] * 2 + [300] * 32, [1 << 16] + [2048] * 3 + [0, 1, 5000], [9000] + [256] * 30])
+def test_uneven_context_batches(gb, orc, sizes):
+    """A few large MSMs among many small ones, whose buckets hold a few entries
+    where the large ones' hold 72."""
+    rng = np.random.default_rng(len(sizes))
+    n = 1 << 16
+    bases = gb.g1_generator_mul(orc.fr_random(n, rng))
+    scal = orc.fr_random(sum(sizes), rng)
+    dv = gb.Bls12_381FrDeviceVec.upload(scal)
+    ctx = gb.Bls12_381G1MsmContext(bases)
+    off = np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(int)
+    got = ctx.device_ragged(dv, [(int(o), i % 7 if m < n - 7 else 0, m) for i, (o, m) in enumerate(zip(off, sizes))])
+    for i, (o, m) in enumerate(zip(off, sizes)):
+        p0 = i % 7 if m < n - 7 else 0
+        assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases[p0:p0 + m], scal[o:o + m]))).all(), i
+    ctx.close()
+    dv.free()

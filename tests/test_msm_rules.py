@@ -26,6 +26,9 @@ def rules(tmp_path_factory):
     L.r_scratch.restype = L.r_rounds_limit.restype = u64
     L.r_groups.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
     L.r_groups.restype = ctypes.c_size_t
+    L.r_typical.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int]
+    L.r_typical.restype = ctypes.c_double
+    L.r_short_span.argtypes = [ctypes.c_double, ctypes.c_double, ctypes.c_uint32]
     return L
 
 
@@ -81,3 +84,24 @@ def test_ordinary_batches_are_one_group(rules):
     assert len(groups(rules, [1 << 18] * 20, 16, 1)) == 2
     assert len(groups(rules, [1 << 20] * 7, 16, 1)) == 2
     assert len(groups(rules, [2049] * 145, 9, 0)) == 2
+
+
+def typical(rules, sizes, c, precomputed):
+    sizes = np.asarray(sizes, dtype=np.uint64)
+    return rules.r_typical(sizes.ctypes.data, len(sizes), c, precomputed)
+
+
+@pytest.mark.parametrize("c,precomputed", [(9, 0), (15, 1), (16, 1)])
+def test_typical_bucket(rules, c, precomputed):
+    """Of equal MSMs the mean; of an uneven batch the large items' buckets, and
+    these may then be added up without the block-wide fix-up."""
+    rows = rules.r_windows(c) if precomputed else 1
+    assert typical(rules, [3000] * 7, c, precomputed) == pytest.approx(3000 * rows / (1 << (c - 1)))
+    assert typical(rules, [0, 0], c, precomputed) == 0
+    for small in (32, 200):
+        sizes = [1 << 16] * 2 + [256] * small
+        large = (1 << 16) * rows / (1 << (c - 1))
+        t = typical(rules, sizes, c, precomputed)
+        assert 0.5 * large < t <= large
+        mean = sum(sizes) / len(sizes) * rows / (1 << (c - 1))
+        assert all(rules.r_short_span(mean, t, L) >= min(32, large / L) for L in range(3, 65))
