@@ -142,7 +142,7 @@ def test_graph_without_room_for_its_scratch(gb, orc, limit):
 
 def test_batches_with_much_scratch_are_not_captured(gb, orc):
     rng = np.random.default_rng(6)
-    n, count = 1 << 18, 8
+    n, count = 1 << 18, 16
     ctx = gb.Bls12_381G1MsmContext(gb.g1_generator_mul(orc.fr_random(n, rng)))
     dv = gb.fr_random_chacha20(bytes(range(32)), 0, n * count)[0]
     captures = gb.msm_graph_stats()[0]
