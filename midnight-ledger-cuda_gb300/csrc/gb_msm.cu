@@ -2241,15 +2241,6 @@ static void msm_host_plain(jacobian_t *out, const affine_t *points, const fr_t *
     plain_run_items(out, d_points, items, s);
 }
 
-// An MSM far smaller than the context's bucket count (2^(c-1)) skips the
-// precomputed windows: with the table it pays for all the buckets (about 30 us
-// for 2^15 of them), as a plain MSM with its own small window far less.  But
-// the plain MSMs are a batch of their own behind the other one (1 to 2 ms), so
-// the line lies well below where the two cost the same alone.  Measured: 64
-// MSMs of 2^10 .. 2^18 points on a 2^18 context, 9 of them below 2^11, 17.8 ms
-// with a ratio of 16 (two batches) and 15.8 ms with 32 and 64 (one).
-static constexpr size_t kPrecomputedMinRatio = 64;  // buckets / points
-
 // Page-locked staging buffers of the asynchronous MSM calls, reused: a
 // cudaFreeHost would synchronise the device, so buffers are kept until exit.
 static std::mutex g_pinned_mu;
@@ -2317,8 +2308,13 @@ static void context_enqueue_items(msm_context_t *ctx, pending_points &pending, c
 {
     std::vector<msm_item> sub[2];
     std::vector<size_t> idx[2];
+    const size_t K = (size_t)1 << (ctx->c - 1);
+    size_t between = 0, points = 0;  // items between the two ratios
+    for (const msm_item &it : items)
+        if (it.n * kTableMinRatio >= K && it.n * kTableRatio < K) between++, points += it.n;
+    const size_t ratio = between && between > table_items(K, points / between) ? kTableRatio : kTableMinRatio;
     for (size_t i = 0; i < items.size(); i++) {
-        const bool big = items[i].n * kPrecomputedMinRatio >= ((size_t)1 << (ctx->c - 1)) || items.size() == 1;
+        const bool big = items[i].n * ratio >= K || items.size() == 1;
         sub[!big].push_back(items[i]);
         idx[!big].push_back(i);
     }

@@ -148,6 +148,28 @@ inline uint32_t short_span(double mean, double typical, uint32_t L)
     return std::min<uint32_t>(kShortSpan, (uint32_t)std::max(6 + 3 * mean / L, 2 + 1.5 * typical / L));
 }
 
+// Of a batch against a context, items of at least 1 / kTableRatio of the
+// context's K buckets use its table: with fewer points the plain engine and a
+// small window is the less work.  But the plain MSMs are a batch of their own
+// behind the other one (1.2 ms), so items down to 1 / kTableMinRatio use the
+// table too, unless there are many.  Measured, ms by the table and plain:
+//   K = 2^15  n = 512    x32 1.75 2.33   x48 3.03 2.85   x512 27.7 12.5
+//             n = 1024   x32 2.10 2.50   x64 3.94 3.73   x512 29.0 14.9
+//             n = 2048   x64 4.25 4.36   x96 6.37 5.89   x512 31.4 19.8
+//             n = 4095   x96 7.32 8.39   x192 14.0 12.3  x512 35.8 29.6
+//   K = 2^14  n = 256    x192 5.92 7.10  x512 14.9 11.0
+//             n = 1024   x192 6.91 8.62  x512 17.0 15.0
+//             n = 2047   x192 7.95 10.4  x512 19.7 19.8
+//   K = 2^12  n = 64     x512 4.67 10.1
+// The number of items up to which the table is taken; n: their mean length.
+static constexpr size_t kTableRatio = 8, kTableMinRatio = 64;
+inline size_t table_items(size_t K, size_t n)
+{
+    if (K >= (size_t)1 << 15) return 32 + n / 40;
+    if (K >= (size_t)1 << 14) return 240 + n / 8;
+    return SIZE_MAX;
+}
+
 // The batch in groups of consecutive items: their first items, and the end.
 // A group holds as many as fit kGroupDigits digits and kGroupBuckets buckets,
 // one at least.

@@ -17,6 +17,7 @@ double r_typical(const size_t *sizes, size_t n, int c, int precomputed)
     return gb::typical_bucket(std::vector<size_t>(sizes, sizes + n), c, precomputed != 0);
 }
 uint32_t r_short_span(double mean, double typical, uint32_t L) { return gb::short_span(mean, typical, L); }
+size_t r_table_items(size_t K, size_t n) { return gb::table_items(K, n); }
 uint64_t r_rounds_limit() { return gb::kRoundsScratch; }
 // the groups' first items and the end into out (n + 1 places at most); how many
 size_t r_groups(const size_t *sizes, size_t n, int c, int precomputed, size_t *out)

@@ -587,3 +587,22 @@ def test_uneven_context_batches(gb, orc, sizes):
         assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases[p0:p0 + m], scal[o:o + m]))).all(), i
     ctx.close()
     dv.free()
+
+
+@pytest.mark.parametrize("small,n", [(8, 300), (50, 512), (50, 600), (4, 20)])
+def test_small_items_of_a_large_context(gb, orc, small, n):
+    """Items below an eighth of a 2^17 context's buckets, few enough for the
+    table and too many, alone and behind a large one."""
+    rng = np.random.default_rng(small + n)
+    bases = gb.g1_generator_mul(orc.fr_random(1 << 17, rng))
+    ctx = gb.Bls12_381G1MsmContext(bases)
+    for large in (0, 5000):
+        sizes = ([large] if large else []) + [n + i for i in range(small)]
+        off = np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(int)
+        scal = orc.fr_random(sum(sizes), rng)
+        dv = gb.Bls12_381FrDeviceVec.upload(scal)
+        got = ctx.device_ragged(dv, [(int(o), i, m) for i, (o, m) in enumerate(zip(off, sizes))])
+        for i, (o, m) in enumerate(zip(off, sizes)):
+            assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases[i:i + m], scal[o:o + m]))).all(), i
+        dv.free()
+    ctx.close()

@@ -25,6 +25,8 @@ def rules(tmp_path_factory):
     L.r_scratch.argtypes = [u64, u64, ctypes.c_int, u64]
     L.r_scratch.restype = L.r_rounds_limit.restype = u64
     L.r_groups.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
+    L.r_table_items.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
+    L.r_table_items.restype = ctypes.c_size_t
     L.r_groups.restype = ctypes.c_size_t
     L.r_typical.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int]
     L.r_typical.restype = ctypes.c_double
@@ -105,3 +107,12 @@ def test_typical_bucket(rules, c, precomputed):
         assert 0.5 * large < t <= large
         mean = sum(sizes) / len(sizes) * rows / (1 << (c - 1))
         assert all(rules.r_short_span(mean, t, L) >= min(32, large / L) for L in range(3, 65))
+
+
+@pytest.mark.parametrize("K,n,count,table", [  # both routes measured, the faster one
+    (1 << 15, 512, 32, True), (1 << 15, 512, 48, False), (1 << 15, 512, 512, False), (1 << 15, 1024, 32, True),
+    (1 << 15, 1024, 64, False), (1 << 15, 2048, 64, True), (1 << 15, 2048, 96, False), (1 << 15, 4095, 96, True),
+    (1 << 15, 4095, 192, False), (1 << 14, 256, 192, True), (1 << 14, 256, 512, False), (1 << 14, 1024, 192, True),
+    (1 << 14, 1024, 512, False), (1 << 14, 2047, 192, True), (1 << 12, 64, 512, True), (1 << 12, 511, 512, True)])
+def test_many_small_items_leave_the_table(rules, K, n, count, table):
+    assert (count <= rules.r_table_items(K, n)) == table
