@@ -1147,14 +1147,15 @@ __device__ void coop_add(const coop_t &c, int a, int q)
     c.sync();
 }
 
-// the GROUPS groups of a block add their SUM slots into group 0's
-template <uint32_t GROUPS>
-__device__ void coop_block_tree(fp_t *sh, const coop_t &c, uint32_t grp)
+// `groups` groups side by side (a power of two; `part` is a group's place among
+// them) add their SUM slots into the first one's; every thread of the block
+// takes part
+__device__ void coop_tree(const coop_t &c, uint32_t part, uint32_t groups)
 {
-    for (uint32_t off = GROUPS / 2; off > 0; off >>= 1) {
+    for (uint32_t off = groups / 2; off > 0; off >>= 1) {
         __syncthreads();
-        if (grp < off) {
-            coop_copy(c, c.s + CO_OPD, sh + (size_t)(grp + off) * CO_SLOTS + CO_SUM);
+        if (part < off) {
+            coop_copy(c, c.s + CO_OPD, c.s + off * CO_SLOTS + CO_SUM);
             coop_add(c, CO_SUM, CO_OPD);
         }
     }
@@ -1245,7 +1246,7 @@ __global__ void __launch_bounds__(kLongGroups *kCoopLanes)
             coop_load(c, CO_OPD, !direct ? share + k : cs + k == ce ? head + ce : tail + cs + k);
             coop_add(c, CO_SUM, CO_OPD);
         }
-        coop_block_tree<kLongGroups>(mem, c, grp);
+        coop_tree(c, grp, kLongGroups);
         if (grp == 0) coop_store(c, CO_SUM, buckets + g);
         __syncthreads();
     }
@@ -1298,58 +1299,63 @@ __global__ void __launch_bounds__(128) msm_line_partial_kernel(const xyzz_t *__r
     partial[seg * 2 * half + to] = acc;
 }
 
-// 8b'. whole line sums, a block a line, from the partials (lm > 0) or the
-//      buckets (lm = 0)
+// 8b'. whole line sums, 2^log_groups groups of lanes a line and a block's 32
+//      groups on as many lines, from the partials (lm > 0) or the buckets (lm =
+//      0).  Few lines take a block each; of many lines, which the number of
+//      resident blocks bounds, short ones share a block (see sum_groups).
 __global__ void __launch_bounds__(128) msm_line_sum_kernel(const xyzz_t *__restrict__ src, line_shape sh, uint32_t lm,
+                                                           uint32_t log_groups, uint32_t total,
                                                            xyzz_t *__restrict__ lines)
 {
     __shared__ __align__(16) fp_t mem[kCoopGroups * CO_SLOTS];
-    const uint32_t grp = threadIdx.x / kCoopLanes;
     const coop_t c(mem);
+    const uint32_t grp = threadIdx.x / kCoopLanes, groups = 1u << log_groups, part = grp & (groups - 1);
+    const uint32_t at = (blockIdx.x * kCoopGroups + grp) >> log_groups;
     const uint32_t lk = sh.lr + sh.lc, rows = 1u << sh.lr;
-    const uint32_t seg = blockIdx.x / sh.lines(), line = blockIdx.x % sh.lines();
+    const uint32_t seg = at / sh.lines(), line = at % sh.lines();
     const bool row = line < rows;
-    const uint32_t n = 1u << ((row ? sh.lc : sh.lr) - lm);
+    const uint32_t n = at < total ? 1u << ((row ? sh.lc : sh.lr) - lm) : 0u;
     const xyzz_t *p = src + ((uint64_t)seg << (lm ? lk + 1 - lm : lk));
     uint32_t step = 1;
     if (row) p += (uint64_t)line * n;
     else if (lm) p += ((uint64_t)1 << (lk - lm)) + (uint64_t)(line - rows) * n;
     else p += line - rows, step = 1u << sh.lc;
     coop_set_inf(c, CO_SUM);
-    for (uint32_t e = grp; e < n; e += kCoopGroups) {
+    for (uint32_t e = part; e < n; e += groups) {
         c.sync();
         coop_load(c, CO_OPD, p + (uint64_t)e * step);
         coop_add(c, CO_SUM, CO_OPD);
     }
-    coop_block_tree<kCoopGroups>(mem, c, grp);
-    if (grp == 0) coop_store(c, CO_SUM, lines + blockIdx.x);
+    coop_tree(c, part, groups);
+    if (part == 0 && n) coop_store(c, CO_SUM, lines + at);
 }
 
-// 8c'. the sums by weight bit, a block a bit: rows weigh i (bits 0 .. lr - 1,
-//      in places 2^lc and up of the result), columns j + 1 (bits 0 .. lc)
-static constexpr uint32_t kBitGroups = 32;
-
-__global__ void __launch_bounds__(kBitGroups *kCoopLanes) msm_bit_sum_kernel(const xyzz_t *__restrict__ lines,
-                                                                             line_shape sh, xyzz_t *__restrict__ bits)
+// 8c'. the sums by weight bit, 2^log_groups groups a bit: rows weigh i (bits 0
+//      .. lr - 1, in places 2^lc and up of the result), columns j + 1 (bits 0 ..
+//      lc)
+__global__ void __launch_bounds__(128) msm_bit_sum_kernel(const xyzz_t *__restrict__ lines, line_shape sh,
+                                                          uint32_t log_groups, uint32_t total,
+                                                          xyzz_t *__restrict__ bits)
 {
-    __shared__ __align__(16) fp_t mem[kBitGroups * CO_SLOTS];
-    const uint32_t grp = threadIdx.x / kCoopLanes;
+    __shared__ __align__(16) fp_t mem[kCoopGroups * CO_SLOTS];
     const coop_t c(mem);
-    const uint32_t seg = blockIdx.x / sh.bits(), place = blockIdx.x % sh.bits(), rows = 1u << sh.lr;
+    const uint32_t grp = threadIdx.x / kCoopLanes, groups = 1u << log_groups, part = grp & (groups - 1);
+    const uint32_t at = (blockIdx.x * kCoopGroups + grp) >> log_groups;
+    const uint32_t seg = at / sh.bits(), place = at % sh.bits(), rows = 1u << sh.lr;
     const bool row = place < sh.lr;
     const uint32_t b = row ? place : place - sh.lr, lw = row ? sh.lr : sh.lc;
     const xyzz_t *p = lines + (uint64_t)seg * sh.lines() + (row ? 0 : rows);
     // weights below 2^lw with bit b, or 2^lc itself for the columns' last bit
-    const uint32_t n = b < lw ? 1u << (lw - 1) : 1u;
+    const uint32_t n = at >= total ? 0u : b < lw ? 1u << (lw - 1) : 1u;
     coop_set_inf(c, CO_SUM);
-    for (uint32_t e = grp; e < n; e += kBitGroups) {
+    for (uint32_t e = part; e < n; e += groups) {
         const uint32_t w = b < lw ? (e >> b) << (b + 1) | 1u << b | (e & ((1u << b) - 1)) : 1u << b;
         c.sync();
         coop_load(c, CO_OPD, p + (row ? w : w - 1));
         coop_add(c, CO_SUM, CO_OPD);
     }
-    coop_block_tree<kBitGroups>(mem, c, grp);
-    if (grp == 0) coop_store(c, CO_SUM, bits + blockIdx.x);
+    coop_tree(c, part, groups);
+    if (part == 0 && n) coop_store(c, CO_SUM, bits + at);
 }
 
 // 8d'. the bit sums of a segment to one point, a block a segment: a group
@@ -1374,7 +1380,7 @@ __global__ void __launch_bounds__(kCombineGroups *kCoopLanes) msm_bit_combine_ke
     } else {
         coop_set_inf(c, CO_SUM);
     }
-    coop_block_tree<kCombineGroups>(mem, c, grp);
+    coop_tree(c, grp, kCombineGroups);
     if (grp == 0) coop_store(c, CO_SUM, seg_sum + blockIdx.x);
 }
 
@@ -1856,14 +1862,18 @@ static void run_planned(const batch_plan &P, const item_desc *d_items, const seg
             GB_CHECK_LAUNCH();
             src = partial;
         }
-        msm_line_sum_kernel<<<sh.lines() * nseg, 128, 0, s>>>(src, sh, lm, lines);
+        const uint32_t nlines = sh.lines() * nseg, lg = sum_groups(nlines, 1u << (sh.lc - lm), sm_count());
+        msm_line_sum_kernel<<<blocks_for((size_t)nlines << lg, kCoopGroups), 128, 0, s>>>(src, sh, lm, lg, nlines,
+                                                                                           lines);
         GB_CHECK_LAUNCH();
         xyzz_t *bit_sum = d_out;
         if (P.tail.kind != msm_tail::BITS) {
             bits = dev_buf<xyzz_t>((size_t)nseg * sh.bits(), s);
             bit_sum = bits;
         }
-        msm_bit_sum_kernel<<<sh.bits() * nseg, kBitGroups * kCoopLanes, 0, s>>>(lines, sh, bit_sum);
+        const uint32_t nbits = sh.bits() * nseg, bg = sum_groups(nbits, 1u << (sh.lc - 1), sm_count());
+        msm_bit_sum_kernel<<<blocks_for((size_t)nbits << bg, kCoopGroups), 128, 0, s>>>(lines, sh, bg, nbits,
+                                                                                         bit_sum);
         GB_CHECK_LAUNCH();
         if (P.tail.kind != msm_tail::BITS) {
             msm_bit_combine_kernel<<<nseg, kCombineGroups * kCoopLanes, 0, s>>>(bits, sh, seg_sum);

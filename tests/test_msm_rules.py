@@ -27,6 +27,7 @@ def rules(tmp_path_factory):
     L.r_groups.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
     L.r_table_items.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
     L.r_table_items.restype = ctypes.c_size_t
+    L.r_sum_groups.argtypes = [u64, ctypes.c_uint32, ctypes.c_int]
     L.r_groups.restype = ctypes.c_size_t
     L.r_typical.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int]
     L.r_typical.restype = ctypes.c_double
@@ -116,3 +117,14 @@ def test_typical_bucket(rules, c, precomputed):
     (1 << 14, 1024, 512, False), (1 << 14, 2047, 192, True), (1 << 12, 64, 512, True), (1 << 12, 511, 512, True)])
 def test_many_small_items_leave_the_table(rules, K, n, count, table):
     assert (count <= rules.r_table_items(K, n)) == table
+
+
+@pytest.mark.parametrize("log_n", range(9))
+def test_groups_a_sum(rules, log_n):
+    """Few sums get all of a block's groups; many get no more than have two
+    points each, so that none of a block's groups is idle."""
+    n = 1 << log_n
+    assert rules.r_sum_groups(8 * 152, n, 152) == 5
+    for sums in (8 * 152 + 1, 1 << 20):
+        groups = 1 << rules.r_sum_groups(sums, n, 152)
+        assert groups == max(1, min(32, n // 2))
