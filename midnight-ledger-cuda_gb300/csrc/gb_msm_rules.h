@@ -168,20 +168,21 @@ inline uint32_t sum_groups(uint64_t sums, uint32_t n, int sms)
 // small window is the less work.  But the plain MSMs are a batch of their own
 // behind the other one (1.2 ms), so items down to 1 / kTableMinRatio use the
 // table too, unless there are many.  Measured, ms by the table and plain:
-//   K = 2^15  n = 512    x32 1.75 2.33   x48 3.03 2.85   x512 27.7 12.5
-//             n = 1024   x32 2.10 2.50   x64 3.94 3.73   x512 29.0 14.9
-//             n = 2048   x64 4.25 4.36   x96 6.37 5.89   x512 31.4 19.8
-//             n = 4095   x96 7.32 8.39   x192 14.0 12.3  x512 35.8 29.6
-//   K = 2^14  n = 256    x192 5.92 7.10  x512 14.9 11.0
-//             n = 1024   x192 6.91 8.62  x512 17.0 15.0
-//             n = 2047   x192 7.95 10.4  x512 19.7 19.8
-//   K = 2^12  n = 64     x512 4.67 10.1
+//   K = 2^15  n = 512   x32 1.75 1.99  x40 2.42 2.15  x128 6.72 4.12  x384 19.4 7.19
+//             n = 1024  x32 2.10 2.16  x40 2.58 2.39  x128 7.08 4.83  x384 20.4 9.13
+//             n = 2048  x40 2.80 2.78  x64 4.00 3.66  x128 7.72 5.98  x384 22.3 12.6
+//             n = 4095  x64 4.63 5.06  x96 6.94 6.94  x128 9.02 8.76  x384 25.6 20.0
+//   K = 2^14  n = 256   x128 3.42 3.72  x192 5.15 5.01  x384 9.86 6.04
+//             n = 512   x192 5.47 5.56  x256 7.04 6.99  x384 10.5 7.19
+//             n = 1024  x192 6.15 6.50  x256 7.90 8.21  x384 11.7 9.09
+//             n = 2047  x192 7.21 8.35  x256 9.24 10.6  x384 13.5 12.6
+//   K = 2^12  n = 64    x384 3.11 5.40;  n = 511  x384 4.25 7.21
 // The number of items up to which the table is taken; n: their mean length.
 static constexpr size_t kTableRatio = 8, kTableMinRatio = 64;
 inline size_t table_items(size_t K, size_t n)
 {
-    if (K >= (size_t)1 << 15) return 32 + n / 40;
-    if (K >= (size_t)1 << 14) return 240 + n / 8;
+    if (K >= (size_t)1 << 15) return 32 + (n * n >> 18);
+    if (K >= (size_t)1 << 14) return 160 + n / 10;
     return SIZE_MAX;
 }
 

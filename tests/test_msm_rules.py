@@ -111,10 +111,11 @@ def test_typical_bucket(rules, c, precomputed):
 
 
 @pytest.mark.parametrize("K,n,count,table", [  # both routes measured, the faster one
-    (1 << 15, 512, 32, True), (1 << 15, 512, 48, False), (1 << 15, 512, 512, False), (1 << 15, 1024, 32, True),
-    (1 << 15, 1024, 64, False), (1 << 15, 2048, 64, True), (1 << 15, 2048, 96, False), (1 << 15, 4095, 96, True),
-    (1 << 15, 4095, 192, False), (1 << 14, 256, 192, True), (1 << 14, 256, 512, False), (1 << 14, 1024, 192, True),
-    (1 << 14, 1024, 512, False), (1 << 14, 2047, 192, True), (1 << 12, 64, 512, True), (1 << 12, 511, 512, True)])
+    (1 << 15, 512, 32, True), (1 << 15, 512, 48, False), (1 << 15, 512, 384, False), (1 << 15, 1024, 32, True),
+    (1 << 15, 1024, 48, False), (1 << 15, 2048, 32, True), (1 << 15, 2048, 64, False), (1 << 15, 4095, 64, True),
+    (1 << 15, 4095, 192, False), (1 << 14, 256, 128, True), (1 << 14, 256, 256, False), (1 << 14, 512, 128, True),
+    (1 << 14, 1024, 192, True), (1 << 14, 1024, 384, False), (1 << 14, 2047, 256, True), (1 << 14, 2047, 384, False),
+    (1 << 12, 64, 384, True), (1 << 12, 511, 384, True)])
 def test_many_small_items_leave_the_table(rules, K, n, count, table):
     assert (count <= rules.r_table_items(K, n)) == table
 
