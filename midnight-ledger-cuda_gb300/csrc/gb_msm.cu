@@ -557,13 +557,18 @@ template <bool REFS>
 __global__ void __launch_bounds__(kPairThreads, kPairBlocks)
     msm_affine_pairs_kernel(const uint32_t *__restrict__ refs, const affine_t *__restrict__ points,
                             affine_t *__restrict__ out, const uint32_t *__restrict__ entries, int round,
-                            uint32_t per_thread, uint4 *__restrict__ prefix)
+                            uint32_t most_per_thread, uint4 *__restrict__ prefix)
 {
     __shared__ fp_t node[2 * kPairThreads];  // product tree: root 1, leaves 128 ..
     __shared__ uint4 stage_mem[15 * kPairThreads];
     const uint32_t tid = threadIdx.x;
     const pair_stage stage{stage_mem + tid};
-    const uint64_t pairs = *entries >> round, tile = (uint64_t)kPairThreads * per_thread;
+    const uint64_t pairs = *entries >> round;
+    // the host knows a bound of the pairs only: of scalars that are zero for the
+    // most part (2^20 of them, one in ten not: 1.98 -> 1.34 ms) the tiles are
+    // shorter, so that every block has one
+    const uint32_t per_thread = min(most_per_thread, pairs_per_thread(pairs, gridDim.x));
+    const uint64_t tile = (uint64_t)kPairThreads * per_thread;
     uint4 *pre = prefix + (uint64_t)blockIdx.x * per_thread * 3 * kPairThreads + tid;
     for (uint64_t base = blockIdx.x * tile + tid; base - tid < pairs; base += gridDim.x * tile) {
         const int turns =

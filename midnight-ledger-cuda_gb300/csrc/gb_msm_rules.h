@@ -61,9 +61,9 @@ static constexpr uint32_t kPairBlocks = 4;
 static constexpr uint32_t kPairsPerThread = 64;
 
 // pairs a thread: whole waves of `slots` tiles of at most kPairsPerThread
-inline uint32_t pairs_per_thread(uint64_t pairs, uint64_t slots)
+GB_RULE uint32_t pairs_per_thread(uint64_t pairs, uint64_t slots)
 {
-    const uint64_t per = std::max<uint64_t>(1, (pairs + slots * kPairThreads - 1) / (slots * kPairThreads));
+    const uint64_t all = (pairs + slots * kPairThreads - 1) / (slots * kPairThreads), per = all ? all : 1;
     const uint64_t waves = (per + kPairsPerThread - 1) / kPairsPerThread;
     return (uint32_t)((per + waves - 1) / waves);
 }

@@ -19,6 +19,7 @@ double r_typical(const size_t *sizes, size_t n, int c, int precomputed)
 uint32_t r_short_span(double mean, double typical, uint32_t L) { return gb::short_span(mean, typical, L); }
 size_t r_table_items(size_t K, size_t n) { return gb::table_items(K, n); }
 uint32_t r_sum_groups(uint64_t sums, uint32_t n, int sms) { return gb::sum_groups(sums, n, sms); }
+uint32_t r_pairs_per_thread(uint64_t pairs, uint64_t slots) { return gb::pairs_per_thread(pairs, slots); }
 uint64_t r_rounds_limit() { return gb::kRoundsScratch; }
 // the groups' first items and the end into out (n + 1 places at most); how many
 size_t r_groups(const size_t *sizes, size_t n, int c, int precomputed, size_t *out)

@@ -606,3 +606,20 @@ def test_small_items_of_a_large_context(gb, orc, small, n):
             assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases[i:i + m], scal[o:o + m]))).all(), i
         dv.free()
     ctx.close()
+
+
+@pytest.mark.parametrize("nonzero", [0, 1, 700, 20000])
+def test_affine_rounds_of_mostly_zero_scalars(gb, orc, nonzero):
+    """Batches planned for 1.8 M pairs a round that have hardly any."""
+    rng = np.random.default_rng(nonzero)
+    n, count = 1 << 16, 3
+    bases = gb.g1_generator_mul(orc.fr_random(n, rng))
+    scal = np.zeros((count, n, 4), dtype=np.uint64)
+    for i in range(count):
+        at = rng.choice(n, size=nonzero, replace=False)
+        scal[i, at] = orc.fr_random(nonzero, rng) if nonzero else 0
+    ctx = gb.Bls12_381G1MsmContext(bases)
+    got = ctx.batch(scal)
+    for i in range(count):
+        assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
+    ctx.close()

@@ -28,6 +28,7 @@ def rules(tmp_path_factory):
     L.r_table_items.argtypes = [ctypes.c_size_t, ctypes.c_size_t]
     L.r_table_items.restype = ctypes.c_size_t
     L.r_sum_groups.argtypes = [u64, ctypes.c_uint32, ctypes.c_int]
+    L.r_pairs_per_thread.argtypes = [u64, u64]
     L.r_groups.restype = ctypes.c_size_t
     L.r_typical.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int]
     L.r_typical.restype = ctypes.c_double
@@ -129,3 +130,19 @@ def test_groups_a_sum(rules, log_n):
     for sums in (8 * 152 + 1, 1 << 20):
         groups = 1 << rules.r_sum_groups(sums, n, 152)
         assert groups == max(1, min(32, n // 2))
+
+
+def test_tiles_of_fewer_pairs_than_planned(rules):
+    """The rounds' kernel makes its tiles from the pairs that there are, with
+    no more a thread than planned: each block then has a tile as long as there
+    are pairs for one, and none is longer than the prefix buffer's."""
+    for lg in np.arange(20, 30, 0.3):
+        planned = int(2 ** lg)
+        most = rules.r_pairs_per_thread(planned, SLOTS)
+        assert 1 <= most <= 64
+        for share in (1, 2, 3, 10, 1000, planned):
+            pairs = planned // share
+            per = min(most, rules.r_pairs_per_thread(pairs, SLOTS))
+            assert 1 <= per <= most
+            tiles = -(-pairs // (per * 128))
+            assert tiles >= min(SLOTS, -(-pairs // 128)) // 2
