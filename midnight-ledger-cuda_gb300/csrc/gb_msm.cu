@@ -1621,7 +1621,7 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
     uint64_t points_total = 0, digits_total = 0;
     for (uint32_t m = 0; m < nitems; m++) {
         const msm_item &it = items[m];
-        if (it.n >= 0x7fffffffull / (uint64_t)nwin) throw cuda_error((int)cudaErrorInvalidValue, "MSM too large");
+        if (it.n >= kMaxDigits / (uint64_t)nwin) throw cuda_error((int)cudaErrorInvalidValue, "MSM too large");
         idesc[m] = item_desc{it.scalars, points_total, digits_total, (uint32_t)it.n};
         for (uint32_t j = 0; j < segs_per_item; j++) {
             seg_desc &sd = sdesc[m * segs_per_item + j];

@@ -32,6 +32,9 @@ GB_RULE int window_offset(int c, int j)
     return j < wide ? j * c : wide * c + (j - wide) * (c - 1);
 }
 
+// an MSM's digits are numbered with 31 bits
+static constexpr uint64_t kMaxDigits = 0x7fffffff;
+
 // Window size for n points, measured on GB300.  With the precomputed table an
 // MSM has 2^(c - 1) buckets in all: ms a call for one and for three MSMs (*
 // chosen)
@@ -51,7 +54,9 @@ inline int choose_window(size_t n, bool precomputed)
 {
     auto upto = [&](int lg) { return n <= (size_t)1 << lg; };
     if (precomputed) return upto(7) ? 8 : upto(11) ? 11 : upto(12) ? 12 : upto(15) ? 13 : upto(16) ? 15 : 16;
-    return upto(11) ? 8 : upto(13) ? 9 : upto(15) ? 10 : upto(17) ? 11 : upto(19) ? 12 : 13;
+    int c = upto(11) ? 8 : upto(13) ? 9 : upto(15) ? 10 : upto(17) ? 11 : upto(19) ? 12 : 13;
+    while (c < kMaxWindowBits && n >= kMaxDigits / windows_for(c)) c++;  // 107 M points with 13 bits, 134 M with 16
+    return c;
 }
 
 // Affine rounds (see msm_affine_pairs_kernel): tiles of kPairThreads x up to

@@ -146,3 +146,13 @@ def test_tiles_of_fewer_pairs_than_planned(rules):
             assert 1 <= per <= most
             tiles = -(-pairs // (per * 128))
             assert tiles >= min(SLOTS, -(-pairs // 128)) // 2
+
+
+def test_no_size_is_refused_for_its_window(rules):
+    """Digits are numbered with 31 bits, and the widest windows have the fewest:
+    whatever these can number, the chosen window can."""
+    for n in [1, 255, 1 << 16, (1 << 24) + 1, 107_374_181, 107_374_182, 113_000_000, 120_000_000, 134_217_726]:
+        assert n < 0x7FFFFFFF // rules.r_windows(16)
+        for precomputed in (0, 1):
+            assert n < 0x7FFFFFFF // rules.r_windows(rules.r_choose_window(n, precomputed)), n
+    assert [rules.r_choose_window(1 << k, 0) for k in (11, 13, 15, 17, 19, 26)] == [8, 9, 10, 11, 12, 13]
