@@ -113,3 +113,17 @@ def test_eval_many_slice_edges(gb, orc, ln, requests):
     for r in range(0, requests, 101):
         assert (got[r][0] == orc.fr_eval_poly(coeffs, points[r])).all()
     dv.free()
+
+
+def test_kate_divide_by_x_is_a_copy(gb, orc):
+    """Point zero: one launch, whatever the length."""
+    ln, count = 5000, 3
+    polys = orc.fr_random(ln * count, np.random.default_rng(9))
+    dv = gb.Bls12_381FrDeviceVec.upload(polys)
+    before = gb.launch_counter()
+    q = gb.fr_device_kate_divide(dv, ln, count, np.zeros(4, dtype=np.uint64))
+    assert gb.launch_counter() == before + 1
+    got, polys = q.download().reshape(count, ln, 4), polys.reshape(count, ln, 4)
+    assert (got[:, :-1] == polys[:, 1:]).all() and (got[:, -1] == 0).all()
+    q.free()
+    dv.free()
