@@ -17,7 +17,7 @@
 
 namespace gb {
 
-static constexpr int kEvalThreads = 256;
+static constexpr int kEvalThreads = 256;  // 2^8
 
 // The loops around products stay loops (unroll 1): these kernels run for
 // microseconds from a cold instruction cache, and a product is 5 KB of code
@@ -38,106 +38,147 @@ struct eval_pair {
     uint32_t row;
 };
 
-// One slice of 256 * per coefficients of one polynomial a block: out[p *
-// slices + slice] = its value at y = points[row]^(2^squarings).  Thread t runs
-// Horner's rule in y^256 over the coefficients t, t + 256, .. of the slice,
-// then the threads are folded by y^128, y^64, .. y.  A chain of 16 + per
-// dependent products bounds it at per = 16, so the coefficients are read 4
-// ahead and one warp has the powers ready (40 polynomials of 2^12 coefficients
-// 48 -> 26 us, of 2^16 87 -> 45).
-// Given flat, polynomial p lies at flat + p * len.
-__global__ void __launch_bounds__(kEvalThreads) eval_slices_kernel(const eval_pair *__restrict__ pairs,
-                                                                   const fr_t *__restrict__ flat, size_t len,
-                                                                   const fr_t *__restrict__ points, int squarings,
-                                                                   int per, uint32_t slices, fr_t *__restrict__ out)
+// One slice of T * per coefficients (T = 2^LOG_T threads, per a multiple of 4)
+// of one polynomial a block: out[p * slices + slice] = its value at y =
+// points[row]^(2^squarings).  Thread t runs Horner's rule in y^T over the
+// coefficients t, t + T, .. of the slice, then the threads are folded by
+// y^(T/2), .. y.  With T = 256 and per = 16 a chain of 16 + per dependent products
+// bounds it, so the coefficients are read 4 ahead and one warp has the powers
+// ready (40 polynomials of 2^12 coefficients 48 -> 26 us, of 2^16 87 -> 45).  T =
+// 32 is for many or short polynomials, which are bound by the products that do
+// not depend on their length: no warp is idle in the folds.  Given flat,
+// polynomial p lies at flat + p * len; without pairs all are evaluated at the
+// first point.  With `ready` the points come with their powers y^(2^s), s = 0 ..
+// LOG_T.
+template <int LOG_T>
+__global__ void __launch_bounds__(1 << LOG_T) eval_slices_kernel(const eval_pair *__restrict__ pairs,
+                                                                 const fr_t *__restrict__ flat, size_t len,
+                                                                 const fr_t *__restrict__ points, bool ready,
+                                                                 int squarings, int per, uint32_t slices,
+                                                                 fr_t *__restrict__ out)
 {
-    __shared__ fr_t sh[kEvalThreads], pw[9];  // pw[s] = y^(2^s)
-    const size_t p = blockIdx.y, lo = (size_t)blockIdx.x * per * kEvalThreads, t = threadIdx.x;
-    const eval_pair e = pairs[p];
+    constexpr size_t T = 1 << LOG_T;
+    __shared__ fr_t sh[T], pw[LOG_T + 1];  // pw[s] = y^(2^s)
+    const size_t p = blockIdx.y, lo = (size_t)blockIdx.x * per * T, t = threadIdx.x;
+    const eval_pair e = pairs ? pairs[p] : eval_pair{nullptr, 0};
     const fr_t *c = (flat ? flat + p * len : e.polys) + lo + t;
-    const size_t left = lo + t < len ? len - (lo + t) : 0;
+    const size_t left = lo + t < len ? len - (lo + t) : 0, row = min(len - lo, T);  // row: threads with coefficients
     auto load = [&](fr_t *v, int k) {  // coefficients k .. k + 3 of the thread
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-            v[u] = (size_t)(k + u) * kEvalThreads < left ? c[(size_t)(k + u) * kEvalThreads] : fr_t::zero();
+        for (int u = 0; u < 4; u++) v[u] = (size_t)(k + u) * T < left ? c[(size_t)(k + u) * T] : fr_t::zero();
     };
     fr_t now[4], next[4];
     load(now, per - 4);
-    if (t < 32) {
+    if (ready) {
+        if (t <= LOG_T) pw[t] = points[e.row * (LOG_T + 1) + t];
+    } else if (t < 32) {
         fr_t y = points[e.row];
 #pragma unroll 1
         for (int k = 0; k < squarings; k++) y = y.sqr();
 #pragma unroll 1
-        for (int k = 0; k < 9; k++) {
+        for (int k = 0; k <= LOG_T && (len - lo > T || ((size_t)1 << k) < row); k++) {
             if (t == 0) pw[k] = y;
-            if (k < 8) y = y.sqr();
+            if (k < LOG_T) y = y.sqr();
         }
     }
     __syncthreads();
-    const fr_t y = pw[8];
+    const fr_t y = pw[LOG_T];
     fr_t acc = fr_t::zero();
+    bool any = false;  // conditions on these rows are the same for the block
     for (int k = per - 4; k >= 0; k -= 4) {
         if (k) load(next, k - 4);
-        if (lo + (size_t)k * kEvalThreads < len) {  // the same for the block
 #pragma unroll
-            for (int u = 3; u >= 0; u--) acc = acc * y + now[u];
+        for (int u = 3; u >= 0; u--) {
+            if (lo + (size_t)(k + u) * T >= len) continue;
+            if (any) acc = acc * y;
+            acc = acc + now[u];
+            any = true;
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) now[u] = next[u];
     }
     sh[t] = acc;
 #pragma unroll 1
-    for (int k = 7; k >= 5; k--) {
+    for (int k = LOG_T - 1; k >= 5; k--) {
         __syncthreads();
         if (t < (1u << k)) sh[t] = sh[t] + sh[t + (1u << k)] * pw[k];
     }
     if (t >= 32) return;
     acc = sh[t];
 #pragma unroll 1
-    for (int k = 4; k >= 0; k--) acc = acc + lane_down(acc, 1u << k) * pw[k];
+    for (int k = 4; k >= 0; k--)
+        if ((1u << k) < row) acc = acc + lane_down(acc, 1u << k) * pw[k];
     if (t == 0) out[p * slices + blockIdx.x] = acc;
 }
 
-// evaluations of pairs (pair p: len coefficients at pairs[p].polys, at the host
-// point points[pairs[p].row]) into d_out; the slices' values are the
-// coefficients of a polynomial in point^slice, evaluated the same way
-static void eval_pairs(fr_t *d_out, const std::vector<eval_pair> &pairs, const RawFr *points, size_t npoints,
-                       size_t len, cudaStream_t s)
+// Values of `total` polynomials of len coefficients into d_out: pair p's at its
+// point, or, without pairs (null), those in a row at `flat` at points[0]; on the
+// host: npoints points.  The slices' values are the coefficients of a polynomial
+// in point^slice, evaluated the same way.
+static void eval_pairs(fr_t *d_out, const std::vector<eval_pair> *pairs, const fr_t *flat, size_t total,
+                       const RawFr *points, size_t npoints, size_t len, cudaStream_t s)
 {
-    const size_t total = pairs.size(), chunk = 65535;  // grid.y limit
+    const size_t chunk = 65535;  // grid.y limit
     if (!total) return;
     if (npoints > 65535 && len <= ((size_t)1 << 24))
         throw cuda_error((int)cudaErrorInvalidValue, "too many evaluation points");
-    dev_buf<fr_t> d_points(npoints, s);
-    h2d(d_points, points, npoints * sizeof(fr_t), s);
-    dev_buf<eval_pair> d_pairs(total, s);
-    h2d(d_pairs, pairs.data(), total * sizeof(eval_pair), s);
+    // A warp a polynomial for short ones and for many (measured, us with 256
+    // threads and with a warp: 1000 polynomials of 256 coefficients 84 35, 20000
+    // 1146 186, 40 of 512 35 36, of 1024 35 45; 600 of 2048 72 70, 1000 of 4096 146
+    // 133)
+    const bool warps = len <= 512 || (len <= 4096 && total >= 456) || (len <= 6144 && total >= 1000);
+    // points of many polynomials each: their powers made here, once
+    const bool ready = warps && npoints * 16 <= total;
+    dev_buf<fr_t> d_points(npoints * (ready ? 6 : 1), s);
+    if (ready) {
+        std::vector<fr_t> powers(npoints * 6);
+        for (size_t q = 0; q < npoints; q++) {
+            powers[6 * q] = from_raw(points[q]);
+            for (int k = 1; k < 6; k++) powers[6 * q + k] = powers[6 * q + k - 1].sqr();
+        }
+        h2d(d_points, powers.data(), powers.size() * sizeof(fr_t), s);
+    } else {
+        h2d(d_points, points, npoints * sizeof(fr_t), s);
+    }
+    dev_buf<eval_pair> d_pairs(pairs ? total : 0, s);
+    if (pairs) h2d(d_pairs, pairs->data(), total * sizeof(eval_pair), s);
     dev_buf<fr_t> values;
-    // 64 coefficients a thread where that leaves two waves of blocks, which
-    // spares the products of the squarings and folds; else 16, to be short
-    const int log_per = total * (len >> 14) >= 608 ? 6 : 4;
+    // Coefficients a thread: up to 64 where that leaves two waves of blocks, or
+    // covers the polynomial and there are many, which spares the products of the
+    // squarings and folds (2000 polynomials of 8192 coefficients 650 -> 407 us);
+    // else 16, to be short
+    auto blocks = [&](int log) { return total * ((len + ((size_t)kEvalThreads << log) - 1) >> (8 + log)); };
+    int log_per = 4;
+    while (log_per < 6 && len > (size_t)kEvalThreads << log_per &&
+           (blocks(log_per + 1) >= 608 || (total >= 304 && len <= (size_t)kEvalThreads << 6)))
+        log_per++;
     for (int squarings = 0;; squarings += 8 + log_per) {
-        const size_t slice = (size_t)kEvalThreads << log_per;
+        const size_t slice = warps ? len : (size_t)kEvalThreads << log_per;
         const uint32_t slices = (uint32_t)((len + slice - 1) / slice);
         dev_buf<fr_t> next(slices > 1 ? total * slices : 0, s);
         fr_t *out = slices > 1 ? next.get() : d_out;
         for (size_t b = 0; b < total; b += chunk) {
-            eval_slices_kernel<<<dim3(slices, (unsigned)std::min(chunk, total - b)), kEvalThreads, 0, s>>>(
-                d_pairs.get() + b, values ? values.get() + b * len : nullptr, len, d_points, squarings, 1 << log_per,
-                slices, out + b * slices);
+            const eval_pair *dp = pairs ? d_pairs.get() + b : nullptr;
+            const fr_t *df = flat ? flat + b * len : nullptr;
+            const dim3 grid(slices, (unsigned)std::min(chunk, total - b));
+            if (warps)
+                eval_slices_kernel<5><<<grid, 32, 0, s>>>(dp, df, len, d_points, ready, 0,
+                                                          (int)((len + 127) / 128 * 4), 1, out + b);
+            else
+                eval_slices_kernel<8><<<grid, kEvalThreads, 0, s>>>(dp, df, len, d_points, false, squarings,
+                                                                    1 << log_per, slices, out + b * slices);
             GB_CHECK_LAUNCH();
         }
         if (slices == 1) return;
         len = slices;
         values = std::move(next);
+        flat = values;
     }
 }
 
 static void eval_polys(fr_t *d_out, const fr_t *polys, size_t len, size_t count, const RawFr &z, cudaStream_t s)
 {
-    std::vector<eval_pair> pairs(count);
-    for (size_t p = 0; p < count; p++) pairs[p] = eval_pair{polys + p * len, 0};
-    eval_pairs(d_out, pairs, &z, 1, len, s);
+    eval_pairs(d_out, nullptr, polys, count, &z, 1, len, s);
 }
 
 // Kate quotient.  With the coefficients taken from the top, a_t =
@@ -403,7 +444,7 @@ static void multiopen_prepare_core(fr_t *d_q, fr_t *d_eval, const std::vector<co
     }
     std::vector<eval_pair> pairs(query_count);
     for (size_t r = 0; r < query_count; r++) pairs[r] = eval_pair{polys[query_poly_indices[r]], query_point_indices[r]};
-    eval_pairs(d_eval, pairs, points, point_count, len, s);
+    eval_pairs(d_eval, &pairs, nullptr, query_count, points, point_count, len, s);
 }
 
 }  // namespace gb
@@ -453,7 +494,7 @@ RustError gb_fr_device_eval_many(RawFr *out_raw, const void *const *vecs, const 
     for (size_t r = 0; r < requests; r++) device_vec_wait(reinterpret_cast<const fr_device_vec *>(vecs[r]), s);
     const size_t total = pairs.size();
     dev_buf<fr_t> d_out(total, s);
-    eval_pairs(d_out, pairs, points_raw, requests, poly_len, s);
+    eval_pairs(d_out, &pairs, nullptr, total, points_raw, requests, poly_len, s);
     d2h(out_raw, d_out, total * sizeof(fr_t), s);
     lane_sync(s);
     return ok();

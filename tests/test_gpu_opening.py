@@ -115,6 +115,37 @@ def test_eval_many_slice_edges(gb, orc, ln, requests):
     dv.free()
 
 
+@pytest.mark.parametrize("ln,count", [(1, 1), (1, 700), (31, 3), (32, 40), (33, 40), (127, 2), (512, 3), (512, 70000),
+                                      (513, 3), (513, 455), (513, 456), (4096, 456), (4097, 304), (4097, 455),
+                                      (4097, 1000), (6145, 1000), (8193, 304), (16385, 304), (16384, 303)])
+def test_eval_polys_forms(gb, orc, ln, count):
+    """Polynomials by a warp and by 256 threads each, with 16, 32 and 64
+    coefficients a thread, one slice and several, in one call and at one point."""
+    rng = np.random.default_rng(ln + count)
+    dv = gb.fr_random_chacha20(bytes(range(32)), 0, ln * count)[0]
+    z = orc.fr_random(1, rng)[0]
+    got = gb.bls12_381_fr_device_eval_polys(dv, ln, count, z)
+    some = sorted({0, count // 2, count - 1} | set(range(0, count, max(1, count // 5))))
+    host = dv.download().reshape(count, ln, 4)
+    for p in some:
+        assert (got[p] == orc.fr_eval_poly(host[p], z)).all(), p
+    dv.free()
+
+
+def test_eval_many_short_at_many_points(gb, orc):
+    """A warp a polynomial with the powers made there (many points) and with
+    the points' powers given (few points, many polynomials each)."""
+    rng = np.random.default_rng(8)
+    for ln, requests, count in ((40, 300, 1), (40, 3, 100), (700, 500, 1), (700, 2, 300)):
+        coeffs, points = orc.fr_random(ln * count, rng), orc.fr_random(requests, rng)
+        dv = gb.Bls12_381FrDeviceVec.upload(coeffs)
+        got = gb.fr_device_eval_many([(dv, count, z) for z in points], ln)
+        for r in range(0, requests, max(1, requests // 7)):
+            for p in range(0, count, max(1, count // 5)):
+                assert (got[r][p] == orc.fr_eval_poly(coeffs[p * ln:(p + 1) * ln], points[r])).all(), (r, p)
+        dv.free()
+
+
 def test_kate_divide_by_x_is_a_copy(gb, orc):
     """Point zero: one launch, whatever the length."""
     ln, count = 5000, 3
