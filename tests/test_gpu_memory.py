@@ -155,3 +155,30 @@ def test_batches_with_much_scratch_are_not_captured(gb, orc):
     assert gb.msm_graph_stats()[0] == captures + 1
     ctx.close()
     dv.free()
+
+
+def test_grand_products_scratch(gb, orc):
+    """12 chained sets over 2^18 rows take their result and little beside it."""
+    rng = np.random.default_rng(7)
+    n, m = 1 << 18, 12
+    cols = gb.fr_random_chacha20(bytes(range(32)), 0, n * m)[0]
+    perms = gb.fr_random_chacha20(bytes(range(1, 33)), 0, n * m)[0]
+    beta, gamma = orc.fr_random(2, rng)
+    deltas, blinds = orc.fr_random(m, rng), orc.fr_random(m, rng)
+    rt, pool, v = _cudart(), ctypes.c_void_p(), ctypes.c_uint64()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+
+    def products():
+        out = gb.fr_permutation_products_device(cols, perms, n, m, 1, beta, gamma, orc.fr_omega(18), deltas, blinds, 1)
+        out.download(1)
+        out.free()
+
+    products()
+    assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(v)) == 0  # cudaMemPoolAttrUsedMemCurrent
+    used = v.value
+    assert rt.cudaMemPoolSetAttribute(pool, 8, ctypes.byref(ctypes.c_uint64(0))) == 0  # cudaMemPoolAttrUsedMemHigh
+    products()
+    assert rt.cudaMemPoolGetAttribute(pool, 8, ctypes.byref(v)) == 0
+    assert v.value - used < 32 * n * m * 1.25
+    cols.free()
+    perms.free()
