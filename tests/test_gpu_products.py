@@ -137,3 +137,75 @@ def test_device_vector_ops(gb, orc):
     assert (da.download() == a2).all()
     with pytest.raises(gb.MsmError):
         da.scatter_host(np.array([300], dtype=np.uint32), vals[:1])
+
+
+def _scalars(orc, rng, *shape):
+    return orc.fr_random(int(np.prod(shape)), rng).reshape(*shape, 4)
+
+
+def _negated_sum(orc, a, b):
+    """-(a + b)"""
+    return orc.fr_from_ints([(-x - y) % orc.R_MOD for x, y in zip(orc.fr_to_ints(a), orc.fr_to_ints(b))])
+
+
+@pytest.mark.parametrize("ln,cc", [(1, 1), (255, 2), (257, 3), (1 << 15, 3), ((1 << 15) + 1, 3), ((1 << 16) + 1, 2),
+                                   (1 << 17, 4), ((1 << 18) - 1, 2), ((1 << 20) + 1300, 3)])
+def test_permutation_products_tile_edges(gb, orc, ln, cc):
+    """1, 2 and 4 rows a thread (above 2^15 and 2^16), lengths that end inside
+    a tile, chained sets, the scan of the tiles' products (above 2^20 rows), and
+    rows whose denominator is zero."""
+    rng = np.random.default_rng(ln + cc)
+    bf = min(5, ln - 1)
+    cols, perms = _scalars(orc, rng, cc, ln), _scalars(orc, rng, cc, ln)
+    beta, gamma = orc.fr_random(2, rng)
+    deltas, blinds = orc.fr_random(cc, rng), orc.fr_random(cc * max(bf, 1), rng)
+    omega = orc.fr_random(1, rng)[0]
+    if ln > 256:  # v + beta s + gamma = 0, late enough for the products before to be seen
+        at = rng.choice(np.arange(ln * 3 // 4, ln), size=3, replace=False)
+        inv = orc.fr_inv(beta)
+        perms[cc - 1, at] = [orc.fr_mul(w, inv) for w in _negated_sum(orc, cols[cc - 1, at], np.tile(gamma, (3, 1)))]
+    flat = lambda a: np.ascontiguousarray(a.reshape(-1, 4))  # noqa: E731
+    want = orc.fr_permutation_products(flat(cols), flat(perms), ln, cc, 1, beta, gamma, omega, deltas, blinds, bf)
+    got = gb.bls12_381_fr_permutation_products(flat(cols), flat(perms), ln, cc, 1, beta, gamma, omega, deltas, blinds,
+                                               bf)
+    assert (got.download() == want).all()
+    got.free()
+
+
+@pytest.mark.parametrize("ln,lc", [(257, 2), ((1 << 15) + 1, 2), ((1 << 16) + 1, 3), ((1 << 20) + 1300, 2)])
+def test_lookup_products_tile_edges(gb, orc, ln, lc):
+    rng = np.random.default_rng(ln + lc)
+    bf = 4
+    ci, ct, pi, pt = (_scalars(orc, rng, lc * ln) for _ in range(4))
+    beta, gamma = orc.fr_random(2, rng)
+    blinds = orc.fr_random(lc * bf, rng)
+    at = rng.choice(np.arange(ln * 3 // 4, ln), size=2, replace=False)
+    pi[at] = _negated_sum(orc, np.tile(beta, (2, 1)), orc.fr_from_ints([0, 0]))
+    want = orc.fr_lookup_products(ci, ct, pi, pt, ln, lc, beta, gamma, blinds, bf)
+    got = gb.bls12_381_fr_lookup_products(ci, ct, pi, pt, ln, lc, beta, gamma, blinds, bf)
+    assert (got.download() == want).all()
+    got.free()
+
+
+@pytest.mark.parametrize("ln", [1, 2, 255, 257, 1024, 1025, (1 << 18) - 1, 1 << 18, (1 << 18) + 1, (1 << 18) + 2049])
+def test_invert_assign_tile_edges(gb, orc, ln):
+    """4 and 8 elements a thread (above 2^18), partial tiles, zeros among them."""
+    rng = np.random.default_rng(ln)
+    v = orc.fr_random(ln, rng)
+    v[::97] = 0
+    assert (gb.bls12_381_fr_invert_assign(v.copy()) == orc.fr_batch_invert(v)).all()
+    assert (gb.bls12_381_fr_invert_assign(np.zeros_like(v)) == 0).all()
+
+
+def test_inversion_with_factors_above_2p18(gb, orc):
+    """num / den of more than 2^18 values: the Lagrange bases of an SRS of
+    2^19, [(tau^n - 1) / n * w^i / (tau - w^i)] G."""
+    k, tau, R = 19, 0x1234567, orc.R_MOD
+    from gb_prover.kzg import ParamsKZG
+    gl = ParamsKZG.unsafe_setup(k, orc.fr_from_ints([tau])[0]).g_lagrange
+    n, w = 1 << k, orc.fr_to_ints(orc.fr_omega(k))[0]
+    rng = np.random.default_rng(19)
+    at = [0, 1, 2047, 2048, n - 1] + [int(i) for i in rng.integers(0, n, size=20)]
+    scale = (pow(tau, n, R) - 1) * pow(n, -1, R) % R
+    terms = [scale * pow(w, i, R) * pow(tau - pow(w, i, R), -1, R) % R for i in at]
+    assert (gl[at] == orc.g1_generator_mul_batch(orc.fr_from_ints(terms))).all()
