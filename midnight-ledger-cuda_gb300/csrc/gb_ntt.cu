@@ -1120,6 +1120,12 @@ const fr_t *pass_twiddles(uint32_t log_n, bool inverse, int s_hi, int g, const f
 }
 }  // namespace
 
+// The staged passes read tables of 64 bytes an element of the transform and go
+// through a scratch copy of the batch.  Where the device has no room for these
+// (a transform of 2^31 values is 64 GiB, its tables 128), the passes that read
+// their twiddles from the common table work in place.
+static bool without_room(const cuda_error &e) { return e.code() == (int)cudaErrorMemoryAllocation; }
+
 // The staged-twiddle transform (variants 4 and 5: 4 or 8 elements per
 // thread), natural order out with the output factors applied.  With two or
 // more passes the first pass writes to a scratch buffer, the middle ones work
@@ -1134,6 +1140,11 @@ static void ntt_staged(fr_t *d, uint32_t log_n, size_t count, bool inverse, cons
     const auto passes = pass_split(log_n);
     const size_t P = passes.size();
     if (in && P < 2) throw cuda_error(-1, "fused NTT input needs two or more passes");
+    // all memory before the first launch: without it nothing is queued, and the
+    // values are as they were (see without_room)
+    const fr_t *tables[4] = {};
+    for (size_t i = 0; i < P; i++)
+        tables[i] = pass_twiddles(log_n, inverse, passes[i].first, passes[i].second, tw, s);
     dev_buf<fr_t> tmp(P > 1 ? count << log_n : 0, s);
     const ntt_factors none{{fr_t::one(), fr_t::one(), fr_t::one()}, 0};
     const ntt_input no_in{nullptr, 0, none};
@@ -1144,7 +1155,7 @@ static void ntt_staged(fr_t *d, uint32_t log_n, size_t count, bool inverse, cons
         const bool last = i + 1 == P;
         const fr_t *src = i == 0 ? d : tmp.get();
         fr_t *dst = last ? d : tmp.get();
-        const fr_t *tab = pass_twiddles(log_n, inverse, s_hi, g, tw, s);
+        const fr_t *tab = tables[i];
         int q = kPassBits - g;
         size_t ctas;
         auto ctas_for = [&](int qq) {
@@ -1309,7 +1320,14 @@ static void ntt_transform(fr_t *d, uint32_t log_n, size_t count, bool inverse, c
 {
     const size_t n = (size_t)1 << log_n;
     if (v >= 4 && log_n >= 3) {
-        ntt_staged(d, log_n, count, inverse, tw, v == 5 ? 3 : 2, fac, status, s);
+        try {
+            ntt_staged(d, log_n, count, inverse, tw, v == 5 ? 3 : 2, fac, status, s);
+        } catch (const cuda_error &e) {
+            if (!without_room(e)) throw;
+            constexpr size_t kMaxY = 65535;
+            for (size_t p = 0; p < count; p += kMaxY)
+                ntt_transform(d + (p << log_n), log_n, std::min(kMaxY, count - p), inverse, tw, 3, fac, status, s);
+        }
         return;
     }
     if (log_n > 0) ntt_passes(d, log_n, count, tw, v >= 4 ? 2 : v, s);
@@ -1395,8 +1413,12 @@ static void ntt_padded(fr_t *out, const fr_t *src, size_t in_len, size_t count, 
     const int v = log_n ? ntt_variant(out, log_n, false, tw, status, s) : 1;
     if (v >= 4 && pass_split(log_n).size() >= 2) {
         const ntt_input in{src, in_len, infac};
-        ntt_staged(out, log_n, count, false, tw, v == 5 ? 3 : 2, outfac, status, s, &in);
-        return;
+        try {
+            ntt_staged(out, log_n, count, false, tw, v == 5 ? 3 : 2, outfac, status, s, &in);
+            return;
+        } catch (const cuda_error &e) {
+            if (!without_room(e)) throw;
+        }
     }
     c2e_factors_kernel<<<blocks_for(n * count, 256), 256, 0, s>>>(out, src, infac, in_len, n, count);
     GB_CHECK_LAUNCH();
@@ -1795,7 +1817,13 @@ RustError gb_fr_device_vec_ntt_ragged(void *device_vec, const size_t *offsets, c
         q_log.push_back(log_ns[j]);
         q_fac.push_back(period3_factors(sc, sc * first, sc * second));
     }
-    ntt_ragged(v->values, q_off.data(), q_log.data(), q_fac.data(), q_off.size(), inverse, st.ptr(), s);
+    try {
+        ntt_ragged(v->values, q_off.data(), q_log.data(), q_fac.data(), q_off.size(), inverse, st.ptr(), s);
+    } catch (const cuda_error &e) {
+        if (!without_room(e)) throw;
+        for (size_t j = 0; j < q_off.size(); j++)
+            ntt_apply(v->values + q_off[j], q_log[j], 1, inverse, q_fac[j], st.ptr(), s);
+    }
     device_vec_mark_ready(v, s);
     return ok();
     GB_ENTRY_END

@@ -182,3 +182,66 @@ def test_grand_products_scratch(gb, orc):
     assert v.value - used < 32 * n * m * 1.25
     cols.free()
     perms.free()
+
+
+def _transformed(gb, log_n, count, inverse, most, limit, values):
+    dv = gb.Bls12_381FrDeviceVec.upload(values["v"])
+    limit(most)
+    dv.ntt_zeta_batch(log_n, count, inverse, values["scale"], values["first"], values["one"])
+    limit(0)
+    out = dv.download()
+    dv.free()
+    return out
+
+
+@pytest.mark.parametrize("inverse", [False, True])
+@pytest.mark.parametrize("log_n,count,most", [(13, 64, 8 << 20),   # no room for the scratch copy (16 MB)
+                                              (23, 1, 400 << 20)])  # for the tables (512 MB, copy 256)
+def test_transforms_without_room_for_the_staged_passes(gb, orc, limit, log_n, count, most, inverse):
+    """They run in place with the common twiddle table, output factors
+    included; the first of 64 is checked against the oracle."""
+    rng = np.random.default_rng(log_n)
+    one, scale, first = orc.fr_const(orc.CONST_ONE), *orc.fr_random(2, rng)
+    values = {"v": orc.fr_random(count << log_n, rng), "one": one, "scale": scale, "first": first}
+    short = _transformed(gb, log_n, count, inverse, most, limit, values)
+    assert (short == _transformed(gb, log_n, count, inverse, 0, limit, values)).all()
+    if log_n == 13:
+        want = orc.fr_ntt(values["v"][:1 << 13], 13, inverse)
+        factors = np.array([orc.fr_mul(scale, f) for f in (one, first, one)])
+        want = np.array([orc.fr_mul(w, factors[i % 3]) for i, w in enumerate(want)])
+        assert (short[:1 << 13] == want).all()
+
+
+def test_extension_without_room_for_the_tables(gb, orc, limit):
+    """2^21 coefficients to 2^24 values: result and copy 512 MB, tables 1 GB."""
+    src = gb.fr_random_chacha20(bytes(range(32)), 0, 1 << 21)[0]
+    limit(700 << 20)
+    short = gb.fr_device_coeff_to_extended_coset_batch(src, 1 << 21, 1, 24)
+    limit(0)
+    full = gb.fr_device_coeff_to_extended_coset_batch(src, 1 << 21, 1, 24)
+    assert (short.download() == full.download()).all()
+    for v in (src, short, full):
+        v.free()
+
+
+def test_ragged_transforms_without_room(gb, orc, limit):
+    rng = np.random.default_rng(8)
+    logs = [16, 3, 12, 10, 14, 1, 0]
+    one, scale, first, second = orc.fr_const(orc.CONST_ONE), *orc.fr_random(3, rng)
+    off = np.concatenate([[0], np.cumsum([1 << lg for lg in logs])[:-1]]).astype(np.uint64)
+    v = orc.fr_random(sum(1 << lg for lg in logs), rng)
+    got = []
+    for most in (2 << 20, 0):  # the scratch copy is 2.8 MB
+        dv = gb.Bls12_381FrDeviceVec.upload(v)
+        limit(most)
+        dv.ntt_ragged(off, logs, True, scale, first, second)
+        limit(0)
+        got.append(dv.download())
+        dv.free()
+    assert (got[0] == got[1]).all()
+    for o, lg in zip(off.astype(int), logs):
+        if lg:
+            want = orc.fr_ntt(v[o:o + (1 << lg)], lg, True)
+            factors = [scale, orc.fr_mul(scale, first), orc.fr_mul(scale, second)]
+            for i in (0, 1, (1 << lg) // 2, (1 << lg) - 1):
+                assert (got[1][o + i] == orc.fr_mul(want[i], factors[i % 3])).all()
