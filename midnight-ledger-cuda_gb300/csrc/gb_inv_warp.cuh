@@ -5,12 +5,16 @@
 // modular inversion", 2019), with delta starting at 1/2: from (f, g) = (p, a)
 // each step replaces (delta, f, g) by (1 - delta, g, (g - f) / 2) when delta >
 // 0 and g is odd, else by (1 + delta, f, (g + (g mod 2) f) / 2), until g = 0
-// and f = +-1.  Thirty steps depend on the low 30 bits of f and g only and are
-// one integer matrix (u v; q r) / 2^30, found by every lane alike; the matrix
-// is applied to f and g, and mod p to (d, e) with d a = f, e a = g (mod p),
-// with one 30-bit limb a lane: two or three products a lane and one carry from
-// each side.  Limbs are signed and carried once, so they stay within 2^30 + 2
-// of zero and the products' sums within 2^62.
+// and f = +-1.  The start at 1/2 and the variable-time order of the steps, runs
+// of zeros and several bits of g at once, are those that libsecp256k1 describes
+// in doc/safegcd_implementation.md.
+//
+// Thirty steps depend on the low 30 bits of f and g only and are one integer
+// matrix (u v; q r) / 2^30, found by every lane alike; the matrix is applied to
+// f and g, and mod p to (d, e) with d a = f, e a = g (mod p), with one 30-bit
+// limb a lane: two or three products a lane and one carry from each side.  Limbs
+// are signed and carried once, so they stay within 2^30 + 2 of zero and the
+// products' sums within 2^62.
 //
 // A dependent chain of 30 (Fr: 20) x about 10 short loops instead of some 460
 // (380) products: about 25 us for one warp against 400 us (150) for a Fermat
@@ -21,7 +25,7 @@
 
 #include "gb_field.cuh"
 
-#if defined(__CUDACC__)
+#if defined(__CUDACC__) || defined(GB_WARP_ON_HOST)  // a test runs the lanes in turn
 namespace gb {
 
 // modulus and 2^(96 N) mod it in 32-bit words, 1 / modulus mod 2^30
@@ -72,10 +76,10 @@ __device__ __forceinline__ int32_t inv_apply(int32_t a, int32_t b, int32_t u, in
     return (lane < LIMBS - 1 ? (int32_t)((uint32_t)n & 0x3fffffffu) : (int32_t)n) + (lane ? from_below : 0);
 }
 
-// the inverse (Montgomery form in and out) of *in, nonzero; every lane of the
-// warp takes part and returns it
+// the division steps' inverse of *in (see inverse_warp), not yet checked.  Only
+// the low bits of F and G count, which wrap around: unsigned.
 template <class Cfg>
-__device__ __noinline__ mont_t<Cfg> inverse_warp(const mont_t<Cfg> *in)
+__device__ __forceinline__ mont_t<Cfg> inverse_steps(const mont_t<Cfg> *in)
 {
     using C = inv_cfg<Cfg>;
     constexpr int L = C::LIMBS, N = Cfg::N;
@@ -86,11 +90,11 @@ __device__ __noinline__ mont_t<Cfg> inverse_warp(const mont_t<Cfg> *in)
     for (int batch = 0; batch < C::BATCHES; batch++) {
         const uint32_t f0 = __shfl_sync(0xffffffffu, f, 0), f1 = __shfl_sync(0xffffffffu, f, 1);
         const uint32_t g0 = __shfl_sync(0xffffffffu, g, 0), g1 = __shfl_sync(0xffffffffu, g, 1);
-        int32_t F = (int32_t)(f0 + (f1 << 30)), G = (int32_t)(g0 + (g1 << 30));
+        uint32_t F = f0 + (f1 << 30), G = g0 + (g1 << 30);
         int32_t u = 1, v = 0, q = 0, r = 1, left = 30;
         for (;;) {  // at most 30 turns: each but the last takes a bit or more
-            const int z = __ffs(G | (int32_t)(0xffffffffu << left)) - 1;
-            G >>= z;
+            const int z = __ffs((int)(G | 0xffffffffu << left)) - 1;
+            G = (uint32_t)((int32_t)G >> z);
             u = (int32_t)((uint32_t)u << z);
             v = (int32_t)((uint32_t)v << z);
             theta += z;
@@ -98,16 +102,17 @@ __device__ __noinline__ mont_t<Cfg> inverse_warp(const mont_t<Cfg> *in)
             if (left == 0) break;
             if (theta >= 0) {
                 theta = -theta - 1;
-                int32_t t = F;
-                F = G, G = -t;
-                t = u, u = q, q = -t;
+                const uint32_t T = F;
+                F = G, G = 0u - T;
+                int32_t t = u;
+                u = q, q = -t;
                 t = v, v = r, r = -t;
             }
             // the next -theta steps keep f, so up to five bits of g go at
             // once: (3 F) ^ 2 is 1 / F mod 32
             const int bits = min(min(left, -theta), 5);
-            const int32_t w = (int32_t)((uint32_t)(-G) * (uint32_t)((3 * F) ^ 2) & ((1u << bits) - 1u));
-            G += F * w;
+            const int32_t w = (int32_t)((0u - G) * ((3u * F) ^ 2u) & ((1u << bits) - 1u));
+            G += F * (uint32_t)w;
             q += u * w;
             r += v * w;
         }
@@ -162,7 +167,15 @@ __device__ __noinline__ mont_t<Cfg> inverse_warp(const mont_t<Cfg> *in)
     mont_t<Cfg> y, r3;
 #pragma unroll
     for (int i = 0; i < N; i++) y.v[i] = w[i], r3.v[i] = C::r3()[i];
-    y = y * r3;
+    return y * r3;
+}
+
+// the inverse (Montgomery form in and out) of *in, nonzero; every lane of the
+// warp takes part and returns it
+template <class Cfg>
+__device__ __noinline__ mont_t<Cfg> inverse_warp(const mont_t<Cfg> *in)
+{
+    mont_t<Cfg> y = inverse_steps<Cfg>(in);
     if (*in * y != mont_t<Cfg>::one()) y = in->inverse();
     return y;
 }
