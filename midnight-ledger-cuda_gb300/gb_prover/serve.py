@@ -31,6 +31,35 @@ from .plonk import GpuBackend, create_proof, create_proofs
 from .rng import ChaCha20Rng
 
 
+# The engine's plan of an MSM batch against a context (csrc/gb_msm_rules.h):
+# window bits by the context's points, and the affine rounds by pairs and
+# entries a bucket.
+_WINDOWS = ((7, 8), (11, 11), (12, 12), (15, 13), (16, 15), (64, 16))
+_ROUNDS = ((9 << 16, 6), (9 << 16, 11), (11 << 16, 40), (1 << 20, 192))
+_ROUNDS_SCRATCH = 16 << 30
+_GROUP_DIGITS = (8 << 30) // 72
+
+
+def msm_scratch_bytes(n, count):
+    """Device bytes that `count` MSMs of n points against an n-point context
+    take while they run: digits and bucket-ordered references, the affine
+    rounds' lists and prefix products, buckets and chunk edges."""
+    bits = next(c for lg, c in _WINDOWS if n <= 1 << lg)
+    windows = 255 // bits + 1
+    count = max(1, min(count, _GROUP_DIGITS // (n * windows)))  # larger batches run in groups
+    digits, buckets = n * count * windows, count << (bits - 1)
+    rounds = 0
+    while (rounds < 4 and digits >> (rounds + 1) >= _ROUNDS[rounds][0]
+           and digits >= buckets * _ROUNDS[rounds][1]):
+        rounds += 1
+    entries = digits + buckets * ((1 << rounds) - 1)
+    lists = 0
+    if rounds:
+        lists = min(entries * (48 if rounds == 1 else 72) + min(24 * entries, 48 * 128 * 608 * 64), _ROUNDS_SCRATCH)
+    chunks = (entries >> rounds) // 8
+    return 4 * (digits + entries) + lists + 192 * buckets + 2 * 192 * chunks
+
+
 def proof_footprint_bytes(circuit):
     """Device bytes one proof of this circuit holds at its peak: extended
     cosets of the advice, permutation and lookup columns and the numerator;
@@ -40,10 +69,7 @@ def proof_footprint_bytes(circuit):
     L, m, sets = circuit.lookups, circuit.m, circuit.permutation_sets
     ext_cols = m + sets + 3 * L + 2
     n_cols = 3 * (m + sets + 3 * L) + 12
-    # 16 windows of at most max(m, 4) polynomials: digits and bucket-ordered
-    # references, the affine rounds' two lists and their prefix products
-    msm_scratch = n * max(m, 4) * 16 * (8 + 72 + 24)
-    return 32 * (ext * ext_cols + n * n_cols) + msm_scratch
+    return 32 * (ext * ext_cols + n * n_cols) + msm_scratch_bytes(n, max(m, 4))
 
 
 class Request:

@@ -156,3 +156,23 @@ def test_no_size_is_refused_for_its_window(rules):
         for precomputed in (0, 1):
             assert n < 0x7FFFFFFF // rules.r_windows(rules.r_choose_window(n, precomputed)), n
     assert [rules.r_choose_window(1 << k, 0) for k in (11, 13, 15, 17, 19, 26)] == [8, 9, 10, 11, 12, 13]
+
+
+@pytest.mark.parametrize("count", [1, 3, 4, 8, 40])
+def test_server_estimate_follows_the_plan(rules, count):
+    """serve.msm_scratch_bytes, the server's admission estimate, covers what the
+    engine allocates for the entries of a batch, and not much more."""
+    from gb_prover import serve
+    for k in range(5, 24):
+        for n in (1 << k, 3 << (k - 1)):
+            c = rules.r_choose_window(n, 1)
+            sizes = np.full(count, n, dtype=np.uint64)
+            first = groups(rules, sizes, c, 1)
+            items = max(b - a for a, b in zip(first, first[1:]))
+            digits, buckets = items * n * rules.r_windows(c), items << (c - 1)
+            r = rules.r_rounds(digits, buckets, SLOTS, rules.r_rounds_limit())
+            lists = rules.r_scratch(digits, buckets, r, SLOTS)
+            entries = digits + buckets * ((1 << r) - 1)
+            known = 4 * (digits + entries) + lists + 192 * buckets
+            got = serve.msm_scratch_bytes(n, count)
+            assert known <= got + 1024 and got <= 1.35 * known + 48 * digits * (r == 0), (n, count, known, got)
