@@ -76,12 +76,9 @@ def f_msm(n):
     return min(FP_MULS_PER_ENTRY * n * windows(c) + FP_MULS_PER_ADD * windows(c) * (1 << c) for c in range(8, 21))
 
 
-def table_bits(n):
-    """The window size the resident-bases context picks for n points."""
-    for lg, c in ((7, 8), (11, 11), (12, 12), (15, 13), (16, 15)):
-        if n <= 1 << lg:
-            return c
-    return 16
+def table_rows(ctx, n):
+    """The windows of a context over n points: its table's rows."""
+    return ctx.device_bytes() // (96 * n)
 
 
 _MAX_MHZ = []
@@ -349,10 +346,10 @@ def main():
     e2e = world * n * args.steps / e2e_s / 1e6
 
     # ---- roofline
-    total_fp, c_table = f_msm(n), table_bits(n)
+    total_fp, rows = f_msm(n), table_rows(ctx, n)
     acc_avg_s = acc_ms / max(acc_n, 1) * 1e-3
     msm_avg_s = msm_ms / max(msm_n, 1) * 1e-3
-    acc_ops = FP_MULS_PER_ENTRY * n * windows(c_table) * MADDS_PER_FP_MUL
+    acc_ops = FP_MULS_PER_ENTRY * n * rows * MADDS_PER_FP_MUL
     achieved = acc_ops / acc_avg_s / 1e12 if acc_avg_s else None
     roofline = {
         "bound": "imad", "unit": "Tmadd/s",
@@ -363,13 +360,13 @@ def main():
                        "unit = one 32x32->64 product",
         "peak_forms": {"wide": probe_forms[0] / 1e12, "rows1": probe_forms[1] / 1e12,
                        "rows2": probe_forms[2] / 1e12, "rows4": probe_forms[3] / 1e12},
-        "algorithmic_per_launch": "6 Fp-mul x n x W(c): one affine addition with a shared inversion per digit, "
-                                  "c=%d, W=%d, 300 madd per Fp-mul" % (c_table, windows(c_table)),
+        "algorithmic_per_launch": "6 Fp-mul x n x W: one affine addition with a shared inversion per digit, "
+                                  "W=%d windows, 300 madd per Fp-mul" % rows,
         "avg_launch_ms": acc_avg_s * 1e3, "launches": acc_n,
         # DRAM bytes of the span: the ncu capture of the n=2^18 launches
         # (dram__bytes_read.sum + dram__bytes_write.sum over 2^18 x 16 digit
         # entries) scaled by this launch's n x W entries
-        "traffic": ACC_DRAM_BYTES_PER_ENTRY * n * windows(c_table),
+        "traffic": ACC_DRAM_BYTES_PER_ENTRY * n * rows,
         "traffic_source": "ncu capture at n=2^18, scaled per digit entry",
     }
     roofline_msm = {
@@ -409,10 +406,11 @@ def main():
             "config": {"workload": "G1 MSM n=2^%d, uniform Fr scalars, bases [r_i]G: KZG commitment of the "
                                    "16x2^20 NTT + coset LDE configuration, resident-bases context"
                                    % args.log_n,
-                       "n": n, "l2": "inputs larger than L2: 2^20 x 16-window base table (1.5 GiB) and 8 "
-                                     "rotating 32 MiB scalar sets", "parallelism": "replicas" if world > 1 else "1gpu",
-                       "table_bytes": n * windows(c_table) * 96,
-                       "table": "the context keeps 2^(16 j) P_i for the 16 windows j (fixed-base precomputation "
+                       "n": n, "l2": "inputs larger than L2: 2^%d x %d-window base table (%.1f GiB) and 8 "
+                                     "rotating sets of scalars" % (args.log_n, rows, n * rows * 96 / 2**30),
+                       "parallelism": "replicas" if world > 1 else "1gpu",
+                       "table_bytes": n * rows * 96,
+                       "table": "the context keeps every base shifted by each of its windows (fixed-base precomputation "
                                 "over the resident SRS; every digit still costs one addition); "
                                 "extra.msm_2p20_resident_no_table_ms is the same MSM without it"},
             "e2e": {"value": e2e, "unit": "Mpts/s", "h2d_bytes_per_step": n * 32, "d2h_bytes_per_step": 144},

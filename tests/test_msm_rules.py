@@ -176,3 +176,21 @@ def test_server_estimate_follows_the_plan(rules, count):
             known = 4 * (digits + entries) + lists + 192 * buckets
             got = serve.msm_scratch_bytes(n, count)
             assert known <= got + 1024 and got <= 1.35 * known + 48 * digits * (r == 0), (n, count, known, got)
+
+
+def test_bench_counts_the_tables_windows(rules):
+    """The roofline's digits are those of the table the context holds."""
+    import sys
+    sys.path.insert(0, REPO)
+    import bench
+
+    class Context:
+        def __init__(self, n):
+            self.bytes = 96 * n * rules.r_windows(rules.r_choose_window(n, 1))
+
+        def device_bytes(self):
+            return self.bytes
+
+    for k in (8, 11, 12, 15, 16, 20):
+        n = 1 << k
+        assert bench.table_rows(Context(n), n) == rules.r_windows(rules.r_choose_window(n, 1))
