@@ -1,8 +1,10 @@
 // Fp and G1 on the host, for the few point operations at the end of an MSM:
 // 6 x 64-bit limbs, Montgomery products with 128-bit intermediates, the binary
 // extended Euclid for inverses (blst's p1_to_affine is what the reference's
-// Rust callers apply to every commitment).  Variable time: commitments are
-// public.  A memory image of these types is that of fp_t and xyzz_t.
+// Rust callers apply to every commitment).  Variable time, as the device's
+// accumulation of the same sums is: commitments are public, and a caller whose
+// scalars may not show in the time of a call masks them (the scrambled entry
+// point).  A memory image of these types is that of fp_t and xyzz_t.
 #pragma once
 
 #include <stdint.h>

@@ -15,10 +15,10 @@
 //                   partials aside
 //   7. fix-up     : buckets spanning chunks add their partials
 //                   (large batches: affine rounds before it)
-//   8. reduce     : sum_k (k+1) B_k per segment, by line and bit sums (few
-//                   buckets) or segmented running sums and a tree, then per
-//                   MSM the window combination; a few MSMs' last dependent
+//   8. reduce     : sum_k (k+1) B_k per segment, by line and bit sums, then
+//                   per MSM the window combination; a few MSMs' last dependent
 //                   steps are the host's.
+// Very large batches go through the stages in groups (gb_msm_rules.h).
 //
 // A "segment" owns 2^(c-1) buckets.  Two modes:
 //   * precomputed (MSM contexts, whose bases are fixed): context creation

@@ -231,21 +231,6 @@ __host__ __device__ __forceinline__ uint32_t ntt_chunk(uint32_t t, uint32_t h, u
     return (r << 3) | ((((t & 3u) << 1) | h) ^ ntt_swz_row(r) ^ x);
 }
 
-__device__ __forceinline__ fr_t ntt_ld(const uint4 *s, uint32_t t, uint32_t x)
-{
-    const uint4 a = s[ntt_chunk(t, 0, x)], b = s[ntt_chunk(t, 1, x)];
-    fr_t r;
-    r.v[0] = a.x, r.v[1] = a.y, r.v[2] = a.z, r.v[3] = a.w;
-    r.v[4] = b.x, r.v[5] = b.y, r.v[6] = b.z, r.v[7] = b.w;
-    return r;
-}
-
-__device__ __forceinline__ void ntt_st(uint4 *s, uint32_t t, uint32_t x, const fr_t &v)
-{
-    s[ntt_chunk(t, 0, x)] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
-    s[ntt_chunk(t, 1, x)] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
-}
-
 // Butterfly arithmetic of the staged passes.  The values between stages and
 // passes are kept in [0, 2r) (Harvey's lazy butterflies): the prepared product
 // of x < 2r by a twiddle is below 2r, and sums and differences are reduced
