@@ -500,7 +500,7 @@ def run_ntt_case(args):
         ms.append(e0.elapsed_time(e1))
     fr_mul = sum((1 << (lg - 1)) * lg for lg in logs)
     print(json.dumps({"case": args.case, "transforms": len(logs), "elements": int(sum(1 << lg for lg in logs)),
-                      "ms": ms, "best_ms": min(ms), "tmadd_per_s": fr_mul * 136 / min(ms) / 1e9}))
+                      "ms": ms, "best_ms": min(ms), "tmadd_per_s": fr_mul * MADDS_PER_TWIDDLE / min(ms) / 1e9}))
 
 
 def mixed_scalars(n, rng):
