@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairBlocks)
     // the host knows a bound of the pairs only: of scalars that are zero for the
     // most part (2^20 of them, one in ten not: 1.98 -> 1.34 ms) the tiles are
     // shorter, so that every block has one
-    const uint32_t per_thread = min(most_per_thread, pairs_per_thread(pairs, gridDim.x));
+    const uint32_t per_thread = min(most_per_thread, pairs_per_thread((uint32_t)pairs, gridDim.x));
     const uint64_t tile = (uint64_t)kPairThreads * per_thread;
     uint4 *pre = prefix + (uint64_t)blockIdx.x * per_thread * 3 * kPairThreads + tid;
     for (uint64_t base = blockIdx.x * tile + tid; base - tid < pairs; base += gridDim.x * tile) {
@@ -1619,6 +1619,7 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
     std::vector<item_desc> idesc(nitems);
     std::vector<seg_desc> sdesc(nseg);
     uint64_t points_total = 0, digits_total = 0;
+    typical_bucket bucket;
     for (uint32_t m = 0; m < nitems; m++) {
         const msm_item &it = items[m];
         if (it.n >= kMaxDigits / (uint64_t)nwin) throw cuda_error((int)cudaErrorInvalidValue, "MSM too large");
@@ -1630,6 +1631,7 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
             sd.n = (uint32_t)std::max<size_t>(it.n, 1);
             sd.point_base = it.point_base;
         }
+        bucket.add(it.n);
         points_total += it.n;
         digits_total += (uint64_t)it.n * nwin;
     }
@@ -1667,9 +1669,7 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
     // 129, 2^14 189 -> 149; 2 x 2^14, 8 entries a thread, 243 and 243, and 2^16
     // 432 and 450)
     const bool pair = variant == 1 && !rounds && digits_total < 6 * (uint64_t)sm_count() * 512;
-    std::vector<size_t> sizes;
-    for (uint32_t m = 0; m < nitems; m++) sizes.push_back(items[m].n);
-    const double typical = typical_bucket(sizes, c, precomputed) / (1 << rounds);
+    const double typical = bucket.entries(c, precomputed) / (1 << rounds);
     const uint32_t L = pair ? pair_chunk_length(digits_total, typical, G)
                             : chunk_length(entries >> rounds, typical, G, variant);
     const uint64_t nchunks = std::max<uint64_t>(1, ((entries >> rounds) + L - 1) / L);
@@ -2095,20 +2095,17 @@ static batch_result msm_run_batch(const std::vector<msm_item> &items, int c, boo
 {
     set_smem_attrs();
     batch_result r;
-    std::vector<size_t> sizes;
-    for (const msm_item &it : items) sizes.push_back(it.n);
-    const std::vector<size_t> first = batch_groups(sizes, c, precomputed);
-    for (size_t g = 0; g + 1 < first.size() && !items.empty(); g++) {
+    for (size_t g = 0, m = 0; g < items.size(); g += m) {
+        m = group_items(g, items.size(), [&](size_t i) { return items[i].n; }, c, precomputed);
         auto plan = [&](uint64_t most_scratch) {
-            return plan_batch(items.data() + first[g], (uint32_t)(first[g + 1] - first[g]), items.size(), c,
-                              precomputed, stride, most_scratch);
+            return plan_batch(items.data() + g, (uint32_t)m, items.size(), c, precomputed, stride, most_scratch);
         };
-        batch_plan P = plan(kRoundsScratch);
+        const batch_plan P = plan(kRoundsScratch);
         if (!g) {
             r.tail = P.tail;
             r.points = dev_buf<xyzz_t>(items.size() * P.tail.points, s);
         }
-        xyzz_t *out = r.points.get() + first[g] * P.tail.points;
+        xyzz_t *out = r.points.get() + g * P.tail.points;
         try {
             launch_planned(P, points, out, s, use_graph);
         } catch (const cuda_error &e) {

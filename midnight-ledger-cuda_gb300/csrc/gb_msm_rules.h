@@ -7,7 +7,6 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <vector>
 
 #if defined(__CUDACC__)
 #define GB_RULE __host__ __device__ constexpr
@@ -65,11 +64,13 @@ static constexpr uint32_t kPairThreads = 128;
 static constexpr uint32_t kPairBlocks = 4;
 static constexpr uint32_t kPairsPerThread = 64;
 
-// pairs a thread: whole waves of `slots` tiles of at most kPairsPerThread
-GB_RULE uint32_t pairs_per_thread(uint64_t pairs, uint64_t slots)
+// pairs a thread: whole waves of `slots` tiles of at most kPairsPerThread (on the
+// device with 32 bits: pairs are below 2^31)
+template <class U>
+GB_RULE uint32_t pairs_per_thread(U pairs, U slots)
 {
-    const uint64_t all = (pairs + slots * kPairThreads - 1) / (slots * kPairThreads), per = all ? all : 1;
-    const uint64_t waves = (per + kPairsPerThread - 1) / kPairsPerThread;
+    const U all = (pairs + slots * kPairThreads - 1) / (slots * kPairThreads), per = all ? all : 1;
+    const U waves = (per + kPairsPerThread - 1) / kPairsPerThread;
     return (uint32_t)((per + waves - 1) / waves);
 }
 
@@ -136,12 +137,14 @@ inline int affine_rounds(uint64_t digits, double avg, uint64_t G, uint64_t slots
 // ones: with chunks and the bound of a thread's span made for the mean, all of
 // these went to the block-wide fix-up (2 MSMs of 2^16 points with 32 of 256
 // points 5.8 ms, with 24 2.9; now 2.2 and 2.0).
-inline double typical_bucket(const std::vector<size_t> &sizes, int c, bool precomputed)
-{
+struct typical_bucket {
     double squares = 0, sum = 0;
-    for (size_t n : sizes) squares += (double)n * (double)n, sum += (double)n;
-    return sum > 0 ? squares / sum * (precomputed ? windows_for(c) : 1) / (double)(1u << (c - 1)) : 0;
-}
+    void add(size_t n) { squares += (double)n * (double)n, sum += (double)n; }
+    double entries(int c, bool precomputed) const
+    {
+        return sum > 0 ? squares / sum * (precomputed ? windows_for(c) : 1) / (double)(1u << (c - 1)) : 0;
+    }
+};
 
 // Chunks that a bucket may span for one thread (or group) to add up its
 // partials, kShortSpan at most: some 3 times the mean bucket's, as a longer
@@ -191,26 +194,20 @@ inline size_t table_items(size_t K, size_t n)
     return SIZE_MAX;
 }
 
-// The batch in groups of consecutive items: their first items, and the end.
-// A group holds as many as fit kGroupDigits digits and kGroupBuckets buckets,
-// one at least.
-inline std::vector<size_t> batch_groups(const std::vector<size_t> &sizes, int c, bool precomputed)
+// One group of a batch: how many of the items from `first` on fit kGroupDigits
+// digits and kGroupBuckets buckets, one at least; size(i) points item i.
+template <class F>
+size_t group_items(size_t first, size_t items, F size, int c, bool precomputed)
 {
     const uint64_t nwin = (uint64_t)windows_for(c), K = (uint64_t)1 << (c - 1);
-    const uint64_t buckets = precomputed ? K : K * nwin;  // an item's
-    std::vector<size_t> first(1, 0);
-    uint64_t digits = 0, items = 0;
-    for (size_t i = 0; i < sizes.size(); i++) {
-        const uint64_t d = sizes[i] * nwin;
-        if (items && (digits + d > kGroupDigits || (items + 1) * buckets > kGroupBuckets)) {
-            first.push_back(i);
-            digits = items = 0;
-        }
-        digits += d;
-        items++;
+    const uint64_t most = kGroupBuckets / (precomputed ? K : K * nwin);
+    uint64_t digits = 0;
+    size_t i = first;
+    for (; i < items; i++) {
+        digits += size(i) * nwin;
+        if (i > first && (digits > kGroupDigits || i - first >= most)) break;
     }
-    first.push_back(sizes.size());
-    return first;
+    return i - first;
 }
 
 }  // namespace gb

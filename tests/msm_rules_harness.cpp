@@ -14,7 +14,9 @@ uint64_t r_scratch(uint64_t digits, uint64_t G, int rounds, uint64_t slots)
 }
 double r_typical(const size_t *sizes, size_t n, int c, int precomputed)
 {
-    return gb::typical_bucket(std::vector<size_t>(sizes, sizes + n), c, precomputed != 0);
+    gb::typical_bucket b;
+    for (size_t i = 0; i < n; i++) b.add(sizes[i]);
+    return b.entries(c, precomputed != 0);
 }
 uint32_t r_short_span(double mean, double typical, uint32_t L) { return gb::short_span(mean, typical, L); }
 size_t r_table_items(size_t K, size_t n) { return gb::table_items(K, n); }
@@ -24,8 +26,9 @@ uint64_t r_rounds_limit() { return gb::kRoundsScratch; }
 // the groups' first items and the end into out (n + 1 places at most); how many
 size_t r_groups(const size_t *sizes, size_t n, int c, int precomputed, size_t *out)
 {
-    const std::vector<size_t> g = gb::batch_groups(std::vector<size_t>(sizes, sizes + n), c, precomputed != 0);
-    std::copy(g.begin(), g.end(), out);
-    return g.size();
+    size_t k = 0, at = 0;
+    for (; at < n; at += gb::group_items(at, n, [&](size_t i) { return sizes[i]; }, c, precomputed != 0)) out[k++] = at;
+    out[k++] = at;
+    return k;
 }
 }
