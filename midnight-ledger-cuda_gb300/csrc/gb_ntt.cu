@@ -1127,10 +1127,10 @@ static void ntt_staged(fr_t *d, uint32_t log_n, size_t count, bool inverse, cons
     if (in && P < 2) throw cuda_error(-1, "fused NTT input needs two or more passes");
     // all memory before the first launch: without it nothing is queued, and the
     // values are as they were (see without_room)
-    const fr_t *tables[4] = {};
+    dev_buf<fr_t> tmp(P > 1 ? count << log_n : 0, s);
+    const fr_t *tables[4] = {};  // these stay, so after the copy
     for (size_t i = 0; i < P; i++)
         tables[i] = pass_twiddles(log_n, inverse, passes[i].first, passes[i].second, tw, s);
-    dev_buf<fr_t> tmp(P > 1 ? count << log_n : 0, s);
     const ntt_factors none{{fr_t::one(), fr_t::one(), fr_t::one()}, 0};
     const ntt_input no_in{nullptr, 0, none};
     const unsigned spins = wait_spins();

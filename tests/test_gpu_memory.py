@@ -245,3 +245,20 @@ def test_ragged_transforms_without_room(gb, orc, limit):
             factors = [scale, orc.fr_mul(scale, first), orc.fr_mul(scale, second)]
             for i in (0, 1, (1 << lg) // 2, (1 << lg) - 1):
                 assert (got[1][o + i] == orc.fr_mul(want[i], factors[i % 3])).all()
+
+
+def test_transform_without_room_builds_no_tables(gb, orc, limit):
+    """Where the scratch copy (512 MB) has no room, the tables (256 MB), which
+    would stay, are not built either."""
+    import torch
+    log_n, count = 22, 4
+    one = orc.fr_const(orc.CONST_ONE)
+    dv = gb.fr_random_chacha20(bytes(range(32)), 0, count << log_n)[0]
+    dv.download(1)
+    free = torch.cuda.mem_get_info()[0]
+    limit(400 << 20)
+    dv.ntt_zeta_batch(log_n, count, True, one, one, one)
+    limit(0)
+    dv.download(1)
+    assert free - torch.cuda.mem_get_info()[0] < 200 << 20  # the common table is 64 MB
+    dv.free()
