@@ -556,14 +556,16 @@ __device__ __forceinline__ int pair_kind(const pair_refs<REFS> &ref, const affin
 template <bool REFS>
 __global__ void __launch_bounds__(kPairThreads, kPairBlocks)
     msm_affine_pairs_kernel(const uint32_t *__restrict__ refs, const affine_t *__restrict__ points,
-                            affine_t *__restrict__ out, const uint32_t *__restrict__ entries, int round,
-                            uint32_t most_per_thread, uint4 *__restrict__ prefix)
+                            affine_t *__restrict__ out, const uint32_t *__restrict__ entries, uint32_t lo,
+                            uint32_t hi, int round, uint32_t most_per_thread, uint4 *__restrict__ prefix)
 {
     __shared__ fp_t node[2 * kPairThreads];  // product tree: root 1, leaves 128 ..
     __shared__ uint4 stage_mem[15 * kPairThreads];
     const uint32_t tid = threadIdx.x;
     const pair_stage stage{stage_mem + tid};
-    const uint64_t pairs = *entries >> round;
+    // of the list's entries lo .. hi - 1 those that there are
+    const uint32_t end = *entries;
+    const uint64_t pairs = (min(end, hi) - min(end, lo)) >> round;
     // the host knows a bound of the pairs only: of scalars that are zero for the
     // most part (2^20 of them, one in ten not: 1.98 -> 1.34 ms) the tiles are
     // shorter, so that every block has one
@@ -1718,14 +1720,15 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
 // that a device without room for them fails before any work is queued.
 struct round_buffers {
     dev_buf<uint4> prefix;
-    dev_buf<affine_t> list_a, list_b;
+    dev_buf<affine_t> list_a, list_b, result;  // result: of all slices
     round_buffers(const batch_plan &P, cudaStream_t s)
     {
         if (!P.rounds) return;
-        const uint64_t slots = (uint64_t)sm_count() * kPairBlocks;
-        prefix = dev_buf<uint4>(slots * pairs_per_thread(P.entries / 2, slots) * 3 * kPairThreads, s);
-        list_a = dev_buf<affine_t>(P.entries / 2 + 1, s);
-        if (P.rounds > 1) list_b = dev_buf<affine_t>(P.entries / 4 + 1, s);
+        const uint64_t slots = (uint64_t)sm_count() * kPairBlocks, slice = slice_entries(P.entries);
+        prefix = dev_buf<uint4>(slots * pairs_per_thread(slice / 2, slots) * 3 * kPairThreads, s);
+        if (sliced(P.entries)) result = dev_buf<affine_t>((P.entries >> P.rounds) + 1, s);
+        if (!result || P.rounds > 1) list_a = dev_buf<affine_t>(slice / 2 + 1, s);
+        if (P.rounds > 1) list_b = dev_buf<affine_t>(slice / 4 + 1, s);
     }
 };
 
@@ -1734,24 +1737,30 @@ struct round_buffers {
 static const affine_t *run_affine_rounds(const batch_plan &P, const uint32_t *sorted, const uint32_t *starts,
                                          const affine_t *points, const round_buffers &buf, cudaStream_t s)
 {
-    const uint64_t slots = (uint64_t)sm_count() * kPairBlocks;
-    const affine_t *in = points;
-    for (int r = 1; r <= P.rounds; r++) {
-        affine_t *out = r & 1 ? buf.list_a.get() : buf.list_b.get();
-        const uint64_t pairs = P.entries >> r;
-        const uint32_t per = std::min(pairs_per_thread(pairs, slots), pairs_per_thread(P.entries / 2, slots));
-        const uint64_t tiles = (pairs + (uint64_t)per * kPairThreads - 1) / ((uint64_t)per * kPairThreads);
-        const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(slots, tiles));
-        if (r == 1)
-            msm_affine_pairs_kernel<true><<<grid, kPairThreads, 0, s>>>(sorted, in, out, starts + P.G, r, per,
-                                                                        buf.prefix);
-        else
-            msm_affine_pairs_kernel<false><<<grid, kPairThreads, 0, s>>>(nullptr, in, out, starts + P.G, r, per,
-                                                                         buf.prefix);
-        GB_CHECK_LAUNCH();
-        in = out;
+    const uint64_t slots = (uint64_t)sm_count() * kPairBlocks, slice = slice_entries(P.entries);
+    const affine_t *in = nullptr;
+    for (uint64_t lo = 0; lo < P.entries; lo += slice) {
+        const uint64_t hi = std::min(P.entries, lo + slice);
+        in = points;
+        for (int r = 1; r <= P.rounds; r++) {
+            affine_t *out = buf.result && r == P.rounds ? buf.result.get() + (lo >> r)
+                            : r & 1                     ? buf.list_a.get()
+                                                        : buf.list_b.get();
+            const uint64_t pairs = (hi - lo) >> r;
+            const uint32_t per = std::min(pairs_per_thread(pairs, slots), pairs_per_thread(slice / 2, slots));
+            const uint64_t tiles = (pairs + (uint64_t)per * kPairThreads - 1) / ((uint64_t)per * kPairThreads);
+            const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(slots, tiles));
+            if (r == 1)
+                msm_affine_pairs_kernel<true><<<grid, kPairThreads, 0, s>>>(
+                    sorted + lo, in, out, starts + P.G, (uint32_t)lo, (uint32_t)hi, r, per, buf.prefix);
+            else
+                msm_affine_pairs_kernel<false><<<grid, kPairThreads, 0, s>>>(
+                    nullptr, in, out, starts + P.G, (uint32_t)lo, (uint32_t)hi, r, per, buf.prefix);
+            GB_CHECK_LAUNCH();
+            in = out;
+        }
     }
-    return in;
+    return buf.result ? buf.result.get() : in;
 }
 
 // The device half: every launch of the batch, its scratch allocated and

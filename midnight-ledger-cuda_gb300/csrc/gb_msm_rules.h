@@ -78,33 +78,42 @@ GB_RULE uint32_t pairs_per_thread(U pairs, U slots)
 inline uint64_t padded_entries(uint64_t digits, uint64_t G, int rounds) { return digits + G * ((1u << rounds) - 1); }
 
 // Scratch of the rounds: the two lists of 96-byte points that they go between
-// (half and a quarter of the entries) and 48-byte prefix products.  Digits and
-// references are 8 bytes an entry, so this is 6 (one round) to 9 times the rest.
+// (half and a quarter of the entries) and 48-byte prefix products, 48 to 72 bytes
+// an entry where digits and references are 8.  Long lists go through the rounds
+// in slices of kSliceEntries, whose results are collected: the two lists are a
+// slice's then, and the last one's length is that of all entries >> rounds (2^24
+// points, 4 rounds: 73.4 ms and 19.5 GB in one piece, 73.2 and 10.4 in 3 slices).
+static constexpr uint64_t kSliceScratch = 8ull << 30;
+static constexpr uint64_t kSliceEntries = kSliceScratch / 72 / 16 * 16;  // whole pairs in every round
+inline uint64_t slice_entries(uint64_t entries) { return entries < kSliceEntries ? entries : kSliceEntries; }
+inline bool sliced(uint64_t entries) { return entries > kSliceEntries; }
 inline uint64_t rounds_scratch(uint64_t entries, int rounds, uint64_t slots)
 {
     if (!rounds) return 0;
-    return 96 * (entries / 2 + 1) + (rounds > 1 ? 96 * (entries / 4 + 1) : 0) +
-           48ull * kPairThreads * slots * pairs_per_thread(entries / 2, slots);
+    const uint64_t slice = slice_entries(entries);
+    const uint64_t prefix = 48ull * kPairThreads * slots * pairs_per_thread(slice / 2, slots);
+    const uint64_t all = sliced(entries) ? 96 * ((entries >> rounds) + 1) : 0;
+    if (rounds == 1 && all) return prefix + all;
+    return prefix + all + 96 * (slice / 2 + 1) + (rounds > 1 ? 96 * (slice / 4 + 1) : 0);
 }
 
-// Rounds are taken while their scratch is below kRoundsScratch, and a batch
-// that would take more than kGroupScratch is run as several, one after the
-// other on the same scratch (7 MSMs of 2^20 points with 16 windows, 35 ms of
-// work, against about 0.3 ms that a batch of its own costs).
-static constexpr uint64_t kRoundsScratch = 16ull << 30, kGroupScratch = 8ull << 30;
+// Rounds are taken while their scratch is below kRoundsScratch, and a batch of
+// more than kGroupDigits digits or kGroupBuckets buckets (192 bytes each) is run
+// as several, one after the other on the same scratch (16 MSMs of 2^20 points with
+// 16 windows, 73 ms of work, against about 0.3 ms that a batch of its own costs).
+static constexpr uint64_t kRoundsScratch = 16ull << 30;
+static constexpr uint64_t kGroupDigits = 1ull << 28, kGroupBuckets = 1ull << 25;
 // Batches with more scratch are not captured as graphs: a graph's memory stays
 // with it between launches, and the gaps between the launches that it spares
 // are less than 0.4 % of such a batch (64 MSMs of 2^10 .. 2^18 points, 3.5 GB
 // of scratch: 14.40 ms as a graph, 14.45 without).
 static constexpr uint64_t kGraphScratch = 4ull << 30;
-// 72 bytes an entry of rounds' scratch, 192 a bucket
-static constexpr uint64_t kGroupDigits = kGroupScratch / 72, kGroupBuckets = 1ull << 25;
 
 // Affine rounds of a batch: as long as a round has pairs enough to fill the
 // GPU (a round costs about 55 us whatever its size: product trees and one
 // inversion a block) and buckets are long enough, as every bucket is padded to
-// a multiple of 2^rounds; and while their scratch is no more than
-// most_scratch.  Measured on GB300, entries and entries a bucket, and
+// a multiple of 2^rounds; none if their scratch is more than most_scratch.
+// Measured on GB300, entries and entries a bucket, and
 // ms a call without rounds and with 1, 2, 3, 4 (* chosen):
 //    1.0 M   80   0.61*  0.68   0.65
 //    1.2 M   72   0.68   0.66*  0.66   0.74   0.79
@@ -125,10 +134,9 @@ inline int affine_rounds(uint64_t digits, double avg, uint64_t G, uint64_t slots
     static constexpr double bucket[4] = {6, 11, 40, 192};
     int r = 0;
     while (r < 4 && digits >> (r + 1) >= pairs[r] && avg >= bucket[r] &&
-           padded_entries(digits, G, r + 1) < 0x80000000ull &&
-           rounds_scratch(padded_entries(digits, G, r + 1), r + 1, slots) <= most_scratch)
+           padded_entries(digits, G, r + 1) < 0x80000000ull)
         r++;
-    return r;
+    return rounds_scratch(padded_entries(digits, G, r), r, slots) <= most_scratch ? r : 0;
 }
 
 // Entries of the bucket that an entry typically lies in: the items' means,

@@ -37,7 +37,8 @@ from .rng import ChaCha20Rng
 _WINDOWS = ((7, 8), (11, 11), (12, 12), (15, 13), (16, 15), (64, 16))
 _ROUNDS = ((9 << 16, 6), (9 << 16, 11), (11 << 16, 40), (1 << 20, 192))
 _ROUNDS_SCRATCH = 16 << 30
-_GROUP_DIGITS = (8 << 30) // 72
+_SLICE = (8 << 30) // 72 // 16 * 16
+_GROUP_DIGITS = 1 << 28
 
 
 def msm_scratch_bytes(n, count):
@@ -55,7 +56,14 @@ def msm_scratch_bytes(n, count):
     entries = digits + buckets * ((1 << rounds) - 1)
     lists = 0
     if rounds:
-        lists = min(entries * (48 if rounds == 1 else 72) + min(24 * entries, 48 * 128 * 608 * 64), _ROUNDS_SCRATCH)
+        part = min(entries, _SLICE)  # longer lists go through the rounds in slices
+        lists = min(24 * part, 48 * 128 * 608 * 64) + (96 * (entries >> rounds) if entries > _SLICE else 0)
+        if rounds > 1:
+            lists += 72 * part
+        elif entries <= _SLICE:
+            lists += 48 * part
+        if lists > _ROUNDS_SCRATCH:
+            lists, rounds, entries = 0, 0, digits
     chunks = (entries >> rounds) // 8
     return 4 * (digits + entries) + lists + 192 * buckets + 2 * 192 * chunks
 

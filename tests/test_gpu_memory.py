@@ -94,17 +94,22 @@ def test_batches_without_room_for_the_affine_rounds(gb, orc, limit, kind):
     ctx.close()
 
 
-def test_batch_divided_into_groups(gb, orc):
-    """5000 MSMs of 1024 points are 123 M digits, more than a group of a batch
-    holds; their results come in order."""
+@pytest.mark.parametrize("count", [5000, 11500])
+def test_batch_in_slices_and_groups(gb, orc, count):
+    """5000 MSMs of 1024 points are 123 M digits, more than a slice of the
+    affine rounds' list; 11500 are more than one group of a batch as well.  Their
+    results come in order."""
     rng = np.random.default_rng(4)
-    n, count = 1024, 5000
+    n = 1024
     bases = gb.g1_generator_mul(orc.fr_random(n, rng))
     dv = gb.fr_random_chacha20(bytes(range(32)), 0, n * count)[0]
     ctx = gb.Bls12_381G1MsmContext(bases)
     got = ctx.device_batch(dv, 0, n, count)
     scal = dv.download().reshape(count, n, 4)
-    for i in list(range(0, count, 500)) + list(range(4840, 4880, 5)) + [count - 1]:
+    some = set(range(0, count, 500)) | set(range(4200, 5000, 40)) | {count - 1}
+    if count > 10923:  # 2^28 digits
+        some |= {10921, 10922, 10923, 10924}
+    for i in sorted(some):
         assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all(), i
     ctx.close()
     dv.free()

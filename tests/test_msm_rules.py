@@ -52,8 +52,10 @@ def test_rounds_scratch_is_bounded(rules, buckets):
 
 
 def test_rounds_of_ordinary_batches(rules):
-    """The bound does not touch what is measured in the rule's table."""
-    for digits, avg, want in ((1 << 20, 80, 0), (4_700_000, 72, 2), (16_800_000, 512, 4), (48_000_000, 23, 2)):
+    """The bound does not touch what is measured in the rule's table, nor long
+    lists, which go through the rounds in slices."""
+    for digits, avg, want in ((1 << 20, 80, 0), (4_700_000, 72, 2), (16_800_000, 512, 4), (48_000_000, 23, 2),
+                              (1 << 28, 8192, 4), (1 << 28, 8, 1), (1 << 30, 32768, 4)):
         assert rules.r_rounds(digits, digits // avg, SLOTS, rules.r_rounds_limit()) == want
 
 
@@ -75,18 +77,18 @@ def test_groups(rules, sizes, c, precomputed):
     parts = [(sum(sizes[a:b]) * nwin, (b - a) * per_item, b - a) for a, b in zip(first, first[1:])]
     for digits, buckets, items in parts:
         if items > 1:
-            assert digits * 72 <= 8 << 30 and buckets <= 1 << 25
+            assert digits <= 1 << 28 and buckets <= 1 << 25
         assert buckets < 1 << 28  # the count scan's range
         r = rules.r_rounds(digits, buckets, SLOTS, rules.r_rounds_limit())
         assert rules.r_scratch(digits, buckets, r, SLOTS) <= rules.r_rounds_limit()
     # no more groups than needed: the next item does not fit
     for (digits, _, items), nxt in zip(parts, first[1:-1]):
-        assert (digits + sizes[nxt] * nwin) * 72 > 8 << 30 or (items + 1) * per_item > 1 << 25
+        assert digits + sizes[nxt] * nwin > 1 << 28 or (items + 1) * per_item > 1 << 25
 
 
 def test_ordinary_batches_are_one_group(rules):
     assert len(groups(rules, [1 << 18] * 20, 16, 1)) == 2
-    assert len(groups(rules, [1 << 20] * 7, 16, 1)) == 2
+    assert len(groups(rules, [1 << 20] * 16, 16, 1)) == 2
     assert len(groups(rules, [2049] * 145, 9, 0)) == 2
 
 
