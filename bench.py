@@ -410,8 +410,8 @@ def main():
                                      "rotating sets of scalars" % (args.log_n, rows, n * rows * 96 / 2**30),
                        "parallelism": "replicas" if world > 1 else "1gpu",
                        "table_bytes": n * rows * 96,
-                       "table": "the context keeps every base shifted by each of its windows (fixed-base precomputation "
-                                "over the resident SRS; every digit still costs one addition); "
+                       "table": "the context keeps every base shifted by each of its windows (fixed-base "
+                                "precomputation over the resident SRS; every digit still costs one addition); "
                                 "extra.msm_2p20_resident_no_table_ms is the same MSM without it"},
             "e2e": {"value": e2e, "unit": "Mpts/s", "h2d_bytes_per_step": n * 32, "d2h_bytes_per_step": 144},
             "gpu_launches": launches,

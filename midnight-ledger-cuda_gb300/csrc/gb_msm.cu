@@ -1925,8 +1925,8 @@ struct graph_key {
     uint64_t points_total = 0, digits_total = 0, nchunks = 0;
     auto tie() const
     {
-        return std::tie(device, stream, points, c, variant, precomputed, fix_by_chunk, tail, stride, nitems, K, segs_per_item,
-                        nseg, G, nblocks, L, short_span, rounds, points_total, digits_total, nchunks);
+        return std::tie(device, stream, points, c, variant, precomputed, fix_by_chunk, tail, stride, nitems, K,
+                        segs_per_item, nseg, G, nblocks, L, short_span, rounds, points_total, digits_total, nchunks);
     }
     bool operator<(const graph_key &o) const { return tie() < o.tie(); }
 };

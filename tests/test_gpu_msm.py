@@ -570,7 +570,8 @@ def test_plain_batches_of_many_buckets(gb, orc, n, count):
         assert (affine_of(orc, got[i]) == affine_of(orc, orc.g1_msm(bases, scal[i]))).all()
 
 
-@pytest.mark.parametrize("sizes", [[1 << 16] * 2 + [300] * 32, [1 << 16] + [2048] * 3 + [0, 1, 5000], [9000] + [256] * 30])
+@pytest.mark.parametrize("sizes", [[1 << 16] * 2 + [300] * 32, [1 << 16] + [2048] * 3 + [0, 1, 5000],
+                                   [9000] + [256] * 30])
 def test_uneven_context_batches(gb, orc, sizes):
     """A few large MSMs among many small ones, whose buckets hold a few entries
     where the large ones' hold 72."""
