@@ -1472,7 +1472,7 @@ static void u32_exclusive_scan(const uint32_t *in, uint32_t n, uint32_t *out, cu
 // that the chunks fill whole waves of resident accumulation blocks (a 2^16
 // MSM's 65536 chunks of 16 fill 84 % of one wave on 152 SMs; chunks of 14
 // fill 96 %; a 2^20 MSM's 3.4 waves of 64 become 3 of 72).
-static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int variant)
+static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int variant, int sms)
 {
     uint32_t L = (uint32_t)std::max(8.0, std::min(64.0, avg * 0.5));
     static device_once once;
@@ -1485,7 +1485,7 @@ static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int varian
         GB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[2], msm_accumulate_kernel<128, 3>, 128, 0));
         for (int k = 0; k < 3; k++) per_sm[dev][k] = std::max(1, b[k]) * (k == 2 ? 128 : 256);
     });
-    const uint64_t wave = (uint64_t)sm_count() * (uint64_t)per_sm[dev][v];  // chunks resident at once
+    const uint64_t wave = (uint64_t)sms * (uint64_t)per_sm[dev][v];  // chunks resident at once
     // short buckets, large batches: chunks long enough for 8 waves, as every
     // chunk's edge costs a fix-up
     if (wave) L = std::max<uint32_t>(L, (uint32_t)std::min<uint64_t>(64, digits / (8 * wave)));
@@ -1515,9 +1515,9 @@ static uint32_t chunk_length(uint64_t digits, double avg, uint32_t G, int varian
 // that (measured, call in us for L = 3, 4, 5, 6, 8: 2^10 points, 11 entries a
 // bucket, 176* 181 186 190 197; 2^12, 20 entries, 220 220 210* 214 224; 2 x
 // 2^12 268 259 268 249* 264).
-static uint32_t pair_chunk_length(uint64_t digits, double avg, uint32_t G)
+static uint32_t pair_chunk_length(uint64_t digits, double avg, uint32_t G, int sms)
 {
-    const uint64_t wave = (uint64_t)sm_count() * kPairSm * kPairChunks;
+    const uint64_t wave = (uint64_t)sms * kPairSm * kPairChunks;
     // a few buckets of hundreds of entries (a window of 8 or 9 bits asked for)
     // have a block each to join their chunks, many at once: 2^12 points in 128
     // buckets 0.37 -> 0.27 ms with 16 in place of 33
@@ -1662,7 +1662,8 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
     const uint32_t nblocks = (uint32_t)bdesc.size();
     const double avg = (double)digits_total / (double)G;
     const int variant = default_acc_variant();
-    const uint64_t slots = (uint64_t)sm_count() * kPairBlocks;
+    const int sms = sm_count();
+    const uint64_t slots = (uint64_t)sms * kPairBlocks;
     const int rounds = affine_rounds(digits_total, avg, G, slots, most_scratch);
     const uint64_t entries = padded_entries(digits_total, G, rounds);
     // a batch of less than 6 entries a resident thread: two lanes a chunk
@@ -1670,10 +1671,10 @@ static batch_plan plan_batch(const msm_item *items, uint32_t nitems, size_t batc
     // 2^10 points 63 -> 25, 2^12 64 -> 44, 2 x 2^12 107 -> 72, 4 x 2^12 151 ->
     // 129, 2^14 189 -> 149; 2 x 2^14, 8 entries a thread, 243 and 243, and 2^16
     // 432 and 450)
-    const bool pair = variant == 1 && !rounds && digits_total < 6 * (uint64_t)sm_count() * 512;
+    const bool pair = variant == 1 && !rounds && digits_total < 6 * (uint64_t)sms * 512;
     const double typical = bucket.entries(c, precomputed) / (1 << rounds);
-    const uint32_t L = pair ? pair_chunk_length(digits_total, typical, G)
-                            : chunk_length(entries >> rounds, typical, G, variant);
+    const uint32_t L = pair ? pair_chunk_length(digits_total, typical, G, sms)
+                            : chunk_length(entries >> rounds, typical, G, variant, sms);
     const uint64_t nchunks = std::max<uint64_t>(1, ((entries >> rounds) + L - 1) / L);
 
     P.pair = pair;

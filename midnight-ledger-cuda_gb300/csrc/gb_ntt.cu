@@ -1134,6 +1134,7 @@ static void ntt_staged(fr_t *d, uint32_t log_n, size_t count, bool inverse, cons
     const ntt_factors none{{fr_t::one(), fr_t::one(), fr_t::one()}, 0};
     const ntt_input no_in{nullptr, 0, none};
     const unsigned spins = wait_spins();
+    const size_t two_each = 2 * (size_t)sm_count();
     for (size_t i = 0; i < P; i++) {
         const int s_hi = passes[i].first, g = passes[i].second;
         const int s_lo = s_hi - g + 1;
@@ -1155,7 +1156,7 @@ static void ntt_staged(fr_t *d, uint32_t log_n, size_t count, bool inverse, cons
         }
         // small transforms: fewer sub-blocks per CTA until there are two
         // CTAs per SM (a single 2^16 transform is otherwise 64 CTAs)
-        while (q > 0 && ctas_for(q) < 2 * (size_t)sm_count()) q--;
+        while (q > 0 && ctas_for(q) < two_each) q--;
         ctas = ctas_for(q);
         const uint32_t nd = 1u << (g + q);
         // the twiddle chunks; a single chunk's data areas go past its first half
